@@ -266,7 +266,6 @@ def ab_reference_kernels(ps, layers, api, rounds=5):
 
     beq = lambda a, b: bool(torch.equal(a.view(torch.uint8), b.view(torch.uint8)))      # bytes: NaN-safe
     med = lambda v: float(np.median(v))
-    api.pf_gemm_set_workspace(ps.gemm_ws)
 
     def one_routing(perm, tiles, ntiles):
         def descs(li):
@@ -520,8 +519,7 @@ def run_ours(args):
         my_macs = float(macs)
         launches = args.steps * ps.launches_per_step
     # dominant kernel: k_pf_gemm_tc (two launches per layer).  Algorithmic int8 operations of this rank's useful slots per
-    # launch / the launches' average CUDA-event duration (the row-gather kernel of the workspace path runs inside the entry
-    # point and is inside that duration).
+    # launch / the launches' average CUDA-event duration.
     n_gemm = max(1, len(gemm_ms))
     avg_launch_ms = float(np.mean(gemm_ms)) if gemm_ms else None
     ops_per_launch = 2.0 * my_macs / n_gemm

@@ -122,7 +122,7 @@ struct Engine {
     float * X, * a_sc, * inv, * h32, * sel, * sig, * w, * a2_sc, * D, * Y, * o;
     int8_t * a_qs, * a2_qs;
     int * idx, * cnt, * off, * tiles, * ntiles, * perm, * toks;
-    void * qh, * gemm_ws; size_t gemm_ws_bytes = 0;
+    void * qh;
 };
 
 lk::QT4 q4(const Pack & p, const std::string & name) { return lk::QT4{p.at(name + ".qs"), p.at(name + ".d")}; }
@@ -185,9 +185,6 @@ void build(Engine & e, int max_seq, int pf_cap) {
         e.tiles = dalloc<int>((size_t) e.max_tiles * 4); e.ntiles = dalloc<int>(1); e.perm = dalloc<int>(ns);
         e.a2_qs = dalloc<int8_t>(ns * I); e.a2_sc = dalloc<float>(ns * (I / 32) * 2); e.D = dalloc<float>(ns * H);
         e.Y = dalloc<float>(m * CONV_ROWS); e.o = dalloc<float>(m * H); e.qh = dalloc<uint16_t>(m * H); e.toks = dalloc<int>(m);
-        lk::check(lkb_pf_gemm_workspace_bytes(e.max_tiles, H, &e.gemm_ws_bytes), "lkb_pf_gemm_workspace_bytes");
-        e.gemm_ws = dalloc<unsigned char>(e.gemm_ws_bytes);
-        lk::check(lkb_pf_gemm_set_workspace(e.gemm_ws, e.gemm_ws_bytes), "lkb_pf_gemm_set_workspace");
     }
 }
 

@@ -343,13 +343,8 @@ int lkb_pf_gemm_config(int cfg);
  * The int32 block sums S_b are exact either way.  Also read once from LKB_PF_ARITH by lkb_init().
  * ref: src/prefill.cu:131-139 (PF_EPI2), 341-342, 381-399 */
 int lkb_pf_gemm_arith(int fold);
-/* Optional workspace of the grouped (perm != NULL) tensor-core form.  With a workspace registered, lkb_pf_gemm_moe /
- * lkb_pf_gemm_swiglu first copy the activation rows into token-tile order (one small kernel) and the GEMM then fetches
- * every 128-token tile with one bulk tensor copy; without one the rows are gathered through perm inside the GEMM, four
- * per copy, which is slower.  Results are identical.  The buffer is the caller's (this library allocates nothing):
- * 256-byte aligned device memory of at least lkb_pf_gemm_workspace_bytes(max_tiles, K of the widest activation)
- * bytes; it is read and written by every grouped GEMM launched afterwards, so calls that share it must be ordered on
- * one stream.  ptr = NULL unregisters.  No counterpart in the reference (its kernel gathers rows with cp.async). */
+/* The tensor-core form gathers the rows of a grouped GEMM through perm itself and needs no workspace; both calls stay
+ * for callers that size and register one (256-byte aligned), which is left alone.  No counterpart in the reference. */
 int lkb_pf_gemm_workspace_bytes(int max_tiles, int k_max, size_t * bytes_out);
 int lkb_pf_gemm_set_workspace(void * ptr, size_t bytes);
 /* Every device-side wait of the tensor-core form is bounded; this SYNCHRONISES the device and
@@ -492,8 +487,7 @@ int lkb_pf_gemm_moe_rows(const lkb_pf_gemm * g, int max_tiles, float * const * o
 /* No counterpart in the reference.  inv_out (optional) of lkb_ep_route_experts receives the received rows' 1/rms as a
  * plane; lkb_pf_gemm_swiglu_packed is lkb_pf_gemm_swiglu reading its activations from PACKED rows of row_pitch bytes
  * (bpr*32 quants, then bpr (d8, 8sum) pairs; g->aqs = the first row, g->asc unused) -- the dispatch rows as they
- * arrived, so no unpack pass is needed.  Needs the registered workspace (the row gather reads the packed rows);
- * tensor-core form only. */
+ * arrived, so no unpack pass is needed; tensor-core form only. */
 int lkb_pf_gemm_swiglu_packed(const lkb_pf_gemm * g, int max_tiles, int row_pitch, lkb_stream_t st);
 /* Publish `phase` of the epoch to every rank, then wait for the same phase of every source (lkb_ep_wait), in one
  * launch.  No counterpart in the reference. */

@@ -72,7 +72,7 @@ def pf_gemm_workspace_bytes(max_tiles, k_max):
 
 
 def pf_gemm_set_workspace(buf):
-    """Register (or with None unregister) the caller-owned workspace of the grouped tensor-core GEMM."""
+    """Accepted for callers that register one; the grouped tensor-core GEMM gathers its rows itself."""
     if buf is None:
         check(lib.lkb_pf_gemm_set_workspace(None, 0))
     else:

@@ -57,16 +57,13 @@ class PrefillStack:
         self.a = api.pf_act(self.a_qs, self.a_sc)
         self.a2 = api.pf_act(self.a2_qs, self.a2_sc)
         self.an = api.pf_act(self.n_qs, self.n_sc)
-        # caller-owned workspace of the grouped GEMM: activation rows in token-tile order (widest: the gate|up input)
-        self.gemm_ws = torch.zeros(api.pf_gemm_workspace_bytes(self.max_tiles, H), dtype=torch.uint8, device=device)
-        self.launches_per_step = 10 * len(layers)       # kernels per layer (the memset is not a kernel)
+        self.launches_per_step = 8 * len(layers)       # kernels per layer (the memset is not a kernel)
 
     def layer(self, i, next_norm_w=None, next_act=None):
         """One MoE FFN layer over the chunk.  next_norm_w / next_act = (PfAct, inv): where the fused combine + norm
         puts the next consumer's quantised activation (the full model: the next mixer's attn_norm, into the live
         activation buffers); by default the next layer's ffn_norm into scratch."""
         l, m = self.layers[i], self.m
-        api.pf_gemm_set_workspace(self.gemm_ws)
         api.k_pf_norm(self.X, l.norm_w, 0, self.a, self.inv, self.h32, m)
         # router + top-4 selection in one launch (the form follows the chunk size: src/engine.cu:1170-1176)
         api.k_pf_router_select(self.h32, m, m <= 256, l.router, l.rbias, self.inv, self.sel, self.sig, self.idx, self.w)
@@ -132,7 +129,7 @@ class PrefillStackEP:
         self.dispatch = dispatch
         self.rank, self.world, self.group = rank, world, group
         # this library's kernels per layer (memsets, the torch division and NCCL's own kernels not counted)
-        self.launches_per_step = (11 if dispatch == "peer" else 15) * len(layers)
+        self.launches_per_step = (9 if dispatch == "peer" else 13) * len(layers)
         self.layers = layers
         self.shards = [shard_layer(l, rank, world) for l in layers]
         self.m = m_total // world
@@ -166,7 +163,6 @@ class PrefillStackEP:
         self.an = api.pf_act(self.n_qs, self.n_sc)
         self.recv_slots = []                                     # per layer: slots this rank computed (load balance)
         self.gemm_events = None
-        self.gemm_ws = torch.zeros(api.pf_gemm_workspace_bytes(self.max_tiles, H), dtype=torch.uint8, device=device)
 
     def _alloc_ep(self, device):
         """Buffers of the device-side dispatch (called once)."""
@@ -288,7 +284,6 @@ class PrefillStackEP:
         ns, per = m * TOPK, E // G
         if not hasattr(self, "send_order"):
             self._alloc_ep(self.X.device)
-        api.pf_gemm_set_workspace(self.gemm_ws)
         api.k_pf_norm(self.X, l.norm_w, 0, self.a, self.inv, self.h32, m)
         # the router form follows the CHUNK size, as on one GPU (ref: src/engine.cu:1170-1176)
         api.k_pf_router_select(self.h32, m, self.m_total <= 256, l.router, l.rbias, self.inv, self.sel, self.sig, self.idx, self.w)

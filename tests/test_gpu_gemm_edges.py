@@ -1,0 +1,86 @@
+"""The tensor-core GEMM at the edges of its tiles: token counts around the 16-column steps of an MMA and the 64-token plan
+tile, row counts that leave half a tile or a single tile, the shortest K.  Bit for bit against the CPU checker; the fused
+SwiGLU form against the CUDA-core form of the same entry point (itself checked in test_gpu_prefill.py)."""
+import numpy as np
+import pytest
+
+from helpers import act_floats, dev, host, nan_f32, rand_q4
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+COUNTS = [1, 2, 15, 16, 17, 31, 32, 33, 47, 48, 49, 63, 64, 65, 0, 129]
+
+
+@pytest.fixture(params=[0, 1], ids=["exact", "fold"])
+def L(request, lkb, orc):
+    lkb.init(0)
+    lkb.pf_gemm_arith(request.param)
+    orc.set_gemm_fold(request.param)
+    lkb.pf_gemm_config(1)
+    yield lkb
+    lkb.pf_gemm_config(-1)
+    lkb.pf_gemm_arith(1)
+    orc.set_gemm_fold(1)
+    assert lkb.lib.lkb_pf_gemm_status() == 0
+
+
+def _plan(rng):
+    """Slots of 16 experts with COUNTS[e] slots each, in a random order: (slots' experts, off-ordered slots, plan tiles)."""
+    idx = rng.permutation(np.repeat(np.arange(len(COUNTS)), COUNTS)).astype(np.int32)
+    perm = np.argsort(idx, kind="stable").astype(np.int32)
+    tiles, off = [], 0
+    for e, c in enumerate(COUNTS):
+        tiles += [[e, off + k, min(64, c - k), 0] for k in range(0, c, 64)]
+        off += c
+    return idx, perm, np.array(tiles, np.int32)
+
+
+@pytest.mark.parametrize("m", [1, 16, 17, 48, 49, 64, 65])
+@pytest.mark.parametrize("N,bpr", [(128, 8), (384, 16)])
+def test_dense(L, orc, m, N, bpr):
+    rng = np.random.default_rng(7 * m + N)
+    qs, d = rand_q4(rng, N, bpr, "ref")
+    aq, asc = orc.pf_quant_rows(act_floats(rng, m * bpr * 32).reshape(m, bpr * 32), bpr)
+    o0 = rng.uniform(-1, 1, size=(m, N)).astype(np.float32)
+    out = dev(o0)
+    L.pf_gemm_dense(L.make_pf_gemm([(dev(qs), dev(d))], [N] * 3, N, bpr, dev(aq), dev(asc), ntok=m, out=out, out_ld=N, add=1))
+    ref = orc.pf_gemm([(qs, d)], [N] * 3, N, bpr, aq, asc, ntok=m, out_init=o0, add=1)
+    assert np.array_equal(host(out), ref)
+
+
+@pytest.mark.parametrize("N,bpr", [(128, 8), (384, 24), (2560, 8)])
+def test_grouped(L, orc, N, bpr):
+    rng = np.random.default_rng(N)
+    idx, perm, tiles = _plan(rng)
+    ns, E = idx.size, len(COUNTS)
+    qs, d = rand_q4(rng, E * N, bpr, "ref")
+    aq, asc = orc.pf_quant_rows(act_floats(rng, ns * bpr * 32).reshape(ns, bpr * 32), bpr)
+    out = nan_f32(ns, N)
+    g = L.make_pf_gemm([(dev(qs), dev(d))], [N] * 3, N, bpr, dev(aq), dev(asc), exp_stride=N * bpr, perm=dev(perm), tiles=dev(tiles),
+                       ntiles=dev(np.array([len(tiles)], np.int32)), out=out, out_ld=N)
+    L.pf_gemm_moe(g, len(tiles))
+    ref = orc.pf_gemm([(qs, d)], [N] * 3, N, bpr, aq, asc, exp_stride=N * bpr, perm=perm, tiles=tiles, out_rows=ns)
+    assert np.array_equal(host(out), ref)
+
+
+@pytest.mark.parametrize("I,bpr", [(64, 8), (192, 16), (256, 64)])
+def test_swiglu(L, orc, I, bpr):
+    rng = np.random.default_rng(I)
+    idx, perm, tiles = _plan(rng)
+    ns, E = idx.size, len(COUNTS)
+    w = [tuple(dev(x) for x in rand_q4(rng, E * I, bpr, "ref")) for _ in range(2)]
+    x = act_floats(rng, ns * bpr * 32).reshape(ns, bpr * 32)
+    x[5] = 0.0                                                       # a row of all-zero blocks
+    aq, asc = (dev(v) for v in orc.pf_quant_rows(x, bpr))
+    scale = dev(rng.uniform(0.01, 0.05, size=ns).astype(np.float32))
+    dperm, dtiles, dnt = dev(perm), dev(tiles), dev(np.array([len(tiles)], np.int32))
+    got = []
+    for cfg in (0, 1):
+        L.pf_gemm_config(cfg)
+        oqs, osc = torch.full((ns, I), 0x5A, dtype=torch.int8, device="cuda"), nan_f32(ns, I // 32, 2)
+        L.pf_gemm_swiglu(L.make_pf_gemm(w, [I] * 3, I, bpr, aq, asc, exp_stride=I * bpr, perm=dperm, tiles=dtiles, ntiles=dnt,
+                                        scale=scale, oqs=oqs, osc=osc, okb=I // 32), len(tiles))
+        got.append((oqs, osc))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    assert int(got[1][0].float().abs().max()) > 0
