@@ -327,6 +327,8 @@ __device__ __forceinline__ bool tc_fold_item(TcSmem & S, TcEpi & X, unsigned tba
 #pragma unroll
                 for (int i = 0; i < NB / 2; ++i) kb[i] = dk[NA / 2 + i];
                 tc_wait_ld();                                                         // the first half is in sva
+                // (polled ahead of the fold and looked at behind it: the answer's latency is hidden)
+                const bool ready = more && tc_mbar_try<0>(&S.tfull[h ^ 1], h == 0 ? u : u ^ 1u);
                 if constexpr (NB > 0) {
 #pragma unroll
                     for (int r = 0; r < R; ++r) tc_ld<NB ? NB : 8>(tcol + h * (2 * TC_TOK) + r * TC_TOK + NA, svb[r]);
@@ -337,7 +339,7 @@ __device__ __forceinline__ bool tc_fold_item(TcSmem & S, TcEpi & X, unsigned tba
                 __syncwarp();
                 tc_mbar_arrive_if(&S.tempty[h], lane == 0);                           // the buffer is free again
                 if (more) {
-                    if (!tc_wait(S, &S.tfull[h ^ 1], h == 0 ? u : u ^ 1u, 31u)) return false;
+                    if (!ready && !tc_wait(S, &S.tfull[h ^ 1], h == 0 ? u : u ^ 1u, 31u)) return false;
                     tc_fence_after();
 #pragma unroll
                     for (int r = 0; r < R; ++r) tc_ld<NA>(tcol + (h ^ 1) * (2 * TC_TOK) + r * TC_TOK, sva[r]);
@@ -537,7 +539,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_pf_gemm_tc(const lkb_pf_gemm 
     extern __shared__ unsigned char tc_smem_raw[];
     // the swizzle patterns are functions of the shared-memory address: stages start on 1024-byte boundaries
     TcSmem & S = *reinterpret_cast<TcSmem *>(tc_smem_raw + ((1024u - (tc_smem_u32(tc_smem_raw) & 1023u)) & 1023u));
-    const int ptid = threadIdx.x, warp = ptid >> 5, lane = ptid & 31;
+    const int ptid = threadIdx.x, warp = __shfl_sync(LKB_FULL, ptid >> 5, 0), lane = ptid & 31;
 
     // ---- item grid: (token tile, row tile), row tiles fastest --------------------
     TcPlan P;
