@@ -1,0 +1,30 @@
+"""Chunk attention around the edges of its tiles (32 or 64 query positions, 128 keys, one or two tiles per block) and with
+rows whose maximum keeps growing along the keys, against float64.  Rows of the cache past the chunk are NaN."""
+import numpy as np
+import pytest
+
+from helpers import host, nan_f32
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m,P,grow", [(31, 97, 0.0), (32, 96, 0.0), (33, 95, 0.0), (65, 63, 0.0), (1, 127, 0.0), (1, 128, 0.0),
+                                      (129, 0, 0.0), (1153, 0, 0.0), (1200, 511, 0.0), (40, 600, 0.02), (1217, 130, 0.01)])
+def test_pf_attn_edges(lkb, orc, m, P, grow):
+    lkb.init(0)
+    rng = np.random.default_rng(m + 31 * P)
+    S = P + m
+    K = rng.standard_normal((S + 1, 8, 64)) * 1.5
+    K *= (1.0 + grow * np.arange(S + 1))[:, None, None]               # later keys score higher: the running maximum moves
+    K = K.astype(np.float16)
+    V = rng.standard_normal((S + 1, 8, 64)).astype(np.float16)
+    Q = (rng.standard_normal((m, 2048)) * 1.5 * 0.125).astype(np.float16)
+    K[S:] = np.nan
+    V[S:] = np.nan
+    f16 = lambda a: torch.from_numpy(a.view(np.int16).copy()).cuda().view(torch.float16)
+    o = nan_f32(m, 2048)
+    lkb.k_pf_attn(f16(Q), m, P, f16(K), f16(V), o)
+    ref = orc.pf_attn_f64(Q.view(np.uint16), m, P, K.view(np.uint16), V.view(np.uint16))
+    assert float(np.max(np.abs(host(o) - ref))) < 2e-3
+    assert lkb.lib.lkb_pf_gemm_status() == 0
