@@ -36,8 +36,12 @@ def ptr(t):
     return t.data_ptr()
 
 
+_raw_stream, _device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+
+
 def stream():
-    return torch.cuda.current_stream().cuda_stream
+    # the handle itself: building torch.cuda.current_stream()'s Stream object took 3.2 us, a third of a launch
+    return _raw_stream(_device())
 
 
 def norm_prod(w=None, h32=None, yq8=None, ssq=None):

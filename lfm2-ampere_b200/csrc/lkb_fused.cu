@@ -130,6 +130,11 @@ __device__ __forceinline__ void grid_arrive(unsigned * bar, FusedSmem & S) {
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" :: "l"(bar) : "memory");
     }
 }
+// The arrival alone, by thread 0, where the data it publishes is thread 0's own.
+__device__ __forceinline__ void grid_arrive_one(unsigned * bar, FusedSmem & S) {
+    S.bar_target += gridDim.x;
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" :: "l"(bar) : "memory");
+}
 // One poll in flight per CTA.  (Keeping four relaxed polls in flight per CTA, a quarter of a round trip apart, was
 // measured: every barrier got 0.4-0.7 us SLOWER -- 148 CTAs x 4 loads on the one L2 line delay the arriving
 // reductions more than the finer sampling gains.  Sleeping 400 / 800 ns before the first poll cost 0.4 / 1.1 us
@@ -588,23 +593,16 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
             FUSED_STAMP(24);
         }
 
-        // ---- A: u = x*w; the 64 router CTAs produce their logit; arrive ----------
+        // ---- A: u = x*w and sums of squares; the 64 router CTAs produce their logit; arrive; quantise u in its shadow ----
+        // (Everyone waits for the logits, so they leave first: dot and 1/rms by warp 0, and thread 0 arrives for the CTA --
+        // its own store is the only one this barrier publishes.  Quantising before the arrival put 0.5 us more on each layer.)
         FUSED_STAMP(0);
         float xv[4], uv[4];
         fused_load_u(S, a.x, nw, xv, uv);
-        if (cta < LKB_N_EXPERTS) {
-            __syncthreads();                                        // S.h complete
-            if (warp == 0) {
-                if (!mbar_wait(&S.mbar_rt, par)) { if (lane == 0) { atomicCAS(status, 0u, 100u + l); S.abort = 1; } }
-                else {
-                    float acc = 0.0f;
-#pragma unroll 16
-                    for (int j = 0; j < LKB_HIDDEN / 32; ++j) acc = fmaf(S.router[j * 32 + lane], S.h[j * 32 + lane], acc);
-                    acc = lkb_warp_sum(acc);
-                    if (lane == 0) S.sel[0] = acc;                   // multiplied by inv below, once inv exists
-                }
-            }
-        } else if (pcta && pf_next) {
+        const float x_own = tid < n_dn ? __ldcg(a.x + dn0 + tid) : 0.0f;    // the residual rows this CTA will update
+        const float sq = lkb_quad_sum(__fmul_rn(xv[0], xv[0]), __fmul_rn(xv[1], xv[1]), __fmul_rn(xv[2], xv[2]), __fmul_rn(xv[3], xv[3]));
+        if ((lane & 7) == 0) S.ssq[tid >> 3] = sq;
+        if (pcta && pf_next) {
             // the next layer's router row (cta - 64) against this layer's input under the next layer's norm weights
             if (!mbar_wait(&S.mbar_rt, par)) { if (lane == 0) { atomicCAS(status, 0u, 100u + l); S.abort = 1; } }
             else {
@@ -616,18 +614,33 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
                 if (lane == 0) S.ppart[warp] = acc;
             }
         }
+        __syncthreads();                                            // S.h, S.ssq (and the guesses' partials) complete
         FUSED_STAMP(1);
-        // ---- B: Q8_1 of u, ssq, inv (needed for the logit scale and for gate|up) --
-        fused_quant_u(S, xv, uv);
-        if (cta < LKB_N_EXPERTS && tid == 0) a.logits[cta] = __fmul_rn(S.sel[0], S.inv);
-        if (pcta && pf_next && tid == 0) {
+        if (warp == 0) {
+            const float inv = lkb_norm_inv(S.ssq, lane, LKB_EPS);
             float acc = 0.0f;
+            if (cta < LKB_N_EXPERTS) {
+                if (!mbar_wait(&S.mbar_rt, par)) { if (lane == 0) { atomicCAS(status, 0u, 100u + l); S.abort = 1; } }
+                else {
+#pragma unroll 16
+                    for (int j = 0; j < LKB_HIDDEN / 32; ++j) acc = fmaf(S.router[j * 32 + lane], S.h[j * 32 + lane], acc);
+                    acc = lkb_warp_sum(acc);
+                }
+            }
+            if (lane == 0) {
+                S.inv = inv;
+                if (cta < LKB_N_EXPERTS) a.logits[cta] = __fmul_rn(acc, inv);
+                if (pcta && pf_next) {
+                    float g = 0.0f;
 #pragma unroll
-            for (int w = 0; w < FUSED_WARPS; ++w) acc += S.ppart[w];
-            a.gu[PF_LOGITS_OFF + cta - LKB_N_EXPERTS] = acc * S.inv;
+                    for (int w = 0; w < FUSED_WARPS; ++w) g += S.ppart[w];
+                    a.gu[PF_LOGITS_OFF + cta - LKB_N_EXPERTS] = g * inv;
+                }
+                grid_arrive_one(a.bar, S);
+            }
         }
+        quad_quant_to_xq(S.xq, uv);
         FUSED_STAMP(2);
-        grid_arrive(a.bar, S);
         // static data of the selection, fetched while the barrier completes
         float rb0 = 0.0f, rb1 = 0.0f;
         if (warp == 0 && ly.rbias) { rb0 = __ldg(ly.rbias + lane); rb1 = __ldg(ly.rbias + lane + 32); }
@@ -902,7 +915,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
             float acc = 0.0f;
 #pragma unroll
             for (int k = 0; k < LKB_TOP_K; ++k) acc = fmaf(S.wk[k], S.dot[k][tid], acc);
-            a.x[dn0 + tid] = __fadd_rn(__ldcg(a.x + dn0 + tid), acc);
+            a.x[dn0 + tid] = __fadd_rn(x_own, acc);
         }
         FUSED_STAMP(7);
         grid_arrive(a.bar, S);
