@@ -49,6 +49,7 @@
 #define PF_MAXL       512
 #define PF_GUESS_OFF  (PF_LOGITS_OFF + 128)
 #define PF_REAL_OFF   (PF_GUESS_OFF + 4 * PF_MAXL)
+static_assert(MAX_DN_ROWS <= FUSED_WARPS, "a down row per warp");
 static_assert(PF_REAL_OFF + 4 * PF_MAXL <= 2 * LKB_TOP_K * LKB_MOE_INTER, "prefetch records must fit the gu scratch");
 
 struct FusedSmem {
@@ -59,7 +60,7 @@ struct FusedSmem {
     alignas(16)  float  router[LKB_HIDDEN];                               // 8192
     alignas(16)  float  h[LKB_HIDDEN];                                    // 8192 raw u = x*w
     alignas(16)  lkb_q8blk xq[LKB_HIDDEN / 32];                           // 2304
-    alignas(16)  int8_t xq2_q[LKB_TOP_K * DN_BPR * 32];                   // 6144: quants of silu(g)*u, 32 B per block
+    alignas(16)  int8_t xq2_q[2][LKB_TOP_K * DN_BPR * 16];                // 6144: quants of silu(g)*u, first and second 16 of every block
     alignas(8)   float2 xq2_s[LKB_TOP_K * DN_BPR];                        // 1536: (float(fp16 d), 8*float(fp16 sum))
     float  ssq[LKB_HIDDEN / 32];
     float  sel[LKB_N_EXPERTS];
@@ -572,6 +573,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
             // ---- M3: the mixer's 2048 outputs, written by their owner CTAs, quantised by every CTA; then this CTA's output-projection rows, added to the residual ----
             {
                 const float4 o4 = __ldcg(reinterpret_cast<const float4 *>(a.mxbuf) + tid);
+                const float xo = lane == 0 && warp < n_dn ? __ldcg(a.x + dn0 + warp) : 0.0f;      // the row this warp will update
                 const float o[4] = {o4.x, o4.y, o4.z, o4.w};
                 quad_quant_to_xq(S.xq, o);
                 __syncthreads();
@@ -580,10 +582,10 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
                 load_xregs<2>(S.xq, GU_BPR, lane, xq, d8, s8);
                 if (!mbar_wait(&S.mbar_mo, par)) { if (lane == 0) { atomicCAS(status, 0u, 500u + l); S.abort = 1; } }
                 else {
-                    for (int j = warp; j < n_dn; j += FUSED_WARPS) {
+                    if (const int j = warp; j < n_dn) {                     // n_dn <= MAX_DN_ROWS = FUSED_WARPS
                         const float acc = lkb_warp_sum(smem_row_partial<2>(S.dn_q + (size_t) j * GU_BPR * 16, S.dn_d + (size_t) j * GU_BPR,
                                                                            GU_BPR, lane, xq, d8, s8));
-                        if (lane == 0) a.x[dn0 + j] = __fadd_rn(__ldcg(a.x + dn0 + j), acc);
+                        if (lane == 0) a.x[dn0 + j] = __fadd_rn(xo, acc);
                     }
                 }
             }
@@ -863,50 +865,60 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
                 float2 sc;
                 const unsigned pk = lkb_quad_quant(v[j], lane, sc);
                 const int b = (warp + FUSED_WARPS * j) * 4 + (lane >> 3);
-                reinterpret_cast<unsigned *>(S.xq2_q)[b * 8 + (lane & 7)] = pk;
+                reinterpret_cast<unsigned *>(S.xq2_q[(lane >> 2) & 1])[b * 4 + (lane & 3)] = pk;
                 if ((lane & 7) == 0) S.xq2_s[b] = sc;
             }
         }
         __syncthreads();
         FUSED_STAMP(11);
-        // one output row per warp, its four expert dots interleaved
-        for (int j = warp; j < n_dn; j += FUSED_WARPS) {
-            bool here[LKB_TOP_K], ok = true;                        // four probes in flight, then the bounded waits if needed
+        // Two output rows and two experts per warp: a block's activation is read from shared memory once for both rows.  This
+        // phase is bound by shared-memory wavefronts; with one row and four experts per warp and 32-byte activation blocks
+        // (two-way bank conflicts) it took 1.6 us, so 1.1.
+        {
+            const int j0 = 2 * (warp >> 1), k0 = 2 * (warp & 1);            // n_dn <= MAX_DN_ROWS = FUSED_WARPS
+            if (j0 < n_dn) {
+                unsigned long long * const m0 = &S.mbar_dn[k0 * dn_ch_per_k + j0 / CH_ROWS], * const m1 = &S.mbar_dn[(k0 + 1) * dn_ch_per_k + j0 / CH_ROWS];
+                const bool h0 = mbar_try_wait(m0, par), h1 = mbar_try_wait(m1, par);      // both probes in flight, then the bounded waits if needed
+                const bool ok = __all_sync(LKB_FULL, (h0 || mbar_wait(m0, par)) && (h1 || mbar_wait(m1, par)));
+                FUSED_STAMP(15);
+                if (!ok) { if (lane == 0) { atomicCAS(status, 0u, 300u + l); S.abort = 1; } }
+                else {
+                    const bool two = j0 + 1 < n_dn;
+                    float acc[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};          // [expert][row]
 #pragma unroll
-            for (int k = 0; k < LKB_TOP_K; ++k) here[k] = mbar_try_wait(&S.mbar_dn[k * dn_ch_per_k + j / CH_ROWS], par);
+                    for (int h = 0; h < 2; ++h) {
+                        const int blk = lane + 32 * h;
+                        if (blk < DN_BPR) {
 #pragma unroll
-            for (int k = 0; k < LKB_TOP_K; ++k) ok = ok && (here[k] || mbar_wait(&S.mbar_dn[k * dn_ch_per_k + j / CH_ROWS], par));
-            ok = __all_sync(LKB_FULL, ok);                          // the shuffles below need the whole warp
-            if (!ok) { if (lane == 0) { atomicCAS(status, 0u, 300u + l); S.abort = 1; } break; }
-            FUSED_STAMP(15);
-            float acc[LKB_TOP_K];
+                            for (int k = 0; k < 2; ++k) {
+                                const int b = (k0 + k) * DN_BPR + blk;
+                                const int4 x0 = *reinterpret_cast<const int4 *>(S.xq2_q[0] + b * 16), x1 = *reinterpret_cast<const int4 *>(S.xq2_q[1] + b * 16);
+                                const int xv8[8] = { x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w };
+                                const float2 sc = S.xq2_s[b];
 #pragma unroll
-            for (int k = 0; k < LKB_TOP_K; ++k) {
-                const unsigned char * wq = S.dn_q + ((size_t) k * MAX_DN_ROWS + j) * DN_BPR * 16;
-                const __half * wd = S.dn_d + ((size_t) k * MAX_DN_ROWS + j) * DN_BPR;
-                float acc_k = 0.0f;
+                                for (int r = 0; r < 2; ++r) {
+                                    const size_t wb = ((size_t) (k0 + k) * MAX_DN_ROWS + j0 + r) * DN_BPR + blk;   // (row n_dn: staged garbage, not stored)
+                                    const uint4 w = *reinterpret_cast<const uint4 *>(S.dn_q + wb * 16);
+                                    acc[k][r] = lkb_block_acc(__half2float(S.dn_d[wb]), sc.x, lkb_sumi(w, xv8), sc.y, acc[k][r]);
+                                }
+                            }
+                        }
+                    }
+                    FUSED_STAMP(14);
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int blk = lane + 32 * h;
-                    if (blk < DN_BPR) {
-                        const uint4 w = *reinterpret_cast<const uint4 *>(wq + (size_t) blk * 16);
-                        const int4 x0 = *reinterpret_cast<const int4 *>(S.xq2_q + (k * DN_BPR + blk) * 32);
-                        const int4 x1 = *reinterpret_cast<const int4 *>(S.xq2_q + (k * DN_BPR + blk) * 32 + 16);
-                        const int xv8[8] = { x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w };
-                        const float2 sc = S.xq2_s[k * DN_BPR + blk];
-                        acc_k = lkb_block_acc(__half2float(wd[blk]), sc.x, lkb_sumi(w, xv8), sc.y, acc_k);
+                    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                        for (int k = 0; k < 2; ++k)
+#pragma unroll
+                            for (int r = 0; r < 2; ++r) acc[k][r] = __fadd_rn(acc[k][r], __shfl_xor_sync(LKB_FULL, acc[k][r], o));
+                    if (lane == 0) {
+#pragma unroll
+                        for (int k = 0; k < 2; ++k) {
+                            S.dot[k0 + k][j0] = acc[k][0];
+                            if (two) S.dot[k0 + k][j0 + 1] = acc[k][1];
+                        }
                     }
                 }
-                acc[k] = acc_k;
-            }
-            FUSED_STAMP(14);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-                for (int k = 0; k < LKB_TOP_K; ++k) acc[k] = __fadd_rn(acc[k], __shfl_xor_sync(LKB_FULL, acc[k], o));
-            if (lane == 0) {
-#pragma unroll
-                for (int k = 0; k < LKB_TOP_K; ++k) S.dot[k][j] = acc[k];
             }
         }
         __syncthreads();
