@@ -34,6 +34,10 @@
 //   * Persistent: one CTA per SM walks the items, expert by expert, so an expert's weights stay in L2.
 // Measured per layer, token lanes with padding -> this form: gate|up 727 -> 676 us at 4096 tokens (Zipf routing), 315 -> 162 at
 // 509, 259 -> 84 at 37; down 379 -> 324, 170 -> 88, 134 -> 50; in_proj 299 -> 287 at 4096, 64 -> 60 at 509.
+// Then, GEMM alone, balanced routing, 4096 / 509 / 37 tokens (weight scales read from their own ring, expansion a stage at a
+// time, no scale barriers, two MMA issuers): gate|up 580 / 111 / 50 -> 526 / 103 / 44 us, down 259 / 57 / 28 -> 244 / 54 / 24,
+// in_proj 247 / 50 / 20 -> 229 / 47 / 19.  A 16384-value block is then 600 cycles of a scheduler: some 320 to 380 of packed
+// FMAs and 200 issue slots of everything else, 300 of synchronisation when the FMAs are left out.
 // No copy in this file is a multicast one; every tensor map covers memory of the GPU the kernel runs on.
 // Every wait is bounded; on expiry a status word is set and all roles drain and exit, freeing TMEM.
 #include "lkb_tc.cuh"
@@ -42,18 +46,19 @@
 #define TC_TOK       64             // tokens per work item (TMEM columns of one tile's block sums)
 #define TC_KB        4              // blocks per pipeline stage = 128 bytes of K per activation row
 #define TC_NS        5              // stages
-#define TC_DBUF      2              // block-sum buffers of 2 x 64 TMEM columns: block j of a stage lands in buffer j & 1
-#define TC_AUNITS    4              // A buffers of two blocks (2 tiles x 2 blocks x 8 TMEM columns): two stages
+#define TC_DBUF      2              // block-sum buffers, 256 TMEM columns in all: block j of a stage lands in buffer j & 1
+#define TC_AUNITS    2              // A buffers of one stage (2 tiles x 4 blocks x 8 TMEM columns)
 #define TC_COL_A     256            // first TMEM column of the A buffers
 #define TC_COL_SEED  384            // 8 columns of the constant A operand
 #define TC_EPI_WARPS 8              // warps 0..7: lane quadrant = warp & 3, column half = warp >> 2
 #define TC_EXP_W0    8              // expansion warps 8..11: quadrant = warp & 3
 #define TC_EXP_WARPS 4
-#define TC_MMA_WARP  12
-#define TC_PROD_WARP 13             // warps 14, 15 only complete the warpgroup that setmaxnreg needs
+#define TC_MMA_WARP  12             // MMA issuers 12, 13
+#define TC_PROD_WARP 14             // warp 15 only completes the warpgroup that setmaxnreg needs
 #define TC_THREADS   512
 #define TC_SC_AHEAD  6              // stages the block scales are requested ahead
-#define TC_SC_RING   8              // stages of scales in shared memory
+#define TC_SC_RING   8              // stages of activation scales in shared memory (read by the thread that requests them)
+#define TC_WS_RING   16             // stages of weight scales: the epilogue reads them up to TC_NS stages behind the expansion
 #define TC_MAGIC_I   0x4B400000
 #define TC_MAGIC_F   12582912.0f
 #define TC_SEED      65536.0f       // 32 products 64 * 32
@@ -64,17 +69,18 @@
 struct TcStage {
     alignas(1024) unsigned char act[TC_TOK * 128];      // activations: row r at r*128, 16-byte chunk c at c ^ (r & 7)
     alignas(1024) unsigned char rawq[2 * TC_ROWS * 64]; // nibbles as in the pack: row r at r*64, chunk c at c ^ ((r >> 1) & 3)
-    alignas(16)   float4 dk[TC_KB][TC_TOK / 2];         // per block and token pair {d8, d8', k, k'}
-    alignas(16)   float  d4[TC_KB][2 * TC_ROWS];        // weight block scales
 };
 static_assert(sizeof(TcStage) % 1024 == 0, "stages keep the 1024-byte alignment of the swizzled operands");
+static_assert(TC_SC_RING > TC_NS, "constants stay until the epilogue has read them: see the expansion warps");
+static_assert(TC_WS_RING >= TC_SC_AHEAD + TC_NS + 2 && !(TC_WS_RING & (TC_WS_RING - 1)), "weight scales stay until the epilogue has read them");
 
 struct TcSmem {
     TcStage st[TC_NS];
     alignas(1024) unsigned seed_b[TC_TOK * 8];                              // constant B operand: 64 rows of 32 bytes
-    alignas(16) uint4  wsc[TC_SC_RING / 2][2 * TC_ROWS];                    // eight fp16 scales per row (two stages)
+    alignas(16) float4 dk[TC_SC_RING][TC_KB][TC_TOK / 2];                   // per stage, block and token pair {d8, d8', k, k'}
+    alignas(16) uint4  wsc[TC_WS_RING / 2][2 * TC_ROWS];                    // eight fp16 scales per row (two stages)
     alignas(16) float4 asc[TC_SC_RING][TC_EXP_WARPS * 32];                  // (d8, 8sum) of two blocks per expansion thread
-    alignas(8) unsigned long long full[TC_NS], empty[TC_NS], kfull[TC_NS], afull[TC_AUNITS], aempty[TC_AUNITS], tfull[TC_DBUF], tempty[TC_DBUF];
+    alignas(8) unsigned long long full[TC_NS], empty[TC_NS], afull[TC_AUNITS], aempty[TC_AUNITS], tfull[2][TC_DBUF], tempty[2][TC_DBUF];
     unsigned tmem_base;
     int      abort;
 };
@@ -119,10 +125,16 @@ __device__ __forceinline__ int tc_seg(const lkb_pf_gemm & g, int row) { return (
 // ---------------------------------------------------------------------------
 // Epilogue state carried from item to item by every epilogue thread.
 // ---------------------------------------------------------------------------
-struct TcEpi {
-    unsigned stg, par;              // the next stage and the parity of its phase
-    __device__ __forceinline__ void next() { if (++stg == TC_NS) { stg = 0; par ^= 1u; } }
+// Block-sum buffers and who fills them.  Free halves (SwiGLU form): each column half has two buffers and an MMA issuer of its
+// own, so the four warps of a half never wait for the other four, which matters where the item ends in the long SwiGLU store
+// (gate|up at 4096 tokens 554 -> 531 us, at 509 107 -> 104, at 37 43 -> 44).  Plain form: one 64-column MMA per tile, common
+// buffers, issuer h for buffer h; half the MMAs (down and in_proj at 37 tokens 4 % faster than with free halves, equal at 4096).
+template <int EPI> struct TcSums {
+    static constexpr int FREE = EPI, TILE = FREE ? TC_TOK / 2 : TC_TOK, BUF = 2 * TILE;      // columns between tiles, between buffers
+    static constexpr int EPI_ARRIVE = FREE ? TC_EPI_WARPS / 2 : TC_EPI_WARPS;
 };
+
+struct TcEpi { unsigned it; };      // the number of the next stage
 
 // Fold NL columns, from column C0 on, of one block into R rows' accumulators.
 template <int FOLD, int R, int NC, int C0, int NL>
@@ -143,35 +155,44 @@ __device__ __forceinline__ void tc_fold(unsigned long long (&acc)[R][NC / 2], co
     }
 }
 
+template <int FOLD> __device__ __forceinline__ float tc_row_scale(__half d4) {
+    const float f = __half2float(d4);
+    return FOLD ? __fmul_rn(f, TC_UP49) : f;
+}
+
 // All blocks of one item for this thread's R rows x NC tokens, as a software pipeline over column halves: while one half's
 // sums are folded the TMEM load of the next half (of this block, or of the next one) is in flight.  (Whole-block double
 // buffering needs 128 registers for the sums beside the 64 accumulators and leaves none to run the scale loads ahead.)
 // Returns false when a wait gave up.
-template <int FOLD, int R, int NC>
+template <int EPI, int FOLD, int R, int NC>
 __device__ __forceinline__ bool tc_fold_item(TcSmem & S, TcEpi & X, unsigned tbase, int half, int row, int lane, int nstage,
                                              unsigned long long (&acc)[R][NC / 2]) {
     constexpr int NA = NC == 24 ? 16 : NC == 8 ? 8 : NC / 2, NB = NC - NA;              // columns of the two halves (8: one piece)
     unsigned sva[R][NA], svb[R][NB ? NB : 8];
-    const unsigned tcol = tbase + half * NC;
+    using L = TcSums<EPI>;
+    const unsigned tcol = tbase + half * (L::FREE ? 2 * L::BUF : NC);
+    unsigned long long * const tfull = S.tfull[L::FREE ? half : 0], * const tempty = S.tempty[L::FREE ? half : 0];
 #pragma unroll
     for (int r = 0; r < R; ++r)
 #pragma unroll
         for (int i = 0; i < NC / 2; ++i) acc[r][i] = 0ull;
-    if (!tc_wait(S, &S.tfull[0], 0u, 31u)) return false;
+    if (!tc_wait(S, &tfull[0], 0u, 31u)) return false;
     tc_fence_after();
 #pragma unroll
-    for (int r = 0; r < R; ++r) tc_ld<NA>(tcol + r * TC_TOK, sva[r]);
+    for (int r = 0; r < R; ++r) tc_ld<NA>(tcol + r * L::TILE, sva[r]);
     for (int ks = 0; ks < nstage; ++ks) {
-        if (!tc_wait(S, &S.kfull[X.stg], X.par, 30u)) return false;                   // the stage's scales are in place
-        const TcStage & T = S.st[X.stg];
+        __half we[2][TC_KB];                                                          // this thread's row scales of the stage
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            *reinterpret_cast<uint2 *>(we[r]) = *(reinterpret_cast<const uint2 *>(&S.wsc[(X.it >> 1) & (TC_WS_RING / 2 - 1)][r * TC_ROWS + row]) + (X.it & 1u));
         // Two blocks per trip: buffers are then fixed (block j -> j & 1) and the phase parity is the trip number (a stage
         // uses each buffer twice), which keeps the synchronisation to a handful of instructions with fixed addresses.
 #pragma unroll
         for (unsigned u = 0; u < 2; ++u) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const float4 * dk = &T.dk[2 * u + h][(half * NC) / 2];
-                const float e0 = T.d4[2 * u + h][row], e1 = R == 2 ? T.d4[2 * u + h][TC_ROWS + row] : 0.0f;
+                const float4 * dk = &S.dk[X.it & (TC_SC_RING - 1)][2 * u + h][(half * NC) / 2];
+                const float e0 = tc_row_scale<FOLD>(we[0][2 * u + h]), e1 = R == 2 ? tc_row_scale<FOLD>(we[1][2 * u + h]) : 0.0f;
                 const unsigned long long ep[2] = {tc_pack(e0, e0), tc_pack(e1, e1)};
                 const bool more = h == 0 || u == 0 || ks < nstage - 1;
                 float4 ka[NA / 2], kb[NB ? NB / 2 : 4];
@@ -181,28 +202,26 @@ __device__ __forceinline__ bool tc_fold_item(TcSmem & S, TcEpi & X, unsigned tba
                 for (int i = 0; i < NB / 2; ++i) kb[i] = dk[NA / 2 + i];
                 tc_wait_ld();                                                         // the first half is in sva
                 // (polled ahead of the fold and looked at behind it: the answer's latency is hidden)
-                const bool ready = more && tc_mbar_try<0>(&S.tfull[h ^ 1], h == 0 ? u : u ^ 1u);
+                const bool ready = more && tc_mbar_try<0>(&tfull[h ^ 1], h == 0 ? u : u ^ 1u);
                 if constexpr (NB > 0) {
 #pragma unroll
-                    for (int r = 0; r < R; ++r) tc_ld<NB ? NB : 8>(tcol + h * (2 * TC_TOK) + r * TC_TOK + NA, svb[r]);
+                    for (int r = 0; r < R; ++r) tc_ld<NB ? NB : 8>(tcol + h * L::BUF + r * L::TILE + NA, svb[r]);
                     tc_fold<FOLD, R, NC, 0, NA>(acc, sva, ka, ep);
                     tc_wait_ld();
                 } else tc_fold<FOLD, R, NC, 0, NA>(acc, sva, ka, ep);
                 tc_fence_before();
                 __syncwarp();
-                tc_mbar_arrive_if(&S.tempty[h], lane == 0);                           // the buffer is free again
+                tc_mbar_arrive_if(&tempty[h], lane == 0);                           // the buffer is free again
                 if (more) {
-                    if (!ready && !tc_wait(S, &S.tfull[h ^ 1], h == 0 ? u : u ^ 1u, 31u)) return false;
+                    if (!ready && !tc_wait(S, &tfull[h ^ 1], h == 0 ? u : u ^ 1u, 31u)) return false;
                     tc_fence_after();
 #pragma unroll
-                    for (int r = 0; r < R; ++r) tc_ld<NA>(tcol + (h ^ 1) * (2 * TC_TOK) + r * TC_TOK, sva[r]);
+                    for (int r = 0; r < R; ++r) tc_ld<NA>(tcol + (h ^ 1) * L::BUF + r * L::TILE, sva[r]);
                 }
                 if constexpr (NB > 0) tc_fold<FOLD, R, NC, NA, NB ? NB : 8>(acc, svb, kb, ep);
             }
         }
-        __syncwarp();
-        tc_mbar_arrive_if(&S.empty[X.stg], lane == 0);
-        X.next();
+        ++X.it;
     }
     return true;
 }
@@ -354,7 +373,7 @@ template <int EPI, int FOLD, int R, int NC>
 __device__ __forceinline__ bool tc_epilogue_item(TcSmem & S, TcEpi & X, const lkb_pf_gemm & g, const TcPlan & P, const TcItem & I, float * const * out_rows,
                                                  unsigned tbase, int half, int quad, int lane) {
     unsigned long long acc[R][NC / 2];
-    if (!tc_fold_item<FOLD, R, NC>(S, X, tbase, half, quad * 32 + lane, lane, P.nstage, acc)) return false;
+    if (!tc_fold_item<EPI, FOLD, R, NC>(S, X, tbase, half, quad * 32 + lane, lane, P.nstage, acc)) return false;
     if constexpr (EPI == 0) tc_store_plain<R, NC>(g, P, I, out_rows, half, quad * 32 + lane, lane, acc);
     else if constexpr (NC == 8) tc_store_swiglu<FOLD, NC, 8>(g, I, half, 0, quad, lane, acc);
     else {
@@ -411,11 +430,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_pf_gemm_tc(const lkb_pf_gemm 
         S.abort = 0;
         for (int i = 0; i < TC_NS; ++i) {
             tc_mbar_init(&S.full[i], 1);                              // the lane that posts the bytes
-            tc_mbar_init(&S.empty[i], 1 + TC_EPI_WARPS);              // MMA commit (nibbles, activations) + epilogue warps (scales)
-            tc_mbar_init(&S.kfull[i], TC_EXP_WARPS);
+            tc_mbar_init(&S.empty[i], 2);                       // both issuers' commits
         }
-        for (int i = 0; i < TC_AUNITS; ++i) { tc_mbar_init(&S.afull[i], TC_EXP_WARPS); tc_mbar_init(&S.aempty[i], 1); }
-        for (int i = 0; i < TC_DBUF; ++i) { tc_mbar_init(&S.tfull[i], 1); tc_mbar_init(&S.tempty[i], TC_EPI_WARPS); }
+        for (int i = 0; i < TC_AUNITS; ++i) { tc_mbar_init(&S.afull[i], TC_EXP_WARPS); tc_mbar_init(&S.aempty[i], 2); }
+        for (int i = 0; i < 2 * TC_DBUF; ++i) { tc_mbar_init(&S.tfull[0][i], 1); tc_mbar_init(&S.tempty[0][i], TcSums<EPI>::EPI_ARRIVE); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -501,54 +519,62 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_pf_gemm_tc(const lkb_pf_gemm 
                 }
             }
         }
-        // ============================ MMA issuer (one warp) ==========================
+        // ============================ MMA issuers (two warps) ========================
+        // Issuer q serves column half q (free halves) or block-sum buffer q, that is blocks q and q + 2 of every stage: polls,
+        // issue and commits of a block take some 200 cycles, and one issuer for everything made that a serial part of the loop.
         // The whole warp runs the loop, so that descriptors and addresses stay in uniform registers; one elected lane issues.
-        else if (warp == TC_MMA_WARP) {
-            unsigned stg = 0, par = 0, apar = 0, ab = 0;          // stage and its parity; A buffers (pairs 0/1, 2/3) and theirs
+        else if (warp < TC_MMA_WARP + 2) {
+            using L = TcSums<EPI>;
+            const unsigned q = warp - TC_MMA_WARP;
+            unsigned stg = 0, par = 0, apar = 0, ab = 0;          // stage and its parity; A buffer and its
             bool ok = true;
             const unsigned long long dseed = tc_desc_seed(tc_smem_u32(S.seed_b));
+            const unsigned d0 = tmem + (L::FREE ? q * (2 * L::BUF) : 0);
+            unsigned long long * const tfull = S.tfull[L::FREE ? q : 0], * const tempty = S.tempty[L::FREE ? q : 0];
             const bool leader = tc_elect();
             TcItem I = tc_item(g, P, blockIdx.x);
             for (int item = blockIdx.x; item < P.n_items && ok; item += gridDim.x) {
-                const unsigned idesc = TC_IDESC(tc_cols(I.tcnt));
+                const unsigned nc = tc_cols(I.tcnt) / 2;          // columns of a half; the MMA's N is a multiple of 16 (rows past the half are dead)
+                const unsigned idesc = TC_IDESC(L::FREE ? (nc + 15) & ~15u : 2 * nc);
                 const bool two = tc_two<EPI>(g, P, I.rt);
                 if (item + (int) gridDim.x < P.n_items) I = tc_item(g, P, item + gridDim.x);
                 for (int ks = 0; ks < P.nstage && ok; ++ks) {
                     if (!tc_wait<TC_HINT_MMA>(S, &S.full[stg], par, 20u)) { ok = false; break; }
-                    const unsigned long long b0 = tc_desc(tc_smem_u32(S.st[stg].act));
+                    if (!tc_wait<TC_HINT_MMA>(S, &S.afull[ab], apar, 22u)) { ok = false; break; }
+                    const unsigned long long b0 = tc_desc(tc_smem_u32(S.st[stg].act) + (L::FREE ? q * nc * 128 : 0));
+                    const unsigned a0 = tmem + TC_COL_A + ab * 64;
 #pragma unroll
-                    for (unsigned u = 0; u < 2; ++u) {
-                        if (!tc_wait<TC_HINT_MMA>(S, &S.afull[ab + u], apar, 22u)) { ok = false; break; }
-#pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            // use k of a buffer waits for phase k: the epilogue releases every buffer once up front
-                            if (!tc_wait<TC_HINT_MMA>(S, &S.tempty[h], u, 21u)) { ok = false; break; }
-                            tc_fence_after();
-                            if (leader) {
-                                const unsigned d = tmem + h * (2 * TC_TOK), a = tmem + TC_COL_A + (ab + u) * 32 + h * 8;
-                                const unsigned long long b = b0 + (2 * u + h) * 2;     // 32 bytes further, in 16-byte units
-                                if (FOLD) {
-                                    tc_mma_i8(d, tmem + TC_COL_SEED, dseed, idesc, 0u);
-                                    if (two) tc_mma_i8(d + TC_TOK, tmem + TC_COL_SEED, dseed, idesc, 0u);
-                                }
-                                tc_mma_i8(d, a, b, idesc, FOLD);
-                                if (two) tc_mma_i8(d + TC_TOK, a + 16, b, idesc, FOLD);
-                                tc_commit(&S.tfull[h]);                                // this block's sums are ready
-                                if (h == 1) tc_commit(&S.aempty[ab + u]);
-                                if (h == 1 && u == 1) tc_commit(&S.empty[stg]);        // the MMAs have finished reading the stage
+                    for (unsigned i = 0; i < (L::FREE ? TC_KB : TC_KB / 2); ++i) {
+                        const unsigned j = L::FREE ? i : 2 * i + q, h = L::FREE ? i & 1 : q;
+                        // use k of a buffer waits for phase k: the epilogue releases every buffer once up front
+                        if (!tc_wait<TC_HINT_MMA>(S, &tempty[h], L::FREE ? i >> 1 : i, 21u)) { ok = false; break; }
+                        tc_fence_after();
+                        if (leader) {
+                            const unsigned d = d0 + h * L::BUF, a = a0 + j * 8;
+                            const unsigned long long b = b0 + j * 2;               // a block is 32 bytes, in 16-byte units
+                            if (FOLD) {
+                                tc_mma_i8(d, tmem + TC_COL_SEED, dseed, idesc, 0u);
+                                if (two) tc_mma_i8(d + L::TILE, tmem + TC_COL_SEED, dseed, idesc, 0u);
                             }
-                            __syncwarp();
+                            tc_mma_i8(d, a, b, idesc, FOLD);
+                            if (two) tc_mma_i8(d + L::TILE, a + 32, b, idesc, FOLD);
+                            tc_commit(&tfull[h]);                                  // this block's sums are ready
+                            if (i + 1 == (L::FREE ? TC_KB : TC_KB / 2)) { tc_commit(&S.aempty[ab]); tc_commit(&S.empty[stg]); }    // the stage has been read
                         }
-                        if (!ok) break;
+                        __syncwarp();
                     }
                     if (++stg == TC_NS) { stg = 0; par ^= 1u; }
-                    ab ^= 2u;
+                    ab ^= 1u;
                     if (ab == 0) apar ^= 1u;
                 }
             }
         }
     }
     // ============================ expansion (four warps) ==========================
+    // The epilogue waits for block sums only: scales and constants are written before afull, the issuers acquire afull before
+    // they issue, and a block's tfull completes after its MMA.  Nor does the epilogue hand them back: a stage comes round
+    // (empty) when the issuers have passed it, and a buffer they reused was released behind every read of the stage before,
+    // so rings of more than TC_NS + 1 stages are never overwritten early.  (Two barriers of their own per stage cost 5 %.)
     // Thread e serves weight rows e and 128 + e of the item and two blocks of token e / 2: it brings their block scales into
     // shared memory (its own cp.async, TC_SC_AHEAD stages ahead), forms the fold's constants, and turns its rows' nibbles
     // into int8 in TMEM (byte i of a block's 16: element i in the low nibble, element i + 16 in the high one).
@@ -581,7 +607,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_pf_gemm_tc(const lkb_pf_gemm 
             if (p_item < P.n_items) {
                 if (p_sc) tc_cp16(&S.asc[p_it % TC_SC_RING][e], p_sc + p_ks * (TC_KB * 8));
                 if (!(p_ks & 1)) {
-                    char * const s0 = (char *) &S.wsc[(p_it >> 1) % (TC_SC_RING / 2)][e];
+                    char * const s0 = (char *) &S.wsc[(p_it >> 1) % (TC_WS_RING / 2)][e];
                     const int o = p_ks * (TC_KB * 2);
                     if (((size_t) p_w0 | (size_t) p_w1) & 8) {                          // planes that are only 8-byte aligned
                         if (p_w0) { tc_cp8(s0, p_w0 + o); tc_cp8(s0 + 8, p_w0 + o + 8); }
@@ -609,29 +635,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_pf_gemm_tc(const lkb_pf_gemm 
                 tc_cp_wait<TC_SC_AHEAD - 1>();                                          // this stage's scales are here
                 if (!tc_wait<TC_HINT_PROD>(S, &S.full[stg], par, 15u)) { ok = false; break; }
                 TcStage & T = S.st[stg];
-#pragma unroll 1
-                for (unsigned u = 0; u < 2; ++u) {
-                    const unsigned au = 2 * (it & 1u) + u;                              // A buffer, its parity turns every other stage
-                    if (!tc_wait<TC_HINT_PROD>(S, &S.aempty[au], ((it >> 1) & 1u) ^ 1u, 16u)) { ok = false; break; }
-                    tc_fence_after();
-#pragma unroll
-                    for (int r = 0; r < 2; ++r) {
-                        if (r && !two) continue;
-                        const unsigned char * rq = T.rawq + (r * TC_ROWS + e) * 64;
-#pragma unroll
-                        for (int jj = 0; jj < 2; ++jj) {
-                            const uint4 w = *reinterpret_cast<const uint4 *>(rq + (((2 * u + jj) ^ ((e >> 1) & 3)) << 4));
-                            tc_st8(ta + au * 32 + r * 16 + jj * 8,
-                                   make_uint4(w.x & 0x0F0F0F0Fu, w.y & 0x0F0F0F0Fu, w.z & 0x0F0F0F0Fu, w.w & 0x0F0F0F0Fu),
-                                   make_uint4((w.x >> 4) & 0x0F0F0F0Fu, (w.y >> 4) & 0x0F0F0F0Fu, (w.z >> 4) & 0x0F0F0F0Fu, (w.w >> 4) & 0x0F0F0F0Fu));
-                        }
-                    }
-                    tc_wait_st();
-                    tc_fence_before();
-                    __syncwarp();
-                    tc_mbar_arrive_if(&S.afull[au], lane == 0);
-                }
-                // the fold's constants, while the MMAs of these blocks run
+                // the fold's constants
                 if (tlive) {
                     const float4 a = S.asc[it % TC_SC_RING][e];
                     const float dd[2] = {a.x, a.z}, ss[2] = {a.y, a.w};
@@ -643,21 +647,29 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_pf_gemm_tc(const lkb_pf_gemm 
                             k = __fmul_rn(fmaf(-TC_SEED, d, fmaf(d, TC_MAGIC_F, -c)), TC_DOWN49);
                             d = __fmul_rn(d, TC_UP100);
                         }
-                        float * const q = reinterpret_cast<float *>(&T.dk[2 * (e & 1) + b][tok >> 1]) + (tok & 1);
+                        float * const q = reinterpret_cast<float *>(&S.dk[it % TC_SC_RING][2 * (e & 1) + b][tok >> 1]) + (tok & 1);
                         q[0] = d; q[2] = k;
                     }
                 }
+                if (!tc_wait<TC_HINT_PROD>(S, &S.aempty[it & 1u], ((it >> 1) & 1u) ^ 1u, 16u)) { ok = false; break; }
+                tc_fence_after();
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
                     if (r && !two) continue;
-                    const uint2 h = *(reinterpret_cast<const uint2 *>(&S.wsc[(it >> 1) % (TC_SC_RING / 2)][r * TC_ROWS + e]) + (it & 1u));
-                    const float2 f01 = __half22float2(*reinterpret_cast<const __half2 *>(&h.x)), f23 = __half22float2(*reinterpret_cast<const __half2 *>(&h.y));
-                    const float f[4] = {f01.x, f01.y, f23.x, f23.y};
+                    const unsigned char * rq = T.rawq + (r * TC_ROWS + e) * 64;
+                    uint4 w[4];
 #pragma unroll
-                    for (int j = 0; j < TC_KB; ++j) T.d4[j][r * TC_ROWS + e] = FOLD ? __fmul_rn(f[j], TC_UP49) : f[j];
+                    for (int j = 0; j < 4; ++j) w[j] = *reinterpret_cast<const uint4 *>(rq + ((j ^ ((e >> 1) & 3)) << 4));
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        tc_st8(ta + (it & 1u) * 64 + r * 32 + j * 8,
+                               make_uint4(w[j].x & 0x0F0F0F0Fu, w[j].y & 0x0F0F0F0Fu, w[j].z & 0x0F0F0F0Fu, w[j].w & 0x0F0F0F0Fu),
+                               make_uint4((w[j].x >> 4) & 0x0F0F0F0Fu, (w[j].y >> 4) & 0x0F0F0F0Fu, (w[j].z >> 4) & 0x0F0F0F0Fu, (w[j].w >> 4) & 0x0F0F0F0Fu));
                 }
+                tc_wait_st();
+                tc_fence_before();
                 __syncwarp();
-                tc_mbar_arrive_if(&S.kfull[stg], lane == 0);
+                tc_mbar_arrive_if(&S.afull[it & 1u], lane == 0);
                 fetch();
                 if (++stg == TC_NS) { stg = 0; par ^= 1u; }
             }
@@ -671,9 +683,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_pf_gemm_tc(const lkb_pf_gemm 
         const unsigned tbase = tmem + ((unsigned) (quad * 32) << 16);
         __syncwarp();
         if (lane == 0)                                          // all block-sum buffers start out free for the MMA issuer
-            for (int i = 0; i < TC_DBUF; ++i) tc_mbar_arrive(&S.tempty[i]);
+            for (int i = 0; i < TC_DBUF; ++i) tc_mbar_arrive(&S.tempty[TcSums<EPI>::FREE ? half : 0][i]);
         TcEpi X;
-        X.stg = X.par = 0;
+        X.it = 0;
         bool ok = true;
         TcItem I = tc_item(g, P, blockIdx.x);
         for (int item = blockIdx.x; item < P.n_items && ok; item += gridDim.x) {
