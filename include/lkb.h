@@ -104,8 +104,11 @@ typedef struct {
 int lkb_init(int device);
 const char * lkb_error_string(int status);
 int lkb_sm_count(void);
-/* 1: launch the decode kernels with programmatic dependent launch so that a
- * kernel's weight prefetch overlaps its predecessor's tail.  Default 0. */
+/* 1: launch the decode kernels that read weights ahead with programmatic
+ * dependent launch, so that the weight prefetch overlaps the predecessor's
+ * tail; no kernel of the stream may then write those weights.  Default 0.
+ * (Kernels that read nothing ahead of their predecessors' completion are
+ * always launched that way.) */
 int lkb_set_pdl(int enable);
 
 /* ------------------------------------------------- activation quantisers */

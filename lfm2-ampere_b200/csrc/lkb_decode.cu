@@ -230,7 +230,7 @@ static int launch_gemv(GemvArgs & a, cudaStream_t st) {
     if (a.bpr > 64) {
         const int wpb = 8;
         int grid = (a.total + wpb - 1) / wpb; if (grid > sms * 8) grid = sms * 8;
-        return lkb_launch(k_gemv_multi_generic, dim3(grid), dim3(wpb * 32), 0, st, a);
+        return lkb_launch_next(k_gemv_multi_generic, dim3(grid), dim3(wpb * 32), 0, st, a);
     }
     // one CTA per SM, 16 warps; fewer CTAs when there are fewer rows than warps
     const int wpb = 16;
@@ -239,13 +239,13 @@ static int launch_gemv(GemvArgs & a, cudaStream_t st) {
     if (need < grid) grid = need;
     const int rows_per_warp = (a.total + grid * wpb - 1) / (grid * wpb);
     if (a.bpr <= 32) {
-        if (rows_per_warp >= 4) return lkb_launch(k_gemv_multi<1, 8>, dim3(grid), dim3(wpb * 32), 0, st, a);
-        return lkb_launch(k_gemv_multi<1, 2>, dim3(grid), dim3(wpb * 32), 0, st, a);
+        if (rows_per_warp >= 4) return lkb_launch_next(k_gemv_multi<1, 8>, dim3(grid), dim3(wpb * 32), 0, st, a);
+        return lkb_launch_next(k_gemv_multi<1, 2>, dim3(grid), dim3(wpb * 32), 0, st, a);
     }
-    if (rows_per_warp >= 5) return lkb_launch(k_gemv_multi<2, 6>, dim3(grid), dim3(wpb * 32), 0, st, a);
-    if (rows_per_warp >= 3) return lkb_launch(k_gemv_multi<2, 4>, dim3(grid), dim3(wpb * 32), 0, st, a);
-    if (rows_per_warp >= 2) return lkb_launch(k_gemv_multi<2, 2>, dim3(grid), dim3(wpb * 32), 0, st, a);
-    return lkb_launch(k_gemv_multi<2, 1>, dim3(grid), dim3(wpb * 32), 0, st, a);
+    if (rows_per_warp >= 5) return lkb_launch_next(k_gemv_multi<2, 6>, dim3(grid), dim3(wpb * 32), 0, st, a);
+    if (rows_per_warp >= 3) return lkb_launch_next(k_gemv_multi<2, 4>, dim3(grid), dim3(wpb * 32), 0, st, a);
+    if (rows_per_warp >= 2) return lkb_launch_next(k_gemv_multi<2, 2>, dim3(grid), dim3(wpb * 32), 0, st, a);
+    return lkb_launch_next(k_gemv_multi<2, 1>, dim3(grid), dim3(wpb * 32), 0, st, a);
 }
 
 // ---------------------------------------------------------------------------
@@ -637,7 +637,7 @@ int lkb_quantize_q8_1(const float * x, lkb_block_q8_1 * y, int nblocks, lkb_stre
     LKB_REQUIRE_INIT();
     if (!x || !y) return LKB_ERR_NULL;
     if (nblocks <= 0) return nblocks == 0 ? LKB_OK : LKB_ERR_SHAPE;
-    return lkb_launch(k_quantize_q8_1, dim3((nblocks + 7) / 8), dim3(256), 0, (cudaStream_t) st,
+    return lkb_launch_next(k_quantize_q8_1, dim3((nblocks + 7) / 8), dim3(256), 0, (cudaStream_t) st,
                       x, reinterpret_cast<lkb_q8blk *>(y), nblocks);
 }
 
@@ -654,7 +654,7 @@ int lkb_norm_produce(const float * x, int n, const lkb_norm_prod_t * np, lkb_str
     LKB_REQUIRE_INIT();
     if (!x || !np || !np->w || !np->yq8 || !np->ssq) return LKB_ERR_NULL;
     if (n <= 0 || n % 32) return LKB_ERR_SHAPE;
-    return lkb_launch(k_norm_prod, dim3((n + 255) / 256), dim3(256), 0, (cudaStream_t) st, x, n, *np);
+    return lkb_launch_next(k_norm_prod, dim3((n + 255) / 256), dim3(256), 0, (cudaStream_t) st, x, n, *np);
 }
 
 int lkb_gemv_q4_0(const void * qs, const void * d, const lkb_block_q8_1 * xq, int out_rows, int bpr,

@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(256) k_ep_pack_push(const int8_t * __restrict_
                                                       const int * __restrict__ offs, int n, int experts_per_rank, EpPeers P, int me, int G,
                                                       const int * __restrict__ epoch_dev, int * __restrict__ pos,
                                                       unsigned * __restrict__ done) {
-    lkb_pdl_wait(); lkb_pdl_trigger();           // programmatic dependent launch: inputs complete from here on
+    lkb_pdl_wait();                              // inputs complete from here on; no early trigger: nothing waits on the SMs while this spins on peers
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int p = blockIdx.x * 8 + warp; p < n; p += gridDim.x * 8) {
         const int slot = send_order[p], t = slot >> 2;
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(256) k_ep_pack_push(const int8_t * __restrict_
 // Wait until every source has published `phase` for this epoch.
 __global__ void __launch_bounds__(32) k_ep_wait(const int * __restrict__ flags, int phase, int G, const int * __restrict__ epoch_dev,
                                                 int * __restrict__ status, unsigned long long limit_ns) {
-    lkb_pdl_wait(); lkb_pdl_trigger();           // programmatic dependent launch: inputs complete from here on
+    lkb_pdl_wait();                              // inputs complete from here on; no early trigger: nothing waits on the SMs while this spins on peers
     const int epoch = *epoch_dev;
     if ((int) threadIdx.x < G) ep_wait_flag(flags, phase, threadIdx.x, epoch, status, 2 + phase, limit_ns);
 }
@@ -173,7 +173,7 @@ __device__ __forceinline__ void ep_route_cta(EpRouteSmem & R, KeyFn key, int n, 
 __global__ void __launch_bounds__(1024) k_ep_route_exchange(const int * __restrict__ idx, int ns, int experts_per_rank, EpPeers P, int me, int G,
                                                             int * __restrict__ epoch_dev, int * __restrict__ send_order, int * __restrict__ doff,
                                                             int * __restrict__ offs, int * __restrict__ status, unsigned long long limit_ns) {
-    lkb_pdl_wait(); lkb_pdl_trigger();           // programmatic dependent launch: inputs complete from here on
+    lkb_pdl_wait();                              // inputs complete from here on; no early trigger: nothing waits on the SMs while this spins on peers
     __shared__ EpRouteSmem R;
     const int t = threadIdx.x;
     ep_route_cta(R, [&](int s) { return idx[s] / experts_per_rank; }, ns, nullptr, doff, nullptr, nullptr, send_order);
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(1024) k_ep_route_experts(const unsigned char *
                                                            int * __restrict__ ntiles, int * __restrict__ perm, int * __restrict__ nrecv_out,
                                                            EpPeers P, float ** __restrict__ home_rows, float * __restrict__ inv_out,
                                                            int * __restrict__ status, unsigned long long limit_ns) {
-    lkb_pdl_wait(); lkb_pdl_trigger();           // programmatic dependent launch: inputs complete from here on
+    lkb_pdl_wait();                              // inputs complete from here on; no early trigger: nothing waits on the SMs while this spins on peers
     __shared__ EpRouteSmem R;
     const int t = threadIdx.x;
     if (t == 0) R.ok = 1;
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(1024) k_ep_route_experts(const unsigned char *
 // GEMM writing result rows straight into their home ranks' buffers) are complete when this kernel starts.
 __global__ void __launch_bounds__(32) k_ep_publish(EpPeers P, int me, int G, int phase, const int * __restrict__ epoch_dev,
                                                    const int * __restrict__ wait_flags, int * __restrict__ status, unsigned long long limit_ns) {
-    lkb_pdl_wait(); lkb_pdl_trigger();           // programmatic dependent launch: inputs complete from here on
+    lkb_pdl_wait();                              // inputs complete from here on; no early trigger: nothing waits on the SMs while this spins on peers
     __threadfence_system();
     const int epoch = *epoch_dev;
     if ((int) threadIdx.x < G) ep_st_release(P.flags[threadIdx.x] + phase * EP_MAX_RANKS + me, epoch);

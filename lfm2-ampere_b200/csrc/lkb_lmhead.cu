@@ -100,7 +100,7 @@ __device__ __forceinline__ int lm_group(const unsigned char * QL, const unsigned
 __global__ void __launch_bounds__(LM_THREADS, 1) k_gemv_q6_K_stream(const unsigned char * __restrict__ ql, const unsigned char * __restrict__ qh,
                                                                     const int8_t * __restrict__ sc, const __half * __restrict__ d,
                                                                     const lkb_q8blk * __restrict__ xq, int out_rows, float * __restrict__ y,
-                                                                    const float * __restrict__ ssq, float eps, int slot, int stat16) {
+                                                                    const float * __restrict__ ssq, float eps, int slot, int stat16, int ahead) {
     extern __shared__ __align__(128) unsigned char lm_raw[];
     LmSmem & S = *reinterpret_cast<LmSmem *>(lm_raw);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -116,7 +116,8 @@ __global__ void __launch_bounds__(LM_THREADS, 1) k_gemv_q6_K_stream(const unsign
     }
     __syncthreads();
 
-    if (warp == LM_WARPS) {                                  // producer: weights do not depend on the previous kernel
+    if (!ahead) lkb_pdl_wait();
+    if (warp == LM_WARPS) {                                  // producer; ahead (lkb_set_pdl): weights do not depend on the previous kernel
         if (lane == 0) {
             unsigned * ctr = g_lm_ticket[slot];
             // Four tickets in flight: one atomic round trip (~1 us) is longer than a chunk's share of the stream.
@@ -216,6 +217,7 @@ __global__ void __launch_bounds__(256) k_gemv_q6_K_simple(const unsigned char * 
                                                           const int8_t * __restrict__ sc, const __half * __restrict__ d,
                                                           const lkb_q8blk * __restrict__ xq, int out_rows, int sbpr, float * __restrict__ y,
                                                           const float * __restrict__ ssq, float eps) {
+    lkb_pdl_wait(); lkb_pdl_trigger();
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (row >= out_rows) return;
     const LmLane m = lm_lane(lane);
@@ -337,11 +339,11 @@ int lkb_gemv_q6_K(const void * ql, const void * qh, const void * sc, const void 
         int grid = lkb_context().sm_count;
         if (grid > (out_rows + LM_ROWS - 1) / LM_ROWS) grid = (out_rows + LM_ROWS - 1) / LM_ROWS;
         static std::atomic<unsigned> seq{0};               // consecutive launches take different ticket counters
-        return lkb_launch(k_gemv_q6_K_stream, dim3(grid), dim3(LM_THREADS), sizeof(LmSmem), (cudaStream_t) st,
+        return lkb_launch_next(k_gemv_q6_K_stream, dim3(grid), dim3(LM_THREADS), sizeof(LmSmem), (cudaStream_t) st,
                           (const unsigned char *) ql, (const unsigned char *) qh, (const int8_t *) sc, (const __half *) d,
-                          (const lkb_q8blk *) xq, out_rows, y, ssq, eps, (int) (seq.fetch_add(1u) % LM_SLOTS), g_lm_static);
+                          (const lkb_q8blk *) xq, out_rows, y, ssq, eps, (int) (seq.fetch_add(1u) % LM_SLOTS), g_lm_static, lkb_context().pdl);
     }
-    return lkb_launch(k_gemv_q6_K_simple, dim3((out_rows + 7) / 8), dim3(256), 0, (cudaStream_t) st,
+    return lkb_launch_next(k_gemv_q6_K_simple, dim3((out_rows + 7) / 8), dim3(256), 0, (cudaStream_t) st,
                       (const unsigned char *) ql, (const unsigned char *) qh, (const int8_t *) sc, (const __half *) d,
                       (const lkb_q8blk *) xq, out_rows, sbpr, y, ssq, eps);
 }
@@ -350,14 +352,14 @@ int lkb_argmax_part(const float * v, int n, float * pv, int * pi, lkb_stream_t s
     if (!lkb_context().inited) return LKB_ERR_NOT_INIT;
     if (!v || !pv || !pi) return LKB_ERR_NULL;
     if (n <= 0) return LKB_ERR_SHAPE;
-    return lkb_launch(k_argmax_part, dim3((n + 1023) / 1024), dim3(256), 0, (cudaStream_t) st, v, n, pv, pi);
+    return lkb_launch_next(k_argmax_part, dim3((n + 1023) / 1024), dim3(256), 0, (cudaStream_t) st, v, n, pv, pi);
 }
 
 int lkb_argmax_final(const float * pv, const int * pi, int n, int * d_token, int * d_pos, lkb_stream_t st) {
     if (!lkb_context().inited) return LKB_ERR_NOT_INIT;
     if (!pv || !pi || !d_token) return LKB_ERR_NULL;
     if (n <= 0) return LKB_ERR_SHAPE;
-    return lkb_launch(k_argmax_final, dim3(1), dim3(256), 0, (cudaStream_t) st, pv, pi, n, d_token, d_pos);
+    return lkb_launch_next(k_argmax_final, dim3(1), dim3(256), 0, (cudaStream_t) st, pv, pi, n, d_token, d_pos);
 }
 
 int lkb_embed_q6_K(const void * ql, const void * qh, const void * sc, const void * d, const int * d_token, int n,

@@ -313,7 +313,7 @@ extern "C" int lkb_pf_attn(const void * qh, int m, int P, const void * kc, const
     if (r != LKB_OK) return r;
     const int two = (m + 2 * FA_POS - 1) / (2 * FA_POS);
     if (two * AT_KVH >= lkb_context().sm_count)
-        return lkb_launch(k_pf_attn_tc<2>, dim3(two, AT_KVH), dim3(FaCfg<2>::THREADS), sizeof(FaSmem<2>) + 1024, (cudaStream_t) st, mq, mk, mv, m, P, o);
-    return lkb_launch(k_pf_attn_tc<1>, dim3((m + FA_POS - 1) / FA_POS, AT_KVH), dim3(FaCfg<1>::THREADS), sizeof(FaSmem<1>) + 1024, (cudaStream_t) st,
+        return lkb_launch_next(k_pf_attn_tc<2>, dim3(two, AT_KVH), dim3(FaCfg<2>::THREADS), sizeof(FaSmem<2>) + 1024, (cudaStream_t) st, mq, mk, mv, m, P, o);
+    return lkb_launch_next(k_pf_attn_tc<1>, dim3((m + FA_POS - 1) / FA_POS, AT_KVH), dim3(FaCfg<1>::THREADS), sizeof(FaSmem<1>) + 1024, (cudaStream_t) st,
                       mq, mk, mv, m, P, o);
 }
