@@ -28,9 +28,10 @@
 //     with the integer add of F's bit pattern.
 //   * The A operand (weights) lives in TMEM: four expansion warps turn staged nibbles into int8 with tcgen05.st, so the
 //     expanded weights never touch shared memory, whose bandwidth the 16-byte fold loads need.
-//   * A producer warp issues bulk tensor copies only: nibble rows (64 B per row and stage), activation rows (dense: 16-row
-//     boxes; grouped: row gathers through perm, four rows per copy).  Block scales travel by 16-byte cp.async, six stages
-//     ahead, because 8 bytes per row and stage are below the copy engine's minimum.
+//   * A producer warp issues bulk tensor copies: nibble rows (64 B per row and stage), activation rows (dense: 16-row boxes;
+//     grouped: row gathers through perm, four rows per copy) and weight scales (16 B per row and two stages: as 16-byte
+//     cp.async they cost the expansion warps 32 lines an instruction, gate|up 67 -> 63 us at 37 tokens of 64 experts, 108 ->
+//     104 at 509, 573 -> 556 at 4096).  Only the activation scales travel by cp.async, six stages ahead.
 //   * Persistent: one CTA per SM walks the items, expert by expert, so an expert's weights stay in L2.
 // Measured per layer, token lanes with padding -> this form: gate|up 727 -> 676 us at 4096 tokens (Zipf routing), 315 -> 162 at
 // 509, 259 -> 84 at 37; down 379 -> 324, 170 -> 88, 134 -> 50; in_proj 299 -> 287 at 4096, 64 -> 60 at 509.
@@ -56,7 +57,7 @@
 #define TC_MMA_WARP  12             // MMA issuers 12, 13
 #define TC_PROD_WARP 14             // warp 15 only completes the warpgroup that setmaxnreg needs
 #define TC_THREADS   512
-#define TC_SC_AHEAD  6              // stages the block scales are requested ahead
+#define TC_SC_AHEAD  6              // stages the activation scales are requested ahead
 #define TC_SC_RING   8              // stages of activation scales in shared memory (read by the thread that requests them)
 #define TC_WS_RING   16             // stages of weight scales: the epilogue reads them up to TC_NS stages behind the expansion
 #define TC_MAGIC_I   0x4B400000
@@ -72,13 +73,13 @@ struct TcStage {
 };
 static_assert(sizeof(TcStage) % 1024 == 0, "stages keep the 1024-byte alignment of the swizzled operands");
 static_assert(TC_SC_RING > TC_NS, "constants stay until the epilogue has read them: see the expansion warps");
-static_assert(TC_WS_RING >= TC_SC_AHEAD + TC_NS + 2 && !(TC_WS_RING & (TC_WS_RING - 1)), "weight scales stay until the epilogue has read them");
+static_assert(TC_WS_RING >= 2 * TC_NS + 2 && !(TC_WS_RING & (TC_WS_RING - 1)), "weight scales stay until the epilogue has read them");
 
 struct TcSmem {
     TcStage st[TC_NS];
     alignas(1024) unsigned seed_b[TC_TOK * 8];                              // constant B operand: 64 rows of 32 bytes
     alignas(16) float4 dk[TC_SC_RING][TC_KB][TC_TOK / 2];                   // per stage, block and token pair {d8, d8', k, k'}
-    alignas(16) uint4  wsc[TC_WS_RING / 2][2 * TC_ROWS];                    // eight fp16 scales per row (two stages)
+    alignas(128) uint4 wsc[TC_WS_RING / 2][2 * TC_ROWS];                    // eight fp16 scales per row (two stages)
     alignas(16) float4 asc[TC_SC_RING][TC_EXP_WARPS * 32];                  // (d8, 8sum) of two blocks per expansion thread
     alignas(8) unsigned long long full[TC_NS], empty[TC_NS], afull[TC_AUNITS], aempty[TC_AUNITS], tfull[2][TC_DBUF], tempty[2][TC_DBUF];
     unsigned tmem_base;
@@ -406,6 +407,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_pf_gemm_tc(const lkb_pf_gemm 
                                                               const __grid_constant__ CUtensorMap map_w0,
                                                               const __grid_constant__ CUtensorMap map_w1,
                                                               const __grid_constant__ CUtensorMap map_w2,
+                                                              const __grid_constant__ CUtensorMap map_d0,
+                                                              const __grid_constant__ CUtensorMap map_d1,
+                                                              const __grid_constant__ CUtensorMap map_d2,
                                                               float * const * __restrict__ out_rows) {
     lkb_pdl_wait(); lkb_pdl_trigger();           // programmatic dependent launch: inputs complete from here on
     extern __shared__ unsigned char tc_smem_raw[];
@@ -463,6 +467,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_pf_gemm_tc(const lkb_pf_gemm 
         asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
         // ============================ producer (one warp) ============================
         if (warp == TC_PROD_WARP) {
+            constexpr int BR = EPI ? 64 : TC_ROWS, NB = 2 * TC_ROWS / BR;       // rows of a box; boxes of an item
             unsigned it = 0;
             bool ok = true;
             TcItem I = tc_item(g, P, blockIdx.x);
@@ -480,37 +485,47 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_pf_gemm_tc(const lkb_pf_gemm 
                     }
                 }
                 const bool glive = g.perm && 4 * lane < I.tcnt;
-                // weight rows: up to four 64-row boxes
-                const CUtensorMap * mw[2];
+                // weight rows: boxes of 64 rows (SwiGLU form, where half a tile may be missing) or of a whole tile
+                const CUtensorMap * mw[2], * md[2];
                 int wrow[2];
                 unsigned boxes = 0;
                 if (EPI) {
-                    mw[0] = &map_w0; mw[1] = &map_w1;
+                    mw[0] = &map_w0; mw[1] = &map_w1; md[0] = &map_d0; md[1] = &map_d1;
                     wrow[0] = wrow[1] = I.expert * rpe + I.rt * TC_ROWS;
                     boxes = (g.N - I.rt * TC_ROWS >= TC_ROWS) ? 15u : 5u;              // N % 64 == 0: half a tile may be missing
                 } else {
 #pragma unroll
                     for (int r = 0; r < 2; ++r) {
                         const int row = tc_tile_row(P, I.rt, r);
-                        if (r && !tc_two<EPI>(g, P, I.rt)) { mw[r] = &map_w0; wrow[r] = 0; continue; }
+                        if (r && !tc_two<EPI>(g, P, I.rt)) { mw[r] = &map_w0; md[r] = &map_d0; wrow[r] = 0; continue; }
                         const int seg = tc_seg(g, row);
                         mw[r] = seg == 0 ? &map_w0 : seg == 1 ? &map_w1 : &map_w2;
+                        md[r] = seg == 0 ? &map_d0 : seg == 1 ? &map_d1 : &map_d2;
                         wrow[r] = I.expert * rpe + row - (seg ? g.seg_end[seg - 1] : 0);
-                        boxes |= 3u << (2 * r);
+                        boxes |= 1u << r;
                     }
                 }
                 const int abox = tc_cols(I.tcnt) / 16, tstart = I.tstart;
-                const unsigned bytes = (unsigned) __popc(boxes) * 4096u + (g.perm ? 512u * (unsigned) ((I.tcnt + 3) >> 2) : 2048u * (unsigned) abox);
+                const unsigned bytes = (unsigned) __popc(boxes) * (BR * 64u) + (g.perm ? 512u * (unsigned) ((I.tcnt + 3) >> 2) : 2048u * (unsigned) abox);
                 if (item + (int) gridDim.x < P.n_items) I = tc_item(g, P, item + gridDim.x);
                 for (int ks = 0; ks < P.nstage; ++ks, ++it) {
                     const unsigned stg = it % TC_NS;
                     if (!tc_wait<TC_HINT_PROD>(S, &S.empty[stg], ((it / TC_NS) & 1u) ^ 1u, 10u)) { ok = false; break; }
                     TcStage & T = S.st[stg];
                     if (lane == 0) {
-                        tc_mbar_arrive_tx(&S.full[stg], bytes);
+                        tc_mbar_arrive_tx(&S.full[stg], bytes + (ks & 1 ? 0u : (unsigned) __popc(boxes) * (BR * 16u)));
 #pragma unroll
-                        for (int b = 0; b < 4; ++b)
-                            if ((boxes >> b) & 1u) tc_tma_tile(T.rawq + b * 4096, mw[b >> 1], ks * (TC_KB * 16), wrow[b >> 1] + 64 * (b & 1), &S.full[stg]);
+                        for (int b = 0; b < NB; ++b) {
+                            const int r = b / (NB / 2);
+                            if ((boxes >> b) & 1u) tc_tma_tile(T.rawq + b * (BR * 64), mw[r], ks * (TC_KB * 16), wrow[r] + BR * b - TC_ROWS * r, &S.full[stg]);
+                        }
+                        if (!(ks & 1)) {                                               // the scales of two stages: 16 bytes a row
+#pragma unroll
+                            for (int b = 0; b < NB; ++b) {
+                                const int r = b / (NB / 2);
+                                if ((boxes >> b) & 1u) tc_tma_tile(&S.wsc[(it >> 1) % (TC_WS_RING / 2)][BR * b], md[r], ks * (TC_KB * 2), wrow[r] + BR * b - TC_ROWS * r, &S.full[stg]);
+                            }
+                        }
                         if (!g.perm)
                             for (int b = 0; b < abox; ++b) tc_tma_tile(T.act + b * 2048, &map_a, ks * 128, tstart + 16 * b, &S.full[stg]);
                     }
@@ -575,7 +590,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_pf_gemm_tc(const lkb_pf_gemm 
     // they issue, and a block's tfull completes after its MMA.  Nor does the epilogue hand them back: a stage comes round
     // (empty) when the issuers have passed it, and a buffer they reused was released behind every read of the stage before,
     // so rings of more than TC_NS + 1 stages are never overwritten early.  (Two barriers of their own per stage cost 5 %.)
-    // Thread e serves weight rows e and 128 + e of the item and two blocks of token e / 2: it brings their block scales into
+    // Thread e serves weight rows e and 128 + e of the item and two blocks of token e / 2: it brings the token's block scales into
     // shared memory (its own cp.async, TC_SC_AHEAD stages ahead), forms the fold's constants, and turns its rows' nibbles
     // into int8 in TMEM (byte i of a block's 16: element i in the low nibble, element i + 16 in the high one).
     else if (warp >= TC_EXP_W0) {
@@ -584,20 +599,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_pf_gemm_tc(const lkb_pf_gemm 
         // ---- the scale requests run ahead of the consumption ----
         int p_item = blockIdx.x, p_ks = 0, n_slot = 0;
         unsigned p_it = 0;
-        const char * p_sc = nullptr, * p_w0 = nullptr, * p_w1 = nullptr;
+        const char * p_sc = nullptr;
         TcItem N = tc_item(g, P, p_item);
         if (g.perm && tok < N.tcnt) n_slot = __ldg(g.perm + N.tstart + tok);
-        auto w_scales = [&](int row, int rt, int expert, int r) -> const char * {       // fp16 scales of one weight row, or null
-            if (EPI) {
-                if (rt * TC_ROWS + e >= g.N) return nullptr;
-                return (const char *) ((const __half *) g.d[r] + (size_t) expert * g.exp_stride + (size_t) (rt * TC_ROWS + e) * g.bpr);
-            }
-            const int seg = tc_seg(g, row);
-            return (const char *) ((const __half *) g.d[seg] + (size_t) expert * g.exp_stride + (size_t) (row - (seg ? g.seg_end[seg - 1] : 0) + e) * g.bpr);
-        };
         auto p_switch = [&]() {                          // N, n_slot describe item p_item: point at its scales, look one item further
-            p_w0 = w_scales(EPI ? 0 : tc_tile_row(P, N.rt, 0), N.rt, N.expert, 0);
-            p_w1 = tc_two<EPI>(g, P, N.rt) ? w_scales(EPI ? 0 : tc_tile_row(P, N.rt, 1), N.rt, N.expert, 1) : nullptr;
             const int arow = g.perm ? n_slot >> g.a_shift : N.tstart + tok;
             p_sc = tok < N.tcnt ? sc_plane + (size_t) arow * s_pitch + (e & 1) * 16 : nullptr;
             if (p_item + (int) gridDim.x < P.n_items) N = tc_item(g, P, p_item + gridDim.x);
@@ -606,17 +611,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_pf_gemm_tc(const lkb_pf_gemm 
         auto fetch = [&]() {
             if (p_item < P.n_items) {
                 if (p_sc) tc_cp16(&S.asc[p_it % TC_SC_RING][e], p_sc + p_ks * (TC_KB * 8));
-                if (!(p_ks & 1)) {
-                    char * const s0 = (char *) &S.wsc[(p_it >> 1) % (TC_WS_RING / 2)][e];
-                    const int o = p_ks * (TC_KB * 2);
-                    if (((size_t) p_w0 | (size_t) p_w1) & 8) {                          // planes that are only 8-byte aligned
-                        if (p_w0) { tc_cp8(s0, p_w0 + o); tc_cp8(s0 + 8, p_w0 + o + 8); }
-                        if (p_w1) { tc_cp8(s0 + TC_ROWS * 16, p_w1 + o); tc_cp8(s0 + TC_ROWS * 16 + 8, p_w1 + o + 8); }
-                    } else {
-                        if (p_w0) tc_cp16(s0, p_w0 + o);
-                        if (p_w1) tc_cp16(s0 + TC_ROWS * 16, p_w1 + o);
-                    }
-                }
                 if (p_ks == 1 && g.perm && tok < N.tcnt) n_slot = __ldg(g.perm + N.tstart + tok);
                 ++p_it;
                 if (++p_ks == P.nstage) { p_ks = 0; p_item += gridDim.x; if (p_item < P.n_items) p_switch(); }
@@ -760,8 +754,8 @@ int lkb_gemm_tc_launch(const lkb_pf_gemm * g, int epi, int fold, int max_tiles, 
     if (((size_t) g->aqs & 15) || (!a_pitch && ((size_t) g->asc & 15))) return LKB_ERR_UNSUPPORTED;
     if (g->exp_stride % g->bpr) return LKB_ERR_UNSUPPORTED;
     const int nseg = epi ? 2 : (g->seg_end[0] >= g->N ? 1 : g->seg_end[1] >= g->N ? 2 : 3);
-    const unsigned qrow = (unsigned) g->bpr * 32u;
-    CUtensorMap ma, mw[3];
+    const unsigned qrow = (unsigned) g->bpr * 32u, box_rows = epi ? 64u : TC_ROWS;
+    CUtensorMap ma, mw[3], md[3];
     // dense: 16-token boxes of consecutive rows; grouped: rows gathered through perm, four per copy.  Packed rows
     // (a_pitch, as the expert-parallel dispatch delivers them): quants first, then the (d8, 8sum) pairs.
     int r = g->perm ? tc_make_map(&ma, g->aqs, qrow, a_pitch ? (unsigned) a_pitch : qrow, TC_ANY_ROWS, 128u, 1u, CU_TENSOR_MAP_SWIZZLE_128B)
@@ -771,17 +765,19 @@ int lkb_gemm_tc_launch(const lkb_pf_gemm * g, int epi, int fold, int max_tiles, 
     const int s_pitch = a_pitch ? a_pitch : g->bpr * 8;
     for (int s = 0; s < 3; ++s) {
         const int src = s < nseg ? s : 0;
-        if (((size_t) g->qs[src] & 15) || ((size_t) g->d[src] & 7)) return LKB_ERR_UNSUPPORTED;
-        r = tc_make_map(&mw[s], g->qs[src], (unsigned) g->bpr * 16u, (unsigned) g->bpr * 16u, TC_ANY_ROWS, 64u, 64u, CU_TENSOR_MAP_SWIZZLE_64B);
+        if (((size_t) g->qs[src] & 15) || ((size_t) g->d[src] & 15)) return LKB_ERR_UNSUPPORTED;
+        r = tc_make_map(&mw[s], g->qs[src], (unsigned) g->bpr * 16u, (unsigned) g->bpr * 16u, TC_ANY_ROWS, 64u, box_rows, CU_TENSOR_MAP_SWIZZLE_64B);
+        if (r != LKB_OK) return r;
+        r = tc_make_map(&md[s], g->d[src], (unsigned) g->bpr * 2u, (unsigned) g->bpr * 2u, TC_ANY_ROWS, 16u, box_rows, CU_TENSOR_MAP_SWIZZLE_NONE);
         if (r != LKB_OK) return r;
     }
     const int rpe = (int) (g->exp_stride / g->bpr);
     const dim3 grid(lkb_context().sm_count), block(TC_THREADS);
     const size_t sm = sizeof(TcSmem) + 1024;
-    if (epi && fold)       LKB_PF_LAUNCH((k_pf_gemm_tc<1, 1>), grid, block, sm, st, *g, max_tiles, rpe, sc_plane, s_pitch, ma, mw[0], mw[1], mw[2], out_rows);
-    else if (epi)          LKB_PF_LAUNCH((k_pf_gemm_tc<1, 0>), grid, block, sm, st, *g, max_tiles, rpe, sc_plane, s_pitch, ma, mw[0], mw[1], mw[2], out_rows);
-    else if (fold)         LKB_PF_LAUNCH((k_pf_gemm_tc<0, 1>), grid, block, sm, st, *g, max_tiles, rpe, sc_plane, s_pitch, ma, mw[0], mw[1], mw[2], out_rows);
-    else                   LKB_PF_LAUNCH((k_pf_gemm_tc<0, 0>), grid, block, sm, st, *g, max_tiles, rpe, sc_plane, s_pitch, ma, mw[0], mw[1], mw[2], out_rows);
+    if (epi && fold)       LKB_PF_LAUNCH((k_pf_gemm_tc<1, 1>), grid, block, sm, st, *g, max_tiles, rpe, sc_plane, s_pitch, ma, mw[0], mw[1], mw[2], md[0], md[1], md[2], out_rows);
+    else if (epi)          LKB_PF_LAUNCH((k_pf_gemm_tc<1, 0>), grid, block, sm, st, *g, max_tiles, rpe, sc_plane, s_pitch, ma, mw[0], mw[1], mw[2], md[0], md[1], md[2], out_rows);
+    else if (fold)         LKB_PF_LAUNCH((k_pf_gemm_tc<0, 1>), grid, block, sm, st, *g, max_tiles, rpe, sc_plane, s_pitch, ma, mw[0], mw[1], mw[2], md[0], md[1], md[2], out_rows);
+    else                   LKB_PF_LAUNCH((k_pf_gemm_tc<0, 0>), grid, block, sm, st, *g, max_tiles, rpe, sc_plane, s_pitch, ma, mw[0], mw[1], mw[2], md[0], md[1], md[2], out_rows);
     return lkb_check_launch();
 }
 
