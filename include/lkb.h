@@ -329,6 +329,8 @@ int lkb_pf_moe_count(const int * idx, int n, int * cnt, lkb_stream_t st);
 int lkb_zero_i32(int * p, int n, lkb_stream_t st);
 int lkb_pf_moe_plan(const int * cnt, int * off, int * tiles, int * ntiles, lkb_stream_t st);
 int lkb_pf_moe_scatter(const int * idx, int n, const int * off, int * perm, lkb_stream_t st);
+/* counts, plan and scatter of n > 0 slots in one call (one launch for a few slots): the same results */
+int lkb_pf_moe_route(const int * idx, int n, int * cnt, int * off, int * tiles, int * ntiles, int * perm, lkb_stream_t st);
 /* ref: src/prefill.cuh:69-71  pf_gemm_dense / pf_gemm_moe / pf_gemm_swiglu */
 int lkb_pf_gemm_dense(const lkb_pf_gemm * g, lkb_stream_t st);
 int lkb_pf_gemm_moe(const lkb_pf_gemm * g, int max_tiles, lkb_stream_t st);
