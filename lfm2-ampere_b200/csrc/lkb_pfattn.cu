@@ -105,6 +105,7 @@ __device__ __forceinline__ bool fa_softmax(FaSmem<NT> & S, int i, unsigned tb, i
             mrow = mn;
             // this half of P has been read; a new maximum also needs the output complete up to the step before
             if (k > 0 && !tc_wait(S, &S.pvdone[i][h], (k - 1) & 1, 61u)) return false;
+            tc_fence_after();                                   // the stores into P below stay behind the MMAs that read it
             if ((k > 0 || h > 0) && __any_sync(LKB_FULL, grown)) {
                 if (!tc_wait(S, &S.pvdone[i][h ^ 1], h ? k & 1 : (k - 1) & 1, 63u)) return false;
                 tc_fence_after();
