@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_pf_gemm_tc(const lkb_pf_gemm 
             tc_mbar_init(&S.empty[i], 2);                       // both issuers' commits
         }
         for (int i = 0; i < TC_AUNITS; ++i) { tc_mbar_init(&S.afull[i], TC_EXP_WARPS); tc_mbar_init(&S.aempty[i], 2); }
-        for (int i = 0; i < 2 * TC_DBUF; ++i) { tc_mbar_init(&S.tfull[0][i], 1); tc_mbar_init(&S.tempty[0][i], TcSums<EPI>::EPI_ARRIVE); }
+        for (int i = 0; i < 2 * TC_DBUF; ++i) { tc_mbar_init(&S.tfull[0][i], 2); tc_mbar_init(&S.tempty[0][i], TcSums<EPI>::EPI_ARRIVE); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -565,6 +565,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_pf_gemm_tc(const lkb_pf_gemm 
                         if (!tc_wait<TC_HINT_MMA>(S, &tempty[h], L::FREE ? i >> 1 : i, 21u)) { ok = false; break; }
                         tc_fence_after();
                         if (leader) {
+                            tc_mbar_arrive(&tfull[h]);                             // releases what full and afull brought: scales, constants
                             const unsigned d = d0 + h * L::BUF, a = a0 + j * 8;
                             const unsigned long long b = b0 + j * 2;               // a block is 32 bytes, in 16-byte units
                             if (FOLD) {
@@ -573,7 +574,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_pf_gemm_tc(const lkb_pf_gemm 
                             }
                             tc_mma_i8(d, a, b, idesc, FOLD);
                             if (two) tc_mma_i8(d + L::TILE, a + 32, b, idesc, FOLD);
-                            tc_commit(&tfull[h]);                                  // this block's sums are ready
+                            tc_commit(&tfull[h]);                                  // this block's sums are ready (the phase's other arrival)
                             if (i + 1 == (L::FREE ? TC_KB : TC_KB / 2)) { tc_commit(&S.aempty[ab]); tc_commit(&S.empty[stg]); }    // the stage has been read
                         }
                         __syncwarp();
@@ -586,10 +587,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_pf_gemm_tc(const lkb_pf_gemm 
         }
     }
     // ============================ expansion (four warps) ==========================
-    // The epilogue waits for block sums only: scales and constants are written before afull, the issuers acquire afull before
-    // they issue, and a block's tfull completes after its MMA.  Nor does the epilogue hand them back: a stage comes round
-    // (empty) when the issuers have passed it, and a buffer they reused was released behind every read of the stage before,
-    // so rings of more than TC_NS + 1 stages are never overwritten early.  (Two barriers of their own per stage cost 5 %.)
+    // The epilogue waits for block sums only.  It reads weight scales (a tensor copy's writes, acquired here with full) and
+    // constants (these warps' own stores) because afull releases them to the issuers, and an issuer's thread arrives on every
+    // tfull itself, beside the commit of its MMAs: what a tcgen05.commit alone makes visible of other threads' writes is not
+    // documented.  (The epilogue waiting for afull as well, once a stage and polled a block ahead, cost 2 to 4 %.)
+    // Nothing is handed back: a stage comes round (empty) when the issuers have passed it, and a buffer they reused was
+    // released behind every read of the stage before, so rings of more than TC_NS + 1 stages are never overwritten early.
     // Thread e serves weight rows e and 128 + e of the item and two blocks of token e / 2: it brings the token's block scales into
     // shared memory (its own cp.async, TC_SC_AHEAD stages ahead), forms the fold's constants, and turns its rows' nibbles
     // into int8 in TMEM (byte i of a block's 16: element i in the low nibble, element i + 16 in the high one).

@@ -1,5 +1,6 @@
 """Hand-overs of the tensor-core kernels, checked on the CPU from their source (a missing wait or fence rarely shows in an output)."""
 import pathlib
+import random
 import re
 
 import pytest
@@ -44,3 +45,122 @@ def test_checker_sees_a_fence_that_may_be_skipped():
 @pytest.mark.parametrize("name", ["lkb_pfattn.cu", "lkb_gemm_tc.cu"])
 def test_every_tmem_access_is_fenced_behind_its_wait(name):
     assert unfenced((CSRC / name).read_text()) == []
+
+
+# ---- the GEMM's rings: the roles of one block as generators over barriers with phases, run in random order ------------------
+GEMM = (CSRC / "lkb_gemm_tc.cu").read_text()
+
+
+def _const(name):
+    return int(re.search(rf"#define {name}\s+(\d+)", GEMM).group(1))
+
+
+NS, AU, SC_RING, WS_RING = _const("TC_NS"), _const("TC_AUNITS"), _const("TC_SC_RING"), _const("TC_WS_RING")
+ISSUERS = GEMM[GEMM.index("// ============================ MMA issuers"):GEMM.index("// ============================ expansion")]
+
+
+class Barrier:
+    """An mbarrier.  What an arriving thread knows (releases) goes to whoever waits for that phase; the arrival of a
+    tcgen05.commit tells that the MMAs are done and nothing about other threads' writes."""
+    def __init__(self, count):
+        self.count, self.left, self.phase, self.gathered, self.known = count, count, 0, {}, {}
+
+    def arrive(self, knows):
+        for k, v in knows.items():
+            self.gathered[k] = max(v, self.gathered.get(k, -1))
+        self.left -= 1
+        assert self.left >= 0, "more arrivals than the phase takes"
+        if self.left == 0:
+            self.left, self.phase, self.known, self.gathered = self.count, self.phase + 1, self.gathered, {}
+
+    def done(self, parity):
+        return (self.phase & 1) != parity
+
+
+def _run_roles(rng, stages, free, tells):
+    full, empty = [Barrier(1) for _ in range(NS)], [Barrier(2) for _ in range(NS)]
+    afull, aempty = [Barrier(1) for _ in range(AU)], [Barrier(2) for _ in range(AU)]
+    tfull = [[Barrier(1 + tells) for _ in range(2)] for _ in range(2)]         # [column half (free form)][buffer]
+    tempty = [[Barrier(1 if free else 2) for _ in range(2)] for _ in range(2)]
+    raw, dk, wsc = {}, {}, {}
+    read = {0: -1, 1: -1, "expansion": -1}                                     # the last stage a reader has finished
+
+    def wait(b, parity, knows):
+        while not b.done(parity):
+            yield
+        for k, v in b.known.items():
+            knows[k] = max(v, knows.get(k, -1))
+
+    def producer():
+        knows = {}
+        for it in range(stages):
+            yield from wait(empty[it % NS], ((it // NS) & 1) ^ 1, knows)
+            assert read["expansion"] >= it - NS, "nibbles overwritten before they were read"
+            raw[it % NS] = it
+            if it % 2 == 0:
+                assert min(read[0], read[1]) >= it - WS_RING + 1, "weight scales overwritten before they were read"
+                wsc[it // 2 % (WS_RING // 2)] = it
+            full[it % NS].arrive({"raw": it, "wsc": it})
+
+    def expansion():
+        knows = {}
+        for it in range(stages):
+            yield from wait(full[it % NS], (it // NS) & 1, knows)
+            assert raw[it % NS] == it and knows["raw"] >= it
+            assert min(read[0], read[1]) >= it - SC_RING, "constants overwritten before they were read"
+            dk[it % SC_RING] = it
+            yield
+            yield from wait(aempty[it % AU], ((it // AU) & 1) ^ 1, knows)
+            read["expansion"] = it
+            afull[it % AU].arrive({**knows, "dk": it})
+
+    def issuer(q):
+        knows = {}
+        for it in range(stages):
+            yield from wait(full[it % NS], (it // NS) & 1, knows)
+            yield from wait(afull[it % AU], (it // AU) & 1, knows)
+            for i in range(4 if free else 2):
+                h = i & 1 if free else q
+                yield from wait(tempty[q if free else 0][h], i >> 1 if free else i, knows)
+                if tells:
+                    tfull[q if free else 0][h].arrive(knows)                   # the thread itself
+                    yield
+                tfull[q if free else 0][h].arrive({})                          # a commit
+                yield
+            aempty[it % AU].arrive({})
+            empty[it % NS].arrive({})
+
+    def epilogue(half):
+        knows, own = {}, half if free else 0
+        for b in tempty[own]:
+            b.arrive({})
+        for it in range(stages):
+            for j in range(4):
+                yield from wait(tfull[own][j & 1], j >> 1, knows)
+                if j == 0:
+                    assert wsc[it // 2 % (WS_RING // 2)] == it // 2 * 2 and knows.get("wsc", -1) >= it // 2 * 2, "weight scales not acquired"
+                assert dk[it % SC_RING] == it and knows.get("dk", -1) >= it, "constants not acquired"
+                yield
+                if j == 3:
+                    read[half] = it
+                tempty[own][j & 1].arrive(knows)
+    roles = [producer(), expansion(), issuer(0), issuer(1), epilogue(0), epilogue(1)]
+    weight = [rng.random() ** 3 + 0.01 for _ in roles]                         # every run has slow and fast roles
+    idle, before = 0, None
+    while roles:
+        i = rng.choices(range(len(roles)), weight)[0]
+        try:
+            next(roles[i])
+        except StopIteration:
+            del roles[i], weight[i]
+        now = [b.phase for b in full + afull + tfull[0] + tfull[1]]
+        idle, before = (0 if now != before else idle + 1), now
+        assert idle < 20000, "the roles wait for one another"
+
+
+@pytest.mark.parametrize("free", [False, True], ids=["plain", "swiglu"])
+def test_epilogue_acquires_what_it_reads(free):
+    """Weight scales (written by a tensor copy) and constants (by the expansion warps) reach the epilogue by releases and
+    acquires of threads, a commit not counted, and no ring is overwritten early."""
+    for seed in range(40):
+        _run_roles(random.Random(seed), stages=60, free=free, tells="tc_mbar_arrive(&tfull[" in ISSUERS)
