@@ -433,6 +433,7 @@ int lkb_shortconv(const float * bcx, int t, const float * conv_w, float * hist, 
  * lkb_pf_qknr: Y = q|k|v output [m][3072]; per-head RMSNorm + NEOX RoPE (base theta; the reference compiles in
  *   1e7); Q leaves as fp16 [m][2048] pre-scaled by 1/8, K and V are appended to the cache.  ref: src/prefill.cu:975-1016
  * lkb_pf_attn: causal GQA attention of the chunk's queries qh over cache positions 0 .. P+m-1, o = fp32 [m][2048].
+ *   Alignment: kc and vc 16 bytes, qh and o 4 bytes (16: Q travels by tensor copies, o in 16-byte stores; same bits).
  *   Definition: float64 softmax over the fp16 inputs; P is rounded to fp16 before the P V product, as in the
  *   reference (gate 4e-3 absolute, ref: tests/test_prefill.cu:244-289).              ref: src/prefill.cu:1029-1268 */
 int lkb_pf_embed(const void * ql, const void * qh, const void * sc, const void * d, const int * toks, float * x, int n, int m,

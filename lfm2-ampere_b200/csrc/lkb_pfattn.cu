@@ -59,6 +59,19 @@ __device__ __forceinline__ unsigned fa_pack(float lo, float hi) {
     return *reinterpret_cast<const unsigned *>(&h);
 }
 
+// One row of Q (this softmax thread's) into the swizzled tile, for a base that no tensor copy takes: 16-byte chunk c of row r
+// at c ^ (r & 7).  Rows past the chunk are zero.
+__device__ __forceinline__ void fa_load_q(unsigned char * tile, const __half * q, int row, bool live) {
+    const unsigned * p = reinterpret_cast<const unsigned *>(q);
+#pragma unroll
+    for (int c = 0; c < AT_D / 8; ++c) {
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (live) v = make_uint4(p[4 * c], p[4 * c + 1], p[4 * c + 2], p[4 * c + 3]);
+        *reinterpret_cast<uint4 *>(tile + row * (AT_D * 2) + ((c ^ (row & 7)) << 4)) = v;
+    }
+    tc_fence_async();                                           // the MMAs read it through the asynchronous proxy
+}
+
 // Softmax of one row (one thread) over all key tiles.  Returns false when a wait gave up.
 template <int NT>
 __device__ __forceinline__ bool fa_softmax(FaSmem<NT> & S, int i, unsigned tb, int lane, int pos, int first_pos, int nkt, float & l_out) {
@@ -150,7 +163,8 @@ template <int NT>
 __global__ void __launch_bounds__(FaCfg<NT>::THREADS, FaCfg<NT>::CTAS) k_pf_attn_tc(const __grid_constant__ CUtensorMap map_q,
                                                                                     const __grid_constant__ CUtensorMap map_k,
                                                                                     const __grid_constant__ CUtensorMap map_v,
-                                                                                    int m, int P, float * __restrict__ o) {
+                                                                                    int m, int P, const __half * __restrict__ q_rows,
+                                                                                    float * __restrict__ o) {
     lkb_pdl_wait(); lkb_pdl_trigger();           // programmatic dependent launch: inputs complete from here on
     typedef FaCfg<NT> C;
     extern __shared__ unsigned char fa_raw[];
@@ -162,7 +176,7 @@ __global__ void __launch_bounds__(FaCfg<NT>::THREADS, FaCfg<NT>::CTAS) k_pf_attn
     const int nkt = (kend + FA_KEYS - 1) / FA_KEYS;
     if (ptid == 0) {
         S.abort = 0;
-        tc_mbar_init(&S.qfull, 1);
+        tc_mbar_init(&S.qfull, q_rows ? 4 * NT : 1);                                // the softmax warps, or the copy's issuer
         for (int s = 0; s < C::SLOTS; ++s) { tc_mbar_init(&S.full[s], 1); tc_mbar_init(&S.empty[s], 1); }
         for (int i = 0; i < NT; ++i) {
             tc_mbar_init(&S.sfull[i], 1); tc_mbar_init(&S.sfree[i], 4);             // MMA commit; the tile's four softmax warps
@@ -181,7 +195,7 @@ __global__ void __launch_bounds__(FaCfg<NT>::THREADS, FaCfg<NT>::CTAS) k_pf_attn
 
     if (warp == C::TMA_WARP) {
         const bool leader = tc_elect();
-        if (leader) {
+        if (leader && !q_rows) {
             tc_mbar_arrive_tx(&S.qfull, NT * FA_TILE);
             for (int i = 0; i < NT; ++i) tc_tma_tile3(S.q[i], &map_q, 0, kvh * AT_GQA, q0 + FA_POS * i, &S.qfull);
         }
@@ -259,6 +273,11 @@ __global__ void __launch_bounds__(FaCfg<NT>::THREADS, FaCfg<NT>::CTAS) k_pf_attn
         const int i = warp >> 2, row = (warp & 3) * 32 + lane;
         const unsigned tb = tmem + 256 * i + ((unsigned) ((warp & 3) * 32) << 16);
         const int q = q0 + FA_POS * i + (row >> 2), head = kvh * AT_GQA + (row & 3);
+        if (q_rows) {
+            fa_load_q(S.q[i], q_rows + (size_t) (q < m ? q : 0) * LKB_HIDDEN + head * AT_D, row, q < m);
+            __syncwarp();
+            tc_mbar_arrive_if(&S.qfull, lane == 0);
+        }
         float l;
         if (fa_softmax<NT>(S, i, tb, lane, P + q, P + q0 + FA_POS * i, nkt, l) && tc_wait(S, &S.pvdone[i][1], (nkt - 1) & 1, 62u)) {
             tc_fence_after();
@@ -268,11 +287,14 @@ __global__ void __launch_bounds__(FaCfg<NT>::THREADS, FaCfg<NT>::CTAS) k_pf_attn
             tc_ld32(tb + 224, r + 32);
             tc_wait_ld();
             if (q < m) {
-                float4 * p = reinterpret_cast<float4 *>(o + (size_t) q * LKB_HIDDEN + head * AT_D);
+                float * const dst = o + (size_t) q * LKB_HIDDEN + head * AT_D;
 #pragma unroll
-                for (int c = 0; c < AT_D / 4; ++c)
-                    p[c] = make_float4(__fmul_rn(__uint_as_float(r[4 * c]), inv), __fmul_rn(__uint_as_float(r[4 * c + 1]), inv),
-                                       __fmul_rn(__uint_as_float(r[4 * c + 2]), inv), __fmul_rn(__uint_as_float(r[4 * c + 3]), inv));
+                for (int c = 0; c < AT_D; c += 4) {
+                    const float4 v = make_float4(__fmul_rn(__uint_as_float(r[c]), inv), __fmul_rn(__uint_as_float(r[c + 1]), inv),
+                                                 __fmul_rn(__uint_as_float(r[c + 2]), inv), __fmul_rn(__uint_as_float(r[c + 3]), inv));
+                    if (((size_t) o & 15) == 0) *reinterpret_cast<float4 *>(dst + c) = v;
+                    else { dst[c] = v.x; dst[c + 1] = v.y; dst[c + 2] = v.z; dst[c + 3] = v.w; }
+                }
             }
         }
     }
@@ -306,15 +328,18 @@ static int fa_make_map(CUtensorMap * t, const void * base, int heads, int rows, 
 extern "C" int lkb_pf_attn(const void * qh, int m, int P, const void * kc, const void * vc, float * o, lkb_stream_t st) {
     if (!lkb_context().inited || !lkb_tensor_map_encoder()) return LKB_ERR_NOT_INIT;
     if (!qh || !kc || !vc || !o) return LKB_ERR_NULL;
-    if (m <= 0 || P < 0 || (((size_t) qh | (size_t) kc | (size_t) vc | (size_t) o) & 15)) return LKB_ERR_SHAPE;
+    // The cache is read by tensor copies alone (16 bytes); Q by one, or from 4-byte words where its base does not allow it.
+    if (m <= 0 || P < 0 || ((size_t) qh & 3) || (((size_t) kc | (size_t) vc) & 15) || ((size_t) o & 3)) return LKB_ERR_SHAPE;
+    const __half * const q_rows = ((size_t) qh & 15) ? (const __half *) qh : nullptr;
     CUtensorMap mq, mk, mv;
-    int r = fa_make_map(&mq, qh, AT_HEADS, m, AT_GQA, FA_POS);
-    if (r == LKB_OK) r = fa_make_map(&mk, kc, AT_KVH, P + m, 1, FA_KEYS);
+    int r = fa_make_map(&mk, kc, AT_KVH, P + m, 1, FA_KEYS);
     if (r == LKB_OK) r = fa_make_map(&mv, vc, AT_KVH, P + m, 1, FA_KEYS);
+    mq = mk;                                                    // (q_rows: never used)
+    if (r == LKB_OK && !q_rows) r = fa_make_map(&mq, qh, AT_HEADS, m, AT_GQA, FA_POS);
     if (r != LKB_OK) return r;
     const int two = (m + 2 * FA_POS - 1) / (2 * FA_POS);
     if (two * AT_KVH >= lkb_context().sm_count)
-        return lkb_launch_next(k_pf_attn_tc<2>, dim3(two, AT_KVH), dim3(FaCfg<2>::THREADS), sizeof(FaSmem<2>) + 1024, (cudaStream_t) st, mq, mk, mv, m, P, o);
+        return lkb_launch_next(k_pf_attn_tc<2>, dim3(two, AT_KVH), dim3(FaCfg<2>::THREADS), sizeof(FaSmem<2>) + 1024, (cudaStream_t) st, mq, mk, mv, m, P, q_rows, o);
     return lkb_launch_next(k_pf_attn_tc<1>, dim3((m + FA_POS - 1) / FA_POS, AT_KVH), dim3(FaCfg<1>::THREADS), sizeof(FaSmem<1>) + 1024, (cudaStream_t) st,
-                      mq, mk, mv, m, P, o);
+                      mq, mk, mv, m, P, q_rows, o);
 }

@@ -28,3 +28,20 @@ def test_pf_attn_edges(lkb, orc, m, P, grow):
     ref = orc.pf_attn_f64(Q.view(np.uint16), m, P, K.view(np.uint16), V.view(np.uint16))
     assert float(np.max(np.abs(host(o) - ref))) < 2e-3
     assert lkb.lib.lkb_pf_gemm_status() == 0
+
+
+@pytest.mark.parametrize("m,P", [(33, 95), (1217, 130)])
+@pytest.mark.parametrize("q_off,o_off", [(2, 0), (4, 1), (0, 2), (6, 3)])
+def test_pf_attn_alignment(lkb, m, P, q_off, o_off):
+    """Q on any 4-byte boundary (q_off halfs past an aligned one) and the output on any float's: the same bits."""
+    lkb.init(0)
+    g = torch.Generator(device="cuda").manual_seed(m)
+    f16 = lambda n: torch.randn(n, device="cuda", generator=g).half()
+    K, V, Q = f16((P + m) * 512), f16((P + m) * 512), f16(m * 2048)
+    want, qb, ob = nan_f32(m, 2048), torch.empty(m * 2048 + 8, dtype=torch.float16, device="cuda"), nan_f32(m * 2048 + 8)
+    lkb.k_pf_attn(Q, m, P, K, V, want)
+    qb[q_off:q_off + m * 2048] = Q
+    lkb.k_pf_attn(qb[q_off:], m, P, K, V, ob[o_off:])
+    assert torch.equal(ob[o_off:o_off + m * 2048].view(m, 2048), want)
+    assert bool(ob[:o_off].isnan().all()) and bool(ob[o_off + m * 2048:].isnan().all())
+    assert lkb.lib.lkb_pf_gemm_status() == 0
