@@ -74,14 +74,14 @@ typedef struct {
 
 /* ref: src/prefill.cuh:45-66 (PfGemm); tiles entries are int4 {expert, start, count, 0} */
 typedef struct {
-    const void *   qs[3];        /* uint4 per block */
-    const void *   d[3];         /* fp16 per block */
+    const void *   qs[3];        /* uint4 per block: 16-byte aligned */
+    const void *   d[3];         /* fp16 per block: 8-byte aligned for the tensor-core form (16: fastest) */
     int            seg_end[3];   /* cumulative row ends, multiples of 128 */
     int            N;            /* output rows (features): multiple of 128 (64 for the SwiGLU form) */
     int            bpr;          /* 32-element blocks per row, multiple of 8 */
     long long      exp_stride;   /* blocks per expert, 0 if dense */
-    const int8_t * aqs;          /* activations, row pitch bpr*32 */
-    const float *  asc;          /* float2 [rows][bpr] */
+    const int8_t * aqs;          /* activations, row pitch bpr*32: 16-byte aligned */
+    const float *  asc;          /* float2 [rows][bpr]: 16-byte aligned for the tensor-core form */
     int            ntok;         /* dense: token rows */
     const int *    perm;         /* MoE: slot ids grouped by expert, or null */
     const int *    tiles;        /* MoE: int4 {expert, start in perm, count, 0} */
@@ -488,13 +488,14 @@ int lkb_ep_route_experts(const void * recv, int cap, const int * flags, int G, c
 /* No counterpart in the reference.  home_rows (optional, with peers) of lkb_ep_route_experts receives, per received
  * row, the address its result row has in its home rank's return buffer; lkb_pf_gemm_moe_rows is lkb_pf_gemm_moe
  * writing the output row of slot s to out_rows[s] instead of out + s * out_ld (plain stores, peer memory included;
- * add must be 0; tensor-core form only, else LKB_ERR_UNSUPPORTED), so the down projection's rows travel home while
- * the GEMM still computes; lkb_ep_publish_wait then announces phase 2 of the epoch to every rank. */
+ * add must be 0; tensor-core form only, else LKB_ERR_UNSUPPORTED: see the alignments in lkb_pf_gemm), so the down
+ * projection's rows travel home while the GEMM still computes; lkb_ep_publish_wait then announces phase 2 of the epoch
+ * to every rank. */
 int lkb_pf_gemm_moe_rows(const lkb_pf_gemm * g, int max_tiles, float * const * out_rows, lkb_stream_t st);
 /* No counterpart in the reference.  inv_out (optional) of lkb_ep_route_experts receives the received rows' 1/rms as a
  * plane; lkb_pf_gemm_swiglu_packed is lkb_pf_gemm_swiglu reading its activations from PACKED rows of row_pitch bytes
  * (bpr*32 quants, then bpr (d8, 8sum) pairs; g->aqs = the first row, g->asc unused) -- the dispatch rows as they
- * arrived, so no unpack pass is needed; tensor-core form only. */
+ * arrived, so no unpack pass is needed; tensor-core form only (else LKB_ERR_UNSUPPORTED); row_pitch % 16 == 0. */
 int lkb_pf_gemm_swiglu_packed(const lkb_pf_gemm * g, int max_tiles, int row_pitch, lkb_stream_t st);
 /* Publish `phase` of the epoch to every rank, then wait for the same phase of every source (lkb_ep_wait), in one
  * launch.  No counterpart in the reference. */

@@ -73,7 +73,7 @@ struct TcStage {
 };
 static_assert(sizeof(TcStage) % 1024 == 0, "stages keep the 1024-byte alignment of the swizzled operands");
 static_assert(TC_SC_RING > TC_NS, "constants stay until the epilogue has read them: see the expansion warps");
-static_assert(TC_WS_RING >= 2 * TC_NS + 2 && !(TC_WS_RING & (TC_WS_RING - 1)), "weight scales stay until the epilogue has read them");
+static_assert(TC_WS_RING >= 2 * TC_NS + 2 && TC_WS_RING >= TC_SC_AHEAD + TC_NS + 2 && !(TC_WS_RING & (TC_WS_RING - 1)), "weight scales stay until the epilogue has read them");
 
 struct TcSmem {
     TcStage st[TC_NS];
@@ -399,8 +399,10 @@ __device__ __forceinline__ bool tc_epilogue_cols(TcSmem & S, TcEpi & X, const lk
 // EPI 0: out (+)= scale * acc           (item: 256 rows, or 128, of one or two weight segments)
 // EPI 1: SwiGLU + Q8_1                  (item: 128 gate rows and the same 128 up rows)
 // rpe = weight rows per expert (exp_stride / bpr).  sc_plane / s_pitch: the (d8, 8sum) pairs of the activation rows.
+// WCOPY 1: weight scales by tensor copy; 0: by the expansion warps' own 8-byte cp.async, for scale planes that start on an
+// 8-byte boundary, where no tensor copy can (for the rest it is the slower one: see the copies above).
 // ---------------------------------------------------------------------------
-template <int EPI, int FOLD>
+template <int EPI, int FOLD, int WCOPY>
 __global__ void __launch_bounds__(TC_THREADS, 1) k_pf_gemm_tc(const lkb_pf_gemm g, const int max_tiles, const int rpe,
                                                               const char * __restrict__ sc_plane, const int s_pitch,
                                                               const __grid_constant__ CUtensorMap map_a,
@@ -513,13 +515,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_pf_gemm_tc(const lkb_pf_gemm 
                     if (!tc_wait<TC_HINT_PROD>(S, &S.empty[stg], ((it / TC_NS) & 1u) ^ 1u, 10u)) { ok = false; break; }
                     TcStage & T = S.st[stg];
                     if (lane == 0) {
-                        tc_mbar_arrive_tx(&S.full[stg], bytes + (ks & 1 ? 0u : (unsigned) __popc(boxes) * (BR * 16u)));
+                        tc_mbar_arrive_tx(&S.full[stg], bytes + (!WCOPY || (ks & 1) ? 0u : (unsigned) __popc(boxes) * (BR * 16u)));
 #pragma unroll
                         for (int b = 0; b < NB; ++b) {
                             const int r = b / (NB / 2);
                             if ((boxes >> b) & 1u) tc_tma_tile(T.rawq + b * (BR * 64), mw[r], ks * (TC_KB * 16), wrow[r] + BR * b - TC_ROWS * r, &S.full[stg]);
                         }
-                        if (!(ks & 1)) {                                               // the scales of two stages: 16 bytes a row
+                        if (WCOPY && !(ks & 1)) {                                      // the scales of two stages: 16 bytes a row
 #pragma unroll
                             for (int b = 0; b < NB; ++b) {
                                 const int r = b / (NB / 2);
@@ -602,18 +604,38 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_pf_gemm_tc(const lkb_pf_gemm 
         // ---- the scale requests run ahead of the consumption ----
         int p_item = blockIdx.x, p_ks = 0, n_slot = 0;
         unsigned p_it = 0;
-        const char * p_sc = nullptr;
+        const char * p_sc = nullptr, * p_w[2] = {nullptr, nullptr};
         TcItem N = tc_item(g, P, p_item);
         if (g.perm && tok < N.tcnt) n_slot = __ldg(g.perm + N.tstart + tok);
         auto p_switch = [&]() {                          // N, n_slot describe item p_item: point at its scales, look one item further
             const int arow = g.perm ? n_slot >> g.a_shift : N.tstart + tok;
             p_sc = tok < N.tcnt ? sc_plane + (size_t) arow * s_pitch + (e & 1) * 16 : nullptr;
+            if constexpr (!WCOPY) {                      // the scales of this thread's two weight rows
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const int row = EPI ? N.rt * TC_ROWS : tc_tile_row(P, N.rt, r), seg = EPI ? r : tc_seg(g, row);
+                    const bool there = EPI ? row + e < g.N : r == 0 || tc_two<EPI>(g, P, N.rt);
+                    p_w[r] = there ? (const char *) g.d[seg] + ((size_t) N.expert * g.exp_stride
+                                     + (size_t) (row - (EPI || !seg ? 0 : g.seg_end[seg - 1]) + e) * g.bpr) * 2 : nullptr;
+                }
+            }
             if (p_item + (int) gridDim.x < P.n_items) N = tc_item(g, P, p_item + gridDim.x);
         };
         p_switch();
         auto fetch = [&]() {
             if (p_item < P.n_items) {
                 if (p_sc) tc_cp16(&S.asc[p_it % TC_SC_RING][e], p_sc + p_ks * (TC_KB * 8));
+                if constexpr (!WCOPY) {
+                    if (!(p_ks & 1)) {
+#pragma unroll
+                        for (int r = 0; r < 2; ++r)
+                            if (p_w[r]) {
+                                char * const w = (char *) &S.wsc[(p_it >> 1) % (TC_WS_RING / 2)][r * TC_ROWS + e];
+                                tc_cp8(w, p_w[r] + p_ks * (TC_KB * 2));
+                                tc_cp8(w + 8, p_w[r] + p_ks * (TC_KB * 2) + 8);
+                            }
+                    }
+                }
                 if (p_ks == 1 && g.perm && tok < N.tcnt) n_slot = __ldg(g.perm + N.tstart + tok);
                 ++p_it;
                 if (++p_ks == P.nstage) { p_ks = 0; p_item += gridDim.x; if (p_item < P.n_items) p_switch(); }
@@ -711,13 +733,17 @@ tc_encode_fn lkb_tensor_map_encoder() { return g_tc_encode; }
 int lkb_pf_attn_init();                    // lkb_pfattn.cu
 int lkb_pf_attn_take_status();
 
+typedef void (*TcKernel)(lkb_pf_gemm, int, int, const char *, int, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap,
+                         CUtensorMap, float * const *);
+static TcKernel const TC_FORMS[8] = {               // 4 epi + 2 fold + weight scales by tensor copy
+    k_pf_gemm_tc<0, 0, 0>, k_pf_gemm_tc<0, 0, 1>, k_pf_gemm_tc<0, 1, 0>, k_pf_gemm_tc<0, 1, 1>,
+    k_pf_gemm_tc<1, 0, 0>, k_pf_gemm_tc<1, 0, 1>, k_pf_gemm_tc<1, 1, 0>, k_pf_gemm_tc<1, 1, 1>};
+
 int lkb_gemm_tc_init() {
     cudaError_t e = cudaSuccess;
     const int sm = (int) sizeof(TcSmem) + 1024;
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_pf_gemm_tc<0, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_pf_gemm_tc<0, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_pf_gemm_tc<1, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_pf_gemm_tc<1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    for (int f = 0; f < 8; ++f)
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(TC_FORMS[f], cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     if (e != cudaSuccess) return -(int) e;
     // the tensor-map encoder is a driver entry point; it is looked up through the runtime so that the
     // library carries no link-time dependency on the driver
@@ -766,21 +792,22 @@ int lkb_gemm_tc_launch(const lkb_pf_gemm * g, int epi, int fold, int max_tiles, 
     if (r != LKB_OK) return r;
     const char * sc_plane = a_pitch ? (const char *) g->aqs + qrow : (const char *) g->asc;
     const int s_pitch = a_pitch ? a_pitch : g->bpr * 8;
+    int wcopy = 1;
+    for (int s = 0; s < nseg; ++s) if ((size_t) g->d[s] & 15) wcopy = 0;
     for (int s = 0; s < 3; ++s) {
         const int src = s < nseg ? s : 0;
-        if (((size_t) g->qs[src] & 15) || ((size_t) g->d[src] & 15)) return LKB_ERR_UNSUPPORTED;
+        if (((size_t) g->qs[src] & 15) || ((size_t) g->d[src] & 7)) return LKB_ERR_UNSUPPORTED;
         r = tc_make_map(&mw[s], g->qs[src], (unsigned) g->bpr * 16u, (unsigned) g->bpr * 16u, TC_ANY_ROWS, 64u, box_rows, CU_TENSOR_MAP_SWIZZLE_64B);
         if (r != LKB_OK) return r;
-        r = tc_make_map(&md[s], g->d[src], (unsigned) g->bpr * 2u, (unsigned) g->bpr * 2u, TC_ANY_ROWS, 16u, box_rows, CU_TENSOR_MAP_SWIZZLE_NONE);
+        md[s] = mw[s];                                                          // (not by tensor copy: never used)
+        if (wcopy) r = tc_make_map(&md[s], g->d[src], (unsigned) g->bpr * 2u, (unsigned) g->bpr * 2u, TC_ANY_ROWS, 16u, box_rows, CU_TENSOR_MAP_SWIZZLE_NONE);
         if (r != LKB_OK) return r;
     }
     const int rpe = (int) (g->exp_stride / g->bpr);
     const dim3 grid(lkb_context().sm_count), block(TC_THREADS);
     const size_t sm = sizeof(TcSmem) + 1024;
-    if (epi && fold)       LKB_PF_LAUNCH((k_pf_gemm_tc<1, 1>), grid, block, sm, st, *g, max_tiles, rpe, sc_plane, s_pitch, ma, mw[0], mw[1], mw[2], md[0], md[1], md[2], out_rows);
-    else if (epi)          LKB_PF_LAUNCH((k_pf_gemm_tc<1, 0>), grid, block, sm, st, *g, max_tiles, rpe, sc_plane, s_pitch, ma, mw[0], mw[1], mw[2], md[0], md[1], md[2], out_rows);
-    else if (fold)         LKB_PF_LAUNCH((k_pf_gemm_tc<0, 1>), grid, block, sm, st, *g, max_tiles, rpe, sc_plane, s_pitch, ma, mw[0], mw[1], mw[2], md[0], md[1], md[2], out_rows);
-    else                   LKB_PF_LAUNCH((k_pf_gemm_tc<0, 0>), grid, block, sm, st, *g, max_tiles, rpe, sc_plane, s_pitch, ma, mw[0], mw[1], mw[2], md[0], md[1], md[2], out_rows);
+    LKB_PF_LAUNCH(TC_FORMS[(epi ? 4 : 0) + (fold ? 2 : 0) + wcopy], grid, block, sm, st, *g, max_tiles, rpe, sc_plane, s_pitch, ma, mw[0], mw[1], mw[2],
+                  md[0], md[1], md[2], out_rows);
     return lkb_check_launch();
 }
 

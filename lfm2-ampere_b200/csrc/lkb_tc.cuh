@@ -175,5 +175,8 @@ __device__ __forceinline__ void tc_tma_gather4(void * dst, const CUtensorMap * m
 __device__ __forceinline__ void tc_cp16(void * dst, const void * src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(tc_smem_u32(dst)), "l"(src) : "memory");
 }
+__device__ __forceinline__ void tc_cp8(void * dst, const void * src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" :: "r"(tc_smem_u32(dst)), "l"(src) : "memory");
+}
 __device__ __forceinline__ void tc_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void tc_cp_wait() { asm volatile("cp.async.wait_group %0;" :: "n"(N) : "memory"); }

@@ -84,3 +84,59 @@ def test_swiglu(L, orc, I, bpr):
         got.append((oqs, osc))
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
     assert int(got[1][0].float().abs().max()) > 0
+
+
+def _past(a, off):
+    """The array's bytes on the device, `off` bytes past an aligned address."""
+    raw = np.ascontiguousarray(a).view(np.uint8).reshape(-1)
+    buf = torch.zeros(raw.size + off, dtype=torch.uint8, device="cuda")
+    buf[off:] = torch.from_numpy(raw.copy()).cuda()
+    return buf[off:]
+
+
+@pytest.mark.parametrize("off", [0, 8])
+def test_scale_planes_on_8_byte_boundaries(L, orc, off):
+    """Every entry point of the tensor-core form takes weight-scale planes that start on an 8-byte boundary: dense with three
+    segments, grouped with row targets, SwiGLU from planar rows and from packed ones (192 rows: half a tile is missing)."""
+    rng = np.random.default_rng(5 + off)
+    N, bpr, m = 640, 16, 70
+    qs, d = rand_q4(rng, N, bpr, "ref")
+    aq, asc = orc.pf_quant_rows(act_floats(rng, m * bpr * 32).reshape(m, bpr * 32), bpr)
+    cut, ends = [slice(0, 256), slice(256, 384), slice(384, N)], [256, 384, N]
+    out = nan_f32(m, N)
+    L.pf_gemm_dense(L.make_pf_gemm([(dev(qs[c]), _past(d[c], off)) for c in cut], ends, N, bpr, dev(aq), dev(asc), ntok=m, out=out, out_ld=N))
+    assert np.array_equal(host(out), orc.pf_gemm([(qs[c], d[c]) for c in cut], ends, N, bpr, aq, asc, ntok=m))
+
+    idx, perm, tiles = _plan(rng)
+    ns, E, I = idx.size, len(COUNTS), 192
+    dperm, dtiles, dnt = dev(perm), dev(tiles), dev(np.array([len(tiles)], np.int32))
+    aq, asc = orc.pf_quant_rows(act_floats(rng, ns * bpr * 32).reshape(ns, bpr * 32), bpr)
+    daq, dasc = dev(aq), dev(asc)
+    plan = dict(perm=dperm, tiles=dtiles, ntiles=dnt)
+    qs, d = rand_q4(rng, E * 256, bpr, "ref")
+    order = torch.from_numpy(rng.permutation(ns).astype(np.int64)).cuda()      # row s of the result goes to row order[s] of the buffer
+    back = nan_f32(ns, 256)
+    rows = back.data_ptr() + order * 1024
+    g = L.make_pf_gemm([(dev(qs), _past(d, off))], [256] * 3, 256, bpr, daq, dasc, exp_stride=256 * bpr, out=back, out_ld=256, **plan)
+    L.pf_gemm_moe_rows(g, len(tiles), rows)
+    ref = orc.pf_gemm([(qs, d)], [256] * 3, 256, bpr, aq, asc, exp_stride=256 * bpr, perm=perm, tiles=tiles, out_rows=ns)
+    assert np.array_equal(host(back)[host(order)], ref)
+
+    w = [rand_q4(rng, E * I, bpr, "ref") for _ in range(2)]
+    pitch = bpr * 40 + 16
+    packed = torch.full((ns, pitch), 0x5A, dtype=torch.uint8, device="cuda")
+    packed[:, :bpr * 32] = daq.view(torch.uint8)
+    packed[:, bpr * 32:bpr * 40] = dasc.reshape(ns, bpr * 2).view(torch.uint8)
+    got = []
+    for form, planes_off in ((0, 0), (1, off), (2, off)):                       # the CUDA-core form; planar; packed
+        L.pf_gemm_config(min(form, 1))
+        oqs, osc = torch.full((ns, I), 0x5A, dtype=torch.int8, device="cuda"), nan_f32(ns, I // 32, 2)
+        g = L.make_pf_gemm([(dev(q), _past(s, planes_off)) for q, s in w], [I] * 3, I, bpr, packed if form == 2 else daq, dasc,
+                           exp_stride=I * bpr, oqs=oqs, osc=osc, okb=I // 32, **plan)
+        if form == 2:
+            L.pf_gemm_swiglu_packed(g, len(tiles), pitch)
+        else:
+            L.pf_gemm_swiglu(g, len(tiles))
+        got.append((oqs, osc))
+    for a, b in got[1:]:
+        assert torch.equal(got[0][0], a) and torch.equal(got[0][1], b)

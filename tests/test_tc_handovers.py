@@ -55,7 +55,7 @@ def _const(name):
     return int(re.search(rf"#define {name}\s+(\d+)", GEMM).group(1))
 
 
-NS, AU, SC_RING, WS_RING = _const("TC_NS"), _const("TC_AUNITS"), _const("TC_SC_RING"), _const("TC_WS_RING")
+NS, AU, SC_RING, WS_RING, AHEAD = (_const(n) for n in ("TC_NS", "TC_AUNITS", "TC_SC_RING", "TC_WS_RING", "TC_SC_AHEAD"))
 ISSUERS = GEMM[GEMM.index("// ============================ MMA issuers"):GEMM.index("// ============================ expansion")]
 
 
@@ -77,7 +77,7 @@ class Barrier:
         return (self.phase & 1) != parity
 
 
-def _run_roles(rng, stages, free, tells):
+def _run_roles(rng, stages, free, tells, wcopy):
     full, empty = [Barrier(1) for _ in range(NS)], [Barrier(2) for _ in range(NS)]
     afull, aempty = [Barrier(1) for _ in range(AU)], [Barrier(2) for _ in range(AU)]
     tfull = [[Barrier(1 + tells) for _ in range(2)] for _ in range(2)]         # [column half (free form)][buffer]
@@ -97,13 +97,19 @@ def _run_roles(rng, stages, free, tells):
             yield from wait(empty[it % NS], ((it // NS) & 1) ^ 1, knows)
             assert read["expansion"] >= it - NS, "nibbles overwritten before they were read"
             raw[it % NS] = it
-            if it % 2 == 0:
-                assert min(read[0], read[1]) >= it - WS_RING + 1, "weight scales overwritten before they were read"
-                wsc[it // 2 % (WS_RING // 2)] = it
-            full[it % NS].arrive({"raw": it, "wsc": it})
+            if wcopy:
+                put_scales(it)
+            full[it % NS].arrive({"raw": it, "wsc": it} if wcopy else {"raw": it})
+
+    def put_scales(it):                                                        # of two stages
+        if it % 2 == 0 and it < stages:
+            assert min(read[0], read[1]) >= it - WS_RING + 1, "weight scales overwritten before they were read"
+            wsc[it // 2 % (WS_RING // 2)] = it
 
     def expansion():
         knows = {}
+        for it in range(AHEAD if not wcopy else 0):
+            put_scales(it)
         for it in range(stages):
             yield from wait(full[it % NS], (it // NS) & 1, knows)
             assert raw[it % NS] == it and knows["raw"] >= it
@@ -112,7 +118,9 @@ def _run_roles(rng, stages, free, tells):
             yield
             yield from wait(aempty[it % AU], ((it // AU) & 1) ^ 1, knows)
             read["expansion"] = it
-            afull[it % AU].arrive({**knows, "dk": it})
+            afull[it % AU].arrive({**knows, "dk": it} if wcopy else {**knows, "dk": it, "wsc": it})
+            if not wcopy:
+                put_scales(it + AHEAD)
 
     def issuer(q):
         knows = {}
@@ -158,9 +166,10 @@ def _run_roles(rng, stages, free, tells):
         assert idle < 20000, "the roles wait for one another"
 
 
+@pytest.mark.parametrize("wcopy", [True, False], ids=["tensor-copy", "cp-async"])
 @pytest.mark.parametrize("free", [False, True], ids=["plain", "swiglu"])
-def test_epilogue_acquires_what_it_reads(free):
-    """Weight scales (written by a tensor copy) and constants (by the expansion warps) reach the epilogue by releases and
+def test_epilogue_acquires_what_it_reads(free, wcopy):
+    """Weight scales (written by a tensor copy or the expansion warps) and constants (by the expansion warps) reach the epilogue by releases and
     acquires of threads, a commit not counted, and no ring is overwritten early."""
     for seed in range(40):
-        _run_roles(random.Random(seed), stages=60, free=free, tells="tc_mbar_arrive(&tfull[" in ISSUERS)
+        _run_roles(random.Random(seed), stages=60, free=free, tells="tc_mbar_arrive(&tfull[" in ISSUERS, wcopy=wcopy)
