@@ -99,7 +99,7 @@ __device__ __forceinline__ bool fa_softmax(FaSmem<NT> & S, int i, unsigned tb, i
         if (k * FA_KEYS + FA_KEYS - 1 > first_pos) {            // the tile reaches past the first row's position (or the cache's end)
             const int last = pos - k * FA_KEYS;                 // last key of the tile that this row may see
 #pragma unroll
-            for (int c = 0; c < FA_KEYS; ++c) if (c > last) su[c] = __float_as_uint(-1e30f);
+            for (int c = 0; c < FA_KEYS; ++c) if (c > last) su[c] = 0xFF800000u;      // -inf: weight 0 under any maximum
         }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {

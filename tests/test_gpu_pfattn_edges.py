@@ -45,3 +45,24 @@ def test_pf_attn_alignment(lkb, m, P, q_off, o_off):
     assert torch.equal(ob[o_off:o_off + m * 2048].view(m, 2048), want)
     assert bool(ob[:o_off].isnan().all()) and bool(ob[o_off + m * 2048:].isnan().all())
     assert lkb.lib.lkb_pf_gemm_status() == 0
+
+
+def _inputs(m, P, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    f16 = lambda n, w: torch.randn(n, w, 64, device="cuda", generator=g).half()
+    return f16(m, 32), f16(P + m, 8), f16(P + m, 8)
+
+
+@pytest.mark.parametrize("m,row", [(40, 3), (200, 131), (1217, 700)])
+def test_pf_attn_row_of_minus_infinities(lkb, m, row):
+    """A query whose every visible score is -inf has no softmax: NaN, and never an average of the keys it may not see."""
+    lkb.init(0)
+    Q, K, V = _inputs(m, 0, m)
+    want, got = nan_f32(m, 32, 64), nan_f32(m, 32, 64)
+    K[:, 0, 0] = -1.0
+    lkb.k_pf_attn(Q, m, 0, K, V, want)
+    Q[row, 0, 0] = float("inf")                                       # head 0 reads KV head 0
+    lkb.k_pf_attn(Q, m, 0, K, V, got)
+    assert bool(got[row, 0].isnan().all())
+    got[row, 0] = want[row, 0]
+    assert torch.equal(got, want)
