@@ -258,10 +258,14 @@ __global__ void __launch_bounds__(FaCfg<NT>::THREADS, FaCfg<NT>::CTAS) k_pf_attn
                     if (!ok) break;
                     tc_fence_after();
                     if (leader) {
+                        // no further than the tile's last key: a key that no row sees has weight 0, but 0 x inf is NaN, and a
+                        // later token's value must not reach rows ahead of its own tile
+                        const int live = P + min(q0 + FA_POS * (i + 1), m) - k * FA_KEYS - FA_STEP * h;
 #pragma unroll
                         for (int kk = 0; kk < FA_STEP / 16; ++kk)
-                            tc_mma_f16_ts(tmem + 256 * i + 192, tmem + 256 * i + 128 + 32 * h + 8 * kk, b + 128 * (4 * h + kk), FA_IDESC_PV,
-                                          (unsigned) (k > 0 || h > 0 || kk > 0));
+                            if (16 * kk < live)
+                                tc_mma_f16_ts(tmem + 256 * i + 192, tmem + 256 * i + 128 + 32 * h + 8 * kk, b + 128 * (4 * h + kk), FA_IDESC_PV,
+                                              (unsigned) (k > 0 || h > 0 || kk > 0));
                         tc_commit(&S.pvdone[i][h]);
                     }
                     __syncwarp();

@@ -66,3 +66,17 @@ def test_pf_attn_row_of_minus_infinities(lkb, m, row):
     assert bool(got[row, 0].isnan().all())
     got[row, 0] = want[row, 0]
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("m,key", [(200, 100), (1217, 1000)])
+def test_pf_attn_reach_of_an_infinite_value(lkb, m, key):
+    """An infinite V of a later token leaves the rows of earlier 32-position tiles alone (0 x inf would be NaN there)."""
+    lkb.init(0)
+    Q, K, V = _inputs(m, 0, m + 1)
+    want, got = nan_f32(m, 32, 64), nan_f32(m, 32, 64)
+    lkb.k_pf_attn(Q, m, 0, K, V, want)
+    V[key, 5, 7] = float("inf")
+    lkb.k_pf_attn(Q, m, 0, K, V, got)
+    first = key // 32 * 32
+    assert torch.equal(got[:first], want[:first])
+    assert not bool(got[key:, 20:24, 7].isfinite().any())              # heads 20..23 read KV head 5
