@@ -715,6 +715,11 @@ static int gemm_check(const lkb_pf_gemm * g, int epi) {
     if (epi ? (g->N % 64) : (g->N % 128)) return LKB_ERR_SHAPE;
     if (!epi && (g->seg_end[0] % 128 || g->seg_end[1] % 128)) return LKB_ERR_SHAPE;
     if (g->perm && (!g->tiles || !g->ntiles)) return LKB_ERR_NULL;
+    // what either form loads or stores at a time (the tensor-core form asks for more and leaves such planes to the other)
+    size_t by16 = (size_t) g->aqs | (size_t) g->tiles, by8 = (size_t) g->asc | (epi ? (size_t) g->osc : 0), by4 = epi ? 0 : (size_t) g->out, by2 = 0;
+    const int nseg = epi ? 2 : (g->seg_end[0] >= g->N ? 1 : g->seg_end[1] >= g->N ? 2 : 3);
+    for (int s = 0; s < nseg; ++s) { by16 |= (size_t) g->qs[s]; by2 |= (size_t) g->d[s]; }
+    if ((by16 & 15) || (by8 & 7) || (by4 & 3) || (by2 & 1)) return LKB_ERR_SHAPE;
     return LKB_OK;
 }
 

@@ -1,6 +1,8 @@
 """The tensor-core GEMM at the edges of its tiles: token counts around the 16-column steps of an MMA and the 64-token plan
 tile, row counts that leave half a tile or a single tile, the shortest K.  Bit for bit against the CPU checker; the fused
 SwiGLU form against the CUDA-core form of the same entry point (itself checked in test_gpu_prefill.py)."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -140,3 +142,21 @@ def test_scale_planes_on_8_byte_boundaries(L, orc, off):
         got.append((oqs, osc))
     for a, b in got[1:]:
         assert torch.equal(got[0][0], a) and torch.equal(got[0][1], b)
+
+
+@pytest.mark.parametrize("cfg", [-1, 0])
+def test_misaligned_planes_are_refused(L, orc, cfg):
+    """Planes off the boundary that both forms' loads need are an error of the call, not of the device."""
+    L.pf_gemm_config(cfg)
+    rng = np.random.default_rng(3)
+    N, bpr, m = 128, 8, 5
+    qs, d = rand_q4(rng, N, bpr, "ref")
+    aq, asc = orc.pf_quant_rows(act_floats(rng, m * bpr * 32).reshape(m, bpr * 32), bpr)
+    buf = torch.zeros(m * N * 4 + 8, dtype=torch.uint8, device="cuda")
+    offs = {"qs": 8, "d": 1, "aqs": 8, "asc": 4, "out": 2}
+    for wrong in [None, *offs]:
+        o = {k: v if k == wrong else 0 for k, v in offs.items()}
+        keep = [_past(qs, o["qs"]), _past(d, o["d"]), _past(aq, o["aqs"]), _past(asc, o["asc"]), buf[o["out"]:]]
+        g = L.make_pf_gemm([(keep[0], keep[1])], [N] * 3, N, bpr, keep[2], keep[3], ntok=m, out=keep[4], out_ld=N)
+        assert L.lib.lkb_pf_gemm_dense(ctypes.byref(g), None) == (0 if wrong is None else -10001), wrong
+    torch.cuda.synchronize()
