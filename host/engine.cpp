@@ -8,7 +8,7 @@
 //
 // The pack (lfm2-ampere_b200/pack.py) holds every tensor in the planar layout the kernels read; it is copied to the
 // device once.  Prompt tokens 0..n-2 run through the batched-prefill call sequence in chunks of LK_PF_CHUNK
-// (dense Q4_0 x Q8_1 GEMMs around the chunk kernels, the MoE FFN as count / plan / scatter + two grouped GEMMs);
+// (dense Q4_0 x Q8_1 GEMMs around the chunk kernels, the MoE FFN as routing + two grouped GEMMs);
 // the last prompt token and every generated token run through the decode step, captured once in a CUDA graph
 // whose inputs (token id, position) live on the device and are advanced by the argmax kernel, so a replay needs
 // no host argument.  All kernels are reached through the C ABI of include/lkb.h (lkb_shim.hpp's wrappers keep
@@ -248,10 +248,7 @@ void prefill_chunk(Engine & e, lk::stream_t st, const int * toks_host, int m, in
         const lkb_moe_layer & l = e.moe[i];
         lk::k_pf_norm(st, m, e.X, l.norm_w, 0, a, e.inv, e.h32);
         lk::check(lkb_pf_router_select(e.h32, m, m <= 256, l.router, l.rbias, e.inv, e.sel, e.sig, e.idx, e.w, st), "k_pf_router + k_pf_select");
-        lk::check(lkb_zero_i32(e.cnt, E, st), "lkb_zero_i32");
-        lk::k_pf_moe_count(st, e.idx, ns, e.cnt);
-        lk::k_pf_moe_plan(st, e.cnt, e.off, e.tiles, e.ntiles);
-        lk::k_pf_moe_scatter(st, e.idx, ns, e.off, e.perm);
+        lk::k_pf_moe_route(st, e.idx, ns, e.cnt, e.off, e.tiles, e.ntiles, e.perm);
         {
             const lk::QT4 segs[2] = {{l.gate_qs, l.gate_d}, {l.up_qs, l.up_d}};
             const int ends[3] = {I, I, I};

@@ -87,6 +87,8 @@ inline int k_pf_moe_plan(stream_t st, const int * cnt, int * off, int * tiles, i
     return check(lkb_pf_moe_plan(cnt, off, tiles, ntiles, st), "k_pf_moe_plan"); }
 inline int k_pf_moe_scatter(stream_t st, const int * idx, int n, const int * off, int * perm) {
     return check(lkb_pf_moe_scatter(idx, n, off, perm, st), "k_pf_moe_scatter"); }
+inline int k_pf_moe_route(stream_t st, const int * idx, int n, int * cnt, int * off, int * tiles, int * ntiles, int * perm) {      // the three above, counts zeroed
+    return check(lkb_pf_moe_route(idx, n, cnt, off, tiles, ntiles, perm, st), "k_pf_moe_route"); }
 inline int k_pf_moe_combine(stream_t st, int m, float * X, const float * D, const float * w) {
     return check(lkb_pf_moe_combine(X, D, w, m, st), "k_pf_moe_combine"); }
 inline int k_pf_moe_combine_norm(stream_t st, int m, float * X, const float * D, const float * w, const float * nw, PfAct a, float * inv_out) {

@@ -45,6 +45,13 @@ def test_engine_refuses_without_pack_or_tokens(engine, tmp_path):
     assert r.returncode == 1 and "LK_MAX_SEQ" in r.stderr
 
 
+def test_engine_routes_a_chunk_in_one_call(engine):
+    """The host reaches the entry points that the Python call sequence does: routing as one call, not its four steps."""
+    used = subprocess.run(["nm", "-D", "--undefined-only", str(engine)], check=True, capture_output=True, text=True).stdout.split()
+    assert {"lkb_pf_moe_route", "lkb_pf_router_select", "lkb_pf_attn"} <= set(used)
+    assert not {"lkb_zero_i32", "lkb_pf_moe_count", "lkb_pf_moe_plan", "lkb_pf_moe_scatter"} & set(used)
+
+
 def test_pack_table_round_trip(tmp_path):
     import importlib
     pack = importlib.import_module("lfm2-ampere_b200.pack")
