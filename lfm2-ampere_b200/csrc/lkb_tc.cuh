@@ -117,10 +117,8 @@ __device__ __forceinline__ void tc_ld32(unsigned taddr, unsigned * r) {
 }
 template <int NC>
 __device__ __forceinline__ void tc_ld(unsigned taddr, unsigned (&r)[NC]) {
-    if constexpr (NC == 8) tc_ld8(taddr, r);
-    else if constexpr (NC == 16) tc_ld16(taddr, r);
-    else if constexpr (NC == 24) { tc_ld16(taddr, r); tc_ld8(taddr + 16, r + 16); }
-    else tc_ld32(taddr, r);
+    static_assert(NC == 8 || NC == 16, "what the epilogue's halves need");
+    if constexpr (NC == 8) tc_ld8(taddr, r); else tc_ld16(taddr, r);
 }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_st8(unsigned taddr, const uint4 a, const uint4 b) {

@@ -66,6 +66,26 @@ def test_grouped(L, orc, N, bpr):
     assert np.array_equal(host(out), ref)
 
 
+def test_registered_workspace_is_left_alone(L, orc):
+    """A caller that sizes and registers one as the header allows gets the same rows, and its buffer back untouched."""
+    rng = np.random.default_rng(11)
+    idx, perm, tiles = _plan(rng)
+    ns, E, N, bpr = idx.size, len(COUNTS), 128, 8
+    qs, d = rand_q4(rng, E * N, bpr, "ref")
+    aq, asc = orc.pf_quant_rows(act_floats(rng, ns * bpr * 32).reshape(ns, bpr * 32), bpr)
+    args = [dev(v) for v in (qs, d, aq, asc, perm, tiles, np.array([len(tiles)], np.int32))]
+    buf = torch.full((L.pf_gemm_workspace_bytes(len(tiles), bpr * 32),), 0x5A, dtype=torch.uint8, device="cuda")
+    got = []
+    for ws in (None, buf):
+        L.pf_gemm_set_workspace(ws)
+        out = nan_f32(ns, N)
+        L.pf_gemm_moe(L.make_pf_gemm([(args[0], args[1])], [N] * 3, N, bpr, args[2], args[3], exp_stride=N * bpr, perm=args[4],
+                                     tiles=args[5], ntiles=args[6], out=out, out_ld=N), len(tiles))
+        got.append(out)
+    L.pf_gemm_set_workspace(None)
+    assert torch.equal(got[0], got[1]) and bool(got[0].isfinite().all()) and bool((buf == 0x5A).all())
+
+
 @pytest.mark.parametrize("I,bpr", [(64, 8), (192, 16), (256, 64)])
 def test_swiglu(L, orc, I, bpr):
     rng = np.random.default_rng(I)

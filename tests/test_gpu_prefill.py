@@ -33,18 +33,6 @@ def fold(request, L, orc):
     orc.set_gemm_fold(1)
 
 
-@pytest.fixture(params=["gather", "tiles"])
-def ws(request, L):
-    """Both activation paths of the grouped tensor-core GEMM: rows gathered through perm inside the kernel (no
-    workspace), or copied into token-tile order first (caller-owned workspace registered)."""
-    buf = None
-    if request.param == "tiles":
-        buf = torch.full((L.pf_gemm_workspace_bytes(4 * 700 // 64 + 64, 2048),), 0x5A, dtype=torch.uint8, device="cuda")
-    L.pf_gemm_set_workspace(buf)
-    yield request.param
-    L.pf_gemm_set_workspace(None)
-
-
 def _f64_gate(got, full, mag, slack, s, bpr, fold):
     """fp32 result against float64 (see the module docstring)."""
     if fold:
@@ -272,7 +260,7 @@ def test_gemm_dense(L, orc, fold, cfg, N, bpr, M, add, scale, three):
 
 @pytest.mark.parametrize("cfg", [0, 1])
 @pytest.mark.parametrize("E,rows,bpr,M,a_shift", [(8, 256, 64, 130, 2), (8, 384, 48, 257, 0), (64, 128, 8, 700, 2)])
-def test_gemm_moe(L, orc, fold, ws, cfg, E, rows, bpr, M, a_shift):
+def test_gemm_moe(L, orc, fold, cfg, E, rows, bpr, M, a_shift):
     L.pf_gemm_config(cfg)
     rng = np.random.default_rng(E * rows + bpr + M)
     NS = M * 4
@@ -310,7 +298,7 @@ def test_gemm_moe(L, orc, fold, ws, cfg, E, rows, bpr, M, a_shift):
 
 
 @pytest.mark.parametrize("cfg", [0, 1])
-def test_gemm_swiglu_fused_equals_unfused(L, orc, fold, ws, cfg):
+def test_gemm_swiglu_fused_equals_unfused(L, orc, fold, cfg):
     L.pf_gemm_config(cfg)
     rng = np.random.default_rng(31)
     E, I, bpr, M = 8, 256, 64, 150
@@ -445,7 +433,7 @@ def _sub_plan(operm, otiles, rng, per_tile=9):
 def test_gemm_moe_full_size_4096_tokens_zipf(L, orc):
     """The benchmark's configuration at full size: 4096 tokens x top-4 = 16384 slots over 64 experts with Zipf(1.1)-skewed
     routing, real layer shapes (gate|up 2 x 1536 x 2048 with the fused SwiGLU quantiser, down 2048 x 1536), through the
-    tensor-core kernel on its workspace path.  Every slot row is checked on the device against the unfused form; more than
+    tensor-core kernel.  Every slot row is checked on the device against the unfused form; more than
     2048 slots (first / middle / last row of every tile and random ones) bit for bit against the CPU checker."""
     rng = np.random.default_rng(4096)
     m, H, I, E = 4096, 2048, 1536, 64
@@ -464,8 +452,6 @@ def test_gemm_moe_full_size_4096_tokens_zipf(L, orc):
     ocnt, ooff, otiles, operm = orc.moe_plan(idx.reshape(-1))
     assert np.array_equal(host(perm), operm) and np.array_equal(host(cnt), ocnt)
     assert ocnt.max() > 4 * ocnt[ocnt > 0].min()                         # the load really is skewed
-    wsb = torch.zeros(L.pf_gemm_workspace_bytes(max_tiles, H), dtype=torch.uint8, device="cuda")
-    L.pf_gemm_set_workspace(wsb)
     L.pf_gemm_config(1)
     dg = [dev(a) for a in (gq, gd, uq, ud, dq_, dd_)]
     daq, dasc, dinv = dev(aq), dev(asc), dev(inv)
@@ -499,7 +485,6 @@ def test_gemm_moe_full_size_4096_tokens_zipf(L, orc):
     oD = orc.pf_gemm([(dq_, dd_)], [H, H, H], H, 48, host(a2q), host(a2s), exp_stride=H * 48, perm=sperm, tiles=stiles,
                      a_shift=0, out_rows=NS)
     assert np.array_equal(gotD[sperm], oD[sperm])                        # down rows, bit for bit
-    L.pf_gemm_set_workspace(None)
     L.pf_gemm_config(-1)
 
 
