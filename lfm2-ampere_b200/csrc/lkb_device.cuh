@@ -261,8 +261,8 @@ int lkb_mixer_init();          // ... of the decode attention kernel
 
 // Launch helpers.  Programmatic dependent launch lets a kernel's launch latency hide behind its predecessor's tail.
 //   lkb_launch_next  always does so: for kernels whose every thread starts with lkb_pdl_wait(), so that none reads or writes
-//                    memory before everything ahead of it in the stream has completed.  Prefill of 2 tokens 4.54 -> 3.81 ms,
-//                    of 37 8.51 -> 7.98, of 509 13.9 -> 13.6, of 4096 54.1 -> 54.1.
+//                    memory before everything ahead of it in the stream has completed.  Without and with: prefill of 37 tokens
+//                    8.06 and 7.44 ms, of 509 behind 1234 13.45 and 13.23, of 4096 53.6 and 53.4; lm_head + argmax 32.8 and 26.3 us.
 //   lkb_launch       only when the caller asked for it (lkb_set_pdl): for kernels that read weights ahead of the wait.
 template <typename... KArgs, typename... Args>
 static int lkb_launch_attr(int pdl, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {

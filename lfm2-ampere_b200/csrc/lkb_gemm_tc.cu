@@ -10,9 +10,11 @@
 //
 // One MMA per 32-element block (K = 32 int8 is one Q4_0 / Q8_1 block): the per-block scales forbid accumulating across
 // blocks in the tensor core, so every block's int32 sums come back through TMEM and are folded into fp32 register
-// accumulators, two FMAs per value.  That fold bounds the kernel: a packed fma.rn.f32x2 takes 2 cycles of a scheduler when
-// it fetches at most two register pairs and 3 when it fetches three (measured), and both FMAs of the fold have three
-// operands that differ, so a 16384-value block costs 320 to 384 cycles; everything else is arranged to cost less.
+// accumulators, two FMAs per value.  That fold bounds the kernel: a packed fma.rn.f32x2 takes 2.1 cycles of a scheduler when
+// it fetches two register pairs and 2.9 when it fetches three (measured, two warps a scheduler), and both FMAs of the fold
+// have three operands that differ, so the 128 of a 16384-value block cost 370 cycles.  Integer instructions do not hide under
+// them: one or two lop3 beside each make it 4.8 or 6.9 cycles.  In gate|up at 4096 tokens packed FMAs are half of the cycles,
+// and with the integer and the remaining FMA-pipe instructions four fifths (ncu's counts times these costs).
 //
 //   * TMEM lanes = weight rows, TMEM columns = tokens.  A work item is 256 weight rows (two 128-lane MMA tiles; the SwiGLU
 //     form: 128 gate rows and the same 128 up rows) x the 1..64 tokens of one plan tile, and the MMA's N is the token count
@@ -29,16 +31,15 @@
 //   * The A operand (weights) lives in TMEM: four expansion warps turn staged nibbles into int8 with tcgen05.st, so the
 //     expanded weights never touch shared memory, whose bandwidth the 16-byte fold loads need.
 //   * A producer warp issues bulk tensor copies: nibble rows (64 B per row and stage), activation rows (dense: 16-row boxes;
-//     grouped: row gathers through perm, four rows per copy) and weight scales (16 B per row and two stages: as 16-byte
-//     cp.async they cost the expansion warps 32 lines an instruction, gate|up 67 -> 63 us at 37 tokens of 64 experts, 108 ->
-//     104 at 509, 573 -> 556 at 4096).  Only the activation scales travel by cp.async, six stages ahead.
+//     grouped: row gathers through perm, four rows per copy) and weight scales (16 B per row and two stages; WCOPY below
+//     has the other way and both times).  Only the activation scales travel by cp.async, six stages ahead.
 //   * Persistent: one CTA per SM walks the items, expert by expert, so an expert's weights stay in L2.
-// Measured per layer, token lanes with padding -> this form: gate|up 727 -> 676 us at 4096 tokens (Zipf routing), 315 -> 162 at
-// 509, 259 -> 84 at 37; down 379 -> 324, 170 -> 88, 134 -> 50; in_proj 299 -> 287 at 4096, 64 -> 60 at 509.
-// Then, GEMM alone, balanced routing, 4096 / 509 / 37 tokens (weight scales read from their own ring, expansion a stage at a
-// time, no scale barriers, two MMA issuers): gate|up 580 / 111 / 50 -> 526 / 103 / 44 us, down 259 / 57 / 28 -> 244 / 54 / 24,
-// in_proj 247 / 50 / 20 -> 229 / 47 / 19.  A 16384-value block is then 600 cycles of a scheduler: some 320 to 380 of packed
-// FMAs and 200 issue slots of everything else, 300 of synchronisation when the FMAs are left out.
+// Measured, one layer's GEMMs, 64 experts, balanced routing, caches flushed before every call, us at 37 / 509 / 4096 tokens:
+//   token lanes padded to 128 (before)       gate|up 284 / 312 / 740   down 152 / 159 / 388   in_proj 37 / 64 / 301
+//   weight rows on lanes, one MMA issuer             82 / 126 / 632         55 /  66 / 285           25 / 53 / 256
+//   ... weight scales in a ring of their own, expansion a stage at a time, no scale barriers, two issuers (this form)
+//                                                    70 / 117 / 569         47 /  64 / 268           23 / 51 / 238
+// With few tokens the hand-over of every block is the bound (300 to 440 cycles of polls, commits and arrivals).
 // No copy in this file is a multicast one; every tensor map covers memory of the GPU the kernel runs on.
 // Every wait is bounded; on expiry a status word is set and all roles drain and exit, freeing TMEM.
 #include "lkb_tc.cuh"
@@ -128,7 +129,7 @@ __device__ __forceinline__ int tc_seg(const lkb_pf_gemm & g, int row) { return (
 // ---------------------------------------------------------------------------
 // Block-sum buffers and who fills them.  Free halves (SwiGLU form): each column half has two buffers and an MMA issuer of its
 // own, so the four warps of a half never wait for the other four, which matters where the item ends in the long SwiGLU store
-// (gate|up at 4096 tokens 554 -> 531 us, at 509 107 -> 104, at 37 43 -> 44).  Plain form: one 64-column MMA per tile, common
+// (gate|up at 4096 tokens -4 %, at 509 -3 %, at 37 +2 %).  Plain form: one 64-column MMA per tile, common
 // buffers, issuer h for buffer h; half the MMAs (down and in_proj at 37 tokens 4 % faster than with free halves, equal at 4096).
 template <int EPI> struct TcSums {
     static constexpr int FREE = EPI, TILE = FREE ? TC_TOK / 2 : TC_TOK, BUF = 2 * TILE;      // columns between tiles, between buffers

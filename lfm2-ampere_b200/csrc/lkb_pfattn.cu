@@ -18,10 +18,12 @@
 // log2 e, the running maximum, l = fma(l, alpha, the step's sum) in four chains of two keys out of eight, O *= alpha -- which
 // touches TMEM only when a row of the warp has a new maximum (alpha is exactly 1 otherwise).
 //
-// What bounds it: the exponentials.  A row and key cost 128 multiply-accumulates (1/32 cycle of the tensor pipe) and one
-// ex2 (1/16 cycle of the SM's special function units): 1024 cycles per 128 x 128 tile against 512.  Two tiles per block
-// (NT = 2: 64 positions, eight softmax warps) keep those units busy across the waits and halve the K / V traffic from L2;
-// a chunk too short to give every SM such a block takes one tile per block.
+// What bounds it: a row and key cost 128 multiply-accumulates (1/32 cycle of the tensor pipe) and one ex2 (1/16 cycle of the
+// SM's special function units): 1024 cycles per 128 x 128 tile against 512.  The exponentials are the busiest unit but do not
+// fill it: 8192 tokens behind 24576 positions take 2.83 ms a layer, 64 % of the special function units' cycles, tensor pipe
+// 32 %, issue 42 % (ncu); the rest is the softmax warps' waits for scores and for the P V product.  Two tiles per block
+// (NT = 2: 64 positions, eight softmax warps) overlap those waits and halve the K / V traffic from L2; a chunk too short to
+// give every SM such a block takes one tile per block.
 // Every wait is bounded; on expiry a status word is set and all roles drain and exit, freeing TMEM.
 #include "lkb_attn.cuh"
 #include "lkb_tc.cuh"
