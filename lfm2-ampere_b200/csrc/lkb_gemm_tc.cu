@@ -568,7 +568,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_pf_gemm_tc(const lkb_pf_gemm 
                         if (!tc_wait<TC_HINT_MMA>(S, &tempty[h], L::FREE ? i >> 1 : i, 21u)) { ok = false; break; }
                         tc_fence_after();
                         if (leader) {
-                            tc_mbar_arrive(&tfull[h]);                             // releases what full and afull brought: scales, constants
                             const unsigned d = d0 + h * L::BUF, a = a0 + j * 8;
                             const unsigned long long b = b0 + j * 2;               // a block is 32 bytes, in 16-byte units
                             if (FOLD) {
@@ -577,7 +576,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_pf_gemm_tc(const lkb_pf_gemm 
                             }
                             tc_mma_i8(d, a, b, idesc, FOLD);
                             if (two) tc_mma_i8(d + L::TILE, a + 32, b, idesc, FOLD);
-                            tc_commit(&tfull[h]);                                  // this block's sums are ready (the phase's other arrival)
+                            tc_commit(&tfull[h]);                                  // this block's sums are ready
+                            tc_mbar_arrive(&tfull[h]);                             // and this thread has acquired the stage's scales and constants
                             if (i + 1 == (L::FREE ? TC_KB : TC_KB / 2)) { tc_commit(&S.aempty[ab]); tc_commit(&S.empty[stg]); }    // the stage has been read
                         }
                         __syncwarp();
