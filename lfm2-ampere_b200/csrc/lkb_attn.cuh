@@ -45,17 +45,24 @@ template <int N> __device__ __forceinline__ void at_wait_group() { asm volatile(
 // One warp; lane i holds dims i (a) and i + 32 (b), the pair that rotates together; returns the rotated pair.
 // The sum of squares follows the halving tree s[i] += s[i + o] (o = 32..1), whose root is what lane 0 of an
 // xor butterfly holds.  ref: src/kernels.cu:871-915, src/kernels.cuh:35-54
-__device__ __forceinline__ void at_norm_rope(float a, float b, const float * __restrict__ nw, float pos, float theta, int lane,
-                                             float & y0, float & y1) {
+// at_rope_angle: the rotation of lane i's pair, the same for every head of a position.  at_norm_rotate: the rest.
+__device__ __forceinline__ void at_rope_angle(float pos, float theta, int lane, float & sn, float & cs) {
+    const float invf = powf(theta, __fdiv_rn(__fmul_rn(-2.0f, (float) lane), (float) AT_D));
+    sincosf(__fmul_rn(pos, invf), &sn, &cs);                // precise form: large arguments (ref: src/kernels.cuh:45-48)
+}
+__device__ __forceinline__ void at_norm_rotate(float a, float b, const float * __restrict__ nw, int lane, float sn, float cs, float & y0, float & y1) {
     float ss = __fadd_rn(__fmul_rn(a, a), __fmul_rn(b, b));
     ss = __shfl_sync(LKB_FULL, lkb_warp_sum(ss), 0);
     const float inv = rsqrtf(__fadd_rn(__fdiv_rn(ss, (float) AT_D), 1e-5f));
     const float x0 = __fmul_rn(__fmul_rn(a, inv), nw[lane]), x1 = __fmul_rn(__fmul_rn(b, inv), nw[lane + 32]);
-    const float invf = powf(theta, __fdiv_rn(__fmul_rn(-2.0f, (float) lane), (float) AT_D));
-    float sn, cs;
-    sincosf(__fmul_rn(pos, invf), &sn, &cs);                // precise form: large arguments (ref: src/kernels.cuh:45-48)
     y0 = __fsub_rn(__fmul_rn(x0, cs), __fmul_rn(x1, sn));
     y1 = __fadd_rn(__fmul_rn(x0, sn), __fmul_rn(x1, cs));
+}
+__device__ __forceinline__ void at_norm_rope(float a, float b, const float * __restrict__ nw, float pos, float theta, int lane,
+                                             float & y0, float & y1) {
+    float sn, cs;
+    at_rope_angle(pos, theta, lane, sn, cs);
+    at_norm_rotate(a, b, nw, lane, sn, cs, y0, y1);
 }
 
 // Warp-level tensor-core step: D(16x8, fp32) += A(16x16, fp16, row) * B(16x8, fp16, col).
@@ -73,6 +80,44 @@ __device__ __forceinline__ void at_split(float x0, float x1, unsigned & hi, unsi
     lo = *reinterpret_cast<const unsigned *>(&l);
 }
 
+// Group i of warp w's share of slice [t0, t1) -> its stage i % STAGES (one cp.async group, empty past the share's end).
+template <int STAGES>
+__device__ __forceinline__ void at_issue(AtWarp<STAGES> & W, const __half * __restrict__ kc, const __half * __restrict__ vc,
+                                         int kvh, int t0, int t1, int warp, int lane, int i) {
+    const int ngrp = (t1 - t0 + AT_G - 1) / AT_G;           // groups of this slice; warp w owns w, w+8, ...
+    const int mine = (ngrp - warp + AT_WARPS - 1) / AT_WARPS;
+    const size_t tstride = (size_t) AT_KVH * AT_D;          // halfs between consecutive tokens
+    const __half * kbase = kc + (size_t) kvh * AT_D, * vbase = vc + (size_t) kvh * AT_D;
+    if (i < mine) {
+        const int st = i % STAGES, g0 = t0 + (warp + i * AT_WARPS) * AT_G;
+        const size_t off0 = (size_t) (g0 + (lane >> 3)) * tstride + (lane & 7) * 8;
+#pragma unroll 4
+        for (int r = 0; r < 8; ++r) {
+            const int j = r * 4 + (lane >> 3);
+            const bool live = g0 + j < t1;
+            // dead rows are zero-filled (size 0) from an address that is always inside the cache
+            const size_t off = live ? off0 + (size_t) r * 4 * tstride : (size_t) t0 * tstride;
+            at_cp16(&W.k[st][j][(lane & 7) * 8], kbase + off, live ? 16 : 0);
+            at_cp16(&W.v[st][j][(lane & 7) * 8], vbase + off, live ? 16 : 0);
+        }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+// Whether group i of the warp holds row seq_len - 1, which the step itself writes: not to be requested before that.
+__device__ __forceinline__ bool at_new_row(int t0, int t1, int seq_len, int warp, int i) {
+    return t1 == seq_len && warp + i * AT_WARPS == (t1 - t0 - 1) / AT_G;
+}
+// Requests the first groups of a slice before its queries exist (all threads of the CTA may call it; staging must be idle).
+template <int STAGES>
+__device__ __forceinline__ void at_prefetch(AtSmem<STAGES> & S, const __half * __restrict__ kc, const __half * __restrict__ vc,
+                                            int kvh, int t0, int t1, int seq_len) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp < AT_WARPS)
+#pragma unroll
+        for (int i = 0; i < STAGES - 1; ++i)
+            if (!at_new_row(t0, t1, seq_len, warp, i)) at_issue<STAGES>(S.w[warp], kc, vc, kvh, t0, t1, warp, lane, i);
+}
+
 // One slice [t0, t1) of one KV head: warps 0..7 of the CTA stream their 32-token groups of K and V through
 // private cp.async rings, keep their own online softmax and are merged at the end into
 // part[(kvh*4 + h)][sp] = {max, sum, acc[64]}.
@@ -83,10 +128,10 @@ __device__ __forceinline__ void at_split(float x0, float x1, unsigned & hi, unsi
 // ~300 instructions per group and warp where the scalar form needed ~1000, which is what makes the slice
 // HBM-bound instead of issue-bound at long context.
 // Every thread of the CTA must call this (it contains CTA barriers); S.q must be filled and visible (a CTA
-// barrier after the fill) before the call.
-template <int STAGES>
+// barrier after the fill) before the call.  AHEAD: at_prefetch was called with the same arguments.
+template <int STAGES, bool AHEAD = false>
 __device__ __forceinline__ void at_slice(AtSmem<STAGES> & S, const __half * __restrict__ kc, const __half * __restrict__ vc,
-                                         int kvh, int sp, int t0, int t1, float * __restrict__ part) {
+                                         int kvh, int sp, int t0, int t1, float * __restrict__ part, int seq_len = 0) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, t4 = lane & 3;
     const bool worker = warp < AT_WARPS;
@@ -94,26 +139,10 @@ __device__ __forceinline__ void at_slice(AtSmem<STAGES> & S, const __half * __re
         AtWarp<STAGES> & W = S.w[warp];
         const int ngrp = (t1 - t0 + AT_G - 1) / AT_G;       // groups of this slice; warp w owns w, w+8, ...
         const int mine = (ngrp - warp + AT_WARPS - 1) / AT_WARPS;
-        const size_t tstride = (size_t) AT_KVH * AT_D;      // halfs between consecutive tokens
-        const __half * kbase = kc + (size_t) kvh * AT_D, * vbase = vc + (size_t) kvh * AT_D;
-        auto issue = [&](int i) {                           // group i of this warp -> stage i % STAGES
-            if (i < mine) {
-                const int st = i % STAGES, g0 = t0 + (warp + i * AT_WARPS) * AT_G;
-                const size_t off0 = (size_t) (g0 + (lane >> 3)) * tstride + (lane & 7) * 8;
+        // (a held-back group is the warp's last one: what at_prefetch issued lies before it)
 #pragma unroll
-                for (int r = 0; r < 8; ++r) {
-                    const int j = r * 4 + (lane >> 3);
-                    const bool live = g0 + j < t1;
-                    // dead rows are zero-filled (size 0) from an address that is always inside the cache
-                    const size_t off = live ? off0 + (size_t) r * 4 * tstride : (size_t) t0 * tstride;
-                    at_cp16(&W.k[st][j][(lane & 7) * 8], kbase + off, live ? 16 : 0);
-                    at_cp16(&W.v[st][j][(lane & 7) * 8], vbase + off, live ? 16 : 0);
-                }
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        };
-#pragma unroll
-        for (int i = 0; i < STAGES - 1; ++i) issue(i);
+        for (int i = 0; i < STAGES - 1; ++i)
+            if (!AHEAD || at_new_row(t0, t1, seq_len, warp, i)) at_issue<STAGES>(W, kc, vc, kvh, t0, t1, warp, lane, i);
         // Q fragments (rows 0..3 = heads, scaled by the exact 1/8): register pair kk holds dims 16 kk + 2 t4 + {0,1}
         // (a0) and + 8 (a2) of head g, as hi and lo parts; rows 8..15 (a1, a3) and heads g >= 4 are zero
         unsigned qh0[4], qh2[4], ql0[4], ql2[4];
@@ -134,8 +163,9 @@ __device__ __forceinline__ void at_slice(AtSmem<STAGES> & S, const __half * __re
         float o[8][4];
 #pragma unroll
         for (int nd = 0; nd < 8; ++nd) { o[nd][0] = o[nd][1] = o[nd][2] = o[nd][3] = 0.0f; }
+#pragma unroll 1
         for (int i = 0; i < mine; ++i) {
-            issue(i + STAGES - 1);
+            at_issue<STAGES>(W, kc, vc, kvh, t0, t1, warp, lane, i + STAGES - 1);
             at_wait_group<STAGES - 1>();
             __syncwarp();
             const int st = i % STAGES, g0 = t0 + (warp + i * AT_WARPS) * AT_G;
@@ -239,23 +269,24 @@ __device__ __forceinline__ float at_combine(const float * __restrict__ part, int
     const int chunk = at_chunk(seq_len, nsl);
     const int nlive = min(nsl, (seq_len + chunk - 1) / chunk);
     const float * P = part + (size_t) head * LKB_ATTN_SPLIT * LKB_ATTN_PARTW;
-    float mv[LKB_ATTN_SPLIT], lv[LKB_ATTN_SPLIT], av[LKB_ATTN_SPLIT];
+    // lane s: slice s (the callers are whole warps); the accumulators of this thread's dim: all slices in flight
+    const int lane = threadIdx.x & 31;
+    const bool mine = lane < nlive;
+    const float m = mine ? __ldcg(P + lane * LKB_ATTN_PARTW) : -1e30f, lv = mine ? __ldcg(P + lane * LKB_ATTN_PARTW + 1) : 0.0f;
+    float av[LKB_ATTN_SPLIT];
 #pragma unroll
-    for (int s = 0; s < LKB_ATTN_SPLIT; ++s) {
-        const bool live = s < nlive;
-        mv[s] = live ? __ldcg(P + s * LKB_ATTN_PARTW) : -1e30f;
-        lv[s] = live ? __ldcg(P + s * LKB_ATTN_PARTW + 1) : 0.0f;
-        av[s] = live ? __ldcg(P + s * LKB_ATTN_PARTW + 2 + d) : 0.0f;
-    }
-    float M = -1e30f;
+    for (int s = 0; s < LKB_ATTN_SPLIT; ++s) av[s] = s < nlive ? __ldcg(P + s * LKB_ATTN_PARTW + 2 + d) : 0.0f;
+    float M = m;
 #pragma unroll
-    for (int s = 0; s < LKB_ATTN_SPLIT; ++s) M = fmaxf(M, mv[s]);
+    for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(LKB_FULL, M, o));
+    M = fmaxf(M, -1e30f);
+    const float es = __expf(__fsub_rn(m, M));
     float L = 0.0f, A = 0.0f;
 #pragma unroll
     for (int s = 0; s < LKB_ATTN_SPLIT; ++s) {
+        const float e = __shfl_sync(LKB_FULL, es, s), l = __shfl_sync(LKB_FULL, lv, s);
         if (s < nlive) {
-            const float e = __expf(__fsub_rn(mv[s], M));
-            L = fmaf(lv[s], e, L);
+            L = fmaf(l, e, L);
             A = fmaf(av[s], e, A);
         }
     }

@@ -90,15 +90,16 @@ __device__ __forceinline__ void lkb_quant_store_planar_fused_epilogue(float xi, 
 // exchanges (xor 4, 2, 1, one per held element) and the last two are adds inside the thread, so every partial
 // sum is the same pair of operands as there (fp32 addition is commutative) and the result has the same bits.
 // ---------------------------------------------------------------------------
+// A lane hands over half of what it holds per level while there is something to split (lane bit 2 keeps elements 0, 1 or 2, 3,
+// bit 1 one of the two), so the five levels take 6 shuffles and 6 additions where summing all four everywhere takes 12 and 15.
 __device__ __forceinline__ float lkb_quad_sum(float a0, float a1, float a2, float a3) {
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) {
-        a0 = __fadd_rn(a0, __shfl_xor_sync(LKB_FULL, a0, o));
-        a1 = __fadd_rn(a1, __shfl_xor_sync(LKB_FULL, a1, o));
-        a2 = __fadd_rn(a2, __shfl_xor_sync(LKB_FULL, a2, o));
-        a3 = __fadd_rn(a3, __shfl_xor_sync(LKB_FULL, a3, o));
-    }
-    return __fadd_rn(__fadd_rn(a0, a2), __fadd_rn(a1, a3));
+    const bool b2 = threadIdx.x & 4, b1 = threadIdx.x & 2;
+    const float k0 = __fadd_rn(b2 ? a2 : a0, __shfl_xor_sync(LKB_FULL, b2 ? a0 : a2, 4));
+    const float k1 = __fadd_rn(b2 ? a3 : a1, __shfl_xor_sync(LKB_FULL, b2 ? a1 : a3, 4));
+    float k = __fadd_rn(b1 ? k1 : k0, __shfl_xor_sync(LKB_FULL, b1 ? k0 : k1, 2));
+    k = __fadd_rn(k, __shfl_xor_sync(LKB_FULL, k, 1));
+    k = __fadd_rn(k, __shfl_xor_sync(LKB_FULL, k, 4));              // elements 0 + 2, 1 + 3
+    return __fadd_rn(k, __shfl_xor_sync(LKB_FULL, k, 2));
 }
 
 // Q8_1 of the block this lane's group of 8 holds: returns the lane's four quants packed low byte first;
@@ -166,13 +167,19 @@ __device__ __forceinline__ float lkb_norm_inv(const float * __restrict__ ssq, in
 
 // Integer block sum: 16 weight bytes (unsigned nibbles) against 32 int8.
 // ref: src/quant.cuh:141-151
+__device__ __forceinline__ int lkb_dp4a_us(unsigned a, int b, int c) {          // unsigned bytes times signed bytes
+    int d;
+    asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
 __device__ __forceinline__ int lkb_sumi(const uint4 q, const int (&x)[8]) {
-    // four independent integer chains (integer addition is exact in any order)
+    // four independent integer chains (integer addition is exact in any order); the high nibbles stay where they are, as
+    // unsigned bytes 16 times as large, so their sum is an exact multiple of 16 and one shift brings it back
     int s0 = __dp4a((int) (q.x & 0x0F0F0F0Fu), x[0], 0), s1 = __dp4a((int) (q.y & 0x0F0F0F0Fu), x[1], 0);
-    int s2 = __dp4a((int) (q.z & 0x0F0F0F0Fu), x[2], 0), s3 = __dp4a((int) (q.w & 0x0F0F0F0Fu), x[3], 0);
-    s0 = __dp4a((int) ((q.x >> 4) & 0x0F0F0F0Fu), x[4], s0); s1 = __dp4a((int) ((q.y >> 4) & 0x0F0F0F0Fu), x[5], s1);
-    s2 = __dp4a((int) ((q.z >> 4) & 0x0F0F0F0Fu), x[6], s2); s3 = __dp4a((int) ((q.w >> 4) & 0x0F0F0F0Fu), x[7], s3);
-    return (s0 + s1) + (s2 + s3);
+    int h0 = lkb_dp4a_us(q.x & 0xF0F0F0F0u, x[4], 0), h1 = lkb_dp4a_us(q.y & 0xF0F0F0F0u, x[5], 0);
+    s0 = __dp4a((int) (q.z & 0x0F0F0F0Fu), x[2], s0); s1 = __dp4a((int) (q.w & 0x0F0F0F0Fu), x[3], s1);
+    h0 = lkb_dp4a_us(q.z & 0xF0F0F0F0u, x[6], h0); h1 = lkb_dp4a_us(q.w & 0xF0F0F0F0u, x[7], h1);
+    return (s0 + s1) + ((h0 + h1) >> 4);
 }
 
 // acc + d4*(d8*sumi - 8*sum): inner = fma(d8, float(sumi), -8sum), acc' = fma(d4, inner, acc).

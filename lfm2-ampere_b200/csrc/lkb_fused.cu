@@ -72,6 +72,7 @@ struct FusedSmem {
     float  ppart[FUSED_WARPS];            // expert prefetch: per-warp partials of the guessed logit
     float  wk[LKB_TOP_K];
     float  inv;
+    float  cs[AT_D / 2], sn[AT_D / 2];    // whole-step kernel: rotation at this step's position
     int    abort;
     unsigned bar_target;
     alignas(8) lkb_moe_layer ly;          // this layer's descriptor (staged: a global read costs ~1 us of latency)
@@ -99,6 +100,7 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long * b, unsigned p
 }
 // Bounded wait; returns false on expiry.
 __device__ __forceinline__ bool mbar_wait(unsigned long long * b, unsigned parity) {
+#pragma unroll 1
     for (unsigned i = 0; i < SPIN_LIMIT; ++i) if (mbar_try_wait(b, parity)) return true;
     return false;
 }
@@ -145,6 +147,7 @@ __device__ __forceinline__ bool grid_wait(unsigned * bar, unsigned * status, Fus
     if (threadIdx.x == 0) {
         const unsigned target = S.bar_target;
         bool ok = false;
+#pragma unroll 1
         for (unsigned i = 0; i < spin_limit; ++i) {
             if (ld_acquire(bar) >= target) { ok = true; break; }
             if ((i & 1023u) == 1023u && ld_acquire(status) != 0u) break;
@@ -168,6 +171,7 @@ __device__ __forceinline__ void issue_rows(const SegView & v, int seg_rows, int 
     unsigned bytes = (unsigned) (g_end - g_begin) * (unsigned) bpr * 18u;
     mbar_expect_tx(mb, bytes);
     int g = g_begin;
+#pragma unroll 1
     while (g < g_end) {
         const int s = g / seg_rows, r = g - s * seg_rows;
         int n = g_end - g; if (n > seg_rows - r) n = seg_rows - r;
@@ -182,6 +186,7 @@ __device__ __forceinline__ void issue_gu_rows(const lkb_moe_layer & ly, const in
                                               unsigned char * sq, __half * sd, unsigned long long * mb) {
     mbar_expect_tx(mb, (unsigned) (g_end - g_begin) * (unsigned) GU_BPR * 18u);
     int g = g_begin;
+#pragma unroll 1
     while (g < g_end) {
         const int seg = g / LKB_MOE_INTER, r = g - seg * LKB_MOE_INTER;
         int n = g_end - g; if (n > LKB_MOE_INTER - r) n = LKB_MOE_INTER - r;
@@ -197,6 +202,7 @@ __device__ __forceinline__ void issue_gu_rows(const lkb_moe_layer & ly, const in
 // The same rows of the guessed experts of the next layer, into L2 only.
 __device__ __forceinline__ void prefetch_gu_rows(const lkb_moe_layer & ly, const int * idx, int g_begin, int g_end) {
     int g = g_begin;
+#pragma unroll 1
     while (g < g_end) {
         const int seg = g / LKB_MOE_INTER, r = g - seg * LKB_MOE_INTER;
         int n = g_end - g; if (n > LKB_MOE_INTER - r) n = LKB_MOE_INTER - r;
@@ -345,6 +351,7 @@ __device__ __forceinline__ void mix_issue_in(FusedSmem & S, const lkb_mixer_laye
     fence_proxy_async();
     if (!mx.is_attn) {
         mbar_expect_tx(&S.mbar_mi, 3u * (unsigned) n_dn * GU_BPR * 18u);
+#pragma unroll 1
         for (int s = 0; s < 3; ++s) {
             const size_t blk = ((size_t) s * LKB_HIDDEN + dn0) * GU_BPR;
             bulk_g2s(S.gu_q + (size_t) s * n_dn * GU_BPR * 16, (const uint4 *) mx.in_qs + blk, (unsigned) n_dn * GU_BPR * 16u, &S.mbar_mi);
@@ -353,6 +360,7 @@ __device__ __forceinline__ void mix_issue_in(FusedSmem & S, const lkb_mixer_laye
     } else {
         mbar_expect_tx(&S.mbar_mi, (unsigned) (a1 - a0) * GU_BPR * 18u);
         unsigned char * sq = S.gu_q; __half * sd = S.gu_d;
+#pragma unroll 1
         for (int g = a0; g < a1; ) {
             const int seg = g < LKB_HIDDEN ? 0 : (g < LKB_HIDDEN + AT_KVH * AT_D ? 1 : 2);
             const int base = seg == 0 ? 0 : (seg == 1 ? LKB_HIDDEN : LKB_HIDDEN + AT_KVH * AT_D);
@@ -399,7 +407,9 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
     if (tid == 0) {
         S.abort = 0;
         S.bar_target = 0u;
+#pragma unroll 1
         for (int i = 0; i < N_GU_CH; ++i) mbar_init(&S.mbar_gu[i], 1);
+#pragma unroll 1
         for (int i = 0; i < N_DN_CH; ++i) mbar_init(&S.mbar_dn[i], 1);
         mbar_init(&S.mbar_rt, 1);
         mbar_init(&S.mbar_mi, 1);
@@ -449,11 +459,13 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
         if (tid < (int) (sizeof(lkb_mixer_layer) / 8))
             reinterpret_cast<unsigned long long *>(&S.mx)[tid] = reinterpret_cast<const unsigned long long *>(&a.mixers[0])[tid];
     }
+    if (MIX && warp == FUSED_WARPS - 1) at_rope_angle((float) pos, a.theta, lane, S.sn[lane], S.cs[lane]);
     __syncthreads();
     if constexpr (MIX) {
         // KV capacity: an attention layer whose descriptor states max_seq refuses a position past its cache.  Every CTA
         // evaluates the same test before anything is in flight, so all leave together (status 600 + layer).
         int over = -1;
+#pragma unroll 1
         for (int l = tid; l < a.n_layers; l += blockDim.x)
             if (a.mixers[l].is_attn && a.mixers[l].max_seq > 0 && pos >= a.mixers[l].max_seq) over = l;
         if (__syncthreads_or(over >= 0)) {
@@ -466,6 +478,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
         }
     }
 
+#pragma unroll 1
     for (int l = 0; l < a.n_layers; ++l) {
         const lkb_moe_layer & ly = S.ly;
         const unsigned par = (unsigned) (l & 1);
@@ -485,6 +498,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
             // ---- M0: the mixer's input activation: layer 0 arrives normalised and quantised; later layers
             //          quantise raw u = x * attn_norm_w and carry 1/rms into the consumer (S.inv) ----
             if (l == 0) {
+#pragma unroll 1
                 for (int i = tid; i < LKB_HIDDEN / 32 * 9; i += FUSED_THREADS)
                     reinterpret_cast<int *>(S.xq)[i] = reinterpret_cast<const int *>(a.xq_first)[i];
                 if (tid == 0) S.inv = 1.0f;
@@ -504,6 +518,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
                 float * mixv = &S.dot[0][0];
                 if (!mbar_wait(&S.mbar_mi, par)) { if (lane == 0) { atomicCAS(status, 0u, 400u + l); S.abort = 1; } }
                 else {
+#pragma unroll 1
                     for (int j = warp; j < nrows; j += FUSED_WARPS) {
                         const float acc = lkb_warp_sum(smem_row_partial<2>(S.gu_q + (size_t) j * GU_BPR * 16, S.gu_d + (size_t) j * GU_BPR,
                                                                            GU_BPR, lane, xq, d8, s8));
@@ -527,36 +542,38 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
             }
             FUSED_STAMP(18);
             grid_arrive(a.bar, S);
+            // ---- M2: one slice of one KV head per CTA; the query heads' norm + rotation are redone by every
+            //          slice, the new K / V row is written by the slice that contains it (the last one).  The first groups
+            //          of the slice, all but the new row's, are requested before q exists: the staging is idle from here. ----
+            const int seq_len = pos + 1, nsl = at_slices(seq_len), chunk = at_chunk(seq_len, nsl);
+            const int kvh = cta & (AT_KVH - 1), sp = cta >> 3;
+            const int t0 = sp * chunk, t1 = min(t0 + chunk, seq_len);
+            const bool slice = is_attn && sp < nsl && t0 < t1;              // CTA-uniform
+            if (slice) at_prefetch<2>(*reinterpret_cast<AtSmem2 *>(fused_smem_raw), reinterpret_cast<const __half *>(mx.kc), reinterpret_cast<const __half *>(mx.vc), kvh, t0, t1, seq_len);
             if (!grid_wait(a.bar, status, S, 1000u + 10u * l + 4u, a.spin_limit)) return;
             FUSED_STAMP(19);
-            const int seq_len = pos + 1;
             if (is_attn) {
-                // ---- M2: one slice of one KV head per CTA; the query heads' norm + rotation are redone by every
-                //          slice, the new K / V row is written by the slice that contains it (the last one) ----
-                const int nsl = at_slices(seq_len), chunk = at_chunk(seq_len, nsl);
-                const int kvh = cta & (AT_KVH - 1), sp = cta >> 3;
-                const int t0 = sp * chunk, t1 = min(t0 + chunk, seq_len);
-                if (sp < nsl && t0 < t1) {                                  // CTA-uniform
+                if (slice) {
                     AtSmem2 & A = *reinterpret_cast<AtSmem2 *>(fused_smem_raw);
                     __half * kc = reinterpret_cast<__half *>(mx.kc), * vc = reinterpret_cast<__half *>(mx.vc);
                     if (warp < AT_GQA) {
                         const float * qh = a.mxbuf + (size_t) (kvh * AT_GQA + warp) * AT_D;
                         float y0, y1;
-                        at_norm_rope(__ldcg(qh + lane), __ldcg(qh + lane + 32), mx.qnorm, (float) pos, a.theta, lane, y0, y1);
+                        at_norm_rotate(__ldcg(qh + lane), __ldcg(qh + lane + 32), mx.qnorm, lane, S.sn[lane], S.cs[lane], y0, y1);
                         reinterpret_cast<float *>(&A.q[lane])[warp] = y0;
                         reinterpret_cast<float *>(&A.q[lane + 32])[warp] = y1;
                     } else if (warp == AT_GQA && t1 == seq_len) {
                         const float * kh = a.mxbuf + LKB_HIDDEN + (size_t) kvh * AT_D;
                         const float * vh = a.mxbuf + LKB_HIDDEN + AT_KVH * AT_D + (size_t) kvh * AT_D;
                         float y0, y1;
-                        at_norm_rope(__ldcg(kh + lane), __ldcg(kh + lane + 32), mx.knorm, (float) pos, a.theta, lane, y0, y1);
+                        at_norm_rotate(__ldcg(kh + lane), __ldcg(kh + lane + 32), mx.knorm, lane, S.sn[lane], S.cs[lane], y0, y1);
                         const size_t off = ((size_t) pos * AT_KVH + kvh) * AT_D;
                         kc[off + lane] = __float2half(y0); kc[off + lane + 32] = __float2half(y1);
                         vc[off + lane] = __float2half(__ldcg(vh + lane)); vc[off + lane + 32] = __float2half(__ldcg(vh + lane + 32));
                         __threadfence();
                     }
                     __syncthreads();
-                    at_slice<2>(A, kc, vc, kvh, sp, t0, t1, a.part);
+                    at_slice<2, true>(A, kc, vc, kvh, sp, t0, t1, a.part, seq_len);
                 }
                 FUSED_STAMP(20);
                 grid_arrive(a.bar, S);
@@ -672,6 +689,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
             float p = 0.0f;
             if (tid < LKB_N_EXPERTS) {
                 float mx = S.sel[0];
+#pragma unroll 1
                 for (int e = 1; e < LKB_N_EXPERTS; ++e) mx = fmaxf(mx, S.sel[e]);
                 p = expf(__fsub_rn(S.sel[tid], mx));
                 S.sig[tid] = p;
@@ -680,6 +698,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
             float pn = 0.0f;
             if (tid < LKB_N_EXPERTS) {
                 float den = 0.0f;
+#pragma unroll 1
                 for (int e = 0; e < LKB_N_EXPERTS; ++e) den = __fadd_rn(den, S.sig[e]);
                 pn = __fdiv_rn(p, den);
             }
@@ -731,6 +750,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
         // ---- D: request every weight row of the layer, one issuing lane per chunk ---
         if (lane == 0) {
             fence_proxy_async();
+#pragma unroll 1
             for (int c = warp; c < n_gu_ch + LKB_TOP_K * dn_ch_per_k; c += FUSED_WARPS) {
                 if (c < n_gu_ch) {
                     const int up = c >= gu_half_ch, ch = up ? c - gu_half_ch : c;
@@ -759,6 +779,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
             int xq[2][8]; float d8[2], s8[2];
             load_xregs<2>(S.xq, GU_BPR, lane, xq, d8, s8);
             const float ninv = S.inv;
+#pragma unroll 1
             for (int j = warp; j < n_gu; j += FUSED_WARPS) {
                 // both probes are issued before either answer is used (a probe takes ~0.1 us even when the rows are there)
                 unsigned long long * const mg = &S.mbar_gu[j / CH_ROWS], * const mu = &S.mbar_gu[gu_half_ch + j / CH_ROWS];
@@ -828,6 +849,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
             // in the chunks of the real request, one or two per issuing lane
             if (lane == 0) {
                 const lkb_moe_layer & nx = S.ly_next;
+#pragma unroll 1
                 for (int c = warp - 1; c < n_gu_ch + LKB_TOP_K * dn_ch_per_k; c += FUSED_WARPS - 1) {
                     if (c < n_gu_ch) {
                         const int up = c >= gu_half_ch, ch = up ? c - gu_half_ch : c;
@@ -952,7 +974,9 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
         float xv[4], uv[4];
         fused_load_u(S, a.x, nw, xv, uv);
         fused_quant_u(S, xv, uv);
+#pragma unroll 1
         for (int i = tid; i < LKB_HIDDEN; i += FUSED_THREADS) if (a.out_h32) a.out_h32[i] = S.h[i];
+#pragma unroll 1
         for (int i = tid; i < LKB_HIDDEN / 32 * 9; i += FUSED_THREADS)
             reinterpret_cast<int *>(a.out_yq8)[i] = reinterpret_cast<const int *>(S.xq)[i];
         if (tid < LKB_HIDDEN / 32) a.out_ssq[tid] = S.ssq[tid];
@@ -965,6 +989,7 @@ static int g_fused_ready = 0;
 int lkb_fused_init() {
     const void * kernels[4] = {(const void *) k_moe_ffn_stack<false, false>, (const void *) k_moe_ffn_stack<false, true>,
                                (const void *) k_moe_ffn_stack<true, false>, (const void *) k_moe_ffn_stack<true, true>};
+#pragma unroll 1
     for (const void * k : kernels) {
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sizeof(FusedSmem));
         if (e != cudaSuccess) return -(int) e;
@@ -1039,8 +1064,11 @@ int lkb_decode_expert_prefetch_hits(const lkb_moe_scratch * scratch, int n_layer
     if (e == cudaSuccess) e = cudaMemcpy(rec[1], scratch->gu + PF_REAL_OFF, sizeof(int) * 4 * nl, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return -(int) e;
     int h = 0;
+#pragma unroll 1
     for (int l = 1; l < nl; ++l)
+#pragma unroll 1
         for (int i = 0; i < 4; ++i)
+#pragma unroll 1
             for (int j = 0; j < 4; ++j) h += rec[0][l * 4 + i] == rec[1][l * 4 + j];
     *hits = h; *guesses = 4 * (nl - 1);
     return LKB_OK;
