@@ -170,7 +170,7 @@ typedef struct {
 /* The fused kernels read x, the norm weights (ffn_norm, attn_norm, the optional final norm) and the scratch vectors 128
  * bits at a time: those pointers must be 16-byte aligned (LKB_ERR_SHAPE where the launcher can see them).
  * Caller-owned global scratch of the fused kernels: 64 floats (router logits), 2*4*1536 floats (exchange of the
- * intermediate activations; the current kernels use the first 4*1536) and
+ * intermediate activations and, in the whole-step kernel, of the residual and the mixers' outputs; any content on entry) and
  * two 32-bit words (barrier counter, status; status != 0 after the kernel means a
  * bounded wait expired: 1000+10*layer+n = grid barrier n, 100/200/300+layer = a copy). */
 #define LKB_MOE_SCRATCH_LOGITS 64

@@ -49,6 +49,10 @@
 #define PF_MAXL       512
 #define PF_GUESS_OFF  (PF_LOGITS_OFF + 128)
 #define PF_REAL_OFF   (PF_GUESS_OFF + 4 * PF_MAXL)
+// Whole-step kernel without expert prefetch: the residual after the mixer and the mixer's outputs have words of their own.
+#define XCH_XB_OFF    (LKB_TOP_K * LKB_MOE_INTER)
+#define XCH_M_OFF     (XCH_XB_OFF + LKB_HIDDEN)
+static_assert(XCH_M_OFF + LKB_HIDDEN <= 2 * LKB_TOP_K * LKB_MOE_INTER, "words must fit the gu scratch");
 static_assert(MAX_DN_ROWS <= FUSED_WARPS, "a down row per warp");
 static_assert(PF_REAL_OFF + 4 * PF_MAXL <= 2 * LKB_TOP_K * LKB_MOE_INTER, "prefetch records must fit the gu scratch");
 
@@ -72,6 +76,7 @@ struct FusedSmem {
     float  ppart[FUSED_WARPS];            // expert prefetch: per-warp partials of the guessed logit
     float  wk[LKB_TOP_K];
     float  inv;
+    float  xown[MAX_DN_ROWS];             // the residual rows this CTA owns
     float  cs[AT_D / 2], sn[AT_D / 2];    // whole-step kernel: rotation at this step's position
     int    abort;
     unsigned bar_target;
@@ -126,17 +131,80 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned * p) {
 // counter reaches (k+1)*gridDim.x: the arrival is a fire-and-forget reduction (no returned
 // ticket to wait for) and the waiter starts polling at once.
 // wait returns false if it expired or another CTA reported a fault.
-__device__ __forceinline__ void grid_arrive(unsigned * bar, FusedSmem & S) {
-    __syncthreads();                                   // this CTA's global writes are issued
-    if (threadIdx.x == 0) {
-        S.bar_target += gridDim.x;
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" :: "l"(bar) : "memory");
-    }
+//
+// What the CTAs exchange -- logits, gate|up outputs, mixer outputs, residual rows: floats, one word each -- is published
+// WITHOUT a release (XCH): a release waits until the stores are acknowledged, some 0.4 us a barrier.  Instead a word that is
+// still due holds XCH_DUE, a NaN that arithmetic does not produce, and a reader that finds it after the barrier loads again.
+// A word is made due again by a CTA that knows everyone has read it (a later barrier is through), followed by a fence, before
+// that CTA arrives at the barrier of the word's next use: the store has been performed on the device when the arrival is
+// sent, so nobody behind that barrier can see the content before.
+// These stores and the fence sit between the arrival and the wait of some barrier, where nobody waits for them (xch_due below).
+// A launch starts with all words due and its first barrier a releasing one.  MoE stack of 40 layers 514 -> 496 us, a token at
+// context 4096 946 -> 930 us.
+#define XCH_DUE 0xFFFFFFFFu
+template <bool XCH>
+__device__ __forceinline__ void xch_put(float * p, float v) {
+    unsigned u = __float_as_uint(v);
+    if (XCH && u == XCH_DUE) u = 0x7FFFFFFFu;                  // (the NaN that arithmetic produces)
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" :: "l"(p), "r"(u) : "memory");
 }
-// The arrival alone, by thread 0, where the data it publishes is thread 0's own.
-__device__ __forceinline__ void grid_arrive_one(unsigned * bar, FusedSmem & S) {
+__device__ __forceinline__ void xch_due(float * p, int i, int n) {       // words i, i + 32, ... below n
+#pragma unroll 1
+    for (; i < n; i += 32) asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" :: "l"(p + i), "r"(XCH_DUE) : "memory");
+}
+__device__ __forceinline__ void xch_due_fence() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+__device__ __forceinline__ uint4 xch_ld4(const float * p) {
+    uint4 v;
+    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ unsigned xch_ld1(const float * p) {
+    unsigned v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ bool xch_missing(const uint4 & v) { return v.x == XCH_DUE || v.y == XCH_DUE || v.z == XCH_DUE || v.w == XCH_DUE; }
+// A word that was due when it was first read: bounded, out of line.  *abort is set when it does not come (`code` as for the
+// barrier in front of it; every phase that reads words ends in a barrier wait, which looks at it).
+__device__ __noinline__ float xch_again(const float * p, unsigned * status, unsigned code, int * abort) {
+#pragma unroll 1
+    for (unsigned i = 0; i < SPIN_LIMIT; ++i) {
+        const unsigned v = xch_ld1(p);
+        if (v != XCH_DUE) return __uint_as_float(v);
+        if ((i & 1023u) == 1023u && ld_acquire(status) != 0u) break;
+    }
+    atomicCAS(status, 0u, code);
+    *abort = 1;
+    return 0.0f;
+}
+template <bool XCH>
+__device__ __forceinline__ float xch_get(const float * p, unsigned * status, int & abort, unsigned code) {
+    const unsigned v = xch_ld1(p);
+    return XCH && v == XCH_DUE ? xch_again(p, status, code, &abort) : __uint_as_float(v);
+}
+// Four words, 16-byte aligned.
+__device__ __noinline__ float4 xch_again4(const float * p, unsigned * status, unsigned code, int * abort) {
+    float4 v;
+    v.x = xch_again(p, status, code, abort); v.y = xch_again(p + 1, status, code, abort);
+    v.z = xch_again(p + 2, status, code, abort); v.w = xch_again(p + 3, status, code, abort);
+    return v;
+}
+template <bool XCH>
+__device__ __forceinline__ float4 xch_get4(const float * p, unsigned * status, int & abort, unsigned code, bool words = true) {
+    const uint4 v = xch_ld4(p);
+    if (XCH && xch_missing(v) && words) return xch_again4(p, status, code, &abort);
+    return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
+}
+template <bool RELEASE = true>
+__device__ __forceinline__ void grid_arrive_one(unsigned * bar, FusedSmem & S, bool release = RELEASE) {
     S.bar_target += gridDim.x;
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" :: "l"(bar) : "memory");
+    if (RELEASE || release) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" :: "l"(bar) : "memory");
+    else                    asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" :: "l"(bar) : "memory");
+}
+template <bool RELEASE = true>
+__device__ __forceinline__ void grid_arrive(unsigned * bar, FusedSmem & S, bool release = RELEASE) {
+    __syncthreads();                                   // this CTA's global writes are issued
+    if (threadIdx.x == 0) grid_arrive_one<RELEASE>(bar, S, release);
 }
 // One poll in flight per CTA.  (Keeping four relaxed polls in flight per CTA, a quarter of a round trip apart, was
 // measured: every barrier got 0.4-0.7 us SLOWER -- 148 CTAs x 4 loads on the one L2 line delay the arriving
@@ -295,7 +363,7 @@ struct FusedArgs {
     int *                 idx_out;     // optional [n_layers][4]
     float *               w_out;       // optional [n_layers][4]
     float *               logits;      // scratch [64]
-    float *               gu;          // scratch [2*4*1536]: silu(gate)*up of the 4*1536 pairs in its first half
+    float *               gu;          // scratch [2*4*1536]: silu(gate)*up of the 4*1536 pairs in its first half; see XCH_*_OFF, PF_*_OFF
     unsigned *            bar;         // scratch [2]: {barrier counter, status}
     int                   softmax;
     unsigned long long *  timing;
@@ -307,14 +375,16 @@ struct FusedArgs {
     const lkb_q8blk *     xq_first;    // layer 0's normalised Q8_1 activation (lkb_rmsnorm_q8_1)
     const int *           d_pos;       // device-side position
     float                 theta;       // RoPE base
-    float *               mxbuf;       // scratch [3072]: q | k | v of an attention layer, or the conv output
+    float *               mxbuf;       // scratch [3072]: q | k | v of an attention layer
     float *               part;        // scratch [32][LKB_ATTN_SPLIT][LKB_ATTN_PARTW]
 };
 
 // Loads x (written by other CTAs -> L2), elements 4*tid .. +3, and forms u = x*w into S.h.
+// words: x is exchanged (the launch's own input may hold any NaN).
+template <bool XCH>
 __device__ __forceinline__ void fused_load_u(FusedSmem & S, const float * __restrict__ x, const float (&nw)[4],
-                                             float (&xv)[4], float (&uv)[4]) {
-    const float4 t = __ldcg(reinterpret_cast<const float4 *>(x) + threadIdx.x);
+                                             float (&xv)[4], float (&uv)[4], bool words, unsigned * status, unsigned code) {
+    const float4 t = xch_get4<XCH>(x + 4 * threadIdx.x, status, S.abort, code, words);
     xv[0] = t.x; xv[1] = t.y; xv[2] = t.z; xv[3] = t.w;
 #pragma unroll
     for (int j = 0; j < 4; ++j) uv[j] = __fmul_rn(xv[j], nw[j]);
@@ -450,8 +520,19 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
         }
     }
     if (tid < LKB_TOP_K) S.pidx[tid] = tid;
+    constexpr bool XCH = !PF;                                        // (with expert prefetch its records take the words' place: released barriers)
+    float * const x_mid = MIX && XCH ? a.gu + XCH_XB_OFF : a.x;      // residual after the mixer
+    float * const m_out = XCH ? a.gu + XCH_M_OFF : a.mxbuf;          // the mixer's outputs
+    if (tid < n_dn) S.xown[tid] = __ldcg(a.x + dn0 + tid);
     // whole-step kernel: row ranges of the mixers, layer 0's descriptor and weight rows
     const int qa0 = (int) (((long long) cta * MIX_QKV_ROWS) / nct), qa1 = (int) (((long long) (cta + 1) * MIX_QKV_ROWS) / nct);
+    if (XCH && warp == 1) {                                          // every word this launch exchanges is due
+        xch_due(a.gu + gu0, lane, n_gu);
+        if (MIX) {
+            xch_due(x_mid + dn0, lane, n_dn); xch_due(m_out + dn0, lane, n_dn); xch_due(a.mxbuf + qa0, lane, qa1 - qa0);
+            if (cta < LKB_N_EXPERTS) xch_due(a.logits + cta, lane, 1);
+        }
+    }
     int pos = 0;
     float anw[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     if constexpr (MIX) {
@@ -505,7 +586,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
                 __syncthreads();
             } else {
                 float xv[4], uv[4];
-                fused_load_u(S, a.x, anw, xv, uv);
+                fused_load_u<XCH>(S, a.x, anw, xv, uv, true, status, 1000u + 10u * (l - 1) + 3u);
                 fused_quant_u(S, xv, uv);
             }
             FUSED_STAMP(17);
@@ -524,7 +605,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
                                                                            GU_BPR, lane, xq, d8, s8));
                         if (lane == 0) {
                             const float v = __fmul_rn(acc, ninv);
-                            if (is_attn) a.mxbuf[qa0 + j] = v; else mixv[j] = v;
+                            if (is_attn) xch_put<XCH>(a.mxbuf + qa0 + j, v); else mixv[j] = v;
                         }
                     }
                 }
@@ -536,12 +617,12 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
                         const float bx = __fmul_rn(mixv[tid], mixv[2 * n_dn + tid]);
                         const float conv = fmaf(bx, cv_w2, fmaf(cv_h.y, cv_w1, __fmul_rn(cv_h.x, cv_w0)));
                         *reinterpret_cast<float2 *>(mx.hist + 2 * ch) = make_float2(cv_h.y, bx);
-                        a.mxbuf[ch] = __fmul_rn(mixv[n_dn + tid], conv);
+                        xch_put<XCH>(m_out + ch, __fmul_rn(mixv[n_dn + tid], conv));
                     }
                 }
             }
             FUSED_STAMP(18);
-            grid_arrive(a.bar, S);
+            grid_arrive<!XCH>(a.bar, S, l == 0);
             // ---- M2: one slice of one KV head per CTA; the query heads' norm + rotation are redone by every
             //          slice, the new K / V row is written by the slice that contains it (the last one).  The first groups
             //          of the slice, all but the new row's, are requested before q exists: the staging is idle from here. ----
@@ -559,17 +640,17 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
                     if (warp < AT_GQA) {
                         const float * qh = a.mxbuf + (size_t) (kvh * AT_GQA + warp) * AT_D;
                         float y0, y1;
-                        at_norm_rotate(__ldcg(qh + lane), __ldcg(qh + lane + 32), mx.qnorm, lane, S.sn[lane], S.cs[lane], y0, y1);
+                        at_norm_rotate(xch_get<XCH>(qh + lane, status, S.abort, 1000u + 10u * l + 4u), xch_get<XCH>(qh + lane + 32, status, S.abort, 1000u + 10u * l + 4u), mx.qnorm, lane, S.sn[lane], S.cs[lane], y0, y1);
                         reinterpret_cast<float *>(&A.q[lane])[warp] = y0;
                         reinterpret_cast<float *>(&A.q[lane + 32])[warp] = y1;
                     } else if (warp == AT_GQA && t1 == seq_len) {
                         const float * kh = a.mxbuf + LKB_HIDDEN + (size_t) kvh * AT_D;
                         const float * vh = a.mxbuf + LKB_HIDDEN + AT_KVH * AT_D + (size_t) kvh * AT_D;
                         float y0, y1;
-                        at_norm_rotate(__ldcg(kh + lane), __ldcg(kh + lane + 32), mx.knorm, lane, S.sn[lane], S.cs[lane], y0, y1);
+                        at_norm_rotate(xch_get<XCH>(kh + lane, status, S.abort, 1000u + 10u * l + 4u), xch_get<XCH>(kh + lane + 32, status, S.abort, 1000u + 10u * l + 4u), mx.knorm, lane, S.sn[lane], S.cs[lane], y0, y1);
                         const size_t off = ((size_t) pos * AT_KVH + kvh) * AT_D;
                         kc[off + lane] = __float2half(y0); kc[off + lane + 32] = __float2half(y1);
-                        vc[off + lane] = __float2half(__ldcg(vh + lane)); vc[off + lane + 32] = __float2half(__ldcg(vh + lane + 32));
+                        vc[off + lane] = __float2half(xch_get<XCH>(vh + lane, status, S.abort, 1000u + 10u * l + 4u)); vc[off + lane + 32] = __float2half(xch_get<XCH>(vh + lane + 32, status, S.abort, 1000u + 10u * l + 4u));
                         __threadfence();
                     }
                     __syncthreads();
@@ -582,15 +663,15 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
                 FUSED_STAMP(21);
                 // merge of the slices: one head per CTA (every CTA reading every partial would cost 150 KB of
                 // L2 sectors per CTA), published through mxbuf like a conv output
-                if (cta < AT_HEADS && tid < AT_D) a.mxbuf[cta * AT_D + tid] = at_combine(a.part, cta, tid, seq_len);
-                grid_arrive(a.bar, S);
+                if (cta < AT_HEADS && tid < AT_D) xch_put<XCH>(m_out + cta * AT_D + tid, at_combine(a.part, cta, tid, seq_len));
+                grid_arrive<!XCH>(a.bar, S);
+                if (XCH && warp == 1) { xch_due(a.mxbuf + qa0, lane, qa1 - qa0); xch_due_fence(); }     // q | k | v: read before the partials' barrier
                 if (!grid_wait(a.bar, status, S, 1000u + 10u * l + 7u, a.spin_limit)) return;
                 FUSED_STAMP(25);
             }
             // ---- M3: the mixer's 2048 outputs, written by their owner CTAs, quantised by every CTA; then this CTA's output-projection rows, added to the residual ----
             {
-                const float4 o4 = __ldcg(reinterpret_cast<const float4 *>(a.mxbuf) + tid);
-                const float xo = lane == 0 && warp < n_dn ? __ldcg(a.x + dn0 + warp) : 0.0f;      // the row this warp will update
+                const float4 o4 = xch_get4<XCH>(m_out + 4 * tid, status, S.abort, 1000u + 10u * l + (is_attn ? 7u : 4u));
                 const float o[4] = {o4.x, o4.y, o4.z, o4.w};
                 quad_quant_to_xq(S.xq, o);
                 __syncthreads();
@@ -602,12 +683,13 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
                     if (const int j = warp; j < n_dn) {                     // n_dn <= MAX_DN_ROWS = FUSED_WARPS
                         const float acc = lkb_warp_sum(smem_row_partial<2>(S.dn_q + (size_t) j * GU_BPR * 16, S.dn_d + (size_t) j * GU_BPR,
                                                                            GU_BPR, lane, xq, d8, s8));
-                        if (lane == 0) a.x[dn0 + j] = __fadd_rn(xo, acc);
+                        if (lane == 0) { const float x = __fadd_rn(S.xown[j], acc); S.xown[j] = x; xch_put<XCH>(x_mid + dn0 + j, x); }
                     }
                 }
             }
             FUSED_STAMP(23);
-            grid_arrive(a.bar, S);
+            grid_arrive<!XCH>(a.bar, S);
+            if (XCH && warp == 1) { xch_due(a.x + dn0, lane, n_dn); xch_due_fence(); }        // the residual before the mixer: read before the mixer's first barrier
             if (!grid_wait(a.bar, status, S, 1000u + 10u * l + 6u, a.spin_limit)) return;
             FUSED_STAMP(24);
         }
@@ -617,8 +699,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
         // its own store is the only one this barrier publishes.  Quantising before the arrival put 0.5 us more on each layer.)
         FUSED_STAMP(0);
         float xv[4], uv[4];
-        fused_load_u(S, a.x, nw, xv, uv);
-        const float x_own = tid < n_dn ? __ldcg(a.x + dn0 + tid) : 0.0f;    // the residual rows this CTA will update
+        fused_load_u<XCH>(S, x_mid, nw, xv, uv, MIX || l > 0, status, MIX ? 1000u + 10u * l + 6u : 1000u + 10u * (l - 1) + 3u);
         const float sq = lkb_quad_sum(__fmul_rn(xv[0], xv[0]), __fmul_rn(xv[1], xv[1]), __fmul_rn(xv[2], xv[2]), __fmul_rn(xv[3], xv[3]));
         if ((lane & 7) == 0) S.ssq[tid >> 3] = sq;
         if (pcta && pf_next) {
@@ -648,18 +729,23 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
             }
             if (lane == 0) {
                 S.inv = inv;
-                if (cta < LKB_N_EXPERTS) a.logits[cta] = __fmul_rn(acc, inv);
+                if (cta < LKB_N_EXPERTS) xch_put<XCH>(a.logits + cta, __fmul_rn(acc, inv));
                 if (pcta && pf_next) {
                     float g = 0.0f;
 #pragma unroll
                     for (int w = 0; w < FUSED_WARPS; ++w) g += S.ppart[w];
                     a.gu[PF_LOGITS_OFF + cta - LKB_N_EXPERTS] = g * inv;
                 }
-                grid_arrive_one(a.bar, S);
+                grid_arrive_one<!XCH>(a.bar, S, !MIX && l == 0);
             }
         }
         quad_quant_to_xq(S.xq, uv);
         FUSED_STAMP(2);
+        if (XCH && warp == 1) {                                     // while the barrier completes: read by everyone before the last barrier
+            if (l > 0) xch_due(a.gu + gu0, lane, n_gu);
+            if (MIX) xch_due(m_out + dn0, lane, n_dn);
+            xch_due_fence();
+        }
         // static data of the selection, fetched while the barrier completes
         float rb0 = 0.0f, rb1 = 0.0f;
         if (warp == 0 && ly.rbias) { rb0 = __ldg(ly.rbias + lane); rb1 = __ldg(ly.rbias + lane + 32); }
@@ -675,7 +761,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
             if (warp == 0) {
                 // both logits are requested before either is used: a shared-memory store between two global
                 // loads would serialise them (the compiler cannot prove the pointers distinct)
-                const float lg0 = __ldcg(a.logits + lane), lg1 = __ldcg(a.logits + lane + 32);
+                const float lg0 = xch_get<XCH>(a.logits + lane, status, S.abort, 1000u + 10u * l + 1u), lg1 = xch_get<XCH>(a.logits + lane + 32, status, S.abort, 1000u + 10u * l + 1u);
                 const float g0 = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-lg0)));
                 const float g1 = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-lg1)));
                 S.sig[lane] = g0; S.sig[lane + 32] = g1;
@@ -684,7 +770,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
                 S.key[lane] = lkb_orderable(s0); S.key[lane + 32] = lkb_orderable(s1);
             }
         } else {
-            if (tid < LKB_N_EXPERTS) S.sel[tid] = __ldcg(a.logits + tid);
+            if (tid < LKB_N_EXPERTS) S.sel[tid] = xch_get<XCH>(a.logits + tid, status, S.abort, 1000u + 10u * l + 1u);
             __syncthreads();
             float p = 0.0f;
             if (tid < LKB_N_EXPERTS) {
@@ -797,11 +883,14 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
                     pu = __fadd_rn(pu, __shfl_xor_sync(LKB_FULL, pu, o));
                 }
                 // v = silu(gate) * up of pair gu0 + j (the stand-alone k_swiglu's arithmetic on the two GEMV outputs)
-                if (lane == 0) a.gu[gu0 + j] = __fmul_rn(lkb_silu(__fmul_rn(pg, ninv)), __fmul_rn(pu, ninv));
+                if (lane == 0) xch_put<XCH>(a.gu + gu0 + j, __fmul_rn(lkb_silu(__fmul_rn(pg, ninv)), __fmul_rn(pu, ninv)));
             }
         }
         FUSED_STAMP(5);
-        grid_arrive(a.bar, S);
+        grid_arrive<!XCH>(a.bar, S);
+        if (XCH && warp == 1) {                                     // read before the logits' barrier: the residual that A read
+            xch_due(x_mid + dn0, lane, n_dn); xch_due_fence();
+        }
         // between arrive and wait: the next layer's router row and norm weights (static data)
         if (l + 1 < a.n_layers) {
             if (cta < LKB_N_EXPERTS && tid == 0) {
@@ -880,7 +969,19 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
             // lane; same quants, scale and raw sum as the one-element-per-lane form (lkb_quad_quant)
             float4 v[3];
 #pragma unroll
-            for (int j = 0; j < 3; ++j) v[j] = __ldcg(reinterpret_cast<const float4 *>(a.gu) + (warp + FUSED_WARPS * j) * 32 + lane);
+            for (int j = 0; j < 3; ++j) {
+                const uint4 t = xch_ld4(a.gu + 4 * ((warp + FUSED_WARPS * j) * 32 + lane));
+                v[j] = make_float4(__uint_as_float(t.x), __uint_as_float(t.y), __uint_as_float(t.z), __uint_as_float(t.w));
+            }
+            if (XCH) {
+#pragma unroll 1
+                for (int j = 0; j < 3; ++j) {                        // rare
+                    const float4 t = j == 0 ? v[0] : j == 1 ? v[1] : v[2];
+                    if (!xch_missing(make_uint4(__float_as_uint(t.x), __float_as_uint(t.y), __float_as_uint(t.z), __float_as_uint(t.w)))) continue;
+                    const float4 n = xch_again4(a.gu + 4 * ((warp + FUSED_WARPS * j) * 32 + lane), status, 1000u + 10u * l + 2u, &S.abort);
+                    if (j == 0) v[0] = n; else if (j == 1) v[1] = n; else v[2] = n;
+                }
+            }
             FUSED_STAMP(10);
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
@@ -949,10 +1050,13 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
             float acc = 0.0f;
 #pragma unroll
             for (int k = 0; k < LKB_TOP_K; ++k) acc = fmaf(S.wk[k], S.dot[k][tid], acc);
-            a.x[dn0 + tid] = __fadd_rn(x_own, acc);
+            const float x = __fadd_rn(S.xown[tid], acc);
+            S.xown[tid] = x;
+            xch_put<XCH>(a.x + dn0 + tid, x);
         }
         FUSED_STAMP(7);
-        grid_arrive(a.bar, S);
+        grid_arrive<!XCH>(a.bar, S);
+        if (XCH && warp == 1 && cta < LKB_N_EXPERTS) { xch_due(a.logits + cta, lane, 1); xch_due_fence(); }      // read before the barrier after gate|up
         if (l + 1 < a.n_layers && tid < (int) (sizeof(lkb_moe_layer) / 8))
             reinterpret_cast<unsigned long long *>(&S.ly)[tid] = reinterpret_cast<const unsigned long long *>(&L[l + 1])[tid];
         if (pf && l + 2 < a.n_layers && tid >= 32 && tid < 32 + (int) (sizeof(lkb_moe_layer) / 8))
@@ -972,7 +1076,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
     if (a.final_norm_w && cta == 0) {
         load4(a.final_norm_w, nw);
         float xv[4], uv[4];
-        fused_load_u(S, a.x, nw, xv, uv);
+        fused_load_u<XCH>(S, a.x, nw, xv, uv, true, status, 1000u + 10u * (a.n_layers - 1) + 3u);
         fused_quant_u(S, xv, uv);
 #pragma unroll 1
         for (int i = tid; i < LKB_HIDDEN; i += FUSED_THREADS) if (a.out_h32) a.out_h32[i] = S.h[i];

@@ -1,0 +1,65 @@
+"""The persistent decode kernels' exchange: whatever the caller's scratch holds on entry, whatever NaN the residual holds, and
+wherever the position falls in the groups of the attention slices (the new row's group is requested later than the rest), the
+results are those of the kernel sequence, bit for bit."""
+import importlib
+
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+H = 2048
+
+
+def _fill(t, pattern):
+    t.view(torch.int32).fill_(pattern)
+
+
+@pytest.mark.parametrize("pattern", [0, -1, 0x3F800000], ids=["zeros", "due", "ones"])
+def test_stack_takes_any_scratch(lkb, pattern):
+    lkb.init(0)
+    synth = importlib.import_module("lfm2-ampere_b200.synth")
+    st = importlib.import_module("lfm2-ampere_b200.decode").DecodeStack(synth.make_model(3, seed=19, zipf_s=1.1))
+    x0 = torch.randn(H, device="cuda", generator=torch.Generator("cuda").manual_seed(2))
+    st.x.copy_(x0); st.step(); ref = st.x.clone()
+    for t in (st.gu, st.logits, st.sync):
+        _fill(t, pattern)
+    for _ in range(2):                                     # the second launch finds what the first one left
+        st.x.copy_(x0); st.step_fused(); torch.cuda.synchronize()
+        assert st.status() == 0 and torch.isfinite(ref).all() and torch.equal(st.x, ref)
+
+
+def test_stack_takes_any_nan(lkb):
+    """A residual with the bit pattern that marks words still due: an input, never waited for."""
+    lkb.init(0)
+    synth = importlib.import_module("lfm2-ampere_b200.synth")
+    st = importlib.import_module("lfm2-ampere_b200.decode").DecodeStack(synth.make_model(2, seed=23))
+    st.x.normal_()
+    st.x.view(torch.int32)[77] = -1
+    st.step_fused(); torch.cuda.synchronize()
+    assert st.status() == 0 and torch.isnan(st.x).any()
+
+
+@pytest.mark.parametrize("pos0", [0, 31, 254, 255, 256, 543, 4605])
+def test_step_at_group_edges(lkb, pos0):
+    """4 layers (conv, conv, attention, conv), three steps from pos0 on: one launch for all layers == one launch per kernel."""
+    lkb.init(0)
+    model = importlib.import_module("lfm2-ampere_b200.model")
+    net = model.make_full_model(n_layers=4, seed=7, vocab=4096)
+    out = []
+    for impl in ("kernels", "mega"):
+        ds = model.DecodeStep(net, max_seq=pos0 + 8, moe_impl=impl)
+        if pos0:
+            ds.fill_kv(pos0, 3)
+        ds.d_token.fill_(11)
+        for t in (ds.gu, ds.logits, ds.mxbuf, ds.part) if impl == "mega" else ():
+            _fill(t, 0x3F800000)
+        xs = []
+        for _ in range(3):
+            ds.step(); torch.cuda.synchronize()
+            xs.append(ds.x.clone())
+        assert ds.status() == 0
+        out.append((torch.stack(xs), ds.kc.clone(), ds.vc.clone(), ds.hist.clone(), ds.logits_v.clone()))
+    assert torch.isfinite(out[0][0]).all()
+    for a, b in zip(*out):
+        assert torch.equal(a, b)
