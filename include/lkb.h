@@ -353,7 +353,7 @@ int lkb_pf_gemm_arith(int fold);
 int lkb_pf_gemm_workspace_bytes(int max_tiles, int k_max, size_t * bytes_out);
 int lkb_pf_gemm_set_workspace(void * ptr, size_t bytes);
 /* Every device-side wait of the tensor-core kernels is bounded; this SYNCHRONISES the device and
- * returns 0, or the code of the first wait that expired since the last call (10 producer,
+ * returns 0, or the code of the first wait that expired since the last call (10 producer, 11 / 33 few-token form,
  * 15/16 expansion, 20-22 MMA issuer, 30/31 epilogue; 50-63 the
  * chunk attention) and clears it.  No counterpart in the reference. */
 int lkb_pf_gemm_status(void);

@@ -695,6 +695,8 @@ __global__ void __launch_bounds__(256) k_pf_gemm_simple(const lkb_pf_gemm g, con
 int lkb_gemm_tc_init();                                      // lkb_gemm_tc.cu
 int lkb_gemm_tc_launch(const lkb_pf_gemm * g, int epi, int fold, int max_tiles, cudaStream_t st, float * const * out_rows, int a_pitch);   // LKB_ERR_UNSUPPORTED if shape not covered
 
+int lkb_gemm_few_launch(const lkb_pf_gemm * g, int epi, int fold, int max_tiles, cudaStream_t st);       // lkb_gemm_few.cu: ... or where another form is faster
+
 static int g_gemm_cfg = -1;        // -1: tensor-core form when it covers the shape; 0: CUDA-core form
 static int g_gemm_fold = 1;        // 1: the reference's shipped per-block term (folded offset); 0: the exact term
 
@@ -729,6 +731,10 @@ static int gemm_dispatch(const lkb_pf_gemm * g, int epi, int max_tiles, cudaStre
     if (r != LKB_OK) return r;
     const int ty = g->perm ? max_tiles : (g->ntok + 63) / 64;
     if (ty <= 0) return g->perm ? LKB_ERR_SHAPE : LKB_OK;
+    if (g_gemm_cfg < 0 && !out_rows && !a_pitch) {
+        const int t = lkb_gemm_few_launch(g, epi, g_gemm_fold, max_tiles, st);
+        if (t != LKB_ERR_UNSUPPORTED) return t;
+    }
     if (g_gemm_cfg != 0) {
         const int t = lkb_gemm_tc_launch(g, epi, g_gemm_fold, max_tiles, st, out_rows, a_pitch);
         if (t != LKB_ERR_UNSUPPORTED) return t;
