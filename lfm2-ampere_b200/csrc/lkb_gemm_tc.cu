@@ -95,12 +95,15 @@ __device__ __forceinline__ unsigned long long tc_desc_seed(unsigned smem_addr) {
 // s8 x s8 -> s32, M = 128, N from the item, B K-major
 #define TC_IDESC(n) (0x20u | (1u << 7) | (1u << 10) | (((unsigned) (n) >> 3) << 17) | ((TC_ROWS >> 4) << 24))
 
+// The dense form's items: tokens per item, and two 128-row tiles or one.  tc_dense_form (host) chooses.
+struct TcDense { int tw, wide; };
 // What every role derives from the launch arguments: the shape of the item grid.
 struct TcPlan {
     int n_rt;            // row tiles per token tile
     int n_items;
     int wide;            // plain form: an item is two 128-row tiles (1) or one (0)
     int nstage;          // pipeline stages per item
+    int tw;              // dense: tokens per item
 };
 struct TcItem { int expert, tstart, tcnt, rt; };
 __device__ __forceinline__ TcItem tc_item(const lkb_pf_gemm & g, const TcPlan & P, int item) {
@@ -111,7 +114,7 @@ __device__ __forceinline__ TcItem tc_item(const lkb_pf_gemm & g, const TcPlan & 
         const int4 tl = __ldg(reinterpret_cast<const int4 *>(g.tiles) + mt);
         I.expert = tl.x; I.tstart = tl.y; I.tcnt = tl.z;
     } else {
-        I.expert = 0; I.tstart = mt * TC_TOK; I.tcnt = min(TC_TOK, g.ntok - I.tstart);
+        I.expert = 0; I.tstart = mt * P.tw; I.tcnt = min(P.tw, g.ntok - I.tstart);
     }
     return I;
 }
@@ -413,7 +416,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_pf_gemm_tc(const lkb_pf_gemm 
                                                               const __grid_constant__ CUtensorMap map_d0,
                                                               const __grid_constant__ CUtensorMap map_d1,
                                                               const __grid_constant__ CUtensorMap map_d2,
-                                                              float * const * __restrict__ out_rows) {
+                                                              float * const * __restrict__ out_rows, const TcDense dense) {
     lkb_pdl_wait(); lkb_pdl_trigger();           // programmatic dependent launch: inputs complete from here on
     extern __shared__ unsigned char tc_smem_raw[];
     // the swizzle patterns are functions of the shared-memory address: stages start on 1024-byte boundaries
@@ -422,12 +425,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_pf_gemm_tc(const lkb_pf_gemm 
 
     // ---- item grid: (token tile, row tile), row tiles fastest --------------------
     TcPlan P;
-    const int n_mt = g.perm ? min(*g.ntiles, max_tiles) : (g.ntok + TC_TOK - 1) / TC_TOK;
+    P.tw = dense.tw;
+    const int n_mt = g.perm ? min(*g.ntiles, max_tiles) : (g.ntok + P.tw - 1) / P.tw;
     P.wide = 1;
     P.n_rt = EPI ? (g.N + TC_ROWS - 1) / TC_ROWS : (g.N + 2 * TC_ROWS - 1) / (2 * TC_ROWS);
-    // A problem with no more 128-row tiles than CTAs (the dense projections of a short prompt) takes them one per item:
-    // an item's time there is the latency of its chain of blocks, and twice the CTAs share the weight stream.
-    if (!EPI && n_mt * (g.N / TC_ROWS) <= (int) gridDim.x) { P.wide = 0; P.n_rt = g.N / TC_ROWS; }
+    // No more 128-row tiles than CTAs: one per item.  An item's time there is the latency of its chain of blocks, and twice the CTAs
+    // share the weight stream.
+    if (!EPI && (g.perm ? n_mt * (g.N / TC_ROWS) <= (int) gridDim.x : !dense.wide)) { P.wide = 0; P.n_rt = g.N / TC_ROWS; }
     P.n_items = n_mt * P.n_rt;
     P.nstage = g.bpr / TC_KB;
     if ((int) blockIdx.x >= P.n_items) return;
@@ -737,7 +741,7 @@ int lkb_gemm_few_init();                   // lkb_gemm_few.cu
 int lkb_gemm_few_take_status();
 
 typedef void (*TcKernel)(lkb_pf_gemm, int, int, const char *, int, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap,
-                         CUtensorMap, float * const *);
+                         CUtensorMap, float * const *, TcDense);
 static TcKernel const TC_FORMS[8] = {               // 4 epi + 2 fold + weight scales by tensor copy
     k_pf_gemm_tc<0, 0, 0>, k_pf_gemm_tc<0, 0, 1>, k_pf_gemm_tc<0, 1, 0>, k_pf_gemm_tc<0, 1, 1>,
     k_pf_gemm_tc<1, 0, 0>, k_pf_gemm_tc<1, 0, 1>, k_pf_gemm_tc<1, 1, 0>, k_pf_gemm_tc<1, 1, 1>};
@@ -776,6 +780,24 @@ int lkb_tc_make_map(CUtensorMap * m, const void * base, unsigned row_bytes, unsi
 }
 #define TC_ANY_ROWS (1ull << 30)            // row bound of a plane whose extent the caller does not state: it only clips
 
+// Items of a dense problem: the token width and height that need the least time, waves of items times an item's.  A block of an item
+// takes about 330 + 6 N cycles with one tile and 350 + 6.2 N with two (measured, N = 16 .. 64), so a problem of less than a wave is
+// cut into narrow items (each reads the weights again, from L2), and one that would leave most of its last wave empty is cut
+// so that the waves fill.  us with 64-token items and with these, caches flushed: in_proj (6144 rows) at 37 / 130 / 509 tokens
+// 22.5 / 26.6 / 51.2 -> 19.5 / 24.6 / 45.0, out_proj (2048 rows) 24.6 / 26.6 / 28.7 -> 18.4 / 20.5 / 26.6; at 4096 tokens the
+// choice is 64 x 256 as before.
+static TcDense tc_dense_form(int ntok, int N, int sms) {
+    TcDense best = {TC_TOK, 1};
+    long long least = 0;
+    for (int wide = 1; wide >= 0; --wide)
+        for (int tw = TC_TOK; tw >= 16; tw -= 16) {
+            const long long items = (long long) ((ntok + tw - 1) / tw) * ((N + (wide ? 2 : 1) * TC_ROWS - 1) / ((wide ? 2 : 1) * TC_ROWS));
+            const long long t = (items + sms - 1) / sms * (wide ? 3500 + 62 * tw : 3300 + 60 * tw);
+            if (!least || t < least) { least = t; best = {tw, wide}; }
+        }
+    return best;
+}
+
 // Shapes the tensor-core form covers; otherwise LKB_ERR_UNSUPPORTED (the caller falls back to the CUDA-core form): the
 // planes must have the alignment the copies ask for.
 int lkb_gemm_tc_launch(const lkb_pf_gemm * g, int epi, int fold, int max_tiles, cudaStream_t st, float * const * out_rows, int a_pitch) {
@@ -811,7 +833,7 @@ int lkb_gemm_tc_launch(const lkb_pf_gemm * g, int epi, int fold, int max_tiles, 
     const dim3 grid(lkb_context().sm_count), block(TC_THREADS);
     const size_t sm = sizeof(TcSmem) + 1024;
     LKB_PF_LAUNCH(TC_FORMS[(epi ? 4 : 0) + (fold ? 2 : 0) + wcopy], grid, block, sm, st, *g, max_tiles, rpe, sc_plane, s_pitch, ma, mw[0], mw[1], mw[2],
-                  md[0], md[1], md[2], out_rows);
+                  md[0], md[1], md[2], out_rows, g->perm ? TcDense{TC_TOK, 1} : tc_dense_form(g->ntok, g->N, lkb_context().sm_count));
     return lkb_check_launch();
 }
 
