@@ -208,33 +208,20 @@ __global__ void __launch_bounds__(256) k_pf_router_token(const float * __restric
 // rows are conflict-free); the multiply loop reads four k-values per load.  With TPT = 4 a warp spends 16 wavefronts
 // (4 loads of router rows, 4 of token rows shared by half a warp) on 64 FMA instructions: the ratio at which the FMA
 // pipes rather than shared memory set the pace.  One CTA barrier per tile.
-#ifndef RT_KT
-#define RT_KT     64                          // measured on B200, 4096 tokens: 32 -> 66 us, 64 -> 55 us, 128 (4 stages) -> 72 us
-#endif
-#define RT_PITCH  (RT_KT + 4)
-#define RT_CPR    (RT_KT / 4)                 // 16-byte copies per staged row
-#ifndef RT_STAGES
-#define RT_STAGES 6
-#endif
-#ifndef RT_L_TPT
-#define RT_L_TPT 4          // long form: 4 warps, 32 tokens per CTA (measured on B200 at 4096 tokens, 32-wide k-tiles: 66 us; 8 warps x 2 tokens 74 us,
-#define RT_L_NW  4          // 8 warps x 4 tokens 94 us, 4 warps x 2 tokens 76 us; the k loop of one CTA is the critical path)
-#endif
-#ifndef RT_S_TPT
-#define RT_S_TPT 2          // middle form: 4 warps, 16 tokens per CTA
-#define RT_S_NW  4
-#endif
+// A tile holds KT k-values, the ring STAGES of them: what a tile costs beside its FMAs (a barrier, the copies' issue) is paid
+// less often with wide tiles, which small CTAs have the shared memory for (see router_tiled).
 __device__ __forceinline__ void rt_cp16(float * dst, const float * src, bool live) {
     const unsigned d = (unsigned) __cvta_generic_to_shared(dst);
     const int n = live ? 16 : 0;                          // 0: the 16 bytes are zero-filled, nothing is read
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(d), "l"(src), "r"(n) : "memory");
 }
-template <int TPT, int NW>
+template <int TPT, int NW, int RT_KT, int RT_STAGES>
 __global__ void __launch_bounds__(32 * NW) k_pf_router_pipe(const float * __restrict__ H, int m, const float * __restrict__ Wr,
                                                         const float * __restrict__ bias, const float * __restrict__ inv,
                                                         float * __restrict__ sel, float * __restrict__ sig,
                                                         int4 * __restrict__ idx, float4 * __restrict__ wout) {
     lkb_pdl_wait(); lkb_pdl_trigger();           // programmatic dependent launch: inputs complete from here on
+    constexpr int RT_PITCH = RT_KT + 4, RT_CPR = RT_KT / 4;            // floats and 16-byte copies per staged row
     constexpr int TT = 2 * NW * TPT, ROWS = TT + LKB_N_EXPERTS, NTILES = LKB_HIDDEN / RT_KT;
     extern __shared__ __align__(16) float rt_ring[];                   // [RT_STAGES][ROWS][RT_PITCH]
     const int tid = threadIdx.x, te = tid & 15, tg = tid >> 4;
@@ -330,19 +317,19 @@ __global__ void __launch_bounds__(32 * NW) k_pf_router_pipe(const float * __rest
         }
     }
 }
-template <int TPT, int NW>
+template <int TPT, int NW, int KT, int STAGES>
 static int rt_launch(const float * H, int m, const float * Wr, const float * bias, const float * inv, float * sel, float * sig,
                      int * idx, float * w, cudaStream_t st) {
     constexpr int TT = 2 * NW * TPT;
-    constexpr size_t smem = (size_t) RT_STAGES * (TT + LKB_N_EXPERTS) * RT_PITCH * sizeof(float);
+    constexpr size_t smem = (size_t) STAGES * (TT + LKB_N_EXPERTS) * (KT + 4) * sizeof(float);
     static int ready[LKB_STATIC_MAX_DEVICES] = {0};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < LKB_STATIC_MAX_DEVICES && !ready[dev]) {
-        if (cudaFuncSetAttribute(k_pf_router_pipe<TPT, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem) != cudaSuccess) return -(int) cudaGetLastError();
+        if (cudaFuncSetAttribute(k_pf_router_pipe<TPT, NW, KT, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem) != cudaSuccess) return -(int) cudaGetLastError();
         ready[dev] = 1;
     }
-    LKB_PF_LAUNCH((k_pf_router_pipe<TPT, NW>), dim3((m + TT - 1) / TT), dim3(32 * NW), smem, st, H, m, Wr, bias, inv, sel, sig,
+    LKB_PF_LAUNCH((k_pf_router_pipe<TPT, NW, KT, STAGES>), dim3((m + TT - 1) / TT), dim3(32 * NW), smem, st, H, m, Wr, bias, inv, sel, sig,
                   reinterpret_cast<int4 *>(idx), reinterpret_cast<float4 *>(w));
     return lkb_check_launch();
 }
@@ -798,15 +785,19 @@ static int router_tiled(const float * H, int m, const float * Wr, const float * 
     LKB_REQUIRE_INIT();
     if (!H || !Wr || !bias || !inv || !sel || !sig) return LKB_ERR_NULL;
     if (m <= 0) return m == 0 ? LKB_OK : LKB_ERR_SHAPE;
-    // The k loop of one CTA is the critical path and its length grows with the tokens per thread, so a token range takes
-    // the smallest CTA shape that still fits one wave (measured on B200, us: 8-token CTAs 36 up to 1184 tokens, 66 at 2048;
-    // 16-token CTAs 43 up to 2368, 68-78 at 4096; 32-token CTAs 55 at any size up to 4736).  A rank's share of an
-    // expert-parallel chunk lands in the first two.  LKB_ROUTER_FORM = 8 / 16 / 32 forces a shape (tuning).
+    // The k loop of one CTA is the critical path and its length grows with the tokens per CTA, so a token range takes the smallest
+    // CTA that still fits one wave.  Measured on B200, us (tiles of 64 k-values, six stages -> of 128, four stages):
+    //   4-token CTAs (two warps)  up to 592 tokens   31.7 -> 21.0   (8-token CTAs there: 32.3)
+    //   8-token CTAs              up to 1184         32.4 -> 29.1
+    //   16-token CTAs             up to 2368         36.5 -> 35.3
+    //   32-token CTAs             at 4096            53.3 -> 69.5: keeps 64
+    // A rank's share of an expert-parallel chunk lands in the first three.  LKB_ROUTER_FORM = 4 / 8 / 16 / 32 forces a shape (tuning).
     static const int form = [] { const char * e = getenv("LKB_ROUTER_FORM"); return e ? atoi(e) : 0; }();
     const int sms = lkb_context().sm_count;
-    if (form == 8 || (form == 0 && m <= 8 * sms)) return rt_launch<1, 4>(H, m, Wr, bias, inv, sel, sig, idx, w, (cudaStream_t) st);
-    if (form == 16 || (form == 0 && m <= 16 * sms)) return rt_launch<RT_S_TPT, RT_S_NW>(H, m, Wr, bias, inv, sel, sig, idx, w, (cudaStream_t) st);
-    return rt_launch<RT_L_TPT, RT_L_NW>(H, m, Wr, bias, inv, sel, sig, idx, w, (cudaStream_t) st);
+    if (form == 4 || (form == 0 && m <= 4 * sms)) return rt_launch<1, 2, 128, 4>(H, m, Wr, bias, inv, sel, sig, idx, w, (cudaStream_t) st);
+    if (form == 8 || (form == 0 && m <= 8 * sms)) return rt_launch<1, 4, 128, 4>(H, m, Wr, bias, inv, sel, sig, idx, w, (cudaStream_t) st);
+    if (form == 16 || (form == 0 && m <= 16 * sms)) return rt_launch<2, 4, 128, 4>(H, m, Wr, bias, inv, sel, sig, idx, w, (cudaStream_t) st);
+    return rt_launch<4, 4, 64, 6>(H, m, Wr, bias, inv, sel, sig, idx, w, (cudaStream_t) st);
 }
 
 int lkb_pf_router_small(const float * H, int m, const float * Wr, const float * bias, const float * inv,
