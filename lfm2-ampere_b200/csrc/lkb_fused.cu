@@ -343,12 +343,18 @@ __device__ __forceinline__ void load4(const float * __restrict__ p, float (&o)[4
     o[0] = t.x; o[1] = t.y; o[2] = t.z; o[3] = t.w;
 }
 // Q8_1 of the block this lane's group of 8 holds -> S.xq[tid >> 3]
+// (Out of line, as the requests of the mixers' rows: a layer is straight-line code that every warp runs once, and the whole-step kernel
+// is larger than the instruction cache.  Four call sites: 130 -> 121 KB, two tokens at context 131000 2760 -> 2720 us.)
+__device__ __noinline__ uint2 quad_quant(float4 v) {
+    __half2 ds;
+    const unsigned pk = lkb_quad_quant_ds(v, ds);
+    return make_uint2(pk, *reinterpret_cast<const unsigned *>(&ds));
+}
 __device__ __forceinline__ void quad_quant_to_xq(lkb_q8blk * xq, const float (&v)[4]) {
     const int b = threadIdx.x >> 3, l8 = threadIdx.x & 7;
-    __half2 ds;
-    const unsigned pk = lkb_quad_quant_ds(make_float4(v[0], v[1], v[2], v[3]), ds);
-    reinterpret_cast<unsigned *>(xq[b].qs)[l8] = pk;
-    if (l8 == 0) xq[b].ds = ds;
+    const uint2 q = quad_quant(make_float4(v[0], v[1], v[2], v[3]));
+    reinterpret_cast<unsigned *>(xq[b].qs)[l8] = q.x;
+    if (l8 == 0) *reinterpret_cast<unsigned *>(&xq[b].ds) = q.y;
 }
 
 struct FusedArgs {
@@ -417,7 +423,7 @@ static_assert(sizeof(AtSmem2) <= offsetof(FusedSmem, router), "attention staging
 
 // One thread: request this CTA's mixer input rows.  Conv: channels [dn0, dn0+n_dn) of B, C and X (rows ch,
 // 2048+ch, 4096+ch of in_proj) -> staged rows s*n_dn + j.  Attention: logical rows [a0, a1) of q | k | v.
-__device__ __forceinline__ void mix_issue_in(FusedSmem & S, const lkb_mixer_layer & mx, int dn0, int n_dn, int a0, int a1) {
+__device__ __noinline__ void mix_issue_in(FusedSmem & S, const lkb_mixer_layer & mx, int dn0, int n_dn, int a0, int a1) {
     fence_proxy_async();
     if (!mx.is_attn) {
         mbar_expect_tx(&S.mbar_mi, 3u * (unsigned) n_dn * GU_BPR * 18u);
@@ -446,7 +452,7 @@ __device__ __forceinline__ void mix_issue_in(FusedSmem & S, const lkb_mixer_laye
     }
 }
 // One thread: request this CTA's rows [dn0, dn0+n_dn) of the mixer's output projection.
-__device__ __forceinline__ void mix_issue_out(FusedSmem & S, const lkb_mixer_layer & mx, int dn0, int n_dn) {
+__device__ __noinline__ void mix_issue_out(FusedSmem & S, const lkb_mixer_layer & mx, int dn0, int n_dn) {
     fence_proxy_async();
     mbar_expect_tx(&S.mbar_mo, (unsigned) n_dn * GU_BPR * 18u);
     bulk_g2s(S.dn_q, (const uint4 *) mx.out_qs + (size_t) dn0 * GU_BPR, (unsigned) n_dn * GU_BPR * 16u, &S.mbar_mo);
@@ -757,7 +763,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
         // the guessed logits of the next layer: requested here, used by warp 1 once the gate|up rows are done
         if (pf_next && warp == 1) { plg0 = __ldcg(a.gu + PF_LOGITS_OFF + lane); plg1 = __ldcg(a.gu + PF_LOGITS_OFF + lane + 32); }
         // ---- C: selection (every CTA, warp 0; the softmax gate takes the 64-thread path) ----
-        if (!a.softmax) {
+        if (MIX || !a.softmax) {                                    // (lkb_decode_layers has the sigmoid gate)
             if (warp == 0) {
                 // both logits are requested before either is used: a shared-memory store between two global
                 // loads would serialise them (the compiler cannot prove the pointers distinct)
