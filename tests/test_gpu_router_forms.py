@@ -1,0 +1,23 @@
+"""The tiled router's CTA shapes at their edges: token counts around a CTA's four, eight and sixteen tokens and around the counts at
+which the launcher goes to the next shape, against one chunk in the largest shape, bit for bit (every logit is the same chain)."""
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+def test_pieces_of_every_shape_equal_one_chunk(lkb):
+    lkb.init(0)
+    sms = lkb.lib.lkb_sm_count()
+    m = 16 * sms + 1                                                 # 32-token CTAs
+    gen = torch.Generator("cuda").manual_seed(31)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    H, W, bias, inv = rnd(m, 2048), 0.03 * rnd(64, 2048), 0.1 * rnd(64), 0.5 + torch.rand(m, device="cuda", generator=gen)
+    out = lambda n: (torch.full((n, 64), float("nan"), device="cuda"), torch.full((n, 64), float("nan"), device="cuda"))
+    sel, sig = out(m)
+    lkb.k_pf_router_tiled(H, m, W, bias, inv, sel, sig)
+    assert bool(torch.isfinite(sel).all())
+    for n in (1, 3, 4, 5, 7, 8, 9, 4 * sms, 4 * sms + 1, 8 * sms, 8 * sms + 1, 16 * sms):
+        sel2, sig2 = out(n)
+        lkb.k_pf_router_tiled(H, n, W, bias, inv, sel2, sig2)
+        assert torch.equal(sel2, sel[:n]) and torch.equal(sig2, sig[:n]), n
