@@ -198,6 +198,49 @@ __global__ void __launch_bounds__(256) k_pf_router_token(const float * __restric
     }
 }
 
+// The same for fewer tokens still: a cluster of eight CTAs per token, a warp per expert.  The selection needs all 64 logits: they meet in
+// the shared memory of the cluster's first CTA.  Bound by the latency of a warp's two rows; see router_small for where it pays.
+#define RC_CTAS 8
+__global__ void __cluster_dims__(RC_CTAS, 1, 1) __launch_bounds__(256) k_pf_router_cluster(const float * __restrict__ H, const float * __restrict__ Wr,
+                                                         const float * __restrict__ bias, const float * __restrict__ inv,
+                                                         float * __restrict__ sel, float * __restrict__ sig,
+                                                         int4 * __restrict__ idx, float4 * __restrict__ wout) {
+    lkb_pdl_wait(); lkb_pdl_trigger();           // programmatic dependent launch: inputs complete from here on
+    __shared__ float s_sel[LKB_N_EXPERTS], s_sig[LKB_N_EXPERTS];
+    if (idx) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");       // the first CTA runs before its memory is written
+    const int t = blockIdx.x / RC_CTAS, rank = blockIdx.x % RC_CTAS, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, e = rank * 8 + warp;
+    const float * h = H + (size_t) t * LKB_HIDDEN, * row = Wr + (size_t) e * LKB_HIDDEN;
+    float acc = 0.0f;
+#pragma unroll
+    for (int j = 0; j < LKB_HIDDEN / 32; ++j) acc = fmaf(__ldg(row + j * 32 + lane), h[j * 32 + lane], acc);
+    acc = lkb_warp_sum(acc);
+    if (idx) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    if (lane == 0) {
+        const float l = __fmul_rn(acc, inv[t]);
+        const float gv = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-l)));
+        const float sv = __fadd_rn(gv, bias[e]);
+        sig[(size_t) t * 64 + e] = gv;
+        sel[(size_t) t * 64 + e] = sv;
+        if (idx) {
+            unsigned a, b;
+            asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"((unsigned) __cvta_generic_to_shared(&s_sig[e])));
+            asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(b) : "r"((unsigned) __cvta_generic_to_shared(&s_sel[e])));
+            asm volatile("st.shared::cluster.f32 [%0], %1;" :: "r"(a), "f"(gv) : "memory");
+            asm volatile("st.shared::cluster.f32 [%0], %1;" :: "r"(b), "f"(sv) : "memory");
+        }
+    }
+    if (idx) {                                             // the selection in the same launch (lkb_pf_select's result)
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (rank == 0 && warp == 0) {
+            int ord[LKB_TOP_K]; float wv[LKB_TOP_K];
+            lkb_router_select(s_sel, s_sig, lane, ord, wv);
+            if (lane == 0) { idx[t] = make_int4(ord[0], ord[1], ord[2], ord[3]); wout[t] = make_float4(wv[0], wv[1], wv[2], wv[3]); }
+        }
+    }
+}
+
 // Tiled form.  Each (token, expert) logit is one FMA chain over k = 0..2047 ascending (reference semantics:
 // src/prefill.cu:1606-1666, same per-logit order), so a CTA runs a long sequential k loop and the kernel is bound by
 // (a) how well the loads of the next k-tiles hide behind the FMAs of the current one and (b) how many FMAs each
@@ -775,6 +818,14 @@ static int router_small(const float * H, int m, const float * Wr, const float * 
     if (!H || !Wr || !bias || !inv || !sel || !sig) return LKB_ERR_NULL;
     if (m <= 0) return m == 0 ? LKB_OK : LKB_ERR_SHAPE;
     if (m > 65535) return LKB_ERR_SHAPE;
+    // A cluster of CTAs a token while that is about a wave: a MoE layer at 2 / 9 / 37 / 64 / 100 tokens 47 / 63 / 114 / 152 / 155 -> 41 / 58 / 109 /
+    // 146 / 150 us; at 180 equal, at 256 182 -> 186.
+    constexpr int MAX_CLUSTERS = 160;
+    if (m <= MAX_CLUSTERS) {
+        LKB_PF_LAUNCH(k_pf_router_cluster, dim3(m * RC_CTAS), dim3(256), 0, (cudaStream_t) st, H, Wr, bias, inv, sel, sig,
+                      reinterpret_cast<int4 *>(idx), reinterpret_cast<float4 *>(w));
+        return lkb_check_launch();
+    }
     LKB_PF_LAUNCH(k_pf_router_token, dim3(m), dim3(256), 0, (cudaStream_t) st, H, Wr, bias, inv, sel, sig,
                   reinterpret_cast<int4 *>(idx), reinterpret_cast<float4 *>(w));
     return lkb_check_launch();

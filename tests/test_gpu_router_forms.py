@@ -21,3 +21,23 @@ def test_pieces_of_every_shape_equal_one_chunk(lkb):
         sel2, sig2 = out(n)
         lkb.k_pf_router_tiled(H, n, W, bias, inv, sel2, sig2)
         assert torch.equal(sel2, sel[:n]) and torch.equal(sig2, sig[:n]), n
+
+
+def test_cluster_form_equals_token_form(lkb):
+    """The short router's two forms, alone and with the selection in the launch, around the count at which the launcher changes."""
+    lkb.init(0)
+    m, gen = 256, torch.Generator("cuda").manual_seed(32)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    H, W, bias, inv = rnd(m, 2048), 0.03 * rnd(64, 2048), 0.1 * rnd(64), 0.5 + torch.rand(m, device="cuda", generator=gen)
+    new = lambda n: [torch.full((n, 64), float("nan"), device="cuda") for _ in range(2)] + [torch.full((n, 4), -1, dtype=torch.int32, device="cuda"),
+                                                                                         torch.full((n, 4), float("nan"), device="cuda")]
+    ref = new(m)
+    lkb.k_pf_router_select(H, m, True, W, bias, inv, *ref)                # 256 tokens: a CTA per token
+    assert all(bool(torch.isfinite(t.float()).all()) for t in ref) and int(ref[2].min()) >= 0
+    for n in (1, 2, 37, 159, 160, 161):
+        got = new(n)
+        lkb.k_pf_router_select(H, n, True, W, bias, inv, *got)
+        assert all(torch.equal(a, b[:n]) for a, b in zip(got, ref)), n
+        alone = new(n)
+        lkb.k_pf_router_small(H, n, W, bias, inv, alone[0], alone[1])
+        assert torch.equal(alone[0], ref[0][:n]) and torch.equal(alone[1], ref[1][:n]), n
