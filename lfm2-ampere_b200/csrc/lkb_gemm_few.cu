@@ -222,7 +222,7 @@ __global__ void __launch_bounds__((FW_WARPS + 1) * 32, FW_CTAS) k_pf_gemm_few(co
 
 // ---------------------------------------------------------------------------
 int lkb_tc_make_map(CUtensorMap * m, const void * base, unsigned row_bytes, unsigned long long pitch, unsigned long long rows,
-                    unsigned box_bytes, unsigned box_rows, CUtensorMapSwizzle sw);           // lkb_gemm_tc.cu
+                    unsigned box_bytes, unsigned box_rows, CUtensorMapSwizzle sw, CUtensorMapL2promotion l2);           // lkb_gemm_tc.cu
 
 typedef void (*FwKernel)(lkb_pf_gemm, int, int, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap);
 static FwKernel const FW_FORMS[4] = {k_pf_gemm_few<0, 0>, k_pf_gemm_few<0, 1>, k_pf_gemm_few<1, 0>, k_pf_gemm_few<1, 1>};      // 2 epi + fold
@@ -244,15 +244,17 @@ int lkb_gemm_few_launch(const lkb_pf_gemm * g, int epi, int fold, int max_tiles,
     if (g->bpr % 8 || (((size_t) g->aqs | (size_t) g->asc) & 15) || g->exp_stride % g->bpr) return LKB_ERR_UNSUPPORTED;
     const int nseg = epi ? 2 : (g->seg_end[0] >= g->N ? 1 : g->seg_end[1] >= g->N ? 2 : 3);
     for (int s = 0; s < nseg; ++s) if (((size_t) g->qs[s] | (size_t) g->d[s]) & 15) return LKB_ERR_UNSUPPORTED;
+    // a stage takes 64 bytes of a row; fetched 256 at a time by L2: 57 against 69 us for gate|up at 37 tokens
+    const CUtensorMapL2promotion l2 = CU_TENSOR_MAP_L2_PROMOTION_L2_256B;
     const unsigned long long any = 1ull << 30;              // row bound of a plane whose extent the caller does not state: it only clips
     CUtensorMap ma, ms, mw[3], md[3];
     const unsigned long long rows = g->perm ? any : (unsigned long long) g->ntok;
-    int r = lkb_tc_make_map(&ma, g->aqs, (unsigned) g->bpr * 32u, (unsigned) g->bpr * 32u, rows, FW_KB * 32u, 1u, CU_TENSOR_MAP_SWIZZLE_NONE);
-    if (r == LKB_OK) r = lkb_tc_make_map(&ms, g->asc, (unsigned) g->bpr * 8u, (unsigned) g->bpr * 8u, rows, FW_KB * 8u, 1u, CU_TENSOR_MAP_SWIZZLE_NONE);
+    int r = lkb_tc_make_map(&ma, g->aqs, (unsigned) g->bpr * 32u, (unsigned) g->bpr * 32u, rows, FW_KB * 32u, 1u, CU_TENSOR_MAP_SWIZZLE_NONE, l2);
+    if (r == LKB_OK) r = lkb_tc_make_map(&ms, g->asc, (unsigned) g->bpr * 8u, (unsigned) g->bpr * 8u, rows, FW_KB * 8u, 1u, CU_TENSOR_MAP_SWIZZLE_NONE, l2);
     for (int s = 0; s < 3 && r == LKB_OK; ++s) {
         const int src = s < nseg ? s : 0;
-        r = lkb_tc_make_map(&mw[s], g->qs[src], (unsigned) g->bpr * 16u, (unsigned) g->bpr * 16u, any, 64u, FW_ROWS, CU_TENSOR_MAP_SWIZZLE_64B);
-        if (r == LKB_OK) r = lkb_tc_make_map(&md[s], g->d[src], (unsigned) g->bpr * 2u, (unsigned) g->bpr * 2u, any, 16u, FW_ROWS, CU_TENSOR_MAP_SWIZZLE_NONE);
+        r = lkb_tc_make_map(&mw[s], g->qs[src], (unsigned) g->bpr * 16u, (unsigned) g->bpr * 16u, any, 64u, FW_ROWS, CU_TENSOR_MAP_SWIZZLE_64B, l2);
+        if (r == LKB_OK) r = lkb_tc_make_map(&md[s], g->d[src], (unsigned) g->bpr * 2u, (unsigned) g->bpr * 2u, any, 16u, FW_ROWS, CU_TENSOR_MAP_SWIZZLE_NONE, l2);
     }
     if (r != LKB_OK) return r;
     const dim3 grid(lkb_context().sm_count * FW_CTAS), block((FW_WARPS + 1) * 32);

@@ -768,13 +768,13 @@ int lkb_gemm_tc_init() {
 // A byte matrix [rows][row_bytes], rows `pitch` bytes apart, as a 2-D tensor; box = box_bytes x box_rows.  Rows past `rows`
 // read as zero.
 int lkb_tc_make_map(CUtensorMap * m, const void * base, unsigned row_bytes, unsigned long long pitch, unsigned long long rows,
-                       unsigned box_bytes, unsigned box_rows, CUtensorMapSwizzle sw) {
+                       unsigned box_bytes, unsigned box_rows, CUtensorMapSwizzle sw, CUtensorMapL2promotion l2) {
     const cuuint64_t dims[2] = {row_bytes, rows};
     const cuuint64_t strides[1] = {pitch};
     const cuuint32_t box[2] = {box_bytes, box_rows};
     const cuuint32_t es[2] = {1, 1};
     const CUresult r = g_tc_encode(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(base), dims, strides, box, es,
-                                   CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                   CU_TENSOR_MAP_INTERLEAVE_NONE, sw, l2,
                                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? LKB_OK : LKB_ERR_UNSUPPORTED;
 }
@@ -813,8 +813,8 @@ int lkb_gemm_tc_launch(const lkb_pf_gemm * g, int epi, int fold, int max_tiles, 
     CUtensorMap ma, mw[3], md[3];
     // dense: 16-token boxes of consecutive rows; grouped: rows gathered through perm, four per copy.  Packed rows
     // (a_pitch, as the expert-parallel dispatch delivers them): quants first, then the (d8, 8sum) pairs.
-    int r = g->perm ? lkb_tc_make_map(&ma, g->aqs, qrow, a_pitch ? (unsigned) a_pitch : qrow, TC_ANY_ROWS, 128u, 1u, CU_TENSOR_MAP_SWIZZLE_128B)
-                    : lkb_tc_make_map(&ma, g->aqs, qrow, qrow, (unsigned long long) g->ntok, 128u, 16u, CU_TENSOR_MAP_SWIZZLE_128B);
+    int r = g->perm ? lkb_tc_make_map(&ma, g->aqs, qrow, a_pitch ? (unsigned) a_pitch : qrow, TC_ANY_ROWS, 128u, 1u, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B)
+                    : lkb_tc_make_map(&ma, g->aqs, qrow, qrow, (unsigned long long) g->ntok, 128u, 16u, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
     if (r != LKB_OK) return r;
     const char * sc_plane = a_pitch ? (const char *) g->aqs + qrow : (const char *) g->asc;
     const int s_pitch = a_pitch ? a_pitch : g->bpr * 8;
@@ -823,10 +823,10 @@ int lkb_gemm_tc_launch(const lkb_pf_gemm * g, int epi, int fold, int max_tiles, 
     for (int s = 0; s < 3; ++s) {
         const int src = s < nseg ? s : 0;
         if (((size_t) g->qs[src] & 15) || ((size_t) g->d[src] & 7)) return LKB_ERR_UNSUPPORTED;
-        r = lkb_tc_make_map(&mw[s], g->qs[src], (unsigned) g->bpr * 16u, (unsigned) g->bpr * 16u, TC_ANY_ROWS, 64u, box_rows, CU_TENSOR_MAP_SWIZZLE_64B);
+        r = lkb_tc_make_map(&mw[s], g->qs[src], (unsigned) g->bpr * 16u, (unsigned) g->bpr * 16u, TC_ANY_ROWS, 64u, box_rows, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
         if (r != LKB_OK) return r;
         md[s] = mw[s];                                                          // (not by tensor copy: never used)
-        if (wcopy) r = lkb_tc_make_map(&md[s], g->d[src], (unsigned) g->bpr * 2u, (unsigned) g->bpr * 2u, TC_ANY_ROWS, 16u, box_rows, CU_TENSOR_MAP_SWIZZLE_NONE);
+        if (wcopy) r = lkb_tc_make_map(&md[s], g->d[src], (unsigned) g->bpr * 2u, (unsigned) g->bpr * 2u, TC_ANY_ROWS, 16u, box_rows, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
         if (r != LKB_OK) return r;
     }
     const int rpe = (int) (g->exp_stride / g->bpr);
