@@ -87,3 +87,21 @@ def test_swiglu(L, orc, I, bpr):
         got.append((oqs, osc))
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
     assert int(got[1][0].float().abs().max()) > 0
+
+
+@pytest.mark.parametrize("m", [3, 20, 60])
+def test_short_stack_replays_from_a_graph(lkb, m):
+    """A short chunk through the MoE stack (few-token GEMMs up to 47 tokens, clustered router): a captured step replays to the
+    residual of an eager one, bit for bit."""
+    import importlib
+    lkb.init(0)
+    ps = importlib.import_module("lfm2-ampere_b200.prefill").PrefillStack(importlib.import_module("lfm2-ampere_b200.synth").make_model(2, seed=41, zipf_s=0.7), m)
+    x0 = torch.randn(m, 2048, device="cuda", generator=torch.Generator("cuda").manual_seed(9))
+    ps.X.copy_(x0); ps.step(); torch.cuda.synchronize()
+    ref = ps.X.clone()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        ps.step()
+    for _ in range(2):
+        ps.X.copy_(x0); g.replay(); torch.cuda.synchronize()
+        assert torch.isfinite(ref).all() and torch.equal(ps.X, ref)
