@@ -39,6 +39,8 @@
 //   weight rows on lanes, one MMA issuer             82 / 126 / 632         55 /  66 / 285           25 / 53 / 256
 //   ... weight scales in a ring of their own, expansion a stage at a time, no scale barriers, two issuers (this form)
 //                                                    70 / 117 / 569         47 /  64 / 268           23 / 51 / 238
+//   ... dense items cut to fill the waves (tc_dense_form)                                            20 / 45 / 236
+// (by itself the launcher takes this form for 48 tokens and more, the few-token form of lkb_gemm_few.cu below)
 // With few tokens the hand-over of every block is the bound (300 to 440 cycles of polls, commits and arrivals).
 // No copy in this file is a multicast one; every tensor map covers memory of the GPU the kernel runs on.
 // Every wait is bounded; on expiry a status word is set and all roles drain and exit, freeing TMEM.
