@@ -49,10 +49,12 @@
 #define PF_MAXL       512
 #define PF_GUESS_OFF  (PF_LOGITS_OFF + 128)
 #define PF_REAL_OFF   (PF_GUESS_OFF + 4 * PF_MAXL)
-// Whole-step kernel without expert prefetch: the residual after the mixer and the mixer's outputs have words of their own.
+// Without expert prefetch: in the whole-step kernel the residual after the mixer and the mixer's outputs have words of their own; behind
+// the records, the logits have two sets of words, used by turns.
 #define XCH_XB_OFF    (LKB_TOP_K * LKB_MOE_INTER)
 #define XCH_M_OFF     (XCH_XB_OFF + LKB_HIDDEN)
-static_assert(XCH_M_OFF + LKB_HIDDEN <= 2 * LKB_TOP_K * LKB_MOE_INTER, "words must fit the gu scratch");
+#define XCH_L_OFF     (PF_REAL_OFF + 4 * PF_MAXL)
+static_assert(XCH_M_OFF + LKB_HIDDEN <= XCH_L_OFF && XCH_L_OFF + 2 * LKB_N_EXPERTS <= 2 * LKB_TOP_K * LKB_MOE_INTER, "words must fit the gu scratch");
 static_assert(MAX_DN_ROWS <= FUSED_WARPS, "a down row per warp");
 static_assert(PF_REAL_OFF + 4 * PF_MAXL <= 2 * LKB_TOP_K * LKB_MOE_INTER, "prefetch records must fit the gu scratch");
 
@@ -135,12 +137,15 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned * p) {
 // What the CTAs exchange -- logits, gate|up outputs, mixer outputs, residual rows: floats, one word each -- is published
 // WITHOUT a release (XCH): a release waits until the stores are acknowledged, some 0.4 us a barrier.  Instead a word that is
 // still due holds XCH_DUE, a NaN that arithmetic does not produce, and a reader that finds it after the barrier loads again.
-// A word is made due again by a CTA that knows everyone has read it (a later barrier is through), followed by a fence, before
-// that CTA arrives at the barrier of the word's next use: the store has been performed on the device when the arrival is
-// sent, so nobody behind that barrier can see the content before.
-// These stores and the fence sit between the arrival and the wait of some barrier, where nobody waits for them (xch_due below).
-// A launch starts with all words due and its first barrier a releasing one.  MoE stack of 40 layers 514 -> 496 us, a token at
-// context 4096 946 -> 930 us.
+//   * A word is made due again by its CTA's warp 1 when a barrier is through that everyone arrived at with the word's value in hand
+//     (tested, so the load is done).
+//   * Behind a later CTA barrier thread 0, which arrives for the CTA, fences (xch_fence).  The fence orders the due stores of the whole CTA
+//     before thread 0's later arrivals, and so before the reads of whoever acquires the barrier of the word's next use: nobody behind
+//     that barrier sees the content from before.  One fence a layer does for all words: it sits behind the request of the weight rows,
+//     where warp 0 would wait for them anyway.  For that the residual is made due as soon as the logits are through, and the logits, read
+//     last before that fence and written first after it, alternate between two sets of words, so that a set has a whole layer to become due.
+//   * At the start of a launch the words of all its later barriers are made due; its first barrier is a releasing one.
+// MoE stack of 40 layers 514 -> 496 us, a token at context 4096 946 -> 930 us.
 #define XCH_DUE 0xFFFFFFFFu
 template <bool XCH>
 __device__ __forceinline__ void xch_put(float * p, float v) {
@@ -152,7 +157,7 @@ __device__ __forceinline__ void xch_due(float * p, int i, int n) {       // word
 #pragma unroll 1
     for (; i < n; i += 32) asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" :: "l"(p + i), "r"(XCH_DUE) : "memory");
 }
-__device__ __forceinline__ void xch_due_fence() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+__device__ __forceinline__ void xch_fence() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 __device__ __forceinline__ uint4 xch_ld4(const float * p) {
     uint4 v;
     asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
@@ -527,6 +532,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
     }
     if (tid < LKB_TOP_K) S.pidx[tid] = tid;
     constexpr bool XCH = !PF;                                        // (with expert prefetch its records take the words' place: released barriers)
+    const bool onward = a.n_layers > 1 || a.final_norm_w != nullptr; // someone reads the residual of a layer (0.15 us of the one-layer call)
     float * const x_mid = MIX && XCH ? a.gu + XCH_XB_OFF : a.x;      // residual after the mixer
     float * const m_out = XCH ? a.gu + XCH_M_OFF : a.mxbuf;          // the mixer's outputs
     if (tid < n_dn) S.xown[tid] = __ldcg(a.x + dn0 + tid);
@@ -534,9 +540,10 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
     const int qa0 = (int) (((long long) cta * MIX_QKV_ROWS) / nct), qa1 = (int) (((long long) (cta + 1) * MIX_QKV_ROWS) / nct);
     if (XCH && warp == 1) {                                          // every word this launch exchanges is due
         xch_due(a.gu + gu0, lane, n_gu);
+        if (cta < LKB_N_EXPERTS && a.n_layers > 1) xch_due(a.gu + XCH_L_OFF + LKB_N_EXPERTS + cta, lane, 1);
         if (MIX) {
+            if (cta < LKB_N_EXPERTS) xch_due(a.gu + XCH_L_OFF + cta, lane, 1);          // (the stack's first logits: behind its releasing barrier)
             xch_due(x_mid + dn0, lane, n_dn); xch_due(m_out + dn0, lane, n_dn); xch_due(a.mxbuf + qa0, lane, qa1 - qa0);
-            if (cta < LKB_N_EXPERTS) xch_due(a.logits + cta, lane, 1);
         }
     }
     int pos = 0;
@@ -570,6 +577,8 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
         const lkb_moe_layer & ly = S.ly;
         const unsigned par = (unsigned) (l & 1);
         const bool pf_next = pf && l + 1 < a.n_layers;              // a next layer to guess for
+        float * const lg = XCH ? a.gu + XCH_L_OFF + par * LKB_N_EXPERTS : a.logits;               // this layer's logits
+        float * const lg_old = a.gu + XCH_L_OFF + (par ^ 1u) * LKB_N_EXPERTS;                     // the last layer's, and the next one's
 
         if constexpr (MIX) {
             const lkb_mixer_layer & mx = S.mx;
@@ -671,7 +680,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
                 // L2 sectors per CTA), published through mxbuf like a conv output
                 if (cta < AT_HEADS && tid < AT_D) xch_put<XCH>(m_out + cta * AT_D + tid, at_combine(a.part, cta, tid, seq_len));
                 grid_arrive<!XCH>(a.bar, S);
-                if (XCH && warp == 1) { xch_due(a.mxbuf + qa0, lane, qa1 - qa0); xch_due_fence(); }     // q | k | v: read before the partials' barrier
+                if (XCH && warp == 1) xch_due(a.mxbuf + qa0, lane, qa1 - qa0);     // q | k | v: read before the partials' barrier
                 if (!grid_wait(a.bar, status, S, 1000u + 10u * l + 7u, a.spin_limit)) return;
                 FUSED_STAMP(25);
             }
@@ -695,7 +704,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
             }
             FUSED_STAMP(23);
             grid_arrive<!XCH>(a.bar, S);
-            if (XCH && warp == 1) { xch_due(a.x + dn0, lane, n_dn); xch_due_fence(); }        // the residual before the mixer: read before the mixer's first barrier
+            if (XCH && warp == 1) xch_due(a.x + dn0, lane, n_dn);        // the residual before the mixer: read before the mixer's first barrier
             if (!grid_wait(a.bar, status, S, 1000u + 10u * l + 6u, a.spin_limit)) return;
             FUSED_STAMP(24);
         }
@@ -735,7 +744,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
             }
             if (lane == 0) {
                 S.inv = inv;
-                if (cta < LKB_N_EXPERTS) xch_put<XCH>(a.logits + cta, __fmul_rn(acc, inv));
+                if (cta < LKB_N_EXPERTS) xch_put<XCH>(lg + cta, __fmul_rn(acc, inv));
                 if (pcta && pf_next) {
                     float g = 0.0f;
 #pragma unroll
@@ -748,9 +757,11 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
         quad_quant_to_xq(S.xq, uv);
         FUSED_STAMP(2);
         if (XCH && warp == 1) {                                     // while the barrier completes: read by everyone before the last barrier
-            if (l > 0) xch_due(a.gu + gu0, lane, n_gu);
+            if (l > 0) {
+                xch_due(a.gu + gu0, lane, n_gu);
+                if (cta < LKB_N_EXPERTS) xch_due(lg_old + cta, lane, 1);
+            }
             if (MIX) xch_due(m_out + dn0, lane, n_dn);
-            xch_due_fence();
         }
         // static data of the selection, fetched while the barrier completes
         float rb0 = 0.0f, rb1 = 0.0f;
@@ -759,6 +770,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
         if (pf_next && warp == 1 && S.ly_next.rbias) { prb0 = __ldg(S.ly_next.rbias + lane); prb1 = __ldg(S.ly_next.rbias + lane + 32); }
         if (!grid_wait(a.bar, status, S, 1000u + 10u * l + 1u, a.spin_limit)) return;
         FUSED_STAMP(3);
+        if (XCH && onward && warp == 1) xch_due(x_mid + dn0, lane, n_dn);     // the residual that A read
 
         // the guessed logits of the next layer: requested here, used by warp 1 once the gate|up rows are done
         if (pf_next && warp == 1) { plg0 = __ldcg(a.gu + PF_LOGITS_OFF + lane); plg1 = __ldcg(a.gu + PF_LOGITS_OFF + lane + 32); }
@@ -767,7 +779,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
             if (warp == 0) {
                 // both logits are requested before either is used: a shared-memory store between two global
                 // loads would serialise them (the compiler cannot prove the pointers distinct)
-                const float lg0 = xch_get<XCH>(a.logits + lane, status, S.abort, 1000u + 10u * l + 1u), lg1 = xch_get<XCH>(a.logits + lane + 32, status, S.abort, 1000u + 10u * l + 1u);
+                const float lg0 = xch_get<XCH>(lg + lane, status, S.abort, 1000u + 10u * l + 1u), lg1 = xch_get<XCH>(lg + lane + 32, status, S.abort, 1000u + 10u * l + 1u);
                 const float g0 = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-lg0)));
                 const float g1 = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-lg1)));
                 S.sig[lane] = g0; S.sig[lane + 32] = g1;
@@ -776,7 +788,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
                 S.key[lane] = lkb_orderable(s0); S.key[lane + 32] = lkb_orderable(s1);
             }
         } else {
-            if (tid < LKB_N_EXPERTS) S.sel[tid] = xch_get<XCH>(a.logits + tid, status, S.abort, 1000u + 10u * l + 1u);
+            if (tid < LKB_N_EXPERTS) S.sel[tid] = xch_get<XCH>(lg + tid, status, S.abort, 1000u + 10u * l + 1u);
             __syncthreads();
             float p = 0.0f;
             if (tid < LKB_N_EXPERTS) {
@@ -863,6 +875,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
                 }
             }
         }
+        if (XCH && onward && tid == 0) xch_fence();                           // the words that warp 1 has made due since the last one
         __syncwarp();
         FUSED_STAMP(4);
 
@@ -894,9 +907,6 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
         }
         FUSED_STAMP(5);
         grid_arrive<!XCH>(a.bar, S);
-        if (XCH && warp == 1) {                                     // read before the logits' barrier: the residual that A read
-            xch_due(x_mid + dn0, lane, n_dn); xch_due_fence();
-        }
         // between arrive and wait: the next layer's router row and norm weights (static data)
         if (l + 1 < a.n_layers) {
             if (cta < LKB_N_EXPERTS && tid == 0) {
@@ -1062,7 +1072,6 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
         }
         FUSED_STAMP(7);
         grid_arrive<!XCH>(a.bar, S);
-        if (XCH && warp == 1 && cta < LKB_N_EXPERTS) { xch_due(a.logits + cta, lane, 1); xch_due_fence(); }      // read before the barrier after gate|up
         if (l + 1 < a.n_layers && tid < (int) (sizeof(lkb_moe_layer) / 8))
             reinterpret_cast<unsigned long long *>(&S.ly)[tid] = reinterpret_cast<const unsigned long long *>(&L[l + 1])[tid];
         if (pf && l + 2 < a.n_layers && tid >= 32 && tid < 32 + (int) (sizeof(lkb_moe_layer) / 8))
