@@ -744,7 +744,11 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
             }
             if (lane == 0) {
                 S.inv = inv;
-                if (cta < LKB_N_EXPERTS) xch_put<XCH>(lg + cta, __fmul_rn(acc, inv));
+                if (cta < LKB_N_EXPERTS) {
+                    const float v = __fmul_rn(acc, inv);
+                    xch_put<XCH>(lg + cta, v);
+                    if (XCH && l + 1 == a.n_layers) a.logits[cta] = v;          // the caller's: nobody reads them here
+                }
                 if (pcta && pf_next) {
                     float g = 0.0f;
 #pragma unroll

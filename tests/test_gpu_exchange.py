@@ -63,3 +63,26 @@ def test_step_at_group_edges(lkb, pos0):
     assert torch.isfinite(out[0][0]).all()
     for a, b in zip(*out):
         assert torch.equal(a, b)
+
+
+def test_logits_scratch_holds_the_last_layers_logits(lkb):
+    """After a launch `scratch->logits` holds what the kernel sequence leaves there: the last layer's router logits."""
+    lkb.init(0)
+    synth = importlib.import_module("lfm2-ampere_b200.synth")
+    st = importlib.import_module("lfm2-ampere_b200.decode").DecodeStack(synth.make_model(3, seed=29, zipf_s=1.1))
+    x0 = torch.randn(H, device="cuda", generator=torch.Generator("cuda").manual_seed(4))
+    st.x.copy_(x0); st.step(); ref = st.logits.clone()
+    for prefetch in (0, 1):
+        lkb.decode_set_expert_prefetch(prefetch)
+        try:
+            st.logits.zero_(); st.x.copy_(x0); st.step_fused(); torch.cuda.synchronize()
+        finally:
+            lkb.decode_set_expert_prefetch(0)
+        assert st.status() == 0 and ref.abs().max() > 0 and torch.equal(st.logits, ref)
+    net = importlib.import_module("lfm2-ampere_b200.model").make_full_model(n_layers=4, seed=7, vocab=4096)
+    left = []
+    for impl in ("kernels", "mega"):
+        ds = importlib.import_module("lfm2-ampere_b200.model").DecodeStep(net, max_seq=16, moe_impl=impl)
+        ds.d_token.fill_(11); ds.step(); torch.cuda.synchronize()
+        left.append(ds.logits.clone())
+    assert left[0].abs().max() > 0 and torch.equal(*left)
