@@ -223,8 +223,9 @@ int lkb_moe_ffn_decode(const lkb_moe_layer * layer, float * x, int * idx_out, fl
  * l+1's router on layer l's input, and each CTA, once its rows of layer l have arrived, asks for its slice of the four
  * guessed experts of layer l+1 to be brought into L2 (cp.async.bulk.prefetch.L2).  Results are unchanged bit for bit:
  * the exact selection decides what is computed, a wrong guess only costs idle HBM bandwidth.  The guesses and the actual
- * choices of the last launch are kept in the second half of scratch->gu; lkb_decode_expert_prefetch_hits waits for
- * `st` and counts how many of the 4*(n_layers-1) guesses were chosen.  The idea of warming L2 with expert rows ahead of
+ * choices of the last launch that made any are kept in the second half of scratch->gu until a whole-step launch (lkb_decode_layers)
+ * without expert prefetch, whose exchange takes their place; lkb_decode_expert_prefetch_hits waits for `st` and counts the
+ * guesses it finds, 4*(n_layers-1) or none, and how many of them were chosen.  The idea of warming L2 with expert rows ahead of
  * their use is the reference's (ref: src/kernels.cu:499-510, there for the current layer's down rows).
  * Off by default (mode 0): on B200, with 74-81% of the guesses chosen, a 40-layer step measured 2-4% slower with it. */
 int lkb_decode_set_expert_prefetch(int mode);

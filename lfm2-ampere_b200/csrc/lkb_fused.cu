@@ -1186,14 +1186,14 @@ int lkb_decode_expert_prefetch_hits(const lkb_moe_scratch * scratch, int n_layer
     if (e == cudaSuccess) e = cudaMemcpy(rec[0], scratch->gu + PF_GUESS_OFF, sizeof(int) * 4 * nl, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = cudaMemcpy(rec[1], scratch->gu + PF_REAL_OFF, sizeof(int) * 4 * nl, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return -(int) e;
-    int h = 0;
-#pragma unroll 1
-    for (int l = 1; l < nl; ++l)
-#pragma unroll 1
-        for (int i = 0; i < 4; ++i)
-#pragma unroll 1
-            for (int j = 0; j < 4; ++j) h += rec[0][l * 4 + i] == rec[1][l * 4 + j];
-    *hits = h; *guesses = 4 * (nl - 1);
+    int h = 0, n = 0;
+    for (int i = 4; i < 4 * nl; ++i) {
+        const int guess = rec[0][i];
+        if (guess < 0 || guess >= LKB_N_EXPERTS) continue;               // no guess: a whole-step launch without prefetch leaves due words there
+        ++n;
+        for (int j = 0; j < 4; ++j) h += guess == rec[1][i / 4 * 4 + j];
+    }
+    *hits = h; *guesses = n;
     return LKB_OK;
 }
 

@@ -445,3 +445,26 @@ def test_expert_prefetch_leaves_results_unchanged(L):
         assert st.status() == 0
     finally:
         L.decode_set_expert_prefetch(0)
+
+
+def test_prefetch_records_after_launches_without(L):
+    """The hit counter counts guesses only: those of the last launch that made any, and none once a whole-step launch without prefetch
+    has used their place for its exchange."""
+    import importlib
+    model = importlib.import_module("lfm2-ampere_b200.model")
+    n = 5
+    ds = model.DecodeStep(model.make_full_model(n_layers=n, seed=3, vocab=2048), max_seq=32, moe_impl="mega")
+    try:
+        L.decode_set_expert_prefetch(2)
+        ds.step(); torch.cuda.synchronize()
+        assert ds.status() == 0
+        hits, guesses = L.decode_expert_prefetch_hits(ds._scratch, n)
+        assert guesses == 4 * (n - 1) and 0 <= hits <= guesses
+        L.decode_set_expert_prefetch(0)
+        L.moe_ffn_decode(ds._descs[0], ds.x, None, None, None, ds._scratch)
+        torch.cuda.synchronize()
+        assert L.decode_expert_prefetch_hits(ds._scratch, n) == (hits, guesses)
+        ds.step(); torch.cuda.synchronize()
+        assert ds.status() == 0 and L.decode_expert_prefetch_hits(ds._scratch, n) == (0, 0)
+    finally:
+        L.decode_set_expert_prefetch(0)
