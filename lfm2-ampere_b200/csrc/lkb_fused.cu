@@ -29,7 +29,7 @@
 // five-kernel sequence.
 //
 // Every wait (grid barrier, mbarrier) is bounded: on expiry the CTA records a code in
-// the status word and leaves; the other CTAs' waits then expire too.
+// the status word, waits for its copies in flight and leaves; the other CTAs' waits then expire too.
 #include <cooperative_groups.h>
 #include "lkb_attn.cuh"
 
@@ -58,6 +58,8 @@ static_assert(XCH_M_OFF + LKB_HIDDEN <= XCH_L_OFF && XCH_L_OFF + 2 * LKB_N_EXPER
 static_assert(MAX_DN_ROWS <= FUSED_WARPS, "a down row per warp");
 static_assert(PF_REAL_OFF + 4 * PF_MAXL <= 2 * LKB_TOP_K * LKB_MOE_INTER, "prefetch records must fit the gu scratch");
 
+struct FusedBar { unsigned long long m; unsigned issued; };     // an mbarrier and how many of its phases copies have been requested for
+
 struct FusedSmem {
     alignas(128) unsigned char gu_q[MAX_GU_ROWS * GU_BPR * 16];          // 98304
     alignas(128) unsigned char dn_q[LKB_TOP_K * MAX_DN_ROWS * DN_BPR * 16]; // 49152
@@ -85,35 +87,35 @@ struct FusedSmem {
     alignas(8) lkb_moe_layer ly;          // this layer's descriptor (staged: a global read costs ~1 us of latency)
     alignas(8) lkb_moe_layer ly_next;     // the next layer's (expert prefetch)
     alignas(8) lkb_mixer_layer mx;        // whole-step kernel: this layer's sequence-mixer descriptor
-    alignas(8) unsigned long long mbar_mi, mbar_mo;   // whole-step kernel: mixer input rows / output rows staged
-    alignas(8) unsigned long long mbar_gu[N_GU_CH];
-    alignas(8) unsigned long long mbar_dn[N_DN_CH];
-    alignas(8) unsigned long long mbar_rt;
+    FusedBar mbar_mi, mbar_mo;            // whole-step kernel: mixer input rows / output rows staged
+    FusedBar mbar_gu[N_GU_CH], mbar_dn[N_DN_CH], mbar_rt;
 };
 
 // ---- PTX wrappers -----------------------------------------------------------
 __device__ __forceinline__ unsigned smem_u32(const void * p) { return (unsigned) __cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(unsigned long long * b, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(b)), "r"(count));
+__device__ __forceinline__ void mbar_init(FusedBar * b) {
+    b->issued = 0u;
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(&b->m)));
 }
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long * b, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(smem_u32(b)), "r"(bytes) : "memory");
+__device__ __forceinline__ void mbar_expect_tx(FusedBar * b, unsigned bytes) {
+    ++b->issued;                                                   // (one thread at a time)
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(smem_u32(&b->m)), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ bool mbar_try_wait(unsigned long long * b, unsigned parity) {
+__device__ __forceinline__ bool mbar_try_wait(FusedBar * b, unsigned parity) {
     unsigned ok;
     asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-                 : "=r"(ok) : "r"(smem_u32(b)), "r"(parity) : "memory");
+                 : "=r"(ok) : "r"(smem_u32(&b->m)), "r"(parity) : "memory");
     return ok != 0;
 }
 // Bounded wait; returns false on expiry.
-__device__ __forceinline__ bool mbar_wait(unsigned long long * b, unsigned parity) {
+__device__ __forceinline__ bool mbar_wait(FusedBar * b, unsigned parity) {
 #pragma unroll 1
     for (unsigned i = 0; i < SPIN_LIMIT; ++i) if (mbar_try_wait(b, parity)) return true;
     return false;
 }
-__device__ __forceinline__ void bulk_g2s(void * dst, const void * src, unsigned bytes, unsigned long long * b) {
+__device__ __forceinline__ void bulk_g2s(void * dst, const void * src, unsigned bytes, FusedBar * b) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 :: "r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(b)) : "memory");
+                 :: "r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(&b->m)) : "memory");
 }
 // Bring [src, src+bytes) into L2 without a destination (16-byte aligned address and size).
 __device__ __forceinline__ void bulk_prefetch_l2(const void * src, unsigned bytes) {
@@ -211,6 +213,17 @@ __device__ __forceinline__ void grid_arrive(unsigned * bar, FusedSmem & S, bool 
     __syncthreads();                                   // this CTA's global writes are issued
     if (threadIdx.x == 0) grid_arrive_one<RELEASE>(bar, S, release);
 }
+// A CTA that leaves early waits for the copies it has requested (bounded): their destination is its shared memory.
+__device__ __noinline__ void fused_drain(FusedSmem & S) {
+    asm volatile("cp.async.wait_all;" ::: "memory");                // this thread's requests of K and V
+    const int i = threadIdx.x;
+    if (i >= N_GU_CH + N_DN_CH + 3) return;
+    FusedBar * const b = i < N_GU_CH ? &S.mbar_gu[i] : i < N_GU_CH + N_DN_CH ? &S.mbar_dn[i - N_GU_CH]
+                       : i == N_GU_CH + N_DN_CH ? &S.mbar_rt : i == N_GU_CH + N_DN_CH + 1 ? &S.mbar_mi : &S.mbar_mo;
+    const unsigned n = b->issued;
+#pragma unroll 1
+    for (unsigned k = 0; n && k < 4096u && !mbar_try_wait(b, (n - 1u) & 1u); ++k) { }
+}
 // One poll in flight per CTA.  (Keeping four relaxed polls in flight per CTA, a quarter of a round trip apart, was
 // measured: every barrier got 0.4-0.7 us SLOWER -- 148 CTAs x 4 loads on the one L2 line delay the arriving
 // reductions more than the finer sampling gains.  Sleeping 400 / 800 ns before the first poll cost 0.4 / 1.1 us
@@ -228,7 +241,9 @@ __device__ __forceinline__ bool grid_wait(unsigned * bar, unsigned * status, Fus
         if (!ok) { atomicCAS(status, 0u, code); S.abort = 1; }
     }
     __syncthreads();
-    return S.abort == 0;
+    if (S.abort == 0) return true;
+    fused_drain(S);
+    return false;
 }
 
 // Rows [j0, j1) of a logical row space made of `nseg` equal segments of `seg_rows`
@@ -239,7 +254,7 @@ struct SegView {
 };
 
 __device__ __forceinline__ void issue_rows(const SegView & v, int seg_rows, int bpr, int g_begin, int g_end,
-                                           unsigned char * sq, __half * sd, unsigned long long * mb) {
+                                           unsigned char * sq, __half * sd, FusedBar * mb) {
     // [g_begin, g_end) may straddle one segment boundary
     unsigned bytes = (unsigned) (g_end - g_begin) * (unsigned) bpr * 18u;
     mbar_expect_tx(mb, bytes);
@@ -256,7 +271,7 @@ __device__ __forceinline__ void issue_rows(const SegView & v, int seg_rows, int 
 
 // Gate|up logical rows g = (half*4 + k)*1536 + row; [g_begin, g_end) may straddle one segment boundary.
 __device__ __forceinline__ void issue_gu_rows(const lkb_moe_layer & ly, const int * idx, int g_begin, int g_end,
-                                              unsigned char * sq, __half * sd, unsigned long long * mb) {
+                                              unsigned char * sq, __half * sd, FusedBar * mb) {
     mbar_expect_tx(mb, (unsigned) (g_end - g_begin) * (unsigned) GU_BPR * 18u);
     int g = g_begin;
 #pragma unroll 1
@@ -489,12 +504,12 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
         S.abort = 0;
         S.bar_target = 0u;
 #pragma unroll 1
-        for (int i = 0; i < N_GU_CH; ++i) mbar_init(&S.mbar_gu[i], 1);
+        for (int i = 0; i < N_GU_CH; ++i) mbar_init(&S.mbar_gu[i]);
 #pragma unroll 1
-        for (int i = 0; i < N_DN_CH; ++i) mbar_init(&S.mbar_dn[i], 1);
-        mbar_init(&S.mbar_rt, 1);
-        mbar_init(&S.mbar_mi, 1);
-        mbar_init(&S.mbar_mo, 1);
+        for (int i = 0; i < N_DN_CH; ++i) mbar_init(&S.mbar_dn[i]);
+        mbar_init(&S.mbar_rt);
+        mbar_init(&S.mbar_mi);
+        mbar_init(&S.mbar_mo);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -557,13 +572,14 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
     __syncthreads();
     if constexpr (MIX) {
         // KV capacity: an attention layer whose descriptor states max_seq refuses a position past its cache.  Every CTA
-        // evaluates the same test before anything is in flight, so all leave together (status 600 + layer).
+        // evaluates the same test before the first barrier, so all leave together (status 600 + layer).
         int over = -1;
 #pragma unroll 1
         for (int l = tid; l < a.n_layers; l += blockDim.x)
             if (a.mixers[l].is_attn && a.mixers[l].max_seq > 0 && pos >= a.mixers[l].max_seq) over = l;
         if (__syncthreads_or(over >= 0)) {
             if (over >= 0) atomicCAS(status, 0u, 600u + (unsigned) over);
+            fused_drain(S);                                         // the first router rows
             return;
         }
         if (tid == 0) {
@@ -870,7 +886,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
                     const int cc = c - n_gu_ch, k = cc / dn_ch_per_k, ch = cc % dn_ch_per_k;
                     const int j0 = ch * CH_ROWS, j1 = min(n_dn, j0 + CH_ROWS);
                     const size_t ed = (size_t) S.idx[k] * LKB_HIDDEN * DN_BPR;
-                    unsigned long long * mb = &S.mbar_dn[k * dn_ch_per_k + ch];
+                    FusedBar * mb = &S.mbar_dn[k * dn_ch_per_k + ch];
                     mbar_expect_tx(mb, (unsigned) (j1 - j0) * DN_BPR * 18u);
                     bulk_g2s(S.dn_q + ((size_t) k * MAX_DN_ROWS + j0) * DN_BPR * 16,
                              (const uint4 *) ly.down_qs + ed + (size_t) (dn0 + j0) * DN_BPR, (unsigned) (j1 - j0) * DN_BPR * 16u, mb);
@@ -891,7 +907,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
 #pragma unroll 1
             for (int j = warp; j < n_gu; j += FUSED_WARPS) {
                 // both probes are issued before either answer is used (a probe takes ~0.1 us even when the rows are there)
-                unsigned long long * const mg = &S.mbar_gu[j / CH_ROWS], * const mu = &S.mbar_gu[gu_half_ch + j / CH_ROWS];
+                FusedBar * const mg = &S.mbar_gu[j / CH_ROWS], * const mu = &S.mbar_gu[gu_half_ch + j / CH_ROWS];
                 const bool hg = mbar_try_wait(mg, par), hu = mbar_try_wait(mu, par);
                 if (__any_sync(LKB_FULL, (!hg && !mbar_wait(mg, par)) || (!hu && !mbar_wait(mu, par)))) {
                     if (lane == 0) { atomicCAS(status, 0u, 200u + l); S.abort = 1; }
@@ -1020,7 +1036,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
         {
             const int j0 = 2 * (warp >> 1), k0 = 2 * (warp & 1);            // n_dn <= MAX_DN_ROWS = FUSED_WARPS
             if (j0 < n_dn) {
-                unsigned long long * const m0 = &S.mbar_dn[k0 * dn_ch_per_k + j0 / CH_ROWS], * const m1 = &S.mbar_dn[(k0 + 1) * dn_ch_per_k + j0 / CH_ROWS];
+                FusedBar * const m0 = &S.mbar_dn[k0 * dn_ch_per_k + j0 / CH_ROWS], * const m1 = &S.mbar_dn[(k0 + 1) * dn_ch_per_k + j0 / CH_ROWS];
                 const bool h0 = mbar_try_wait(m0, par), h1 = mbar_try_wait(m1, par);      // both probes in flight, then the bounded waits if needed
                 const bool ok = __all_sync(LKB_FULL, (h0 || mbar_wait(m0, par)) && (h1 || mbar_wait(m1, par)));
                 FUSED_STAMP(15);

@@ -111,3 +111,25 @@ def test_words_are_due_before_the_next_ones_are_published(layers):
     words = {w for _, w in ev if w}
     assert {"a.gu", "a.x"} <= words and ("moe" in layers or {"x_mid", "m_out"} <= words) and sum(k == "put" for k, _ in ev) >= 3 * len(layers)
     assert faults(ev) == []
+
+
+def _function(head):
+    return _block(re.sub(r"//[^\n]*", "", SRC[SRC.index(head):]), 0)[1]
+
+
+def test_every_way_out_waits_for_the_copies_in_flight():
+    """A CTA that leaves early has no copy into its shared memory under way: every `return` of the kernel follows a barrier wait that gave up,
+    which drains, or a drain of its own; the one exception leaves before anything is requested.  The drain knows the phases that
+    copies were requested for from the one function that announces their bytes."""
+    kernel = _function("k_moe_ffn_stack(const FusedArgs a) {")
+    requests = kernel.index("mbar_expect_tx(")
+    for t in re.finditer(r"\breturn;", kernel):
+        before = kernel[:t.start()].rstrip()
+        assert before.endswith("fused_drain(S);") or re.search(r"if \(!grid_wait\([^;]*\)$", before) or t.start() < requests, before[-120:]
+    assert re.search(r"if \(S\.abort == 0\) return true;\s*fused_drain\(S\);\s*return false;\s*}$", _function("bool grid_wait("))
+    announce = _function("void mbar_expect_tx(")
+    assert "++b->issued;" in announce and SRC.count("mbarrier.arrive.expect_tx") == announce.count("mbarrier.arrive.expect_tx") == 1
+    drain = _function("void fused_drain(")
+    assert "cp.async.wait_all" in drain
+    for bar in set(re.findall(r"\bmbar_(?:gu|dn|rt|mi|mo)\b", kernel)):
+        assert f"S.{bar}" in drain
