@@ -246,29 +246,6 @@ __device__ __forceinline__ bool grid_wait(unsigned * bar, unsigned * status, Fus
     return false;
 }
 
-// Rows [j0, j1) of a logical row space made of `nseg` equal segments of `seg_rows`
-// rows; segment s lives at base_q[s]/base_d[s].  Issues the bulk copies of chunk c.
-struct SegView {
-    const uint4 *  q[8];
-    const __half * d[8];
-};
-
-__device__ __forceinline__ void issue_rows(const SegView & v, int seg_rows, int bpr, int g_begin, int g_end,
-                                           unsigned char * sq, __half * sd, FusedBar * mb) {
-    // [g_begin, g_end) may straddle one segment boundary
-    unsigned bytes = (unsigned) (g_end - g_begin) * (unsigned) bpr * 18u;
-    mbar_expect_tx(mb, bytes);
-    int g = g_begin;
-#pragma unroll 1
-    while (g < g_end) {
-        const int s = g / seg_rows, r = g - s * seg_rows;
-        int n = g_end - g; if (n > seg_rows - r) n = seg_rows - r;
-        bulk_g2s(sq, v.q[s] + (size_t) r * bpr, (unsigned) n * bpr * 16u, mb);
-        bulk_g2s(sd, v.d[s] + (size_t) r * bpr, (unsigned) n * bpr * 2u, mb);
-        sq += (size_t) n * bpr * 16; sd += (size_t) n * bpr; g += n;
-    }
-}
-
 // Gate|up logical rows g = (half*4 + k)*1536 + row; [g_begin, g_end) may straddle one segment boundary.
 __device__ __forceinline__ void issue_gu_rows(const lkb_moe_layer & ly, const int * idx, int g_begin, int g_end,
                                               unsigned char * sq, __half * sd, FusedBar * mb) {
