@@ -84,6 +84,7 @@ struct FusedSmem {
     float  cs[AT_D / 2], sn[AT_D / 2];    // whole-step kernel: rotation at this step's position
     int    abort;
     unsigned bar_target;
+    unsigned spin_limit;                  // polls a wait for other CTAs may take
     alignas(8) lkb_moe_layer ly;          // this layer's descriptor (staged: a global read costs ~1 us of latency)
     alignas(8) lkb_moe_layer ly_next;     // the next layer's (expert prefetch)
     alignas(8) lkb_mixer_layer mx;        // whole-step kernel: this layer's sequence-mixer descriptor
@@ -171,35 +172,36 @@ __device__ __forceinline__ unsigned xch_ld1(const float * p) {
     return v;
 }
 __device__ __forceinline__ bool xch_missing(const uint4 & v) { return v.x == XCH_DUE || v.y == XCH_DUE || v.z == XCH_DUE || v.w == XCH_DUE; }
-// A word that was due when it was first read: bounded, out of line.  *abort is set when it does not come (`code` as for the
+// A word that was due when it was first read: bounded, out of line.  S.abort is set when it does not come (`code` as for the
 // barrier in front of it; every phase that reads words ends in a barrier wait, which looks at it).
-__device__ __noinline__ float xch_again(const float * p, unsigned * status, unsigned code, int * abort) {
+__device__ __noinline__ float xch_again(const float * p, unsigned * status, unsigned code, FusedSmem & S) {
+    const unsigned limit = S.spin_limit;
 #pragma unroll 1
-    for (unsigned i = 0; i < SPIN_LIMIT; ++i) {
+    for (unsigned i = 0; i < limit; ++i) {
         const unsigned v = xch_ld1(p);
         if (v != XCH_DUE) return __uint_as_float(v);
         if ((i & 1023u) == 1023u && ld_acquire(status) != 0u) break;
     }
     atomicCAS(status, 0u, code);
-    *abort = 1;
+    S.abort = 1;
     return 0.0f;
 }
 template <bool XCH>
-__device__ __forceinline__ float xch_get(const float * p, unsigned * status, int & abort, unsigned code) {
+__device__ __forceinline__ float xch_get(const float * p, unsigned * status, FusedSmem & S, unsigned code) {
     const unsigned v = xch_ld1(p);
-    return XCH && v == XCH_DUE ? xch_again(p, status, code, &abort) : __uint_as_float(v);
+    return XCH && v == XCH_DUE ? xch_again(p, status, code, S) : __uint_as_float(v);
 }
 // Four words, 16-byte aligned.
-__device__ __noinline__ float4 xch_again4(const float * p, unsigned * status, unsigned code, int * abort) {
+__device__ __noinline__ float4 xch_again4(const float * p, unsigned * status, unsigned code, FusedSmem & S) {
     float4 v;
-    v.x = xch_again(p, status, code, abort); v.y = xch_again(p + 1, status, code, abort);
-    v.z = xch_again(p + 2, status, code, abort); v.w = xch_again(p + 3, status, code, abort);
+    v.x = xch_again(p, status, code, S); v.y = xch_again(p + 1, status, code, S);
+    v.z = xch_again(p + 2, status, code, S); v.w = xch_again(p + 3, status, code, S);
     return v;
 }
 template <bool XCH>
-__device__ __forceinline__ float4 xch_get4(const float * p, unsigned * status, int & abort, unsigned code, bool words = true) {
+__device__ __forceinline__ float4 xch_get4(const float * p, unsigned * status, FusedSmem & S, unsigned code, bool words = true) {
     const uint4 v = xch_ld4(p);
-    if (XCH && xch_missing(v) && words) return xch_again4(p, status, code, &abort);
+    if (XCH && xch_missing(v) && words) return xch_again4(p, status, code, S);
     return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
 }
 template <bool RELEASE = true>
@@ -319,7 +321,8 @@ __device__ __forceinline__ void load_xregs(const lkb_q8blk * xq, int bpr, int la
 #ifdef LKB_TUNING
 static unsigned long long * g_fused_timing = nullptr;
 #endif
-static int g_fused_absent_cta = -1;              // test hook, see lkb_debug_fused_absent_cta
+static int g_fused_absent_cta = -1;              // test hooks, see lkb_debug_fused_absent_cta, lkb_debug_fused_withheld
+static int g_fused_withheld = -1;
 static unsigned g_fused_spin_limit = 0;          // 0: default
 static int g_fused_prefetch = 0;                 // bit 0: MoE stack, bit 1: whole-step kernel (lkb_decode_set_expert_prefetch)
 #ifdef LKB_TUNING
@@ -371,7 +374,8 @@ struct FusedArgs {
     int                   softmax;
     unsigned long long *  timing;
     int                   absent_cta;  // test hook: this CTA leaves at once and never arrives (-1: none)
-    unsigned              spin_limit;  // iterations a grid-barrier wait may spin
+    int                   withheld;    // test hook: the logit that is not published, layer * 64 + expert (-1: none)
+    unsigned              spin_limit;  // polls that a wait for other CTAs -- a barrier, a word due -- may take
     int                   prefetch;    // expert prefetch on
     // whole-step kernel only
     const lkb_mixer_layer * mixers;    // device array [n_layers]
@@ -387,7 +391,7 @@ struct FusedArgs {
 template <bool XCH>
 __device__ __forceinline__ void fused_load_u(FusedSmem & S, const float * __restrict__ x, const float (&nw)[4],
                                              float (&xv)[4], float (&uv)[4], bool words, unsigned * status, unsigned code) {
-    const float4 t = xch_get4<XCH>(x + 4 * threadIdx.x, status, S.abort, code, words);
+    const float4 t = xch_get4<XCH>(x + 4 * threadIdx.x, status, S, code, words);
     xv[0] = t.x; xv[1] = t.y; xv[2] = t.z; xv[3] = t.w;
 #pragma unroll
     for (int j = 0; j < 4; ++j) uv[j] = __fmul_rn(xv[j], nw[j]);
@@ -480,6 +484,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
     if (tid == 0) {
         S.abort = 0;
         S.bar_target = 0u;
+        S.spin_limit = a.spin_limit;
 #pragma unroll 1
         for (int i = 0; i < N_GU_CH; ++i) mbar_init(&S.mbar_gu[i]);
 #pragma unroll 1
@@ -648,17 +653,17 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
                     if (warp < AT_GQA) {
                         const float * qh = a.mxbuf + (size_t) (kvh * AT_GQA + warp) * AT_D;
                         float y0, y1;
-                        at_norm_rotate(xch_get<XCH>(qh + lane, status, S.abort, 1000u + 10u * l + 4u), xch_get<XCH>(qh + lane + 32, status, S.abort, 1000u + 10u * l + 4u), mx.qnorm, lane, S.sn[lane], S.cs[lane], y0, y1);
+                        at_norm_rotate(xch_get<XCH>(qh + lane, status, S, 1000u + 10u * l + 4u), xch_get<XCH>(qh + lane + 32, status, S, 1000u + 10u * l + 4u), mx.qnorm, lane, S.sn[lane], S.cs[lane], y0, y1);
                         reinterpret_cast<float *>(&A.q[lane])[warp] = y0;
                         reinterpret_cast<float *>(&A.q[lane + 32])[warp] = y1;
                     } else if (warp == AT_GQA && t1 == seq_len) {
                         const float * kh = a.mxbuf + LKB_HIDDEN + (size_t) kvh * AT_D;
                         const float * vh = a.mxbuf + LKB_HIDDEN + AT_KVH * AT_D + (size_t) kvh * AT_D;
                         float y0, y1;
-                        at_norm_rotate(xch_get<XCH>(kh + lane, status, S.abort, 1000u + 10u * l + 4u), xch_get<XCH>(kh + lane + 32, status, S.abort, 1000u + 10u * l + 4u), mx.knorm, lane, S.sn[lane], S.cs[lane], y0, y1);
+                        at_norm_rotate(xch_get<XCH>(kh + lane, status, S, 1000u + 10u * l + 4u), xch_get<XCH>(kh + lane + 32, status, S, 1000u + 10u * l + 4u), mx.knorm, lane, S.sn[lane], S.cs[lane], y0, y1);
                         const size_t off = ((size_t) pos * AT_KVH + kvh) * AT_D;
                         kc[off + lane] = __float2half(y0); kc[off + lane + 32] = __float2half(y1);
-                        vc[off + lane] = __float2half(xch_get<XCH>(vh + lane, status, S.abort, 1000u + 10u * l + 4u)); vc[off + lane + 32] = __float2half(xch_get<XCH>(vh + lane + 32, status, S.abort, 1000u + 10u * l + 4u));
+                        vc[off + lane] = __float2half(xch_get<XCH>(vh + lane, status, S, 1000u + 10u * l + 4u)); vc[off + lane + 32] = __float2half(xch_get<XCH>(vh + lane + 32, status, S, 1000u + 10u * l + 4u));
                         __threadfence();
                     }
                     __syncthreads();
@@ -679,7 +684,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
             }
             // ---- M3: the mixer's 2048 outputs, written by their owner CTAs, quantised by every CTA; then this CTA's output-projection rows, added to the residual ----
             {
-                const float4 o4 = xch_get4<XCH>(m_out + 4 * tid, status, S.abort, 1000u + 10u * l + (is_attn ? 7u : 4u));
+                const float4 o4 = xch_get4<XCH>(m_out + 4 * tid, status, S, 1000u + 10u * l + (is_attn ? 7u : 4u));
                 const float o[4] = {o4.x, o4.y, o4.z, o4.w};
                 quad_quant_to_xq(S.xq, o);
                 __syncthreads();
@@ -737,7 +742,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
             }
             if (lane == 0) {
                 S.inv = inv;
-                if (cta < LKB_N_EXPERTS) {
+                if (cta < LKB_N_EXPERTS && (!XCH || a.withheld != l * LKB_N_EXPERTS + cta)) {
                     const float v = __fmul_rn(acc, inv);
                     xch_put<XCH>(lg + cta, v);
                     if (XCH && l + 1 == a.n_layers) a.logits[cta] = v;          // the caller's: nobody reads them here
@@ -776,7 +781,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
             if (warp == 0) {
                 // both logits are requested before either is used: a shared-memory store between two global
                 // loads would serialise them (the compiler cannot prove the pointers distinct)
-                const float lg0 = xch_get<XCH>(lg + lane, status, S.abort, 1000u + 10u * l + 1u), lg1 = xch_get<XCH>(lg + lane + 32, status, S.abort, 1000u + 10u * l + 1u);
+                const float lg0 = xch_get<XCH>(lg + lane, status, S, 1000u + 10u * l + 1u), lg1 = xch_get<XCH>(lg + lane + 32, status, S, 1000u + 10u * l + 1u);
                 const float g0 = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-lg0)));
                 const float g1 = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-lg1)));
                 S.sig[lane] = g0; S.sig[lane + 32] = g1;
@@ -785,7 +790,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
                 S.key[lane] = lkb_orderable(s0); S.key[lane + 32] = lkb_orderable(s1);
             }
         } else {
-            if (tid < LKB_N_EXPERTS) S.sel[tid] = xch_get<XCH>(lg + tid, status, S.abort, 1000u + 10u * l + 1u);
+            if (tid < LKB_N_EXPERTS) S.sel[tid] = xch_get<XCH>(lg + tid, status, S, 1000u + 10u * l + 1u);
             __syncthreads();
             float p = 0.0f;
             if (tid < LKB_N_EXPERTS) {
@@ -991,7 +996,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
                 for (int j = 0; j < 3; ++j) {                        // rare
                     const float4 t = j == 0 ? v[0] : j == 1 ? v[1] : v[2];
                     if (!xch_missing(make_uint4(__float_as_uint(t.x), __float_as_uint(t.y), __float_as_uint(t.z), __float_as_uint(t.w)))) continue;
-                    const float4 n = xch_again4(a.gu + 4 * ((warp + FUSED_WARPS * j) * 32 + lane), status, 1000u + 10u * l + 2u, &S.abort);
+                    const float4 n = xch_again4(a.gu + 4 * ((warp + FUSED_WARPS * j) * 32 + lane), status, 1000u + 10u * l + 2u, S);
                     if (j == 0) v[0] = n; else if (j == 1) v[1] = n; else v[2] = n;
                 }
             }
@@ -1136,6 +1141,7 @@ static int fused_launch(FusedArgs & a, cudaStream_t st) {
     a.timing = nullptr;
 #endif
     a.absent_cta = g_fused_absent_cta;
+    a.withheld = g_fused_withheld;
     a.spin_limit = g_fused_spin_limit ? g_fused_spin_limit : SPIN_LIMIT;
     a.prefetch = (g_fused_prefetch >> (a.mixers ? 1 : 0)) & 1;
     cudaLaunchConfig_t cfg = {};
@@ -1162,6 +1168,12 @@ __attribute__((visibility("default"))) int lkb_debug_fused_timing(unsigned long 
 // instead of hanging.  cta = -1 restores normal operation.  Nothing faults, traps or spins without a bound.
 __attribute__((visibility("default"))) int lkb_debug_fused_absent_cta(int cta, unsigned spin_limit) {
     g_fused_absent_cta = cta; g_fused_spin_limit = spin_limit; return LKB_OK;
+}
+
+// Test hook (not in the public header): the next launches do not publish one logit of one layer, so every CTA's wait for that word runs out
+// after `spin_limit` polls, behind a barrier that everyone has reached.  layer = -1 restores normal operation.
+__attribute__((visibility("default"))) int lkb_debug_fused_withheld(int layer, int expert, unsigned spin_limit) {
+    g_fused_withheld = layer < 0 ? -1 : layer * LKB_N_EXPERTS + expert; g_fused_spin_limit = spin_limit; return LKB_OK;
 }
 
 int lkb_decode_set_expert_prefetch(int mode) {

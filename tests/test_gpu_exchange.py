@@ -1,7 +1,9 @@
 """The persistent decode kernels' exchange: whatever the caller's scratch holds on entry, whatever NaN the residual holds, and
 wherever the position falls in the groups of the attention slices (the new row's group is requested later than the rest), the
 results are those of the kernel sequence, bit for bit."""
+import ctypes
 import importlib
+import time
 
 import pytest
 
@@ -86,3 +88,47 @@ def test_logits_scratch_holds_the_last_layers_logits(lkb):
         ds.d_token.fill_(11); ds.step(); torch.cuda.synchronize()
         left.append(ds.logits.clone())
     assert left[0].abs().max() > 0 and torch.equal(*left)
+
+
+@pytest.fixture
+def withheld(lkb):
+    """lkb_debug_fused_withheld(layer, expert, polls): that logit is not published."""
+    lkb.init(0)
+    f = lkb.lib.lkb_debug_fused_withheld
+    f.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_uint]
+    yield f
+    f(-1, 0, 0)
+
+
+@pytest.mark.parametrize("form", ["stack", "step"])
+def test_wait_for_a_word_is_bounded(lkb, withheld, form):
+    """A word that never comes, behind a barrier that everyone has reached: the launch ends with that barrier's code after the caller's
+    limit of polls (16384 are some 10 ms, the default 4 M some seconds), and the next one is right again."""
+    layer = 2
+    if form == "stack":
+        synth = importlib.import_module("lfm2-ampere_b200.synth")
+        st = importlib.import_module("lfm2-ampere_b200.decode").DecodeStack(synth.make_model(4, seed=31))
+        go = st.step_fused
+    else:
+        model = importlib.import_module("lfm2-ampere_b200.model")
+        st = model.DecodeStep(model.make_full_model(n_layers=4, seed=9, vocab=2048), max_seq=16, moe_impl="mega")
+        go = st.step
+    x0 = torch.randn(H, device="cuda", generator=torch.Generator("cuda").manual_seed(6))
+
+    def launch():
+        st.x.copy_(x0)
+        if form == "step":
+            st.d_token.fill_(11); st.d_pos.zero_(); st.hist.zero_()
+        torch.cuda.synchronize()
+        t = time.perf_counter()
+        go()
+        torch.cuda.synchronize()
+        return time.perf_counter() - t
+    launch()
+    good = st.x.clone()
+    assert st.status() == 0 and torch.isfinite(good).all()
+    withheld(layer, 37, 1 << 14)
+    assert launch() < 1.0 and st.status() == 1000 + 10 * layer + 1
+    withheld(-1, 0, 0)
+    launch()
+    assert st.status() == 0 and torch.equal(st.x, good)
