@@ -172,7 +172,8 @@ typedef struct {
  * Caller-owned global scratch of the fused kernels: 64 floats (router logits), 2*4*1536 floats (exchange of the
  * intermediate activations and, in the whole-step kernel, of the residual and the mixers' outputs; any content on entry) and
  * two 32-bit words (barrier counter, status; status != 0 after the kernel means a
- * bounded wait expired: 1000+10*layer+n = grid barrier n, 100/200/300+layer = a copy). */
+ * bounded wait expired: 1000+10*layer+n = grid barrier n or a value published ahead of it, 100/200/300+layer = a copy; x then
+ * holds, row by row, what its CTA had last added up, and nothing else that the launch writes is of use). */
 #define LKB_MOE_SCRATCH_LOGITS 64
 #define LKB_MOE_SCRATCH_GU     (2 * LKB_TOP_K * LKB_MOE_INTER)
 #define LKB_MOE_SCRATCH_SYNC   2

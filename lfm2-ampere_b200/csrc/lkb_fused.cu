@@ -85,6 +85,7 @@ struct FusedSmem {
     int    abort;
     unsigned bar_target;
     unsigned spin_limit;                  // polls a wait for other CTAs may take
+    float *  x_own; int n_own;            // the residual rows this CTA owns, in the caller's vector
     alignas(8) lkb_moe_layer ly;          // this layer's descriptor (staged: a global read costs ~1 us of latency)
     alignas(8) lkb_moe_layer ly_next;     // the next layer's (expert prefetch)
     alignas(8) lkb_mixer_layer mx;        // whole-step kernel: this layer's sequence-mixer descriptor
@@ -215,10 +216,12 @@ __device__ __forceinline__ void grid_arrive(unsigned * bar, FusedSmem & S, bool 
     __syncthreads();                                   // this CTA's global writes are issued
     if (threadIdx.x == 0) grid_arrive_one<RELEASE>(bar, S, release);
 }
-// A CTA that leaves early waits for the copies it has requested (bounded): their destination is its shared memory.
+// A CTA that leaves early waits for the copies it has requested (bounded): their destination is its shared memory.  And the words of
+// its residual rows may be due: what it last added up goes back (nobody gets past the next barrier any more).
 __device__ __noinline__ void fused_drain(FusedSmem & S) {
     asm volatile("cp.async.wait_all;" ::: "memory");                // this thread's requests of K and V
     const int i = threadIdx.x;
+    if (S.abort && i < S.n_own) S.x_own[i] = S.xown[i];
     if (i >= N_GU_CH + N_DN_CH + 3) return;
     FusedBar * const b = i < N_GU_CH ? &S.mbar_gu[i] : i < N_GU_CH + N_DN_CH ? &S.mbar_dn[i - N_GU_CH]
                        : i == N_GU_CH + N_DN_CH ? &S.mbar_rt : i == N_GU_CH + N_DN_CH + 1 ? &S.mbar_mi : &S.mbar_mo;
@@ -485,6 +488,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
         S.abort = 0;
         S.bar_target = 0u;
         S.spin_limit = a.spin_limit;
+        S.x_own = a.x + dn0; S.n_own = n_dn;
 #pragma unroll 1
         for (int i = 0; i < N_GU_CH; ++i) mbar_init(&S.mbar_gu[i]);
 #pragma unroll 1

@@ -129,6 +129,13 @@ def test_wait_for_a_word_is_bounded(lkb, withheld, form):
     assert st.status() == 0 and torch.isfinite(good).all()
     withheld(layer, 37, 1 << 14)
     assert launch() < 1.0 and st.status() == 1000 + 10 * layer + 1
+    left = st.x.clone()                                        # the residual as that layer's FFN found it: nothing still due
     withheld(-1, 0, 0)
     launch()
-    assert st.status() == 0 and torch.equal(st.x, good)
+    assert st.status() == 0 and torch.equal(st.x, good) and torch.isfinite(left).all()
+    if form == "stack":
+        st.x.copy_(x0)
+        for i in range(layer):
+            lkb.moe_ffn_decode(st._descs[i], st.x, None, None, None, st._scratch)
+        torch.cuda.synchronize()
+        assert torch.equal(left, st.x)
