@@ -253,7 +253,7 @@ void prefill_chunk(Engine & e, lk::stream_t st, const int * toks_host, int m, in
             const lk::QT4 segs[2] = {{l.gate_qs, l.gate_d}, {l.up_qs, l.up_d}};
             const int ends[3] = {I, I, I};
             lk::PfGemm g = gemm_desc(segs, 2, ends, I, BPR, e.a_qs, e.a_sc);
-            g.exp_stride = (long long) I * BPR; g.perm = e.perm; g.tiles = e.tiles; g.ntiles = e.ntiles; g.a_shift = 2; g.scale = e.inv;
+            g.ntok = ns; g.exp_stride = (long long) I * BPR; g.perm = e.perm; g.tiles = e.tiles; g.ntiles = e.ntiles; g.a_shift = 2; g.scale = e.inv;
             g.oqs = e.a2_qs; g.osc = e.a2_sc; g.okb = I / 32;
             lk::pf_gemm_swiglu(g, e.max_tiles, st);
         }
@@ -261,7 +261,7 @@ void prefill_chunk(Engine & e, lk::stream_t st, const int * toks_host, int m, in
             const lk::QT4 seg{l.down_qs, l.down_d};
             const int ends[3] = {H, H, H};
             lk::PfGemm g = gemm_desc(&seg, 1, ends, H, I / 32, e.a2_qs, e.a2_sc);
-            g.exp_stride = (long long) H * (I / 32); g.perm = e.perm; g.tiles = e.tiles; g.ntiles = e.ntiles; g.a_shift = 0;
+            g.ntok = ns; g.exp_stride = (long long) H * (I / 32); g.perm = e.perm; g.tiles = e.tiles; g.ntiles = e.ntiles; g.a_shift = 0;
             g.out = e.D; g.out_ld = H;
             lk::pf_gemm_moe(g, e.max_tiles, st);
         }

@@ -82,7 +82,7 @@ typedef struct {
     long long      exp_stride;   /* blocks per expert, 0 if dense */
     const int8_t * aqs;          /* activations, row pitch bpr*32: 16-byte aligned */
     const float *  asc;          /* float2 [rows][bpr]: 16-byte aligned for the tensor-core form */
-    int            ntok;         /* dense: token rows */
+    int            ntok;         /* dense: token rows; MoE: the slots in perm, 0 = not stated (chooses the form, see lkb_pf_gemm_config) */
     const int *    perm;         /* MoE: slot ids grouped by expert, or null */
     const int *    tiles;        /* MoE: int4 {expert, start in perm, count, 0} */
     const int *    ntiles;       /* MoE: device-side tile count */
@@ -338,8 +338,10 @@ int lkb_pf_gemm_dense(const lkb_pf_gemm * g, lkb_stream_t st);
 int lkb_pf_gemm_moe(const lkb_pf_gemm * g, int max_tiles, lkb_stream_t st);
 int lkb_pf_gemm_swiglu(const lkb_pf_gemm * g, int max_tiles, lkb_stream_t st);
 /* Kernel-configuration selector of the three launchers above: -1 (default) the
- * tensor-core form wherever it covers the shape, 0 the CUDA-core form, 1 the
- * tensor-core form or an error.  Also read once from the environment variable
+ * tensor-core form wherever it covers the shape, and for a few tokens -- dense up to 4, MoE up to 188
+ * slots (g->ntok) with max_tiles >= 64 -- a form that streams the weights once; 0 the CUDA-core form, 1 the
+ * tensor-core form or an error.  The results are the same bits in every form.  max_tiles bounds the tiles the plan may
+ * have and says nothing about how full they are.  Also read once from the environment variable
  * LKB_PF_CFG by lkb_init().  ref: src/prefill.cu:813-848 (LK_PF_CFG_DENSE/MOE/SWIGLU) */
 int lkb_pf_gemm_config(int cfg);
 /* Per-block term of the three launchers above.  1 (default): the reference's shipped form -- the block sum

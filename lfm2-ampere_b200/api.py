@@ -222,7 +222,7 @@ def k_pf_moe_scatter(idx, n, off, perm):
 
 def make_pf_gemm(segs, seg_end, N, bpr, aqs, asc, *, ntok=0, exp_stride=0, perm=None, tiles=None, ntiles=None,
                  a_shift=0, scale=None, out=None, out_ld=0, add=0, oqs=None, osc=None, okb=0):
-    """lkb_pf_gemm from tensors; segs = [(qs, d), ...] (1 to 3 stacked weight tensors)."""
+    """lkb_pf_gemm from tensors; segs = [(qs, d), ...] (1 to 3 stacked weight tensors); ntok = token rows, with perm its slots (0: not stated)."""
     g = PfGemm()
     for i in range(3):
         q, d = segs[min(i, len(segs) - 1)]

@@ -29,12 +29,12 @@
 #define FW_WS     4                  // pairs of stages of weight scales
 #define FW_CTAS   3                  // per SM
 #define FW_WARPS  4                  // dot warps; warp 4 fetches
-// Where the forms cross.  Grouped: the plan tiles the caller allows for, which without the counts on the host is one per expert and one per
-// 64 slots: 64 .. 66 is up to 47 tokens of four slots (the crossing is near 45 tokens with skewed routing and near 75 with
-// balanced); fewer than 64 say nothing about how full the tiles are.  Dense: a projection of 2048 rows is 8 items
+// Where the forms cross.  Grouped: by the slots the caller states, spread over 64 experts: the crossing is near 45 tokens of four slots with
+// skewed routing and near 75 with balanced.  A plan that cannot have a tile per expert is one of fewer experts, whose tiles may be
+// full; it takes the other form, as does a call that does not state its slots.  Dense: a projection of 2048 rows is 8 items
 // here and the chain of its 64 blocks shows: 2 tokens 85 against 88 us a layer, 9 tokens 104 against 100.
 #define FW_MIN_TILES LKB_N_EXPERTS
-#define FW_MAX_TILES (LKB_N_EXPERTS + 2)
+#define FW_MAX_SLOTS (47 * LKB_TOP_K)
 #define FW_MAX_DENSE 4
 static_assert(2 * FW_WS >= FW_NS + 4, "weight scales stay until their stages have been read");
 
@@ -236,10 +236,16 @@ int lkb_gemm_few_init() {
 }
 int lkb_gemm_few_take_status() { return tc_take_status(); }
 
+static bool fw_better(const lkb_pf_gemm * g, int max_tiles) {
+    return g->perm ? max_tiles >= FW_MIN_TILES && g->ntok > 0 && g->ntok <= FW_MAX_SLOTS : g->ntok <= FW_MAX_DENSE;
+}
+// Test hook (not in the public header): whether a call of few tokens takes this form by itself, if its planes allow it.
+extern "C" __attribute__((visibility("default"))) int lkb_debug_gemm_few_better(const lkb_pf_gemm * g, int max_tiles) { return fw_better(g, max_tiles); }
+
 // LKB_ERR_UNSUPPORTED where another form is the better one or the planes do not have the alignment the copies ask for.
 int lkb_gemm_few_launch(const lkb_pf_gemm * g, int epi, int fold, int max_tiles, cudaStream_t st) {
     if (!lkb_tensor_map_encoder()) return LKB_ERR_UNSUPPORTED;
-    if (g->perm ? max_tiles < FW_MIN_TILES || max_tiles > FW_MAX_TILES : g->ntok > FW_MAX_DENSE) return LKB_ERR_UNSUPPORTED;
+    if (!fw_better(g, max_tiles)) return LKB_ERR_UNSUPPORTED;
     if (epi ? (g->N % FW_ROWS) : (g->N % (2 * FW_ROWS))) return LKB_ERR_UNSUPPORTED;
     if (g->bpr % 8 || (((size_t) g->aqs | (size_t) g->asc) & 15) || g->exp_stride % g->bpr) return LKB_ERR_UNSUPPORTED;
     const int nseg = epi ? 2 : (g->seg_end[0] >= g->N ? 1 : g->seg_end[1] >= g->N ? 2 : 3);

@@ -69,11 +69,11 @@ class PrefillStack:
         api.k_pf_router_select(self.h32, m, m <= 256, l.router, l.rbias, self.inv, self.sel, self.sig, self.idx, self.w)
         api.k_pf_moe_route(self.idx, self.ns, self.cnt, self.off, self.tiles, self.ntiles, self.perm)
         g = api.make_pf_gemm([(l.gate_qs, l.gate_d), (l.up_qs, l.up_d)], [I, I, I], I, H // 32, self.a_qs, self.a_sc,
-                             exp_stride=I * (H // 32), perm=self.perm, tiles=self.tiles, ntiles=self.ntiles,
+                             ntok=self.ns, exp_stride=I * (H // 32), perm=self.perm, tiles=self.tiles, ntiles=self.ntiles,
                              a_shift=2, scale=self.inv, oqs=self.a2_qs, osc=self.a2_sc, okb=I // 32)
         _timed(self, api.pf_gemm_swiglu, g, self.max_tiles)
         dn = api.make_pf_gemm([(l.down_qs, l.down_d)], [H, H, H], H, I // 32, self.a2_qs, self.a2_sc,
-                              exp_stride=H * (I // 32), perm=self.perm, tiles=self.tiles, ntiles=self.ntiles,
+                              ntok=self.ns, exp_stride=H * (I // 32), perm=self.perm, tiles=self.tiles, ntiles=self.ntiles,
                               a_shift=0, out=self.D, out_ld=H)
         _timed(self, api.pf_gemm_moe, dn, self.max_tiles)
         if next_norm_w is None:

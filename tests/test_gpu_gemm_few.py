@@ -2,6 +2,8 @@
 chunks of eight and the row gathers' groups of four, tiles of more than one chunk, the shortest K and an odd number of stage
 pairs, one and several items a CTA, weight segments, residual add.  Bit for bit against the CPU checker; the fused SwiGLU form
 against the CUDA-core form (itself checked in test_gpu_prefill.py)."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -10,8 +12,8 @@ from helpers import act_floats, dev, host, nan_f32, rand_q4
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
-MAX_TILES = 65                                          # what a caller passes for a few tokens: one tile per expert, one per 64 slots
-COUNTS = [1, 2, 3, 4, 5, 7, 8, 9, 0, 12, 16, 17, 40, 64, 66]
+MAX_TILES = 66                                          # what a caller passes for a few tokens: one tile per expert, one per 64 slots
+COUNTS = [1, 2, 3, 4, 5, 7, 8, 9, 0, 12, 16, 17, 38, 66]   # 188 slots: the most this form takes
 
 
 @pytest.fixture(params=[0, 1], ids=["exact", "fold"])
@@ -34,7 +36,12 @@ def _plan(rng):
     for e, c in enumerate(COUNTS):
         tiles += [[e, off + k, min(64, c - k), 0] for k in range(0, c, 64)]
         off += c
+    assert perm.size == 188
     return perm, np.array(tiles, np.int32)
+
+
+def _takes(L, g, max_tiles=MAX_TILES):
+    return L.lib.lkb_debug_gemm_few_better(ctypes.byref(g), max_tiles) == 1
 
 
 @pytest.mark.parametrize("m", [1, 2, 3, 4])
@@ -46,7 +53,9 @@ def test_dense(L, orc, m, N, ends, bpr):
     aq, asc = orc.pf_quant_rows(act_floats(rng, m * bpr * 32).reshape(m, bpr * 32), bpr)
     o0 = rng.uniform(-1, 1, size=(m, N)).astype(np.float32)
     out = dev(o0)
-    L.pf_gemm_dense(L.make_pf_gemm([(dev(qs[c]), dev(d[c])) for c in cut], list(ends), N, bpr, dev(aq), dev(asc), ntok=m, out=out, out_ld=N, add=1))
+    g = L.make_pf_gemm([(dev(qs[c]), dev(d[c])) for c in cut], list(ends), N, bpr, dev(aq), dev(asc), ntok=m, out=out, out_ld=N, add=1)
+    assert _takes(L, g)
+    L.pf_gemm_dense(g)
     ref = orc.pf_gemm([(qs[c], d[c]) for c in cut], list(ends), N, bpr, aq, asc, ntok=m, out_init=o0, add=1)
     assert np.array_equal(host(out), ref)
 
@@ -59,8 +68,9 @@ def test_grouped(L, orc, N, bpr):
     qs, d = rand_q4(rng, E * N, bpr, "ref")
     aq, asc = orc.pf_quant_rows(act_floats(rng, ns * bpr * 32).reshape(ns, bpr * 32), bpr)
     out = nan_f32(ns, N)
-    g = L.make_pf_gemm([(dev(qs), dev(d))], [N] * 3, N, bpr, dev(aq), dev(asc), exp_stride=N * bpr, perm=dev(perm), tiles=dev(tiles),
+    g = L.make_pf_gemm([(dev(qs), dev(d))], [N] * 3, N, bpr, dev(aq), dev(asc), ntok=ns, exp_stride=N * bpr, perm=dev(perm), tiles=dev(tiles),
                        ntiles=dev(np.array([len(tiles)], np.int32)), out=out, out_ld=N)
+    assert _takes(L, g)
     L.pf_gemm_moe(g, MAX_TILES)
     ref = orc.pf_gemm([(qs, d)], [N] * 3, N, bpr, aq, asc, exp_stride=N * bpr, perm=perm, tiles=tiles, out_rows=ns)
     assert np.array_equal(host(out), ref)
@@ -82,8 +92,10 @@ def test_swiglu(L, orc, I, bpr):
     for cfg in (0, -1):
         L.pf_gemm_config(cfg)
         oqs, osc = torch.full((ns, I), 0x5A, dtype=torch.int8, device="cuda"), nan_f32(ns, I // 32, 2)
-        L.pf_gemm_swiglu(L.make_pf_gemm(w, [I] * 3, I, bpr, aq, asc, exp_stride=I * bpr, perm=dperm, tiles=dtiles, ntiles=dnt,
-                                        a_shift=2, scale=scale, oqs=oqs, osc=osc, okb=I // 32), MAX_TILES)
+        g = L.make_pf_gemm(w, [I] * 3, I, bpr, aq, asc, ntok=ns, exp_stride=I * bpr, perm=dperm, tiles=dtiles, ntiles=dnt,
+                           a_shift=2, scale=scale, oqs=oqs, osc=osc, okb=I // 32)
+        assert _takes(L, g)
+        L.pf_gemm_swiglu(g, MAX_TILES)
         got.append((oqs, osc))
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
     assert int(got[1][0].float().abs().max()) > 0
