@@ -800,6 +800,12 @@ static TcDense tc_dense_form(int ntok, int N, int sms) {
     return best;
 }
 
+// Test hook (not in the public header): the items a dense problem is cut into, tokens * 1000 + weight rows.
+extern "C" __attribute__((visibility("default"))) int lkb_debug_gemm_dense_item(int ntok, int N) {
+    const TcDense d = tc_dense_form(ntok, N, lkb_context().sm_count);
+    return d.tw * 1000 + (d.wide ? 2 : 1) * TC_ROWS;
+}
+
 // Shapes the tensor-core form covers; otherwise LKB_ERR_UNSUPPORTED (the caller falls back to the CUDA-core form): the
 // planes must have the alignment the copies ask for.
 int lkb_gemm_tc_launch(const lkb_pf_gemm * g, int epi, int fold, int max_tiles, cudaStream_t st, float * const * out_rows, int a_pitch) {

@@ -51,6 +51,23 @@ def test_dense(L, orc, m, N, bpr):
     assert np.array_equal(host(out), ref)
 
 
+@pytest.mark.parametrize("item,N,ends,m,bpr", [
+    ((16, 256), 2176, (2176,) * 3, 161, 24), ((32, 128), 1152, (1152,) * 3, 497, 8), ((32, 256), 2176, (2176,) * 3, 305, 8),
+    ((32, 256), 3072, (2048, 2560, 3072), 289, 16), ((48, 256), 3072, (2048, 2560, 3072), 401, 8), ((48, 256), 2176, (2176,) * 3, 593, 24),
+    ((64, 256), 3072, (2048, 2560, 3072), 577, 8), ((64, 256), 6272, (6272,) * 3, 289, 8)])
+def test_dense_items(L, orc, item, N, ends, m, bpr):
+    """The items that a dense problem is cut into to fill the waves: each width and height, with the last token item short, a last row item of
+    one tile where N has an odd number of them, and weight segments that end inside and between row items."""
+    assert L.sm_count() != 148 or L.lib.lkb_debug_gemm_dense_item(m, N) == item[0] * 1000 + item[1]
+    rng = np.random.default_rng(m + N)
+    qs, d = rand_q4(rng, N, bpr, "ref")
+    cut = [slice(a, b) for a, b in zip((0,) + ends[:2], ends) if b > a]
+    aq, asc = orc.pf_quant_rows(act_floats(rng, m * bpr * 32).reshape(m, bpr * 32), bpr)
+    out = nan_f32(m, N)
+    L.pf_gemm_dense(L.make_pf_gemm([(dev(qs[c]), dev(d[c])) for c in cut], list(ends), N, bpr, dev(aq), dev(asc), ntok=m, out=out, out_ld=N))
+    assert np.array_equal(host(out), orc.pf_gemm([(qs[c], d[c]) for c in cut], list(ends), N, bpr, aq, asc, ntok=m))
+
+
 @pytest.mark.parametrize("N,bpr", [(128, 8), (384, 24), (2560, 8)])
 def test_grouped(L, orc, N, bpr):
     rng = np.random.default_rng(N)
