@@ -203,7 +203,7 @@ typedef struct {
     const void *  out_qs; const void * out_d;       /* out_proj / attn_output, 2048 x 2048 */
 } lkb_mixer_layer;
 /* Caller-owned global scratch of the whole-step kernel, beside lkb_moe_scratch. */
-#define LKB_STEP_SCRATCH_MX   3072                  /* floats: q | k | v of an attention layer, or the conv output */
+#define LKB_STEP_SCRATCH_MX   3072                  /* floats: q | k | v of an attention layer (with expert prefetch also the mixers' outputs) */
 #define LKB_STEP_SCRATCH_PART (32 * 18 * 66)        /* floats: attention partials */
 typedef struct {
     float * mx;

@@ -347,7 +347,7 @@ __device__ __forceinline__ void load4(const float * __restrict__ p, float (&o)[4
 }
 // Q8_1 of the block this lane's group of 8 holds -> S.xq[tid >> 3]
 // (Out of line, as the requests of the mixers' rows: a layer is straight-line code that every warp runs once, and the whole-step kernel
-// is larger than the instruction cache.  Four call sites: 130 -> 121 KB, two tokens at context 131000 2760 -> 2720 us.)
+// is larger than the instruction cache: 118 KB, 130 before both were.  Together: two tokens at context 131000 2760 -> 2720 us.)
 __device__ __noinline__ uint2 quad_quant(float4 v) {
     __half2 ds;
     const unsigned pk = lkb_quad_quant_ds(v, ds);
@@ -679,7 +679,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
                 if (!grid_wait(a.bar, status, S, 1000u + 10u * l + 5u, a.spin_limit)) return;
                 FUSED_STAMP(21);
                 // merge of the slices: one head per CTA (every CTA reading every partial would cost 150 KB of
-                // L2 sectors per CTA), published through mxbuf like a conv output
+                // L2 sectors per CTA), published like a conv output
                 if (cta < AT_HEADS && tid < AT_D) xch_put<XCH>(m_out + cta * AT_D + tid, at_combine(a.part, cta, tid, seq_len));
                 grid_arrive<!XCH>(a.bar, S);
                 if (XCH && warp == 1) xch_due(a.mxbuf + qa0, lane, qa1 - qa0);     // q | k | v: read before the partials' barrier
@@ -1114,7 +1114,6 @@ static int g_fused_ready = 0;
 int lkb_fused_init() {
     const void * kernels[4] = {(const void *) k_moe_ffn_stack<false, false>, (const void *) k_moe_ffn_stack<false, true>,
                                (const void *) k_moe_ffn_stack<true, false>, (const void *) k_moe_ffn_stack<true, true>};
-#pragma unroll 1
     for (const void * k : kernels) {
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sizeof(FusedSmem));
         if (e != cudaSuccess) return -(int) e;

@@ -15,7 +15,10 @@
 // Measured, a whole MoE layer of 64 experts at 2 / 9 / 20 / 37 / 64 tokens, us (router, norms and routing included):
 //   tensor-core form   55 / 92 / 120 / 140 / 152 with balanced routing    54 / 88 / 112 / 127 / 147 with Zipf(1.1) routing
 //   this form          47 / 63 /  87 / 113 / 145                          45 / 62 /  87 / 118 / 158
-// What bounds it: at 37 tokens about 205 MB of gate|up weights in 45 us (4.5 TB/s); the dots, two cycles an instruction, from there on.
+// What bounds it: whole waves of items.  gate|up, caches flushed before every call, CUDA events: 28 / 48 / 61 of 64 experts hit by 9 / 20 / 37 tokens
+// are 99 / 170 / 216 MB in 32 / 50 / 62 us, 3.1 to 3.5 TB/s (tensor-core form 46 / 58 / 69 us), down 50 / 85 / 108 MB in 22 / 30 / 40 us.  At 20 tokens
+// that is 576 gate|up items on 444 CTAs, 1.3 waves, and 0.9 of a wave of down items: a third of the CTA time is idle, and
+// the dots wait for their stages (ncu: long scoreboard first, issue 40 %).  From 37 tokens on the dots, two cycles an instruction, count too.
 // Tried: 128 bytes of a row per stage (37 tokens +15 %), tiles of 64 and 32 rows with more CTAs (+35 %), two stages and four
 // CTAs (+4 %), one CTA of five stages (+29 %).
 // No copy in this file is a multicast one; every tensor map covers memory of the GPU the kernel runs on.
@@ -32,7 +35,8 @@
 // Where the forms cross.  Grouped: by the slots the caller states, spread over 64 experts: the crossing is near 45 tokens of four slots with
 // skewed routing and near 75 with balanced.  A plan that cannot have a tile per expert is one of fewer experts, whose tiles may be
 // full; it takes the other form, as does a call that does not state its slots.  Dense: a projection of 2048 rows is 8 items
-// here and the chain of its 64 blocks shows: 2 tokens 85 against 88 us a layer, 9 tokens 104 against 100.
+// here and the chain of its 64 blocks shows, more from the second row gather on.  A whole layer (grouped part here both times) at
+// 2 / 3 / 4 / 5 / 6 / 7 / 9 tokens: 71.2 / 71.6 / 73.2 / 82.4 / 85.1 / 93.6 / 98.9 us dense here, 73.8 / 76.7 / 79.4 / 82.7 / 85.4 / 89.0 / 94.1 there.
 #define FW_MIN_TILES LKB_N_EXPERTS
 #define FW_MAX_SLOTS (47 * LKB_TOP_K)
 #define FW_MAX_DENSE 4
@@ -250,7 +254,7 @@ int lkb_gemm_few_launch(const lkb_pf_gemm * g, int epi, int fold, int max_tiles,
     if (g->bpr % 8 || (((size_t) g->aqs | (size_t) g->asc) & 15) || g->exp_stride % g->bpr) return LKB_ERR_UNSUPPORTED;
     const int nseg = epi ? 2 : (g->seg_end[0] >= g->N ? 1 : g->seg_end[1] >= g->N ? 2 : 3);
     for (int s = 0; s < nseg; ++s) if (((size_t) g->qs[s] | (size_t) g->d[s]) & 15) return LKB_ERR_UNSUPPORTED;
-    // a stage takes 64 bytes of a row; fetched 256 at a time by L2: 57 against 69 us for gate|up at 37 tokens
+    // a stage takes 64 bytes of a row; fetched 256 at a time by L2 gate|up at 37 tokens took 12 us less
     const CUtensorMapL2promotion l2 = CU_TENSOR_MAP_L2_PROMOTION_L2_256B;
     const unsigned long long any = 1ull << 30;              // row bound of a plane whose extent the caller does not state: it only clips
     CUtensorMap ma, ms, mw[3], md[3];

@@ -40,7 +40,7 @@
 //   ... weight scales in a ring of their own, expansion a stage at a time, no scale barriers, two issuers (this form)
 //                                                    70 / 117 / 569         47 /  64 / 268           23 / 51 / 238
 //   ... dense items cut to fill the waves (tc_dense_form)                                            20 / 45 / 236
-// (by itself the launcher takes this form for 48 tokens and more, the few-token form of lkb_gemm_few.cu below)
+// (by itself the launcher takes this form above 188 slots (47 tokens of four) grouped and above 4 tokens dense, below them that of lkb_gemm_few.cu)
 // With few tokens the hand-over of every block is the bound (300 to 440 cycles of polls, commits and arrivals).
 // No copy in this file is a multicast one; every tensor map covers memory of the GPU the kernel runs on.
 // Every wait is bounded; on expiry a status word is set and all roles drain and exit, freeing TMEM.
@@ -783,7 +783,8 @@ int lkb_tc_make_map(CUtensorMap * m, const void * base, unsigned row_bytes, unsi
 #define TC_ANY_ROWS (1ull << 30)            // row bound of a plane whose extent the caller does not state: it only clips
 
 // Items of a dense problem: the token width and height that need the least time, waves of items times an item's.  A block of an item
-// takes about 330 + 6 N cycles with one tile and 350 + 6.2 N with two (measured, N = 16 .. 64), so a problem of less than a wave is
+// takes about 330 + 6 N cycles with one tile and 350 + 6.2 N with two (measured at N = 16 .. 64 and 64 blocks a row; what an item takes besides its blocks is
+// left out, and weighs more where a row has fewer), so a problem of less than a wave is
 // cut into narrow items (each reads the weights again, from L2), and one that would leave most of its last wave empty is cut
 // so that the waves fill.  us with 64-token items and with these, caches flushed: in_proj (6144 rows) at 37 / 130 / 509 tokens
 // 22.5 / 26.6 / 51.2 -> 19.5 / 24.6 / 45.0, out_proj (2048 rows) 24.6 / 26.6 / 28.7 -> 18.4 / 20.5 / 26.6; at 4096 tokens the
