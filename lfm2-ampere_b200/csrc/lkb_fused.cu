@@ -1189,7 +1189,7 @@ int lkb_decode_expert_prefetch_hits(const lkb_moe_scratch * scratch, int n_layer
     if (!scratch || !scratch->gu || !hits || !guesses) return LKB_ERR_NULL;
     if (n_layers < 2) return LKB_ERR_SHAPE;
     const int nl = n_layers < PF_MAXL ? n_layers : PF_MAXL;
-    static int rec[2][4 * PF_MAXL];
+    int rec[2][4 * PF_MAXL];
     cudaError_t e = cudaStreamSynchronize((cudaStream_t) st);
     if (e == cudaSuccess) e = cudaMemcpy(rec[0], scratch->gu + PF_GUESS_OFF, sizeof(int) * 4 * nl, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = cudaMemcpy(rec[1], scratch->gu + PF_REAL_OFF, sizeof(int) * 4 * nl, cudaMemcpyDeviceToHost);
