@@ -58,6 +58,11 @@ static_assert(XCH_M_OFF + LKB_HIDDEN <= XCH_L_OFF && XCH_L_OFF + 2 * LKB_N_EXPER
 static_assert(MAX_DN_ROWS <= FUSED_WARPS, "a down row per warp");
 static_assert(PF_REAL_OFF + 4 * PF_MAXL <= 2 * LKB_TOP_K * LKB_MOE_INTER, "prefetch records must fit the gu scratch");
 
+#define MB_DN   N_GU_CH                         // the first down chunk's barrier (the gate|up chunks' are in front)
+#define MB_RT   (MB_DN + N_DN_CH)
+#define MB_MI   (MB_RT + 1)
+#define MB_MO   (MB_MI + 1)
+#define N_BARS  (MB_MO + 1)
 struct FusedBar { unsigned long long m; unsigned issued; };     // an mbarrier and how many of its phases copies have been requested for
 
 struct FusedSmem {
@@ -89,8 +94,7 @@ struct FusedSmem {
     alignas(8) lkb_moe_layer ly;          // this layer's descriptor (staged: a global read costs ~1 us of latency)
     alignas(8) lkb_moe_layer ly_next;     // the next layer's (expert prefetch)
     alignas(8) lkb_mixer_layer mx;        // whole-step kernel: this layer's sequence-mixer descriptor
-    FusedBar mbar_mi, mbar_mo;            // whole-step kernel: mixer input rows / output rows staged
-    FusedBar mbar_gu[N_GU_CH], mbar_dn[N_DN_CH], mbar_rt;
+    FusedBar mbar[N_BARS];                // gate|up chunks, down chunks, router row, whole-step kernel: mixer input rows / output rows
 };
 
 // ---- PTX wrappers -----------------------------------------------------------
@@ -222,9 +226,8 @@ __device__ __noinline__ void fused_drain(FusedSmem & S) {
     asm volatile("cp.async.wait_all;" ::: "memory");                // this thread's requests of K and V
     const int i = threadIdx.x;
     if (S.abort && i < S.n_own) S.x_own[i] = S.xown[i];
-    if (i >= N_GU_CH + N_DN_CH + 3) return;
-    FusedBar * const b = i < N_GU_CH ? &S.mbar_gu[i] : i < N_GU_CH + N_DN_CH ? &S.mbar_dn[i - N_GU_CH]
-                       : i == N_GU_CH + N_DN_CH ? &S.mbar_rt : i == N_GU_CH + N_DN_CH + 1 ? &S.mbar_mi : &S.mbar_mo;
+    if (i >= N_BARS) return;
+    FusedBar * const b = &S.mbar[i];
     const unsigned n = b->issued;
 #pragma unroll 1
     for (unsigned k = 0; n && k < 4096u && !mbar_try_wait(b, (n - 1u) & 1u); ++k) { }
@@ -430,15 +433,15 @@ static_assert(sizeof(AtSmem2) <= offsetof(FusedSmem, router), "attention staging
 __device__ __noinline__ void mix_issue_in(FusedSmem & S, const lkb_mixer_layer & mx, int dn0, int n_dn, int a0, int a1) {
     fence_proxy_async();
     if (!mx.is_attn) {
-        mbar_expect_tx(&S.mbar_mi, 3u * (unsigned) n_dn * GU_BPR * 18u);
+        mbar_expect_tx(&S.mbar[MB_MI], 3u * (unsigned) n_dn * GU_BPR * 18u);
 #pragma unroll 1
         for (int s = 0; s < 3; ++s) {
             const size_t blk = ((size_t) s * LKB_HIDDEN + dn0) * GU_BPR;
-            bulk_g2s(S.gu_q + (size_t) s * n_dn * GU_BPR * 16, (const uint4 *) mx.in_qs + blk, (unsigned) n_dn * GU_BPR * 16u, &S.mbar_mi);
-            bulk_g2s(S.gu_d + (size_t) s * n_dn * GU_BPR, (const __half *) mx.in_d + blk, (unsigned) n_dn * GU_BPR * 2u, &S.mbar_mi);
+            bulk_g2s(S.gu_q + (size_t) s * n_dn * GU_BPR * 16, (const uint4 *) mx.in_qs + blk, (unsigned) n_dn * GU_BPR * 16u, &S.mbar[MB_MI]);
+            bulk_g2s(S.gu_d + (size_t) s * n_dn * GU_BPR, (const __half *) mx.in_d + blk, (unsigned) n_dn * GU_BPR * 2u, &S.mbar[MB_MI]);
         }
     } else {
-        mbar_expect_tx(&S.mbar_mi, (unsigned) (a1 - a0) * GU_BPR * 18u);
+        mbar_expect_tx(&S.mbar[MB_MI], (unsigned) (a1 - a0) * GU_BPR * 18u);
         unsigned char * sq = S.gu_q; __half * sd = S.gu_d;
 #pragma unroll 1
         for (int g = a0; g < a1; ) {
@@ -449,8 +452,8 @@ __device__ __noinline__ void mix_issue_in(FusedSmem & S, const lkb_mixer_layer &
             const void * q = seg == 0 ? mx.wq_qs : (seg == 1 ? mx.wk_qs : mx.wv_qs);
             const void * d = seg == 0 ? mx.wq_d : (seg == 1 ? mx.wk_d : mx.wv_d);
             const size_t blk = (size_t) (g - base) * GU_BPR;
-            bulk_g2s(sq, (const uint4 *) q + blk, (unsigned) n * GU_BPR * 16u, &S.mbar_mi);
-            bulk_g2s(sd, (const __half *) d + blk, (unsigned) n * GU_BPR * 2u, &S.mbar_mi);
+            bulk_g2s(sq, (const uint4 *) q + blk, (unsigned) n * GU_BPR * 16u, &S.mbar[MB_MI]);
+            bulk_g2s(sd, (const __half *) d + blk, (unsigned) n * GU_BPR * 2u, &S.mbar[MB_MI]);
             sq += (size_t) n * GU_BPR * 16; sd += (size_t) n * GU_BPR; g += n;
         }
     }
@@ -458,9 +461,9 @@ __device__ __noinline__ void mix_issue_in(FusedSmem & S, const lkb_mixer_layer &
 // One thread: request this CTA's rows [dn0, dn0+n_dn) of the mixer's output projection.
 __device__ __noinline__ void mix_issue_out(FusedSmem & S, const lkb_mixer_layer & mx, int dn0, int n_dn) {
     fence_proxy_async();
-    mbar_expect_tx(&S.mbar_mo, (unsigned) n_dn * GU_BPR * 18u);
-    bulk_g2s(S.dn_q, (const uint4 *) mx.out_qs + (size_t) dn0 * GU_BPR, (unsigned) n_dn * GU_BPR * 16u, &S.mbar_mo);
-    bulk_g2s(S.dn_d, (const __half *) mx.out_d + (size_t) dn0 * GU_BPR, (unsigned) n_dn * GU_BPR * 2u, &S.mbar_mo);
+    mbar_expect_tx(&S.mbar[MB_MO], (unsigned) n_dn * GU_BPR * 18u);
+    bulk_g2s(S.dn_q, (const uint4 *) mx.out_qs + (size_t) dn0 * GU_BPR, (unsigned) n_dn * GU_BPR * 16u, &S.mbar[MB_MO]);
+    bulk_g2s(S.dn_d, (const __half *) mx.out_d + (size_t) dn0 * GU_BPR, (unsigned) n_dn * GU_BPR * 2u, &S.mbar[MB_MO]);
 }
 
 template <bool MIX, bool PF>
@@ -490,12 +493,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
         S.spin_limit = a.spin_limit;
         S.x_own = a.x + dn0; S.n_own = n_dn;
 #pragma unroll 1
-        for (int i = 0; i < N_GU_CH; ++i) mbar_init(&S.mbar_gu[i]);
-#pragma unroll 1
-        for (int i = 0; i < N_DN_CH; ++i) mbar_init(&S.mbar_dn[i]);
-        mbar_init(&S.mbar_rt);
-        mbar_init(&S.mbar_mi);
-        mbar_init(&S.mbar_mo);
+        for (int i = 0; i < N_BARS; ++i) mbar_init(&S.mbar[i]);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -503,8 +501,8 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
     const lkb_moe_layer * L = a.layers ? a.layers : &a.one;
     // first layer's router row, first layer's norm weights
     if (cta < LKB_N_EXPERTS && tid == 0) {
-        mbar_expect_tx(&S.mbar_rt, LKB_HIDDEN * 4);
-        bulk_g2s(S.router, L[0].router + (size_t) cta * LKB_HIDDEN, LKB_HIDDEN * 4, &S.mbar_rt);
+        mbar_expect_tx(&S.mbar[MB_RT], LKB_HIDDEN * 4);
+        bulk_g2s(S.router, L[0].router + (size_t) cta * LKB_HIDDEN, LKB_HIDDEN * 4, &S.mbar[MB_RT]);
     }
     float nw[4];
     load4(L[0].norm_w, nw);
@@ -525,8 +523,8 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
             reinterpret_cast<unsigned long long *>(&S.ly_next)[tid] = reinterpret_cast<const unsigned long long *>(&L[1])[tid];
         if (pcta) {
             if (tid == 0) {
-                mbar_expect_tx(&S.mbar_rt, LKB_HIDDEN * 4);
-                bulk_g2s(S.router, L[1].router + (size_t) (cta - LKB_N_EXPERTS) * LKB_HIDDEN, LKB_HIDDEN * 4, &S.mbar_rt);
+                mbar_expect_tx(&S.mbar[MB_RT], LKB_HIDDEN * 4);
+                bulk_g2s(S.router, L[1].router + (size_t) (cta - LKB_N_EXPERTS) * LKB_HIDDEN, LKB_HIDDEN * 4, &S.mbar[MB_RT]);
             }
             load4(L[1].norm_w, pnw);
         }
@@ -614,7 +612,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
                 const float ninv = S.inv;
                 const int nrows = is_attn ? (qa1 - qa0) : 3 * n_dn;
                 float * mixv = &S.dot[0][0];
-                if (!mbar_wait(&S.mbar_mi, par)) { if (lane == 0) { atomicCAS(status, 0u, 400u + l); S.abort = 1; } }
+                if (!mbar_wait(&S.mbar[MB_MI], par)) { if (lane == 0) { atomicCAS(status, 0u, 400u + l); S.abort = 1; } }
                 else {
 #pragma unroll 1
                     for (int j = warp; j < nrows; j += FUSED_WARPS) {
@@ -695,7 +693,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
                 FUSED_STAMP(22);
                 int xq[2][8]; float d8[2], s8[2];
                 load_xregs<2>(S.xq, GU_BPR, lane, xq, d8, s8);
-                if (!mbar_wait(&S.mbar_mo, par)) { if (lane == 0) { atomicCAS(status, 0u, 500u + l); S.abort = 1; } }
+                if (!mbar_wait(&S.mbar[MB_MO], par)) { if (lane == 0) { atomicCAS(status, 0u, 500u + l); S.abort = 1; } }
                 else {
                     if (const int j = warp; j < n_dn) {                     // n_dn <= MAX_DN_ROWS = FUSED_WARPS
                         const float acc = lkb_warp_sum(smem_row_partial<2>(S.dn_q + (size_t) j * GU_BPR * 16, S.dn_d + (size_t) j * GU_BPR,
@@ -721,7 +719,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
         if ((lane & 7) == 0) S.ssq[tid >> 3] = sq;
         if (pcta && pf_next) {
             // the next layer's router row (cta - 64) against this layer's input under the next layer's norm weights
-            if (!mbar_wait(&S.mbar_rt, par)) { if (lane == 0) { atomicCAS(status, 0u, 100u + l); S.abort = 1; } }
+            if (!mbar_wait(&S.mbar[MB_RT], par)) { if (lane == 0) { atomicCAS(status, 0u, 100u + l); S.abort = 1; } }
             else {
                 float acc = 0.0f;
 #pragma unroll
@@ -737,7 +735,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
             const float inv = lkb_norm_inv(S.ssq, lane, LKB_EPS);
             float acc = 0.0f;
             if (cta < LKB_N_EXPERTS) {
-                if (!mbar_wait(&S.mbar_rt, par)) { if (lane == 0) { atomicCAS(status, 0u, 100u + l); S.abort = 1; } }
+                if (!mbar_wait(&S.mbar[MB_RT], par)) { if (lane == 0) { atomicCAS(status, 0u, 100u + l); S.abort = 1; } }
                 else {
 #pragma unroll 16
                     for (int j = 0; j < LKB_HIDDEN / 32; ++j) acc = fmaf(S.router[j * 32 + lane], S.h[j * 32 + lane], acc);
@@ -867,12 +865,12 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
                     const int j0 = ch * CH_ROWS, j1 = min(n_gu, j0 + CH_ROWS);
                     const int g0 = up * GU_PAIRS + gu0, s0 = up * gu_pad + j0;       // logical rows: gate 0..6143, up 6144..12287
                     issue_gu_rows(ly, S.idx, g0 + j0, g0 + j1, S.gu_q + (size_t) s0 * GU_BPR * 16,
-                                  S.gu_d + (size_t) s0 * GU_BPR, &S.mbar_gu[c]);
+                                  S.gu_d + (size_t) s0 * GU_BPR, &S.mbar[c]);
                 } else {
                     const int cc = c - n_gu_ch, k = cc / dn_ch_per_k, ch = cc % dn_ch_per_k;
                     const int j0 = ch * CH_ROWS, j1 = min(n_dn, j0 + CH_ROWS);
                     const size_t ed = (size_t) S.idx[k] * LKB_HIDDEN * DN_BPR;
-                    FusedBar * mb = &S.mbar_dn[k * dn_ch_per_k + ch];
+                    FusedBar * mb = &S.mbar[MB_DN + k * dn_ch_per_k + ch];
                     mbar_expect_tx(mb, (unsigned) (j1 - j0) * DN_BPR * 18u);
                     bulk_g2s(S.dn_q + ((size_t) k * MAX_DN_ROWS + j0) * DN_BPR * 16,
                              (const uint4 *) ly.down_qs + ed + (size_t) (dn0 + j0) * DN_BPR, (unsigned) (j1 - j0) * DN_BPR * 16u, mb);
@@ -893,7 +891,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
 #pragma unroll 1
             for (int j = warp; j < n_gu; j += FUSED_WARPS) {
                 // both probes are issued before either answer is used (a probe takes ~0.1 us even when the rows are there)
-                FusedBar * const mg = &S.mbar_gu[j / CH_ROWS], * const mu = &S.mbar_gu[gu_half_ch + j / CH_ROWS];
+                FusedBar * const mg = &S.mbar[j / CH_ROWS], * const mu = &S.mbar[gu_half_ch + j / CH_ROWS];
                 const bool hg = mbar_try_wait(mg, par), hu = mbar_try_wait(mu, par);
                 if (__any_sync(LKB_FULL, (!hg && !mbar_wait(mg, par)) || (!hu && !mbar_wait(mu, par)))) {
                     if (lane == 0) { atomicCAS(status, 0u, 200u + l); S.abort = 1; }
@@ -917,8 +915,8 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
         if (l + 1 < a.n_layers) {
             if (cta < LKB_N_EXPERTS && tid == 0) {
                 fence_proxy_async();
-                mbar_expect_tx(&S.mbar_rt, LKB_HIDDEN * 4);
-                bulk_g2s(S.router, L[l + 1].router + (size_t) cta * LKB_HIDDEN, LKB_HIDDEN * 4, &S.mbar_rt);
+                mbar_expect_tx(&S.mbar[MB_RT], LKB_HIDDEN * 4);
+                bulk_g2s(S.router, L[l + 1].router + (size_t) cta * LKB_HIDDEN, LKB_HIDDEN * 4, &S.mbar[MB_RT]);
             }
             load4(L[l + 1].norm_w, nw);
             if constexpr (MIX) {
@@ -932,8 +930,8 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
             FUSED_STAMP1(26);
             if (pcta && l + 2 < a.n_layers && tid == 32) {
                 fence_proxy_async();
-                mbar_expect_tx(&S.mbar_rt, LKB_HIDDEN * 4);
-                bulk_g2s(S.router, L[l + 2].router + (size_t) (cta - LKB_N_EXPERTS) * LKB_HIDDEN, LKB_HIDDEN * 4, &S.mbar_rt);
+                mbar_expect_tx(&S.mbar[MB_RT], LKB_HIDDEN * 4);
+                bulk_g2s(S.router, L[l + 2].router + (size_t) (cta - LKB_N_EXPERTS) * LKB_HIDDEN, LKB_HIDDEN * 4, &S.mbar[MB_RT]);
             }
             // rank the 64 guesses by the rule of the selection: warp 1 forms the keys, thread e counts who beats expert e
             if (warp <= 2) {
@@ -1022,7 +1020,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
         {
             const int j0 = 2 * (warp >> 1), k0 = 2 * (warp & 1);            // n_dn <= MAX_DN_ROWS = FUSED_WARPS
             if (j0 < n_dn) {
-                FusedBar * const m0 = &S.mbar_dn[k0 * dn_ch_per_k + j0 / CH_ROWS], * const m1 = &S.mbar_dn[(k0 + 1) * dn_ch_per_k + j0 / CH_ROWS];
+                FusedBar * const m0 = &S.mbar[MB_DN + k0 * dn_ch_per_k + j0 / CH_ROWS], * const m1 = &S.mbar[MB_DN + (k0 + 1) * dn_ch_per_k + j0 / CH_ROWS];
                 const bool h0 = mbar_try_wait(m0, par), h1 = mbar_try_wait(m1, par);      // both probes in flight, then the bounded waits if needed
                 const bool ok = __all_sync(LKB_FULL, (h0 || mbar_wait(m0, par)) && (h1 || mbar_wait(m1, par)));
                 FUSED_STAMP(15);

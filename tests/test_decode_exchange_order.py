@@ -131,5 +131,4 @@ def test_every_way_out_waits_for_the_copies_in_flight():
     assert "++b->issued;" in announce and SRC.count("mbarrier.arrive.expect_tx") == announce.count("mbarrier.arrive.expect_tx") == 1
     drain = _function("void fused_drain(")
     assert "cp.async.wait_all" in drain
-    for bar in set(re.findall(r"\bmbar_(?:gu|dn|rt|mi|mo)\b", kernel)):
-        assert f"S.{bar}" in drain
+    assert "if (i >= N_BARS) return;" in drain and "&S.mbar[i]" in drain and "FusedBar mbar[N_BARS];" in SRC and SRC.count("FusedBar mbar") == 1
