@@ -86,9 +86,8 @@ __device__ __forceinline__ void lkb_quant_store_planar_fused_epilogue(float xi, 
 // ---------------------------------------------------------------------------
 // Four elements per lane.  A 32-element block lives in 8 adjacent lanes, lane l holding elements 4(l&7) .. +3
 // (one 128-bit load), so a warp covers four blocks = 512 contiguous bytes per step.  The xor-butterfly of the
-// one-element-per-lane form pairs element i with i^16, i^8, i^4, i^2, i^1: here the first three levels are lane
-// exchanges (xor 4, 2, 1, one per held element) and the last two are adds inside the thread, so every partial
-// sum is the same pair of operands as there (fp32 addition is commutative) and the result has the same bits.
+// one-element-per-lane form pairs element i with i^16, i^8, i^4, i^2, i^1: lanes 4, 2 and 1 apart, then elements 2 and 1 apart.
+// Every partial sum is the same pair of operands as there (fp32 addition is commutative), so the result has the same bits.
 // ---------------------------------------------------------------------------
 // A lane hands over half of what it holds per level while there is something to split (lane bit 2 keeps elements 0, 1 or 2, 3,
 // bit 1 one of the two), so the five levels take 6 shuffles and 6 additions where summing all four everywhere takes 12 and 15.

@@ -343,7 +343,7 @@ static int g_fused_prefetch = 0;                 // bit 0: MoE stack, bit 1: who
 // Thread t holds elements 4t .. 4t+3 of a 2048-vector (one 128-bit access): a 32-element block lives in 8 adjacent
 // lanes, a warp covers four blocks, the 16 warps the 64 blocks.  Quantisation and sums of squares go through
 // lkb_quad_quant_ds / lkb_quad_sum, whose pairings are those of the one-element-per-lane butterfly (same bits), with
-// 6 shuffles per block instead of 10 plus a redux, and a reciprocal with an exact fallback instead of 32 divisions.
+// 9 shuffles for four blocks instead of 5 and a redux for each, and a reciprocal with an exact fallback instead of 32 divisions.
 __device__ __forceinline__ void load4(const float * __restrict__ p, float (&o)[4]) {
     const float4 t = reinterpret_cast<const float4 *>(p)[threadIdx.x];
     o[0] = t.x; o[1] = t.y; o[2] = t.z; o[3] = t.w;
