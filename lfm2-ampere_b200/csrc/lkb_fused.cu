@@ -492,8 +492,14 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
         S.bar_target = 0u;
         S.spin_limit = a.spin_limit;
         S.x_own = a.x + dn0; S.n_own = n_dn;
+        if (MIX) {                                                  // (by a thread each as below: more spills in this larger instantiation)
 #pragma unroll 1
-        for (int i = 0; i < N_BARS; ++i) mbar_init(&S.mbar[i]);
+            for (int i = 0; i < N_BARS; ++i) mbar_init(&S.mbar[i]);
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+    }
+    if (!MIX && tid < N_BARS) {                                     // a loop of 23 by one thread: 0.3 us of the one-layer call
+        mbar_init(&S.mbar[tid]);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -744,10 +750,10 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
             }
             if (lane == 0) {
                 S.inv = inv;
+                float v = 0.0f;
                 if (cta < LKB_N_EXPERTS && (!XCH || a.withheld != l * LKB_N_EXPERTS + cta)) {
-                    const float v = __fmul_rn(acc, inv);
+                    v = __fmul_rn(acc, inv);
                     xch_put<XCH>(lg + cta, v);
-                    if (XCH && l + 1 == a.n_layers) a.logits[cta] = v;          // the caller's: nobody reads them here
                 }
                 if (pcta && pf_next) {
                     float g = 0.0f;
@@ -756,6 +762,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1) k_moe_ffn_stack(const FusedA
                     a.gu[PF_LOGITS_OFF + cta - LKB_N_EXPERTS] = g * inv;
                 }
                 grid_arrive_one<!XCH>(a.bar, S, !MIX && l == 0);
+                if (XCH && cta < LKB_N_EXPERTS && l + 1 == a.n_layers) a.logits[cta] = v;      // the caller's: nobody reads them here
             }
         }
         quad_quant_to_xq(S.xq, uv);
