@@ -789,7 +789,7 @@ int lkb_tc_make_map(CUtensorMap * m, const void * base, unsigned row_bytes, unsi
 // so that the waves fill.  us with 64-token items and with these, caches flushed: in_proj (6144 rows) at 37 / 130 / 509 tokens
 // 22.5 / 26.6 / 51.2 -> 19.5 / 24.6 / 45.0, out_proj (2048 rows) 24.6 / 26.6 / 28.7 -> 18.4 / 20.5 / 26.6; at 4096 tokens the
 // choice is 64 x 256 as before.
-static TcDense tc_dense_form(int ntok, int N, int sms) {
+static TcDense tc_dense_form(int ntok, int N, int sms, long long * cost = nullptr) {
     TcDense best = {TC_TOK, 1};
     long long least = 0;
     for (int wide = 1; wide >= 0; --wide)
@@ -798,7 +798,14 @@ static TcDense tc_dense_form(int ntok, int N, int sms) {
             const long long t = (items + sms - 1) / sms * (wide ? 3500 + 62 * tw : 3300 + 60 * tw);
             if (!least || t < least) { least = t; best = {tw, wide}; }
         }
+    if (cost) *cost = least;
     return best;
+}
+// What a block of all its items' waves takes, in ns: the above at 1.87 GHz.
+int lkb_gemm_tc_dense_ns(int ntok, int N, int sms) {
+    long long c = 0;
+    tc_dense_form(ntok, N, sms, &c);
+    return (int) (c * 100 / 1870 < (1 << 30) ? c * 100 / 1870 : 1 << 30);
 }
 
 // Test hook (not in the public header): the items a dense problem is cut into, tokens * 1000 + weight rows.

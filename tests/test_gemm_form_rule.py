@@ -26,3 +26,19 @@ def test_grouped(lkb, slots, max_tiles, few):
 @pytest.mark.parametrize("m", range(1, 10))
 def test_dense(lkb, m):
     assert _better(lkb, ntok=m, perm=None) == (m <= 4)
+
+
+@pytest.mark.parametrize("slots,max_tiles,width", [(4, 64, 16), (188, 66, 16), (189, 66, 16), (800, 76, 16), (801, 76, 32), (1536, 88, 32), (1537, 88, 0), (4096, 128, 0), (0, 66, 0), (400, 63, 0)])
+def test_width_of_grouped_items(lkb, slots, max_tiles, width):
+    g = lkb.PfGemm()
+    g.ntok, g.perm, g.N, g.bpr = slots, 64, 2048, 64
+    assert lkb.lib.lkb_debug_gemm_few_width(ctypes.byref(g), max_tiles, 148) == width
+
+
+@pytest.mark.parametrize("m,N,bpr,width", [(1, 2048, 64, 8), (4, 6144, 8, 8), (5, 2048, 8, 0), (37, 6144, 64, 8), (64, 6144, 64, 16), (128, 6144, 64, 0), (144, 2048, 64, 8), (180, 2048, 64, 16),
+                                           (300, 2048, 64, 0), (4096, 6144, 64, 0)])
+def test_width_of_dense_items(lkb, m, N, bpr, width):
+    """By the waves of items over 148 SMs in either form."""
+    g = lkb.PfGemm()
+    g.ntok, g.N, g.bpr = m, N, bpr
+    assert lkb.lib.lkb_debug_gemm_few_width(ctypes.byref(g), 0, 148) == width
