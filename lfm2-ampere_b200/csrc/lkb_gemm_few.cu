@@ -195,15 +195,19 @@ __device__ __forceinline__ bool fw_store_swiglu(FwSmem<TOK> & S, const int * slo
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
         float x[2][2];                                                   // [row][token]
+        const float s0 = scls[8 * n + 2 * q], s1 = scls[8 * n + 2 * q + 1];
+        const unsigned long long scl = tc_pack(s0, s1);
+        bool sure = true;
 #pragma unroll
-        for (int p = 0; p < 2; ++p) {
-            const float scl = scls[8 * n + 2 * q + p];
+        for (int k = 0; k < 2; ++k) tc_unpack(tc_fmul2(tc_silu2(tc_fmul2(acc[0][n][k], scl), sure), tc_fmul2(acc[1][n][k], scl)), x[k][0], x[k][1]);
+        if (!sure) {
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
                 float gx[2], ux[2];
                 tc_unpack(acc[0][n][k], gx[0], gx[1]);
                 tc_unpack(acc[1][n][k], ux[0], ux[1]);
-                x[k][p] = __fmul_rn(lkb_silu(__fmul_rn(gx[p], scl)), __fmul_rn(ux[p], scl));
+                x[k][0] = __fmul_rn(lkb_silu(__fmul_rn(gx[0], s0)), __fmul_rn(ux[0], s0));
+                x[k][1] = __fmul_rn(lkb_silu(__fmul_rn(gx[1], s1)), __fmul_rn(ux[1], s1));
             }
         }
         v[n][0] = mine ? x[0][1] : x[0][0]; v[n][1] = mine ? x[1][1] : x[1][0];
@@ -483,6 +487,26 @@ static int fw_width(const lkb_pf_gemm * g, int max_tiles, int sms) {
 }
 // Test hook (not in the public header): the items' token width where a call takes this form, if its planes allow it; else 0.
 extern "C" __attribute__((visibility("default"))) int lkb_debug_gemm_few_width(const lkb_pf_gemm * g, int max_tiles, int sms) { return fw_width(g, max_tiles, sms); }
+
+// Test hook (not in the public header): over `count` float bit patterns from `first` on, counts[0] += those whose tc_silu2 is sure of another
+// result than lkb_silu's, counts[1] += those it is not sure of.
+__global__ void k_debug_silu(unsigned first, unsigned long long count, unsigned long long * __restrict__ counts) {
+    unsigned long long wrong = 0, unsure = 0;
+    for (unsigned long long i = blockIdx.x * (unsigned long long) blockDim.x + threadIdx.x; i < count; i += (unsigned long long) gridDim.x * blockDim.x) {
+        const float v = __uint_as_float(first + (unsigned) i);
+        bool sure = true;
+        float q, o;
+        tc_unpack(tc_silu2(tc_pack(v, 1.0f), sure), q, o);
+        unsure += !sure;
+        wrong += sure && __float_as_uint(q) != __float_as_uint(lkb_silu(v));
+    }
+    if (wrong) atomicAdd(counts, wrong);
+    if (unsure) atomicAdd(counts + 1, unsure);
+}
+extern "C" __attribute__((visibility("default"))) int lkb_debug_silu(unsigned first, unsigned long long count, unsigned long long * counts, lkb_stream_t st) {
+    k_debug_silu<<<1184, 256, 0, (cudaStream_t) st>>>(first, count, counts);
+    return lkb_check_launch();
+}
 
 // LKB_ERR_UNSUPPORTED where another form is the better one or the planes do not have the alignment the copies ask for.
 int lkb_gemm_few_launch(const lkb_pf_gemm * g, int epi, int fold, int max_tiles, cudaStream_t st) {

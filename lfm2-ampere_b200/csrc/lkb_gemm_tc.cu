@@ -240,16 +240,28 @@ template <int NC> __device__ __forceinline__ float tc_col(const unsigned long lo
     return (c & 1) ? y : x;
 }
 
+// What lane i knows of token half * NC + i: its slot and its row scale.  Asked for ahead of an item's fold: two loads, one after the other,
+// that the item's store would wait for.
+struct TcTok { int slot; float scl; bool live; };
+template <int NC>
+__device__ __forceinline__ TcTok tc_tok(const lkb_pf_gemm & g, const TcItem & I, int half, int lane) {
+    TcTok K;
+    const int tl = half * NC + lane;
+    K.live = lane < NC && tl < I.tcnt;
+    K.slot = K.live ? (g.perm ? __ldg(g.perm + I.tstart + tl) : I.tstart + tl) : 0;
+    K.scl = (K.live && g.scale) ? __ldg(g.scale + (K.slot >> g.a_shift)) : 1.0f;
+    return K;
+}
+
 // Plain output: lane = weight row, so a token's 32 rows of a warp are one 128-byte store.
 template <int R, int NC>
-__device__ __forceinline__ void tc_store_plain(const lkb_pf_gemm & g, const TcPlan & P, const TcItem & I, float * const * out_rows, int half,
+__device__ __forceinline__ void tc_store_plain(const lkb_pf_gemm & g, const TcPlan & P, const TcItem & I, const TcTok & K, float * const * out_rows, int half,
                                                int row, int lane, const unsigned long long (&acc)[R][NC / 2]) {
-    // lane i: where token half * NC + i goes, and its row scale.  out_rows: a row address of its own per slot (the
-    // expert-parallel form: the row goes straight into its home rank's buffer, a peer's memory included -- plain stores)
-    const int tl = half * NC + lane;
-    const bool live = lane < NC && tl < I.tcnt;
-    const int slot = live ? (g.perm ? __ldg(g.perm + I.tstart + tl) : I.tstart + tl) : 0;
-    const float scl = (live && g.scale) ? __ldg(g.scale + (slot >> g.a_shift)) : 1.0f;
+    // out_rows: a row address of its own per slot (the expert-parallel form: the row goes straight into its home rank's buffer, a
+    // peer's memory included -- plain stores)
+    const bool live = K.live;
+    const int slot = K.slot;
+    const float scl = K.scl;
     const unsigned long long rp = !live ? 0ull : (unsigned long long) (out_rows ? out_rows[slot] : g.out + (size_t) slot * g.out_ld);
     const int o0 = tc_tile_row(P, I.rt, 0) + row;
     const int nlive = I.tcnt - half * NC;                                             // live tokens of this warp
@@ -307,21 +319,32 @@ __device__ __forceinline__ void tc_sum_level(float (&t)[N], int lane) {
 
 // SwiGLU + Q8_1 of NT tokens (columns c0.. of the accumulators): a warp holds one 32-row output block (lane = row).
 template <int FOLD, int NC, int NT>
-__device__ __forceinline__ void tc_store_swiglu(const lkb_pf_gemm & g, const TcItem & I, int half, int c0, int quad, int lane,
+__device__ __forceinline__ void tc_store_swiglu(const lkb_pf_gemm & g, const TcItem & I, const TcTok & K, int half, int c0, int quad, int lane,
                                                 const unsigned long long (&acc)[2][NC / 2]) {
     const int row0 = I.rt * TC_ROWS + quad * 32;                                      // first output row of this warp's block
     const int nlive = I.tcnt - (half * NC + c0);
     if (row0 >= g.N || nlive <= 0) return;
-    const int tl = half * NC + c0 + lane;
-    const bool live = lane < NT && tl < I.tcnt;
-    const int slot = live ? (g.perm ? __ldg(g.perm + I.tstart + tl) : I.tstart + tl) : 0;
-    const float scl = (live && g.scale) ? __ldg(g.scale + (slot >> g.a_shift)) : 1.0f;
+    const int slot = __shfl_sync(LKB_FULL, K.slot, c0 + lane);                        // lane t: token c0 + t
+    const bool live = lane < NT && half * NC + c0 + lane < I.tcnt;
     float v[NT], t[NT];
     unsigned my_am = 0;
+    bool sure = true;
+#pragma unroll
+    for (int c = 0; c < NT; c += 2) {                                                 // two tokens at a time
+        const unsigned long long s = tc_pack(__shfl_sync(LKB_FULL, K.scl, c0 + c), __shfl_sync(LKB_FULL, K.scl, c0 + c + 1));
+        bool ok = true;
+        tc_unpack(tc_fmul2(tc_silu2(tc_fmul2(acc[0][(c0 + c) / 2], s), ok), tc_fmul2(acc[1][(c0 + c) / 2], s)), v[c], v[c + 1]);
+        sure = sure && (ok || c >= nlive);
+    }
+    if (!__all_sync(LKB_FULL, sure)) {
+#pragma unroll
+        for (int c = 0; c < NT; ++c) {
+            const float s = __shfl_sync(LKB_FULL, K.scl, c0 + c);
+            v[c] = __fmul_rn(lkb_silu(__fmul_rn(tc_col<NC>(acc[0], c0 + c), s)), __fmul_rn(tc_col<NC>(acc[1], c0 + c), s));
+        }
+    }
 #pragma unroll
     for (int c = 0; c < NT; ++c) {
-        const float s = __shfl_sync(LKB_FULL, scl, c);
-        v[c] = __fmul_rn(lkb_silu(__fmul_rn(tc_col<NC>(acc[0], c0 + c), s)), __fmul_rn(tc_col<NC>(acc[1], c0 + c), s));
         t[c] = v[c];
         const unsigned am = __reduce_max_sync(LKB_FULL, __float_as_uint(fabsf(v[c])));
         if (lane == c) my_am = am;
@@ -350,7 +373,7 @@ __device__ __forceinline__ void tc_store_swiglu(const lkb_pf_gemm & g, const TcI
     for (int b = 0; b < NT; b += 8) {
         if (b < nlive) {
             float q[8];
-            bool sure = true;
+            sure = true;
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
                 const float rd = __shfl_sync(LKB_FULL, rd_l, b + c);
@@ -380,13 +403,14 @@ template <int EPI, int FOLD, int R, int NC>
 __device__ __forceinline__ bool tc_epilogue_item(TcSmem & S, TcEpi & X, const lkb_pf_gemm & g, const TcPlan & P, const TcItem & I, float * const * out_rows,
                                                  unsigned tbase, int half, int quad, int lane) {
     unsigned long long acc[R][NC / 2];
+    const TcTok K = tc_tok<NC>(g, I, half, lane);
     if (!tc_fold_item<EPI, FOLD, R, NC>(S, X, tbase, half, quad * 32 + lane, lane, P.nstage, acc)) return false;
-    if constexpr (EPI == 0) tc_store_plain<R, NC>(g, P, I, out_rows, half, quad * 32 + lane, lane, acc);
-    else if constexpr (NC == 8) tc_store_swiglu<FOLD, NC, 8>(g, I, half, 0, quad, lane, acc);
+    if constexpr (EPI == 0) tc_store_plain<R, NC>(g, P, I, K, out_rows, half, quad * 32 + lane, lane, acc);
+    else if constexpr (NC == 8) tc_store_swiglu<FOLD, NC, 8>(g, I, K, half, 0, quad, lane, acc);
     else {
-        tc_store_swiglu<FOLD, NC, 16>(g, I, half, 0, quad, lane, acc);
-        if constexpr (NC == 24) tc_store_swiglu<FOLD, NC, 8>(g, I, half, 16, quad, lane, acc);
-        if constexpr (NC == 32) tc_store_swiglu<FOLD, NC, 16>(g, I, half, 16, quad, lane, acc);
+        tc_store_swiglu<FOLD, NC, 16>(g, I, K, half, 0, quad, lane, acc);
+        if constexpr (NC == 24) tc_store_swiglu<FOLD, NC, 8>(g, I, K, half, 16, quad, lane, acc);
+        if constexpr (NC == 32) tc_store_swiglu<FOLD, NC, 16>(g, I, K, half, 16, quad, lane, acc);
     }
     return true;
 }
