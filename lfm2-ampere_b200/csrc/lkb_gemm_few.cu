@@ -9,15 +9,15 @@
 // and 16 + 4q + i, which is the A fragment after a mask and a shift), the sums start from the bit pattern of 12582912.0f and are folded
 // from the registers they arrive in.  Measured without copies, ns a 256-row block at 8 / 16 / 32 / 64 tokens: 69 / 99 / 182 / 313 (35 for
 // the rows, 4.3 a token, half of it MMA and half fold; they do not overlap), the other form 230 / 230 / 290 / 350.
-//   * One CTA an SM: one item takes a whole SM for some 7 us, and few SMs idle behind the last wave.  Eight dot warps, one warp
-//     that issues the weights' copies, one the activations' gathers (a copy costs its thread 80 to 100 cycles: one warp for both was the bound), and one
-//     that turns a stage's (d8, 8sum) into the constants of token pairs (in the dot warps, eight times over, that doubled a block's time).
+//   * One CTA an SM: one item takes a whole SM for some 7 us, and few SMs idle behind the last wave.  Eight dot warps, three that
+//     issue copies (one costs its thread 80 to 100 cycles: a single warp for all was the bound, one for all activations cost 5 % at 256 tokens), and
+//     one that turns a stage's (d8, 8sum) into the constants of token pairs (in the dot warps, eight times over, that doubled a block's time).
 //   * Stages of eight blocks: 128 bytes of a weight row, half the copies and waits of four (m = 128: gate|up 78 -> 66 us).
 //   * 16 or 32 tokens an item; the part of a stage that activations leave goes into stages: five or four, 110 to 180 KB in flight.
 // Measured, 64 experts, balanced routing, caches flushed before every call, us at 9 / 20 / 37 / 64 / 128 / 256 / 384 / 509 tokens:
 //   gate|up  dp4a form, three CTAs an SM (before, to 47 tokens)  32 / 50 / 62;  tensor-core form  80 / 82 / 89 / 103 / 121 from 64 on
-//            this form                                           33 / 44 / 52 / 57 / 60 / 79 / 100 / 119
-//   down     before  22 / 30 / 40;  49 / 53 / 59 / 58 / 65       this form  21 / 29 / 32 / 35 / 36 / 43 / 53 / 67
+//            this form                                           33 / 43 / 52 / 57 / 61 / 72 / 93 / 117
+//   down     before  22 / 30 / 40;  49 / 53 / 59 / 58 / 65       this form  21 / 29 / 33 / 35 / 39 / 41 / 50 / 66
 // What bounds it: to some 100 tokens whole waves of items (768 on 148 SMs: 5.2) of 4.5 TB/s each and 5 to 7 us of launch, fill and drain;
 // then the MMAs and the fold.
 // No copy in this file is a multicast one; every tensor map covers memory of the GPU the kernel runs on.
@@ -27,10 +27,10 @@
 #define FW_ROWS   128                // rows of a tile; an item has two (SwiGLU form: gate and up rows)
 #define FW_KB     8                  // blocks per stage
 #define FW_WARPS  8                  // dot warps: 16 rows of each tile
-#define FW_W_WARP 8                  // fetches weights and their scales
-#define FW_A_WARP 9                  // fetches activations and their scales
-#define FW_C_WARP 10                 // forms the token constants of a stage
-#define FW_THREADS 352
+#define FW_W_WARP 8                  // fetches weights and their scales, and the activations' scales
+#define FW_A_WARP 9                  // this one and the next fetch activations, four blocks of a stage each
+#define FW_C_WARP 11                 // forms the token constants of a stage
+#define FW_THREADS 384
 #define FW_UNITS  2048               // parts of plan tiles that are listed
 
 // The two sizes, by the most tokens of an item, and the stages that fit beside each.
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(FW_THREADS, 1) k_pf_gemm_few(const lkb_pf_gemm
     const int n_rt = EPI ? g.N / FW_ROWS : g.N / (2 * FW_ROWS), nstage = g.bpr / FW_KB;
     if (tid == 0) {
         S.abort = 0;
-        for (int i = 0; i < S.NS; ++i) { tc_mbar_init(&S.full[i], 2); tc_mbar_init(&S.ready[i], 1); tc_mbar_init(&S.empty[i], FW_WARPS); }
+        for (int i = 0; i < S.NS; ++i) { tc_mbar_init(&S.full[i], 3); tc_mbar_init(&S.ready[i], 1); tc_mbar_init(&S.empty[i], FW_WARPS); }
         for (int i = 0; i < FW_WARPS / 2; ++i) { tc_mbar_init(&S.xfull[i], 2); tc_mbar_init(&S.xempty[i], 2); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -320,8 +320,8 @@ __global__ void __launch_bounds__(FW_THREADS, 1) k_pf_gemm_few(const lkb_pf_gemm
     __syncthreads();
     const int n_items = (g.perm ? S.n_units : (g.ntok + tw - 1) / tw) * n_rt;
     unsigned it = 0;
-    if (warp == FW_W_WARP || warp == FW_A_WARP) {
-        // ============================ producers (two warps) ==========================
+    if (warp >= FW_W_WARP && warp < FW_C_WARP) {
+        // ============================ producers (three warps) ========================
         bool ok = true;
         for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
             const FwItem I = fw_item<TOK>(S, g, tw, n_rt, item);
@@ -330,12 +330,10 @@ __global__ void __launch_bounds__(FW_THREADS, 1) k_pf_gemm_few(const lkb_pf_gemm
             const int n_g = (I.cnt + 3) >> 2;
             const CUtensorMap * mw[2], * md[2];
             int wrow[2];
-            if (warp == FW_A_WARP) {
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int t = I.tstart + min(4 * (lane & (TOK / 4 - 1)) + q, I.cnt - 1);
-                    crd[q] = g.perm ? __ldg(g.perm + t) >> g.a_shift : t;
-                }
+            for (int q = 0; q < 4; ++q) {
+                const int t = I.tstart + min(4 * (lane & (TOK / 4 - 1)) + q, I.cnt - 1);
+                crd[q] = g.perm ? __ldg(g.perm + t) >> g.a_shift : t;
             }
 #pragma unroll
             for (int r = 0; r < 2; ++r) {
@@ -351,23 +349,21 @@ __global__ void __launch_bounds__(FW_THREADS, 1) k_pf_gemm_few(const lkb_pf_gemm
                 FwStage<TOK> & T = S.st[stg];
                 if (warp == FW_W_WARP) {
                     if (lane == 0) {
-                        tc_mbar_arrive_tx(&S.full[stg], 2u * FW_ROWS * (128u + 16u));
+                        tc_mbar_arrive_tx(&S.full[stg], 2u * FW_ROWS * (128u + 16u) + (unsigned) n_g * (4u * 64u));
 #pragma unroll
                         for (int r = 0; r < 2; ++r) tc_tma_tile(T.q + r * (FW_ROWS * 128), mw[r], ks * (FW_KB * 16), wrow[r], &S.full[stg]);
 #pragma unroll
                         for (int r = 0; r < 2; ++r) tc_tma_tile(&T.ws[r * FW_ROWS], md[r], ks * (FW_KB * 2), wrow[r], &S.full[stg]);
                     }
                     __syncwarp();
+                    if (lane < n_g) tc_tma_gather4(&T.asc[4 * lane][0], &map_s, ks * (FW_KB * 8), crd[0], crd[1], crd[2], crd[3], &S.full[stg]);
                 } else {
-                    if (lane == 0) tc_mbar_arrive_tx(&S.full[stg], (unsigned) n_g * (4u * 256u + 4u * 64u));
+                    const int h = warp - FW_A_WARP;
+                    if (lane == 0) tc_mbar_arrive_tx(&S.full[stg], (unsigned) n_g * (4u * 128u));
                     __syncwarp();
-                    if (lane < n_g) {
-                        tc_tma_gather4(&T.asc[4 * lane][0], &map_s, ks * (FW_KB * 8), crd[0], crd[1], crd[2], crd[3], &S.full[stg]);
-#pragma unroll
-                        for (int h = 0; h < 2; ++h) tc_tma_gather4(T.act[h] + 512 * lane, &map_a, ks * (FW_KB * 32) + 128 * h, crd[0], crd[1], crd[2], crd[3], &S.full[stg]);
-                    }
-                    __syncwarp();
+                    if (lane < n_g) tc_tma_gather4(T.act[h] + 512 * lane, &map_a, ks * (FW_KB * 32) + 128 * h, crd[0], crd[1], crd[2], crd[3], &S.full[stg]);
                 }
+                __syncwarp();
             }
         }
         if (!ok)                                                         // copies in flight land before the block leaves (bounded)
@@ -447,13 +443,13 @@ int lkb_gemm_few_init() {
 int lkb_gemm_few_take_status() { return tc_take_status(); }
 
 // Where the forms cross.  Grouped: by the slots the caller states, spread over 64 experts.  Up to FW_MAX_SLOTS this form is better whatever the
-// skew; beyond, gate|up + down at 64 / 128 / 256 / 384 / 509 / 700 tokens of four slots take 92 / 96 / 122 / 154 / 187 / 242 us here and 129 / 135 / 149 / 162 / 187 /
-// 233 in the tensor-core form with balanced routing: the line lies at 384.  Items of 16 tokens to 200 tokens (at 180: 104 us, 113 with
-// 32), of 32 beyond (at 384: 154, 160 with 16).  A plan that cannot have a tile per expert is one of fewer experts, whose tiles may be
+// skew; beyond, a MoE layer at 400 / 440 / 480 / 520 / 600 tokens of four slots takes 196 / 214 / 223 / 241 / 268 us here and 212 / 220 / 224 / 240 / 260 in the
+// tensor-core form with balanced routing, 209 / 212 / 223 / 235 / 260 and 235 / 239 / 242 / 250 / 270 with Zipf(1.1): the line lies at 480.  Items of 16 tokens to 200 tokens (at
+// 180 gate|up 64 us, 68 with 32; the fifth stage is worth 7 % of a layer at 37 tokens), of 32 beyond.  A plan that cannot have a tile per expert is one of fewer experts, whose tiles may be
 // full; it takes the other form, as does a call that does not state its slots.
 #define FW_MIN_TILES LKB_N_EXPERTS
 #define FW_MAX_SLOTS (47 * LKB_TOP_K)
-#define FW_MORE_SLOTS (384 * LKB_TOP_K)
+#define FW_MORE_SLOTS (480 * LKB_TOP_K)
 #define FW_16_SLOTS  (200 * LKB_TOP_K)
 // Dense: up to FW_MAX_DENSE tokens always, beyond by the time of either form's waves of items (fw_dense_width).
 #define FW_MAX_DENSE 4

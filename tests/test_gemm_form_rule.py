@@ -28,7 +28,7 @@ def test_dense(lkb, m):
     assert _better(lkb, ntok=m, perm=None) == (m <= 4)
 
 
-@pytest.mark.parametrize("slots,max_tiles,width", [(4, 64, 16), (188, 66, 16), (189, 66, 16), (800, 76, 16), (801, 76, 32), (1536, 88, 32), (1537, 88, 0), (4096, 128, 0), (0, 66, 0), (400, 63, 0)])
+@pytest.mark.parametrize("slots,max_tiles,width", [(4, 64, 16), (188, 66, 16), (189, 66, 16), (800, 76, 16), (801, 76, 32), (1920, 94, 32), (1921, 94, 0), (4096, 128, 0), (0, 66, 0), (400, 63, 0)])
 def test_width_of_grouped_items(lkb, slots, max_tiles, width):
     g = lkb.PfGemm()
     g.ntok, g.perm, g.N, g.bpr = slots, 64, 2048, 64
