@@ -765,6 +765,7 @@ int lkb_pf_attn_init();                    // lkb_pfattn.cu
 int lkb_pf_attn_take_status();
 int lkb_gemm_few_init();                   // lkb_gemm_few.cu
 int lkb_gemm_few_take_status();
+int lkb_prefill_take_status();             // lkb_prefill.cu: the tiled router
 
 typedef void (*TcKernel)(lkb_pf_gemm, int, int, const char *, int, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap,
                          CUtensorMap, float * const *, TcDense);
@@ -891,7 +892,7 @@ int lkb_pf_gemm_set_workspace(void * ptr, size_t bytes) {
 }
 int lkb_pf_gemm_status(void) {
     if (cudaDeviceSynchronize() != cudaSuccess) return -1;
-    const int a = tc_take_status(), b = lkb_pf_attn_take_status(), c = lkb_gemm_few_take_status();
-    return a ? a : b ? b : c;
+    const int a = tc_take_status(), b = lkb_pf_attn_take_status(), c = lkb_gemm_few_take_status(), d = lkb_prefill_take_status();
+    return a ? a : b ? b : c ? c : d;
 }
 }

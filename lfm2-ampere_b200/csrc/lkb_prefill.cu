@@ -5,7 +5,7 @@
 // serves as the always-available configuration (the tensor-core form lives in
 // lkb_gemm_tc.cu).  Each kernel evaluates the per-token formula of its decode
 // twin, so per-token results are bit-identical to the decode kernels.
-#include "lkb_device.cuh"
+#include "lkb_tc.cuh"
 #include <cstdlib>
 
 #define LKB_REQUIRE_INIT() do { if (!lkb_context().inited) return LKB_ERR_NOT_INIT; } while (0)
@@ -377,6 +377,161 @@ static int rt_launch(const float * H, int m, const float * Wr, const float * bia
     return lkb_check_launch();
 }
 
+// Tiled form of longer chunks: the same chains, bound by
+// shared memory's return path: a 128-bit load writes 512 bytes of registers, four cycles of the SM's, whatever it reads, so the eight loads
+// of a thread's 4 tokens x 4 experts x 4 k-values cost the four warps 128 cycles and their 64 FMAs each 64.  CTA = NW warps of 4 TPT tokens x
+// 32 experts (a thread: tokens l / 8, + 4, ..., experts l % 8, + 8, + 16, + 24), 4 * TPT independent chains a thread, and one warp that copies:
+// k-tiles of the CTA's token rows and of all 64 router rows travel global -> shared by tensor copies, 128 bytes of every row at a time
+// (swizzled: 128-bit loads of eight neighbouring rows are conflict-free), through a ring of RT_STAGES buffers handed over by mbarriers.
+// us at 1184 / 2048 / 4096 / 8192 tokens: 31.5 / 36.4 / 54.5 / 106 in the form above, 26.9 / 30.5 / 44.6 / 86 here (without the shared loads 16 / 17 / 22 /
+// 39; with a bulk copy per row, 67 cycles each, 44 / 54 / 118 / 234).  At 509 tokens 22.8 there, 29.4 here with the same four-token CTAs.
+// Waits are bounded; on expiry a status word is set and all roles leave, the copying warp after its copies have landed.
+__device__ __forceinline__ float4 rt_lds(unsigned addr) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+template <int TPT, int NW, int RT_KT, int RT_STAGES> struct RtShape {
+    static constexpr int TT = 2 * NW * TPT, H_BYTES = (TT * 128 + 1023) / 1024 * 1024, SUB = LKB_N_EXPERTS * 128 + H_BYTES;    // 32 k-values: router rows, token rows
+    static constexpr int STAGE = RT_KT / 32 * SUB, NTILES = LKB_HIDDEN / RT_KT;
+    static constexpr size_t SMEM = (size_t) RT_STAGES * STAGE + 1024;
+};
+template <int TPT, int NW, int RT_KT, int RT_STAGES>
+__global__ void __launch_bounds__(32 * NW + 32) k_pf_router_tma(int m, const __grid_constant__ CUtensorMap map_h, const __grid_constant__ CUtensorMap map_w,
+                                                        const float * __restrict__ bias, const float * __restrict__ inv,
+                                                        float * __restrict__ sel, float * __restrict__ sig,
+                                                        int4 * __restrict__ idx, float4 * __restrict__ wout) {
+    using F = RtShape<TPT, NW, RT_KT, RT_STAGES>;
+    constexpr int TT = F::TT, NTILES = F::NTILES;
+    extern __shared__ unsigned char rt_raw[];
+    unsigned char * const ring = rt_raw + ((1024u - (tc_smem_u32(rt_raw) & 1023u)) & 1023u);         // swizzled tiles start on 1024-byte boundaries
+    __shared__ alignas(8) unsigned long long full[RT_STAGES], empty[RT_STAGES];
+    __shared__ struct { int abort; } S;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, te = (warp & 1) * 32 + (lane & 7), tg = (warp >> 1) * (4 * TPT) + (lane >> 3);
+    const int t0 = blockIdx.x * TT;
+    if (tid == 0) {
+        S.abort = 0;
+        for (int i = 0; i < RT_STAGES; ++i) { tc_mbar_init(&full[i], 1); tc_mbar_init(&empty[i], NW); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    lkb_pdl_wait(); lkb_pdl_trigger();           // programmatic dependent launch: inputs complete from here on
+    float acc[TPT][4];
+#pragma unroll
+    for (int i = 0; i < TPT; ++i)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[i][q] = 0.0f;
+    if (warp == NW) {
+        int tile = 0;
+        for (; tile < NTILES; ++tile) {
+            const int stg = tile % RT_STAGES;
+            if (!tc_wait<TC_HINT_PROD>(S, &empty[stg], ((unsigned) (tile / RT_STAGES) & 1u) ^ 1u, 41u)) break;
+            if (lane == 0) tc_mbar_arrive_tx(&full[stg], (TT + LKB_N_EXPERTS) * RT_KT * 4);
+            __syncwarp();
+            unsigned char * const st = ring + stg * F::STAGE;
+            if (lane < RT_KT / 32) {                                   // lane: 32 k-values (tokens past the chunk read as zero)
+                tc_tma_tile(st + lane * F::SUB, &map_w, (tile * RT_KT + lane * 32) * 4, 0, &full[stg]);
+                tc_tma_tile(st + lane * F::SUB + LKB_N_EXPERTS * 128, &map_h, (tile * RT_KT + lane * 32) * 4, t0, &full[stg]);
+            }
+        }
+        if (tile < NTILES)                                             // copies in flight land before the block leaves (bounded)
+            for (int k = max(0, tile - RT_STAGES); k < tile; ++k)
+                for (unsigned i = 0; i < 4096u && !tc_mbar_try<TC_HINT_PROD>(&full[k % RT_STAGES], (unsigned) (k / RT_STAGES) & 1u); ++i) { }
+    } else for (int tile = 0; tile < NTILES; ++tile) {
+        const int stg = tile % RT_STAGES;
+        if (!tc_wait(S, &full[stg], (unsigned) (tile / RT_STAGES) & 1u, 42u)) break;
+        const unsigned st = tc_smem_u32(ring) + stg * F::STAGE, sw = st + te * 128 + ((te & 7) << 4);
+        float4 w[2][4], h[2][TPT];                          // four k-values in use, the next four on their way
+        auto load = [&](int b, int c) {
+            const unsigned at = (c >> 5) * F::SUB, part = ((c >> 2) & 7) << 4;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) w[b][q] = rt_lds((sw ^ part) + at + q * (8 * 128));
+#pragma unroll
+            for (int i = 0; i < TPT; ++i) {
+                const int row = tg + 4 * i;
+                h[b][i] = rt_lds(((st + LKB_N_EXPERTS * 128 + row * 128 + ((row & 7) << 4)) ^ part) + at);
+            }
+        };
+        load(0, 0);
+#pragma unroll
+        for (int c = 0; c < RT_KT; c += 4) {
+            const int b = (c >> 2) & 1;
+            if (c + 4 < RT_KT) load(b ^ 1, c + 4);
+            // k-major order: consecutive FMAs belong to different chains, so none waits for its predecessor
+#pragma unroll
+            for (int i = 0; i < TPT; ++i)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) acc[i][q] = fmaf(h[b][i].x, w[b][q].x, acc[i][q]);
+#pragma unroll
+            for (int i = 0; i < TPT; ++i)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) acc[i][q] = fmaf(h[b][i].y, w[b][q].y, acc[i][q]);
+#pragma unroll
+            for (int i = 0; i < TPT; ++i)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) acc[i][q] = fmaf(h[b][i].z, w[b][q].z, acc[i][q]);
+#pragma unroll
+            for (int i = 0; i < TPT; ++i)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) acc[i][q] = fmaf(h[b][i].w, w[b][q].w, acc[i][q]);
+        }
+        __syncwarp();
+        tc_mbar_arrive_if(&empty[stg], lane == 0);
+    }
+    // the ring is free after the last tile: the CTA's sel / sig rows pass through it to the selection warps
+    float * s_sel = reinterpret_cast<float *>(ring), * s_sig = s_sel + TT * LKB_N_EXPERTS;
+    if (idx) __syncthreads();
+    if (warp < NW)
+#pragma unroll
+    for (int i = 0; i < TPT; ++i) {
+        const int tl = tg + 4 * i, tk = t0 + tl;
+        if (tk >= m) continue;
+        const float iv = inv[tk];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int e = te + 8 * q;
+            const float l = __fmul_rn(acc[i][q], iv);
+            const float gv = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-l)));
+            const float sv = __fadd_rn(gv, bias[e]);
+            sig[(size_t) tk * 64 + e] = gv;
+            sel[(size_t) tk * 64 + e] = sv;
+            if (idx) { s_sig[tl * LKB_N_EXPERTS + e] = gv; s_sel[tl * LKB_N_EXPERTS + e] = sv; }
+        }
+    }
+    if (idx) {                                             // the selection in the same launch (lkb_pf_select's result)
+        __syncthreads();
+        for (int tl = warp; tl < TT; tl += NW + 1) {
+            const int tk = t0 + tl;
+            if (tk >= m) break;
+            int ord[LKB_TOP_K]; float wv[LKB_TOP_K];
+            lkb_router_select(s_sel + tl * LKB_N_EXPERTS, s_sig + tl * LKB_N_EXPERTS, lane, ord, wv);
+            if (lane == 0) { idx[tk] = make_int4(ord[0], ord[1], ord[2], ord[3]); wout[tk] = make_float4(wv[0], wv[1], wv[2], wv[3]); }
+        }
+    }
+}
+int lkb_tc_make_map(CUtensorMap * m, const void * base, unsigned row_bytes, unsigned long long pitch, unsigned long long rows,
+                    unsigned box_bytes, unsigned box_rows, CUtensorMapSwizzle sw, CUtensorMapL2promotion l2);           // lkb_gemm_tc.cu
+template <int TPT, int NW, int KT, int STAGES>
+static int rt_launch_tma(const float * H, int m, const float * Wr, const float * bias, const float * inv, float * sel, float * sig,
+                     int * idx, float * w, cudaStream_t st) {
+    using F = RtShape<TPT, NW, KT, STAGES>;
+    static int ready[LKB_STATIC_MAX_DEVICES] = {0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < LKB_STATIC_MAX_DEVICES && !ready[dev]) {
+        if (cudaFuncSetAttribute(k_pf_router_tma<TPT, NW, KT, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) F::SMEM) != cudaSuccess) return -(int) cudaGetLastError();
+        ready[dev] = 1;
+    }
+    if (((size_t) H | (size_t) Wr) & 15) return LKB_ERR_SHAPE;         // 16-byte copies of the rows
+    CUtensorMap mh, mw;
+    int r = lkb_tc_make_map(&mh, H, LKB_HIDDEN * 4, LKB_HIDDEN * 4, (unsigned long long) m, 128u, F::TT, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+    if (r == LKB_OK) r = lkb_tc_make_map(&mw, Wr, LKB_HIDDEN * 4, LKB_HIDDEN * 4, LKB_N_EXPERTS, 128u, LKB_N_EXPERTS, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+    if (r != LKB_OK) return r;
+    LKB_PF_LAUNCH((k_pf_router_tma<TPT, NW, KT, STAGES>), dim3((m + F::TT - 1) / F::TT), dim3(32 * NW + 32), F::SMEM, st, m, mh, mw, bias, inv, sel, sig,
+                  reinterpret_cast<int4 *>(idx), reinterpret_cast<float4 *>(w));
+    return lkb_check_launch();
+}
+
 // Top-4 of 64 per token: warps stride over the tokens (any grid); the selection itself is the redux-based
 // lkb_router_select shared with the decode router.  ref semantics: src/prefill.cu:1696-1708
 __global__ void __launch_bounds__(256) k_pf_select(const float * __restrict__ sel, const float * __restrict__ sig, int m,
@@ -730,6 +885,7 @@ int lkb_gemm_few_launch(const lkb_pf_gemm * g, int epi, int fold, int max_tiles,
 static int g_gemm_cfg = -1;        // -1: tensor-core form when it covers the shape; 0: CUDA-core form
 static int g_gemm_fold = 1;        // 1: the reference's shipped per-block term (folded offset); 0: the exact term
 
+int lkb_prefill_take_status() { return tc_take_status(); }
 int lkb_prefill_init() {
     const char * v = getenv("LKB_PF_CFG");
     if (v) g_gemm_cfg = atoi(v);
@@ -837,18 +993,18 @@ static int router_tiled(const float * H, int m, const float * Wr, const float * 
     if (!H || !Wr || !bias || !inv || !sel || !sig) return LKB_ERR_NULL;
     if (m <= 0) return m == 0 ? LKB_OK : LKB_ERR_SHAPE;
     // The k loop of one CTA is the critical path and its length grows with the tokens per CTA, so a token range takes the smallest
-    // CTA that still fits one wave.  Measured on B200, us (tiles of 64 k-values, six stages -> of 128, four stages):
-    //   4-token CTAs (two warps)  up to 592 tokens   31.7 -> 21.0   (8-token CTAs there: 32.3)
-    //   8-token CTAs              up to 1184         32.4 -> 29.1
-    //   16-token CTAs             up to 2368         36.5 -> 35.3
-    //   32-token CTAs             at 4096            53.3 -> 69.5: keeps 64
+    // CTA that still fits one wave.  Measured on B200, us, copies by every thread and by tensor copies:
+    //   4-token CTAs (two warps)         up to 592 tokens   22.8   29.4
+    //   8-token CTAs (two warps)         up to 1184         31.0   26.9
+    //   16-token CTAs                    up to 2368         36.3   30.5
+    //   32-token CTAs, 64 k-values a tile  at 4096          54.5   44.6
     // A rank's share of an expert-parallel chunk lands in the first three.  LKB_ROUTER_FORM = 4 / 8 / 16 / 32 forces a shape (tuning).
     static const int form = [] { const char * e = getenv("LKB_ROUTER_FORM"); return e ? atoi(e) : 0; }();
     const int sms = lkb_context().sm_count;
     if (form == 4 || (form == 0 && m <= 4 * sms)) return rt_launch<1, 2, 128, 4>(H, m, Wr, bias, inv, sel, sig, idx, w, (cudaStream_t) st);
-    if (form == 8 || (form == 0 && m <= 8 * sms)) return rt_launch<1, 4, 128, 4>(H, m, Wr, bias, inv, sel, sig, idx, w, (cudaStream_t) st);
-    if (form == 16 || (form == 0 && m <= 16 * sms)) return rt_launch<2, 4, 128, 4>(H, m, Wr, bias, inv, sel, sig, idx, w, (cudaStream_t) st);
-    return rt_launch<4, 4, 64, 6>(H, m, Wr, bias, inv, sel, sig, idx, w, (cudaStream_t) st);
+    if (form == 8 || (form == 0 && m <= 8 * sms)) return rt_launch_tma<2, 2, 128, 4>(H, m, Wr, bias, inv, sel, sig, idx, w, (cudaStream_t) st);
+    if (form == 16 || (form == 0 && m <= 16 * sms)) return rt_launch_tma<2, 4, 128, 4>(H, m, Wr, bias, inv, sel, sig, idx, w, (cudaStream_t) st);
+    return rt_launch_tma<4, 4, 64, 6>(H, m, Wr, bias, inv, sel, sig, idx, w, (cudaStream_t) st);
 }
 
 int lkb_pf_router_small(const float * H, int m, const float * Wr, const float * bias, const float * inv,
