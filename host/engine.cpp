@@ -235,8 +235,7 @@ void prefill_chunk(Engine & e, lk::stream_t st, const int * toks_host, int m, in
             lk::PfGemm g = gemm_desc(&mx.in_proj, 1, ends, CONV_ROWS, BPR, e.a_qs, e.a_sc);
             g.ntok = m; g.scale = scale; g.out = e.Y; g.out_ld = CONV_ROWS;
             lk::pf_gemm_dense(g, st);
-            lk::k_pf_conv(st, m, e.Y, mx.conv_w, mx.hist, a);
-            lk::k_pf_conv_hist(st, e.Y, m, mx.hist);
+            lk::k_pf_conv_next(st, m, e.Y, mx.conv_w, mx.hist, a);
         }
         {   // out_proj / attn_output, added onto the residual stream
             const int ends[3] = {H, H, H};
@@ -246,8 +245,8 @@ void prefill_chunk(Engine & e, lk::stream_t st, const int * toks_host, int m, in
         }
         // MoE FFN.  ref: src/engine.cu:1170-1241
         const lkb_moe_layer & l = e.moe[i];
-        lk::k_pf_norm(st, m, e.X, l.norm_w, 0, a, e.inv, e.h32);
-        lk::check(lkb_pf_router_select(e.h32, m, m <= 256, l.router, l.rbias, e.inv, e.sel, e.sig, e.idx, e.w, st), "k_pf_router + k_pf_select");
+        lk::check(lkb_pf_norm_router_select(e.X, l.norm_w, a, e.inv, e.h32, m, m <= 256, l.router, l.rbias, e.sel, e.sig, e.idx, e.w, st),
+                  "k_pf_norm + k_pf_router + k_pf_select");
         lk::k_pf_moe_route(st, e.idx, ns, e.cnt, e.off, e.tiles, e.ntiles, e.perm);
         {
             const lk::QT4 segs[2] = {{l.gate_qs, l.gate_d}, {l.up_qs, l.up_d}};

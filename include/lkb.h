@@ -324,6 +324,10 @@ int lkb_pf_select(const float * sel, const float * sig, int m, int * idx, float 
  * results as the two calls.  No counterpart in the reference (its engine launches the two kernels, src/engine.cu:1170-1180). */
 int lkb_pf_router_select(const float * H, int m, int small_form, const float * Wr, const float * bias, const float * inv,
                          float * sel, float * sig, int * idx, float * w, lkb_stream_t st);
+/* lkb_pf_norm (plain = 0) followed by lkb_pf_router_select on its h32: up to 160 tokens of the small form in one launch, which
+ * leaves h32 (m x 2048 floats of the caller's) untouched.  Same results as the two calls. */
+int lkb_pf_norm_router_select(const float * X, const float * nw, lkb_pf_act a, float * inv, float * h32, int m, int small_form,
+                              const float * Wr, const float * bias, float * sel, float * sig, int * idx, float * w, lkb_stream_t st);
 /* ref: src/prefill.cuh:117-122  k_pf_moe_count / _plan / _scatter.  cnt must be
  * zero on entry to count (the engine memsets it, ref: src/engine.cu:1182). */
 int lkb_pf_moe_count(const int * idx, int n, int * cnt, lkb_stream_t st);
@@ -434,6 +438,7 @@ int lkb_shortconv(const float * bcx, int t, const float * conv_w, float * hist, 
  * lkb_pf_embed: x[t][0..n) = dequantised Q6_K row toks[t].                         ref: src/prefill.cu:856-868
  * lkb_pf_conv: Y = in_proj output [m][6144] (B | C | X); planar Q8_1 rows of C * conv into a; hist is read.
  * lkb_pf_conv_hist: the two-tap history after the chunk (run after lkb_pf_conv).   ref: src/prefill.cu:937-970
+ * lkb_pf_conv_next: both in one launch: hist is read and then holds the history after the chunk.
  * lkb_pf_qknr: Y = q|k|v output [m][3072]; per-head RMSNorm + NEOX RoPE (base theta; the reference compiles in
  *   1e7); Q leaves as fp16 [m][2048] pre-scaled by 1/8, K and V are appended to the cache.  ref: src/prefill.cu:975-1016
  * lkb_pf_attn: causal GQA attention of the chunk's queries qh over cache positions 0 .. P+m-1, o = fp32 [m][2048].
@@ -444,6 +449,7 @@ int lkb_pf_embed(const void * ql, const void * qh, const void * sc, const void *
                  lkb_stream_t st);
 int lkb_pf_conv(const float * Y, const float * cw, const float * hist, lkb_pf_act a, int m, lkb_stream_t st);
 int lkb_pf_conv_hist(const float * Y, int m, float * hist, lkb_stream_t st);
+int lkb_pf_conv_next(const float * Y, const float * cw, float * hist, lkb_pf_act a, int m, lkb_stream_t st);
 int lkb_pf_qknr(const float * Y, const float * qn, const float * kn, int P, void * qh, void * kc, void * vc, int m, float theta,
                 lkb_stream_t st);
 int lkb_pf_attn(const void * qh, int m, int P, const void * kc, const void * vc, float * o, lkb_stream_t st);

@@ -124,6 +124,8 @@ inline int k_pf_embed(stream_t st, int m, const uint8_t * ql, const uint8_t * qh
     return check(lkb_pf_embed(ql, qh, sc, d, toks, x, LKB_HIDDEN, m, st), "k_pf_embed"); }
 inline int k_pf_conv(stream_t st, int m, const float * Y, const float * cw, const float * hist, PfAct a) {
     return check(lkb_pf_conv(Y, cw, hist, a, m, st), "k_pf_conv"); }
+inline int k_pf_conv_next(stream_t st, int m, const float * Y, const float * cw, float * hist, PfAct a) {
+    return check(lkb_pf_conv_next(Y, cw, hist, a, m, st), "k_pf_conv_next"); }
 inline int k_pf_conv_hist(stream_t st, const float * Y, int m, float * hist) { return check(lkb_pf_conv_hist(Y, m, hist, st), "k_pf_conv_hist"); }
 inline int k_pf_qknr(stream_t st, int m, const float * Y, const float * qn, const float * kn, int P, void * qh, void * kc, void * vc) {
     return check(lkb_pf_qknr(Y, qn, kn, P, qh, kc, vc, m, 10000000.0f, st), "k_pf_qknr"); }

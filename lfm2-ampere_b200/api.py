@@ -17,14 +17,14 @@ __all__ = [
     "k_quantize_q8_1", "k_rmsnorm_q8_1", "norm_produce", "k_gemv_q4_0", "k_gemv_q4_0_prod", "k_gemv_q4_0_3",
     "k_gemv_q4_0_exp2", "k_gemv_q4_0_exp", "k_swiglu", "k_moe_accum4", "k_moe_down_accum", "k_router_dot",
     "k_router_top4", "router_top4_softmax", "block_sumi", "k_pf_norm", "k_pf_quant_rows", "k_pf_swiglu",
-    "k_pf_router", "k_pf_router_small", "k_pf_router_tiled", "k_pf_router_select", "k_pf_select", "k_pf_moe_count", "k_pf_moe_plan", "k_pf_moe_scatter", "k_pf_moe_route",
+    "k_pf_router", "k_pf_router_small", "k_pf_router_tiled", "k_pf_router_select", "k_pf_norm_router_select", "k_pf_select", "k_pf_moe_count", "k_pf_moe_plan", "k_pf_moe_scatter", "k_pf_moe_route",
     "pf_gemm_dense", "pf_gemm_moe", "pf_gemm_swiglu", "k_pf_moe_combine", "k_pf_moe_combine_norm",
     "k_pf_pack_q8_1", "zero_i32", "moe_layer_desc", "moe_scratch", "moe_ffn_decode", "moe_ffn_decode_stack",
     "layer_descs_to_device", "ep_pack_rows", "ep_unpack_rows", "k_pf_moe_combine_norm_gather", "moe_ffn_decode_stack_static", "set_pdl", "pf_gemm_config", "pf_gemm_arith", "pf_gemm_workspace_bytes", "pf_gemm_set_workspace", "sm_count",
     "k_gemv_q6_K", "k_argmax_part", "k_argmax_final", "k_embed_q6_K", "gemv_q6_K_status",
     "k_attn_split", "k_attn_combine", "k_qk_norm_rope", "k_shortconv", "ATTN_SPLIT", "ATTN_PARTW",
     "mixer_layer_desc", "step_scratch", "decode_layers",
-    "k_pf_embed", "k_pf_conv", "k_pf_conv_hist", "k_pf_qknr", "k_pf_attn",
+    "k_pf_embed", "k_pf_conv", "k_pf_conv_hist", "k_pf_conv_next", "k_pf_qknr", "k_pf_attn",
     "decode_set_expert_prefetch", "decode_expert_prefetch_hits", "ep_peers", "EP_ROW_BYTES", "ep_set_wait_limit_ms", "ep_route_exchange", "ep_route_experts", "pf_gemm_moe_rows", "pf_gemm_swiglu_packed", "ep_publish_wait", "ep_pack_push", "ep_wait",
 ]
 
@@ -184,6 +184,11 @@ def k_pf_router(H, m, Wr, bias, inv, sel, sig):
 def k_pf_router_select(H, m, small_form, Wr, bias, inv, sel, sig, idx, w):
     check(lib.lkb_pf_router_select(ptr(H), m, int(bool(small_form)), ptr(Wr), ptr(bias), ptr(inv), ptr(sel), ptr(sig), ptr(idx), ptr(w),
                                    stream()), "k_pf_router_select")
+
+
+def k_pf_norm_router_select(X, w, a, inv, h32, m, small_form, Wr, bias, sel, sig, idx, wout):
+    check(lib.lkb_pf_norm_router_select(ptr(X), ptr(w), a, ptr(inv), ptr(h32), m, int(bool(small_form)), ptr(Wr), ptr(bias), ptr(sel), ptr(sig),
+                                        ptr(idx), ptr(wout), stream()), "k_pf_norm_router_select")
 
 
 def k_pf_router_tiled(H, m, Wr, bias, inv, sel, sig):
@@ -399,6 +404,10 @@ def k_pf_embed(ql, qh, sc, d, toks, x, n, m):
 
 def k_pf_conv(Y, cw, hist, a, m):
     check(lib.lkb_pf_conv(ptr(Y), ptr(cw), ptr(hist), a, m, stream()), "k_pf_conv")
+
+
+def k_pf_conv_next(Y, cw, hist, a, m):
+    check(lib.lkb_pf_conv_next(ptr(Y), ptr(cw), ptr(hist), a, m, stream()), "k_pf_conv_next")
 
 
 def k_pf_conv_hist(Y, m, hist):

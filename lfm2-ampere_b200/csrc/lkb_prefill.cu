@@ -201,6 +201,7 @@ __global__ void __launch_bounds__(256) k_pf_router_token(const float * __restric
 // The same for fewer tokens still: a cluster of eight CTAs per token, a warp per expert.  The selection needs all 64 logits: they meet in
 // the shared memory of the cluster's first CTA.  Bound by the latency of a warp's two rows; see router_small for where it pays.
 #define RC_CTAS 8
+#define RC_MAX_TOKENS 160            // see router_small
 __global__ void __cluster_dims__(RC_CTAS, 1, 1) __launch_bounds__(256) k_pf_router_cluster(const float * __restrict__ H, const float * __restrict__ Wr,
                                                          const float * __restrict__ bias, const float * __restrict__ inv,
                                                          float * __restrict__ sel, float * __restrict__ sig,
@@ -238,6 +239,71 @@ __global__ void __cluster_dims__(RC_CTAS, 1, 1) __launch_bounds__(256) k_pf_rout
             lkb_router_select(s_sel, s_sig, lane, ord, wv);
             if (lane == 0) { idx[t] = make_int4(ord[0], ord[1], ord[2], ord[3]); wout[t] = make_float4(wv[0], wv[1], wv[2], wv[3]); }
         }
+    }
+}
+
+// ffn_norm (k_pf_token_norm<0>) and the router above in one launch, while a cluster of eight CTAs a token is the form: each CTA forms u = x * w itself for
+// its eight experts' rows, quantises an eighth of it, and the first one gets logits and blocks' sums of squares through its shared memory and
+// ends with 1 / rms, the gates and the selection.  Same sums in the same order.  Two launches took 5.5 + 8.5 us at 9 tokens and 5.7 + 8.2 at 37 (ncu), this 5.9 and 8.4.
+__global__ void __cluster_dims__(RC_CTAS, 1, 1) __launch_bounds__(256) k_pf_norm_router_cluster(const float * __restrict__ X, const float * __restrict__ nw,
+                                                         int8_t * __restrict__ aqs, float2 * __restrict__ asc, float * __restrict__ inv_out,
+                                                         const float * __restrict__ Wr, const float * __restrict__ bias,
+                                                         float * __restrict__ sel, float * __restrict__ sig,
+                                                         int4 * __restrict__ idx, float4 * __restrict__ wout) {
+    lkb_pdl_wait(); lkb_pdl_trigger();           // programmatic dependent launch: inputs complete from here on
+    __shared__ float s_u[LKB_HIDDEN], s_acc[LKB_N_EXPERTS], s_sq[LKB_HIDDEN / 32], s_sel[LKB_N_EXPERTS], s_sig[LKB_N_EXPERTS];
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");                // the first CTA runs before its memory is written
+    const int t = blockIdx.x / RC_CTAS, rank = blockIdx.x % RC_CTAS, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, e = rank * 8 + warp;
+    const float4 * x4 = reinterpret_cast<const float4 *>(X + (size_t) t * LKB_HIDDEN), * w4 = reinterpret_cast<const float4 *>(nw);
+    const float * row = Wr + (size_t) e * LKB_HIDDEN;
+    auto to_first = [](float * p, float v) {
+        unsigned a;
+        asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"((unsigned) __cvta_generic_to_shared(p)));
+        asm volatile("st.shared::cluster.f32 [%0], %1;" :: "r"(a), "f"(v) : "memory");
+    };
+    float r[LKB_HIDDEN / 32];
+#pragma unroll
+    for (int j = 0; j < LKB_HIDDEN / 32; ++j) r[j] = __ldg(row + j * 32 + lane);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const float4 xv = x4[threadIdx.x + 256 * j], wv = __ldg(w4 + threadIdx.x + 256 * j);
+        reinterpret_cast<float4 *>(s_u)[threadIdx.x + 256 * j] = make_float4(__fmul_rn(xv.x, wv.x), __fmul_rn(xv.y, wv.y), __fmul_rn(xv.z, wv.z), __fmul_rn(xv.w, wv.w));
+    }
+    float sq = 0.0f;
+    if (warp < 2) {                                        // the CTA's eight blocks, four a warp
+        const int i4 = (rank * 8 + warp * 4) * 8 + lane;
+        const float4 xv = x4[i4], wv = __ldg(w4 + i4);
+        float2 s2;
+        reinterpret_cast<unsigned *>(aqs + (size_t) t * LKB_HIDDEN)[i4] = lkb_quad_quant(make_float4(__fmul_rn(xv.x, wv.x), __fmul_rn(xv.y, wv.y), __fmul_rn(xv.z, wv.z), __fmul_rn(xv.w, wv.w)), lane, s2);
+        sq = lkb_quad_sum(__fmul_rn(xv.x, xv.x), __fmul_rn(xv.y, xv.y), __fmul_rn(xv.z, xv.z), __fmul_rn(xv.w, xv.w));
+        if ((lane & 7) == 0) asc[(size_t) t * (LKB_HIDDEN / 32) + rank * 8 + warp * 4 + (lane >> 3)] = s2;
+    }
+    __syncthreads();
+    float acc = 0.0f;
+#pragma unroll
+    for (int j = 0; j < LKB_HIDDEN / 32; ++j) acc = fmaf(r[j], s_u[j * 32 + lane], acc);
+    acc = lkb_warp_sum(acc);
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    if (lane == 0) to_first(&s_acc[e], acc);
+    if (warp < 2 && (lane & 7) == 0) to_first(&s_sq[rank * 8 + warp * 4 + (lane >> 3)], sq);
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (rank == 0 && warp == 0) {
+        const float sv = lkb_warp_sum(__fadd_rn(s_sq[lane], s_sq[lane + 32])), inv = rsqrtf(fmaf(sv, 1.0f / (float) LKB_HIDDEN, LKB_EPS));
+#pragma unroll
+        for (int q = lane; q < LKB_N_EXPERTS; q += 32) {
+            const float l = __fmul_rn(s_acc[q], inv);
+            const float gv = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-l)));
+            const float v = __fadd_rn(gv, bias[q]);
+            sig[(size_t) t * 64 + q] = gv;
+            sel[(size_t) t * 64 + q] = v;
+            s_sig[q] = gv; s_sel[q] = v;
+        }
+        __syncwarp();
+        int ord[LKB_TOP_K]; float wv[LKB_TOP_K];
+        lkb_router_select(s_sel, s_sig, lane, ord, wv);
+        if (lane == 0) { idx[t] = make_int4(ord[0], ord[1], ord[2], ord[3]); wout[t] = make_float4(wv[0], wv[1], wv[2], wv[3]); inv_out[t] = inv; }
     }
 }
 
@@ -976,8 +1042,7 @@ static int router_small(const float * H, int m, const float * Wr, const float * 
     if (m > 65535) return LKB_ERR_SHAPE;
     // A cluster of CTAs a token while that is about a wave: a MoE layer at 2 / 9 / 37 / 64 / 100 tokens 47 / 63 / 114 / 152 / 155 -> 41 / 58 / 109 /
     // 146 / 150 us; at 180 equal, at 256 182 -> 186.
-    constexpr int MAX_CLUSTERS = 160;
-    if (m <= MAX_CLUSTERS) {
+    if (m <= RC_MAX_TOKENS) {
         LKB_PF_LAUNCH(k_pf_router_cluster, dim3(m * RC_CTAS), dim3(256), 0, (cudaStream_t) st, H, Wr, bias, inv, sel, sig,
                       reinterpret_cast<int4 *>(idx), reinterpret_cast<float4 *>(w));
         return lkb_check_launch();
@@ -1024,6 +1089,20 @@ int lkb_pf_router_select(const float * H, int m, int small_form, const float * W
                          float * sel, float * sig, int * idx, float * w, lkb_stream_t st) {
     if (!idx || !w) return LKB_ERR_NULL;
     return small_form ? router_small(H, m, Wr, bias, inv, sel, sig, idx, w, st) : router_tiled(H, m, Wr, bias, inv, sel, sig, idx, w, st);
+}
+
+int lkb_pf_norm_router_select(const float * X, const float * nw, lkb_pf_act a, float * inv, float * h32, int m, int small_form, const float * Wr,
+                              const float * bias, float * sel, float * sig, int * idx, float * w, lkb_stream_t st) {
+    LKB_REQUIRE_INIT();
+    if (!X || !nw || !a.qs || !a.sc || !inv || !h32 || !Wr || !bias || !sel || !sig || !idx || !w) return LKB_ERR_NULL;
+    if (m <= 0) return m == 0 ? LKB_OK : LKB_ERR_SHAPE;
+    if (small_form && m <= RC_MAX_TOKENS) {
+        LKB_PF_LAUNCH(k_pf_norm_router_cluster, dim3(m * RC_CTAS), dim3(256), 0, (cudaStream_t) st, X, nw, a.qs, reinterpret_cast<float2 *>(a.sc), inv, Wr, bias, sel, sig,
+                      reinterpret_cast<int4 *>(idx), reinterpret_cast<float4 *>(w));
+        return lkb_check_launch();
+    }
+    const int r = lkb_pf_norm(X, nw, 0, a, inv, h32, m, st);
+    return r != LKB_OK ? r : lkb_pf_router_select(h32, m, small_form, Wr, bias, inv, sel, sig, idx, w, st);
 }
 
 int lkb_pf_select(const float * sel, const float * sig, int m, int * idx, float * w, lkb_stream_t st) {

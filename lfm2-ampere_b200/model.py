@@ -221,7 +221,7 @@ class PrefillChunk:
         self.o = torch.zeros(m, H, **f32)
         self.toks = torch.zeros(m, dtype=torch.int32, device=device)
         n_attn = sum(mx.is_attn for mx in model.mixers)
-        self.launches_per_step = 1 + 1 + sum((6 if mx.is_attn else 4) for mx in model.mixers) + (6 if 4 * m <= 2048 else 8) * len(model.mixers)
+        self.launches_per_step = 1 + 1 + sum((6 if mx.is_attn else 3) for mx in model.mixers) + (5 if m <= 160 else 6 if 4 * m <= 2048 else 8) * len(model.mixers)
 
     def macs_per_step(self):
         m, n = self.m_, len(self.model.mixers)
@@ -255,8 +255,7 @@ class PrefillChunk:
                 g = api.make_pf_gemm([(mx.in_qs, mx.in_d)], [CONV_ROWS] * 3, CONV_ROWS, bpr, self.a_qs, self.a_sc, ntok=m,
                                      scale=scale, out=self.Y, out_ld=CONV_ROWS)
                 api.pf_gemm_dense(g)
-                api.k_pf_conv(self.Y, mx.conv_w, st.hist[ci], self.a, m)
-                api.k_pf_conv_hist(self.Y, m, st.hist[ci])
+                api.k_pf_conv_next(self.Y, mx.conv_w, st.hist[ci], self.a, m)
                 ci += 1
             og = api.make_pf_gemm([(mx.out_qs, mx.out_d)], [H] * 3, H, bpr, self.a_qs, self.a_sc, ntok=m,
                                   out=self.X, out_ld=H, add=1)

@@ -1,7 +1,7 @@
 """Batched prefill of the MoE FFN stack on one GPU: the host-side call sequence of the
 reference's pf_chunk() for this path (ref: src/engine.cu:1170-1241), one C-ABI call per
 reference kernel / launcher:
-  k_pf_norm(ffn_norm) -> k_pf_router + k_pf_select (one launch) -> k_pf_moe_route (up to 2048 slots;
+  k_pf_norm(ffn_norm) -> k_pf_router + k_pf_select (one launch; with the norm up to 160 tokens) -> k_pf_moe_route (up to 2048 slots;
   beyond: memset(cnt) -> k_pf_moe_count -> k_pf_moe_plan -> k_pf_moe_scatter) -> pf_gemm_swiglu (gate|up, a_shift 2, scale inv) ->
   pf_gemm_moe (down, a_shift 0) -> k_pf_moe_combine_norm (next layer's first norm)."""
 from __future__ import annotations
@@ -57,16 +57,15 @@ class PrefillStack:
         self.a = api.pf_act(self.a_qs, self.a_sc)
         self.a2 = api.pf_act(self.a2_qs, self.a2_sc)
         self.an = api.pf_act(self.n_qs, self.n_sc)
-        self.launches_per_step = (6 if self.ns <= 2048 else 8) * len(layers)       # kernels per layer (the memset is not a kernel)
+        self.launches_per_step = (5 if m <= 160 else 6 if self.ns <= 2048 else 8) * len(layers)       # kernels per layer (the memset is not a kernel)
 
     def layer(self, i, next_norm_w=None, next_act=None):
         """One MoE FFN layer over the chunk.  next_norm_w / next_act = (PfAct, inv): where the fused combine + norm
         puts the next consumer's quantised activation (the full model: the next mixer's attn_norm, into the live
         activation buffers); by default the next layer's ffn_norm into scratch."""
         l, m = self.layers[i], self.m
-        api.k_pf_norm(self.X, l.norm_w, 0, self.a, self.inv, self.h32, m)
-        # router + top-4 selection in one launch (the form follows the chunk size: src/engine.cu:1170-1176)
-        api.k_pf_router_select(self.h32, m, m <= 256, l.router, l.rbias, self.inv, self.sel, self.sig, self.idx, self.w)
+        # ffn_norm, router + top-4 selection (the form follows the chunk size: src/engine.cu:1170-1176)
+        api.k_pf_norm_router_select(self.X, l.norm_w, self.a, self.inv, self.h32, m, m <= 256, l.router, l.rbias, self.sel, self.sig, self.idx, self.w)
         api.k_pf_moe_route(self.idx, self.ns, self.cnt, self.off, self.tiles, self.ntiles, self.perm)
         g = api.make_pf_gemm([(l.gate_qs, l.gate_d), (l.up_qs, l.up_d)], [I, I, I], I, H // 32, self.a_qs, self.a_sc,
                              ntok=self.ns, exp_stride=I * (H // 32), perm=self.perm, tiles=self.tiles, ntiles=self.ntiles,

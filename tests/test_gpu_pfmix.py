@@ -34,6 +34,25 @@ def test_pf_embed_rows(L, orc):
         assert np.array_equal(host(x)[i], orc.embed_q6_K(ql, qh, sc, d, int(t), sb))
 
 
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 37])
+def test_pf_conv_next_equals_both_launches(L, golden_dir, m):
+    """One launch, with fewer tokens than a run, a whole one and more: activations and the history after the chunk, bit for bit."""
+    cw = dev(np.load(golden_dir / "conv_taps.npz")["conv_w"])
+    rng = np.random.default_rng(m)
+    Y = dev(rng.uniform(-1, 1, (m, 3 * H)).astype(np.float32))
+    got = []
+    for one in (False, True):
+        a_qs, a_sc = torch.full((m, H), 0x55, dtype=torch.int8, device="cuda"), nan_f32(m, H // 32, 2)
+        hist = dev((0.5 * np.random.default_rng(9).uniform(-1, 1, 2 * H)).astype(np.float32))
+        if one:
+            L.k_pf_conv_next(Y, cw, hist, L.pf_act(a_qs, a_sc), m)
+        else:
+            L.k_pf_conv(Y, cw, hist, L.pf_act(a_qs, a_sc), m)
+            L.k_pf_conv_hist(Y, m, hist)
+        got.append((a_qs, a_sc, hist))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
 @pytest.mark.parametrize("m", [1, 2, 3, 37])
 def test_pf_conv_equals_decode_steps(L, orc, golden_dir, m):
     cw = np.load(golden_dir / "conv_taps.npz")["conv_w"]

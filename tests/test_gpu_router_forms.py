@@ -41,3 +41,23 @@ def test_cluster_form_equals_token_form(lkb):
         alone = new(n)
         lkb.k_pf_router_small(H, n, W, bias, inv, alone[0], alone[1])
         assert torch.equal(alone[0], ref[0][:n]) and torch.equal(alone[1], ref[1][:n]), n
+
+
+def test_norm_and_router_in_one_launch_equal_two(lkb):
+    """Up to 160 tokens the norm shares the short router's launch: activations, 1 / rms, gates and selection, bit for bit; and the counts behind."""
+    lkb.init(0)
+    m, gen = 300, torch.Generator("cuda").manual_seed(33)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    X, nw, W, bias = rnd(m, 2048) * torch.exp(rnd(m, 1)), 1 + 0.1 * rnd(2048), 0.03 * rnd(64, 2048), 0.1 * rnd(64)
+    X[3], X[5, :32] = 0.0, 0.0                                         # a row and a block of zeros
+    def new(n):
+        full = lambda *s, **k: torch.full(s, k.pop("fill", float("nan")), device="cuda", **k)
+        return (full(n, 2048, fill=0x55, dtype=torch.int8), full(n, 64, 2), full(n), full(n, 64), full(n, 64), full(n, 4, fill=-1, dtype=torch.int32), full(n, 4), full(n, 2048))
+    for n in (1, 2, 37, 159, 160, 161, 256, 300):
+        qs, sc, inv, sel, sig, idx, w, h = new(n)
+        lkb.k_pf_norm(X, nw, 0, lkb.pf_act(qs, sc), inv, h, n)
+        lkb.k_pf_router_select(h, n, n <= 256, W, bias, inv, sel, sig, idx, w)
+        got = new(n)
+        lkb.k_pf_norm_router_select(X, nw, lkb.pf_act(*got[:2]), got[2], got[7], n, n <= 256, W, bias, *got[3:7])
+        assert all(torch.equal(a, b) for a, b in zip(got[:7], (qs, sc, inv, sel, sig, idx, w))), n
+        assert bool(torch.isnan(got[7]).all()) == (n <= 160)
