@@ -245,8 +245,13 @@ void prefill_chunk(Engine & e, lk::stream_t st, const int * toks_host, int m, in
         }
         // MoE FFN.  ref: src/engine.cu:1170-1241
         const lkb_moe_layer & l = e.moe[i];
-        lk::check(lkb_pf_norm_router_select(e.X, l.norm_w, a, e.inv, e.h32, m, m <= 256, l.router, l.rbias, e.sel, e.sig, e.idx, e.w, st),
-                  "k_pf_norm + k_pf_router + k_pf_select");
+        if (m <= 160) {                                                       // one launch
+            lk::check(lkb_pf_norm_router_select(e.X, l.norm_w, a, e.inv, e.h32, m, 1, l.router, l.rbias, e.sel, e.sig, e.idx, e.w, st),
+                      "k_pf_norm + k_pf_router + k_pf_select");
+        } else {
+            lk::k_pf_norm(st, m, e.X, l.norm_w, 0, a, e.inv, e.h32);
+            lk::check(lkb_pf_router_select(e.h32, m, m <= 256, l.router, l.rbias, e.inv, e.sel, e.sig, e.idx, e.w, st), "k_pf_router + k_pf_select");
+        }
         lk::k_pf_moe_route(st, e.idx, ns, e.cnt, e.off, e.tiles, e.ntiles, e.perm);
         {
             const lk::QT4 segs[2] = {{l.gate_qs, l.gate_d}, {l.up_qs, l.up_d}};
