@@ -10,7 +10,7 @@ import ctypes as C
 
 import torch
 
-from . import EpPeers, MixerLayer, MoeLayer, MoeScratch, NormProd, PfAct, PfGemm, StepScratch, check, lib
+from . import _fast, EpPeers, MixerLayer, MoeLayer, MoeScratch, NormProd, PfAct, PfGemm, StepScratch, check, lib
 
 __all__ = [
     "ptr", "stream", "norm_prod", "pf_act", "make_pf_gemm",
@@ -29,11 +29,7 @@ __all__ = [
 ]
 
 
-def ptr(t):
-    if t is None:
-        return None
-    assert t.is_cuda and t.is_contiguous(), "device-resident contiguous tensors only"
-    return t.data_ptr()
+ptr = _fast.ptr            # a tensor's address (device-resident, contiguous), None for None
 
 
 # torch's handle lookups by themselves: building torch.cuda.current_stream()'s Stream object took 3.2 us, a third of a launch.
@@ -46,6 +42,9 @@ if _raw_stream and _device:
 else:
     def stream():
         return torch.cuda.current_stream().cuda_stream
+
+
+_fast.set_stream_lookup(*((_raw_stream, _device) if _raw_stream and _device else (stream, None)))
 
 
 def norm_prod(w=None, h32=None, yq8=None, ssq=None):
@@ -97,7 +96,7 @@ def k_quantize_q8_1(x, y, nblocks):
 
 
 def k_rmsnorm_q8_1(x, w, n, eps, y32, y16, yq8):
-    check(lib.lkb_rmsnorm_q8_1(ptr(x), ptr(w), n, eps, ptr(y32), ptr(y16), ptr(yq8), stream()), "k_rmsnorm_q8_1")
+    check(_fast.rmsnorm_q8_1(x, w, n, eps, y32, y16, yq8), "k_rmsnorm_q8_1")
 
 
 def norm_produce(x, n, np_):
@@ -105,8 +104,7 @@ def norm_produce(x, n, np_):
 
 
 def k_gemv_q4_0(qs, d, xq, out_rows, bpr, y, add_residual=0, ssq=None, eps=1e-5):
-    check(lib.lkb_gemv_q4_0(ptr(qs), ptr(d), ptr(xq), out_rows, bpr, ptr(y), add_residual, ptr(ssq), eps, stream()),
-          "k_gemv_q4_0")
+    check(_fast.gemv_q4_0(qs, d, xq, out_rows, bpr, y, add_residual, ssq, eps), "k_gemv_q4_0")
 
 
 def k_gemv_q4_0_prod(qs, d, xq, out_rows, bpr, y, add_residual, np_):
@@ -166,11 +164,11 @@ def block_sumi(qs, xq, rows, bpr, out):
 
 # ----------------------------------------------------------------- prefill --
 def k_pf_norm(X, w, plain, a, inv_out, h32, m):
-    check(lib.lkb_pf_norm(ptr(X), ptr(w), plain, a, ptr(inv_out), ptr(h32), m, stream()), "k_pf_norm")
+    check(_fast.pf_norm(X, w, plain, a, inv_out, h32, m), "k_pf_norm")
 
 
 def k_pf_quant_rows(X, ld, kb, a, rows):
-    check(lib.lkb_pf_quant_rows(ptr(X), ld, kb, a, rows, stream()), "k_pf_quant_rows")
+    check(_fast.pf_quant_rows(X, ld, kb, a, rows), "k_pf_quant_rows")
 
 
 def k_pf_swiglu(Y, ld, up_off, kb, a, rows):
@@ -187,8 +185,7 @@ def k_pf_router_select(H, m, small_form, Wr, bias, inv, sel, sig, idx, w):
 
 
 def k_pf_norm_router_select(X, w, a, inv, h32, m, small_form, Wr, bias, sel, sig, idx, wout):
-    check(lib.lkb_pf_norm_router_select(ptr(X), ptr(w), a, ptr(inv), ptr(h32), m, int(bool(small_form)), ptr(Wr), ptr(bias), ptr(sel), ptr(sig),
-                                        ptr(idx), ptr(wout), stream()), "k_pf_norm_router_select")
+    check(_fast.pf_norm_router_select(X, w, a, inv, h32, m, bool(small_form), Wr, bias, sel, sig, idx, wout), "k_pf_norm_router_select")
 
 
 def k_pf_router_tiled(H, m, Wr, bias, inv, sel, sig):
@@ -218,7 +215,7 @@ def k_pf_moe_plan(cnt, off, tiles, ntiles):
 
 
 def k_pf_moe_route(idx, n, cnt, off, tiles, ntiles, perm):
-    check(lib.lkb_pf_moe_route(ptr(idx), n, ptr(cnt), ptr(off), ptr(tiles), ptr(ntiles), ptr(perm), stream()), "k_pf_moe_route")
+    check(_fast.pf_moe_route(idx, n, cnt, off, tiles, ntiles, perm), "k_pf_moe_route")
 
 
 def k_pf_moe_scatter(idx, n, off, perm):
@@ -229,30 +226,20 @@ def make_pf_gemm(segs, seg_end, N, bpr, aqs, asc, *, ntok=0, exp_stride=0, perm=
                  a_shift=0, scale=None, out=None, out_ld=0, add=0, oqs=None, osc=None, okb=0):
     """lkb_pf_gemm from tensors; segs = [(qs, d), ...] (1 to 3 stacked weight tensors); ntok = token rows, with perm its slots (0: not stated)."""
     g = PfGemm()
-    for i in range(3):
-        q, d = segs[min(i, len(segs) - 1)]
-        g.qs[i] = ptr(q)
-        g.d[i] = ptr(d)
-        g.seg_end[i] = seg_end[min(i, len(seg_end) - 1)]
-    g.N, g.bpr, g.exp_stride = N, bpr, exp_stride
-    g.aqs, g.asc, g.ntok = ptr(aqs), ptr(asc), ntok
-    g.perm, g.tiles, g.ntiles = ptr(perm), ptr(tiles), ptr(ntiles)
-    g.a_shift, g.scale = a_shift, ptr(scale)
-    g.out, g.out_ld, g.add = ptr(out), out_ld, add
-    g.oqs, g.osc, g.okb = ptr(oqs), ptr(osc), okb
+    _fast.fill_pf_gemm(g, segs, seg_end, N, bpr, aqs, asc, ntok, exp_stride, perm, tiles, ntiles, a_shift, scale, out, out_ld, add, oqs, osc, okb)
     return g
 
 
 def pf_gemm_dense(g):
-    check(lib.lkb_pf_gemm_dense(C.byref(g), stream()), "pf_gemm_dense")
+    check(_fast.pf_gemm_dense(g), "pf_gemm_dense")
 
 
 def pf_gemm_moe(g, max_tiles):
-    check(lib.lkb_pf_gemm_moe(C.byref(g), max_tiles, stream()), "pf_gemm_moe")
+    check(_fast.pf_gemm_moe(g, max_tiles), "pf_gemm_moe")
 
 
 def pf_gemm_swiglu(g, max_tiles):
-    check(lib.lkb_pf_gemm_swiglu(C.byref(g), max_tiles, stream()), "pf_gemm_swiglu")
+    check(_fast.pf_gemm_swiglu(g, max_tiles), "pf_gemm_swiglu")
 
 
 def k_pf_moe_combine(X, D, w, m):
@@ -260,8 +247,7 @@ def k_pf_moe_combine(X, D, w, m):
 
 
 def k_pf_moe_combine_norm(X, D, w, nw, a, inv_out, m):
-    check(lib.lkb_pf_moe_combine_norm(ptr(X), ptr(D), ptr(w), ptr(nw), a, ptr(inv_out), m, stream()),
-          "k_pf_moe_combine_norm")
+    check(_fast.pf_moe_combine_norm(X, D, w, nw, a, inv_out, m), "k_pf_moe_combine_norm")
 
 
 def k_pf_pack_q8_1(a, t, y):
@@ -336,8 +322,7 @@ def k_pf_moe_combine_norm_gather(X, D, pos, w, nw, a, inv_out, m):
 
 # ------------------------------------------------ output projection / embedding --
 def k_gemv_q6_K(ql, qh, sc, d, xq, out_rows, sbpr, y, ssq=None, eps=1e-5):
-    check(lib.lkb_gemv_q6_K(ptr(ql), ptr(qh), ptr(sc), ptr(d), ptr(xq), out_rows, sbpr, ptr(y), ptr(ssq), eps, stream()),
-          "k_gemv_q6_K")
+    check(_fast.gemv_q6_K(ql, qh, sc, d, xq, out_rows, sbpr, y, ssq, eps), "k_gemv_q6_K")
 
 
 def gemv_q6_K_status():
@@ -345,11 +330,11 @@ def gemv_q6_K_status():
 
 
 def k_argmax_part(v, n, pv, pi):
-    check(lib.lkb_argmax_part(ptr(v), n, ptr(pv), ptr(pi), stream()), "k_argmax_part")
+    check(_fast.argmax_part(v, n, pv, pi), "k_argmax_part")
 
 
 def k_argmax_final(pv, pi, n, d_token, d_pos=None):
-    check(lib.lkb_argmax_final(ptr(pv), ptr(pi), n, ptr(d_token), ptr(d_pos), stream()), "k_argmax_final")
+    check(_fast.argmax_final(pv, pi, n, d_token, d_pos), "k_argmax_final")
 
 
 def k_embed_q6_K(ql, qh, sc, d, d_token, n, x):
@@ -399,7 +384,7 @@ def decode_layers(moe_dev, mixers_dev, n_layers, x, xq_first, d_pos, theta, next
 
 # ------------------------------------------------------------ prefill mixers --
 def k_pf_embed(ql, qh, sc, d, toks, x, n, m):
-    check(lib.lkb_pf_embed(ptr(ql), ptr(qh), ptr(sc), ptr(d), ptr(toks), ptr(x), n, m, stream()), "k_pf_embed")
+    check(_fast.pf_embed(ql, qh, sc, d, toks, x, n, m), "k_pf_embed")
 
 
 def k_pf_conv(Y, cw, hist, a, m):
@@ -407,7 +392,7 @@ def k_pf_conv(Y, cw, hist, a, m):
 
 
 def k_pf_conv_next(Y, cw, hist, a, m):
-    check(lib.lkb_pf_conv_next(ptr(Y), ptr(cw), ptr(hist), a, m, stream()), "k_pf_conv_next")
+    check(_fast.pf_conv_next(Y, cw, hist, a, m), "k_pf_conv_next")
 
 
 def k_pf_conv_hist(Y, m, hist):
@@ -415,11 +400,11 @@ def k_pf_conv_hist(Y, m, hist):
 
 
 def k_pf_qknr(Y, qn, kn, P, qh, kc, vc, m, theta=1e7):
-    check(lib.lkb_pf_qknr(ptr(Y), ptr(qn), ptr(kn), P, ptr(qh), ptr(kc), ptr(vc), m, theta, stream()), "k_pf_qknr")
+    check(_fast.pf_qknr(Y, qn, kn, P, qh, kc, vc, m, theta), "k_pf_qknr")
 
 
 def k_pf_attn(qh, m, P, kc, vc, o):
-    check(lib.lkb_pf_attn(ptr(qh), m, P, ptr(kc), ptr(vc), ptr(o), stream()), "k_pf_attn")
+    check(_fast.pf_attn(qh, m, P, kc, vc, o), "k_pf_attn")
 
 
 # ------------------------------------------------ expert-parallel exchange over peer memory --

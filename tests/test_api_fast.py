@@ -1,0 +1,46 @@
+"""The native bindings: what they refuse, and the descriptors they fill, against the fields set one by one."""
+import ctypes
+import importlib
+
+import pytest
+
+torch = pytest.importorskip("torch")
+
+
+def test_refusals(lkb):
+    api, fast = importlib.import_module("lfm2-ampere_b200.api"), importlib.import_module("lfm2-ampere_b200._fast")
+    assert api.ptr(None) is None
+    with pytest.raises(AssertionError):
+        api.ptr(torch.zeros(4))                                            # host memory
+    with pytest.raises(TypeError):
+        api.ptr(1234)
+    with pytest.raises(TypeError):
+        fast.pf_gemm_dense(lkb.PfAct())                                    # a structure of another type
+    with pytest.raises(TypeError):
+        fast.pf_gemm_dense()
+    with pytest.raises((TypeError, AssertionError)):
+        fast.pf_moe_route(None, 1.5, None, None, None, None, None)
+    with pytest.raises(IndexError):
+        fast.fill_pf_gemm(lkb.PfGemm(), [], [1], *range(17))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_seg", [1, 2, 3])
+def test_descriptor_fields(lkb, n_seg):
+    new = lambda n, d: torch.zeros(n, dtype=d, device="cuda")
+    segs = [(new(64, torch.uint8), new(8, torch.float16)) for _ in range(n_seg)]
+    ends = [128, 256, 384][:n_seg]
+    t = {k: new(16, torch.int32) for k in ("aqs", "asc", "perm", "tiles", "ntiles", "scale", "out", "oqs", "osc")}
+    g = lkb.make_pf_gemm(segs, ends, 384, 24, t["aqs"], t["asc"], ntok=7, exp_stride=1 << 40, perm=t["perm"], tiles=t["tiles"], ntiles=t["ntiles"], a_shift=2,
+                         scale=t["scale"], out=t["out"], out_ld=5, add=1, oqs=t["oqs"], osc=t["osc"], okb=9)
+    last = n_seg - 1
+    for i in range(3):
+        q, d = segs[min(i, last)]
+        assert (g.qs[i], g.d[i], g.seg_end[i]) == (q.data_ptr(), d.data_ptr(), ends[min(i, last)])
+    assert all(getattr(g, k) == v.data_ptr() for k, v in t.items())
+    assert (g.N, g.bpr, g.ntok, g.exp_stride, g.a_shift, g.out_ld, g.add, g.okb) == (384, 24, 7, 1 << 40, 2, 5, 1, 9)
+    assert importlib.import_module("lfm2-ampere_b200._fast").pf_moe_route(None, 4, None, None, None, None, None) != 0       # the entry point's refusal
+    h = lkb.make_pf_gemm(segs, ends, 384, 24, t["aqs"], t["asc"])
+    assert h.perm is None and h.out is None and h.ntok == 0 and ctypes.sizeof(h) == ctypes.sizeof(g)
+    with pytest.raises(AssertionError):
+        lkb.make_pf_gemm([(segs[0][0][::2], segs[0][1])], ends, 384, 24, t["aqs"], t["asc"])        # not contiguous
