@@ -459,17 +459,18 @@ static bool fw_better(const lkb_pf_gemm * g, int max_tiles) {
 // Test hook (not in the public header): whether a call takes this form whatever the other's time.
 extern "C" __attribute__((visibility("default"))) int lkb_debug_gemm_few_better(const lkb_pf_gemm * g, int max_tiles) { return fw_better(g, max_tiles); }
 
-// The token width of a dense problem's items, or 0 where the tensor-core form is faster: waves x the time of an item's block, which is 95 or
-// 128 ns at 8 or 16 tokens here (64 blocks a row: a wave more takes 6.1 or 8.2 us; 225 ns at 32, never better) against tc_dense_ns there, and 5 us more
-// an item for launch, fill and drain.  us in the tensor-core form and here, caches flushed: in_proj (6144 rows) at 37 / 64 / 96 tokens 19.5 / 24.6 / 24.6 -> 14.3 / 16.4 / 16.4
-// (at 256 28.7 there, 32.8 here), out_proj (2048 rows) at 37 / 128 / 256 18.4 / 20.5 / 24.6 -> 12.3 / 12.3 / 16.4.
+// The token width of a dense problem's items, or 0 where the tensor-core form is faster: waves x the time of an item's block, which is 95, 128 or
+// 176 ns at 8, 16 or 24 tokens here (64 blocks a row: a wave more takes 6.1, 8.2 or 11.3 us; 225 ns at 32, never better) against tc_dense_ns there, and 5 us more
+// an item for launch, fill and drain.  us in the tensor-core form and here, caches flushed: in_proj (6144 rows) at 37 / 64 / 96 / 128 / 144 / 432 tokens
+// 19.5 / 24.6 / 24.6 / 23.6 / 24.6 / 46.1 -> 14.3 / 16.4 / 16.4 / 18.9 / 19.0 / 39.9 (at 256 28.7 there, 32.8 here), out_proj (2048 rows) at 37 / 128 / 256 / 300 / 432
+// 18.4 / 20.5 / 24.6 / 23.5 / 24.0 -> 12.3 / 12.3 / 16.4 / 17.9 / 18.9.
 int lkb_gemm_tc_dense_ns(int ntok, int N, int sms);      // lkb_gemm_tc.cu
 static int fw_dense_width(int ntok, int N, int bpr, int sms, bool always) {
-    static const int ns[2] = {95, 128};
+    static const int ns[3] = {95, 128, 176};
     int best = 0;
     long long least = always ? 1ll << 62 : lkb_gemm_tc_dense_ns(ntok, N, sms) - 5000 / bpr;
-    for (int i = 0; i < 2; ++i) {
-        const int tw = 8 << i;
+    for (int i = 0; i < 3; ++i) {
+        const int tw = 8 * (i + 1);
         const long long items = (long long) ((ntok + tw - 1) / tw) * (N / (2 * FW_ROWS)), t = (items + sms - 1) / sms * ns[i];
         if (t < least) { least = t; best = tw; }
     }

@@ -35,8 +35,8 @@ def test_width_of_grouped_items(lkb, slots, max_tiles, width):
     assert lkb.lib.lkb_debug_gemm_few_width(ctypes.byref(g), max_tiles, 148) == width
 
 
-@pytest.mark.parametrize("m,N,bpr,width", [(1, 2048, 64, 8), (4, 6144, 8, 8), (5, 2048, 8, 0), (37, 6144, 64, 8), (64, 6144, 64, 16), (128, 6144, 64, 0), (144, 2048, 64, 8), (180, 2048, 64, 16),
-                                           (300, 2048, 64, 0), (4096, 6144, 64, 0)])
+@pytest.mark.parametrize("m,N,bpr,width", [(1, 2048, 64, 8), (4, 6144, 8, 8), (5, 2048, 8, 0), (37, 6144, 64, 8), (64, 6144, 64, 16), (96, 6144, 64, 16), (97, 6144, 64, 24), (144, 6144, 64, 24), (145, 6144, 64, 0),
+                                           (144, 2048, 64, 8), (180, 2048, 64, 16), (289, 2048, 64, 24), (432, 2048, 64, 24), (433, 2048, 64, 0), (4096, 6144, 64, 0)])
 def test_width_of_dense_items(lkb, m, N, bpr, width):
     """By the waves of items over 148 SMs in either form."""
     g = lkb.PfGemm()

@@ -103,7 +103,7 @@ def test_swiglu(L, orc, I, bpr, width, off):
 
 
 @pytest.mark.parametrize("m,N,ends,bpr,width", [(5, 256, (256,) * 3, 64, 8), (37, 1024, (512, 640, 1024), 40, 8), (130, 2048, (2048,) * 3, 64, 8), (251, 2048, (2048,) * 3, 64, 16),
-                                                (90, 6144, (6144,) * 3, 64, 16), (128, 6144, (6144,) * 3, 64, 0), (37, 256, (256,) * 3, 8, 0)])
+                                                (90, 6144, (6144,) * 3, 64, 16), (97, 6144, (6144,) * 3, 64, 24), (143, 6144, (2048, 4096, 6144), 64, 24), (300, 2048, (2048,) * 3, 64, 24), (145, 6144, (6144,) * 3, 64, 0), (37, 256, (256,) * 3, 8, 0)])
 def test_dense(L, orc, m, N, ends, bpr, width):
     rng = np.random.default_rng(7 * m + N)
     qs, d = rand_q4(rng, N, bpr, "ref")
