@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(FW_THREADS, 1) k_pf_gemm_few(const lkb_pf_gemm
         unsigned n_item = 0;
         for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++n_item) {
             const FwItem I = fw_item<TOK>(S, g, tw, n_rt, item);
-            if (I.cnt <= 0) continue;
+            if (I.cnt <= 0) { --n_item; continue; }                      // (only items with tokens count)
             if (lane < TOK) {                                            // (no later than the item's first constants)
                 const int slot = lane < I.cnt ? (g.perm ? __ldg(g.perm + I.tstart + lane) : I.tstart + lane) : 0;
                 const float scl = lane < I.cnt && g.scale ? __ldg(g.scale + (slot >> g.a_shift)) : 1.0f;
@@ -407,7 +407,7 @@ __global__ void __launch_bounds__(FW_THREADS, 1) k_pf_gemm_few(const lkb_pf_gemm
         unsigned n_item = 0;
         for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++n_item) {
             const FwItem I = fw_item<TOK>(S, g, tw, n_rt, item);
-            if (I.cnt <= 0) continue;
+            if (I.cnt <= 0) { --n_item; continue; }                      // (only items with tokens count)
             const int nt = (I.cnt + 7) >> 3;
             if (nt == 1) ok = fw_do_item<EPI, FOLD, TOK, 1>(S, it, n_item, g, I, nstage, warp, lane);
             if (nt == 2) ok = fw_do_item<EPI, FOLD, TOK, 2>(S, it, n_item, g, I, nstage, warp, lane);

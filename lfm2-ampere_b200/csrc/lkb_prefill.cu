@@ -314,9 +314,8 @@ __global__ void __cluster_dims__(RC_CTAS, 1, 1) __launch_bounds__(256) k_pf_norm
 // four experts (lane, lane + 16, + 32, + 48): 4 * TPT independent chains.  Tiles of RT_KT k-values of the CTA's token
 // rows and of all 64 router rows travel global -> shared by 16-byte asynchronous copies through a ring of RT_STAGES
 // buffers (rows keep their [row][k] layout, pitch RT_KT + 4 floats: nothing is transposed and 128-bit loads of 16 different
-// rows are conflict-free); the multiply loop reads four k-values per load.  With TPT = 4 a warp spends 16 wavefronts
-// (4 loads of router rows, 4 of token rows shared by half a warp) on 64 FMA instructions: the ratio at which the FMA
-// pipes rather than shared memory set the pace.  One CTA barrier per tile.
+// rows are conflict-free); the multiply loop reads four k-values per load.  Instantiated for 4-token CTAs
+// (TPT = 1: up to 592 tokens, one wave); larger ones take k_pf_router_tma below.  One CTA barrier per tile.
 // A tile holds KT k-values, the ring STAGES of them: what a tile costs beside its FMAs (a barrier, the copies' issue) is paid
 // less often with wide tiles, which small CTAs have the shared memory for (see router_tiled).
 __device__ __forceinline__ void rt_cp16(float * dst, const float * src, bool live) {

@@ -74,6 +74,25 @@ def test_more_parts_than_are_listed(L, orc):
     assert np.array_equal(host(out), ref)
 
 
+def test_more_parts_than_are_listed_swiglu(L, orc):
+    """As above with three row tiles, so that a block meets empty parts between others."""
+    rng = np.random.default_rng(6)
+    I, bpr, E, ns = 384, 8, 3, 2100
+    perm, tiles = _plan(rng, [ns // E] * E, tile=1)
+    w = [tuple(dev(x) for x in rand_q4(rng, E * I, bpr, "ref")) for _ in range(2)]
+    aq, asc = (dev(v) for v in orc.pf_quant_rows(act_floats(rng, ns * bpr * 32).reshape(ns, bpr * 32), bpr))
+    dperm, dtiles, dnt = dev(perm), dev(tiles), dev(np.array([ns], np.int32))
+    got = []
+    for cfg in (0, -1):
+        L.pf_gemm_config(cfg)
+        oqs, osc = torch.full((ns, I), 0x5A, dtype=torch.int8, device="cuda"), nan_f32(ns, I // 32, 2)
+        g = L.make_pf_gemm(w, [I] * 3, I, bpr, aq, asc, ntok=300, exp_stride=I * bpr, perm=dperm, tiles=dtiles, ntiles=dnt, oqs=oqs, osc=osc, okb=I // 32)
+        assert _width(L, g, ns) == 16
+        L.pf_gemm_swiglu(g, ns)
+        got.append((oqs, osc))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1].view(torch.int32), got[1][1].view(torch.int32))
+
+
 @pytest.mark.parametrize("width", [16, 32])
 @pytest.mark.parametrize("I,bpr", [(128, 8), (384, 40)])
 @pytest.mark.parametrize("off", [0, 1])
