@@ -54,13 +54,29 @@ template <int TOK> struct FwSmem {
     int abort, n_units, listed;
 };
 
-struct FwItem { int expert, tstart, cnt, rt; };             // cnt <= 0: nothing to do
+struct FwItem { int expert, tstart, cnt, rt, r0, rows; };   // cnt <= 0: nothing to do; rows r0 .. r0 + rows - 1 of both tiles
+// The blocks' work: items, of which those from `whole` on -- a last wave that would leave half of the blocks or more without one -- are cut
+// into 1 << cut parts of fewer rows, one a block, whose first warps have rows (an item's time is its weights' way into one SM).  us, whole -> cut, caches
+// flushed: down at 2 / 20 tokens 15.3 -> 13.3, 29.7 -> 27.7; out_proj (2048 rows) at 2 to 64 tokens 13.3 -> 11.3, in_proj at 2 13.3 -> 11.3; a layer of 2 / 9 / 20 / 37 /
+// 64 tokens 59.4 / 84.4 / 100.6 / 114.3 / 122.3 -> 55.6 / 79.2 / 96.3 / 111.3 / 119.8.  A choice of the width that counts a part as 0.6 of an item
+// changed nothing (-1 % at 70 tokens, +0.5 % at 200).
+struct FwWork { int whole, cut, n; };
+__device__ __forceinline__ FwWork fw_work(int n_items, int cut, int blocks) {
+    FwWork W;
+    const int rem = n_items % blocks;
+    W.cut = rem << cut <= blocks ? cut : 0;
+    W.whole = n_items - rem;
+    W.n = W.whole + (rem << W.cut);
+    return W;
+}
 // Items by token unit (dense: tw tokens; grouped: a plan tile or a part of one) and row tile, row tiles fastest.
 template <int TOK>
-__device__ __forceinline__ FwItem fw_item(const FwSmem<TOK> & S, const lkb_pf_gemm & g, int tw, int n_rt, int item) {
+__device__ __forceinline__ FwItem fw_item(const FwSmem<TOK> & S, const lkb_pf_gemm & g, int tw, int n_rt, const FwWork & W, int n) {
     FwItem I;
-    const int u = item / n_rt;
+    const int over = max(n - W.whole, 0), cut = n < W.whole ? 0 : W.cut, item = min(n, W.whole) + (over >> W.cut), u = item / n_rt;
     I.rt = item - u * n_rt;
+    I.rows = FW_ROWS >> cut;
+    I.r0 = (over & ((1 << cut) - 1)) * I.rows;
     if (g.perm) {
         const int t = S.listed ? S.unit[u] : u, t0 = (t % (64 / TOK)) * TOK;
         const int4 tl = __ldg(reinterpret_cast<const int4 *>(g.tiles) + t / (64 / TOK));
@@ -160,7 +176,7 @@ __device__ __forceinline__ bool fw_dots(FwSmem<TOK> & S, unsigned & it, int nsta
 // out (+)= scale * acc: a store of a warp is 8 rows (a sector) of four tokens.
 template <int NT>
 __device__ __forceinline__ void fw_store_plain(const int * slots, const float * scls, const lkb_pf_gemm & g, const FwItem & I, int warp, int lane, const unsigned long long (&acc)[2][NT][2]) {
-    const int o0 = I.rt * (2 * FW_ROWS) + 16 * warp + (lane >> 2);
+    const int o0 = I.rt * (2 * FW_ROWS) + I.r0 + 16 * warp + (lane >> 2);
 #pragma unroll
     for (int n = 0; n < NT; ++n)
 #pragma unroll
@@ -189,7 +205,7 @@ __device__ __forceinline__ void fw_store_plain(const int * slots, const float * 
 template <int FOLD, int TOK, int NT>
 __device__ __forceinline__ bool fw_store_swiglu(FwSmem<TOK> & S, const int * slots, const float * scls, unsigned xpar, const lkb_pf_gemm & g, const FwItem & I, int warp, int lane,
                                                 const unsigned long long (&acc)[2][NT][2]) {
-    const int row0 = I.rt * FW_ROWS + (warp >> 1) * 32, gr = lane >> 2, mine = warp & 1, q = lane & 3;
+    const int row0 = I.rt * FW_ROWS + I.r0 + (warp >> 1) * 32, gr = lane >> 2, mine = warp & 1, q = lane & 3;
     float v[NT][2];                                                      // my token of pair n, my two rows
     if (!tc_wait(S, &S.xempty[warp >> 1], xpar ^ 1u, 34u)) return false; // what was handed over last has been read
 #pragma unroll
@@ -281,11 +297,13 @@ __device__ __forceinline__ bool fw_do_item(FwSmem<TOK> & S, unsigned & it, unsig
     return true;
 }
 
+// Nibbles and scales of the three row segments, in boxes of 128 rows and of a part's.
+struct FwMaps { CUtensorMap w[2][3], d[2][3]; };
+
 template <int EPI, int FOLD, int TOK>
-__global__ void __launch_bounds__(FW_THREADS, 1) k_pf_gemm_few(const lkb_pf_gemm g, const int max_tiles, const int rpe, const int tw,
+__global__ void __launch_bounds__(FW_THREADS, 1) k_pf_gemm_few(const lkb_pf_gemm g, const int max_tiles, const int rpe, const int tw, const int cut,
         const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_s,
-        const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUtensorMap map_w2,
-        const __grid_constant__ CUtensorMap map_d0, const __grid_constant__ CUtensorMap map_d1, const __grid_constant__ CUtensorMap map_d2) {
+        const __grid_constant__ FwMaps maps) {
     lkb_pdl_wait(); lkb_pdl_trigger();           // programmatic dependent launch: inputs complete from here on
     extern __shared__ unsigned char fw_smem_raw[];
     FwSmem<TOK> & S = *reinterpret_cast<FwSmem<TOK> *>(fw_smem_raw + ((1024u - (tc_smem_u32(fw_smem_raw) & 1023u)) & 1023u));
@@ -318,13 +336,13 @@ __global__ void __launch_bounds__(FW_THREADS, 1) k_pf_gemm_few(const lkb_pf_gemm
         }
     }
     __syncthreads();
-    const int n_items = (g.perm ? S.n_units : (g.ntok + tw - 1) / tw) * n_rt;
+    const FwWork W = fw_work((g.perm ? S.n_units : (g.ntok + tw - 1) / tw) * n_rt, cut, gridDim.x);
     unsigned it = 0;
     if (warp >= FW_W_WARP && warp < FW_C_WARP) {
         // ============================ producers (three warps) ========================
         bool ok = true;
-        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-            const FwItem I = fw_item<TOK>(S, g, tw, n_rt, item);
+        for (int item = blockIdx.x; item < W.n && ok; item += gridDim.x) {
+            const FwItem I = fw_item<TOK>(S, g, tw, n_rt, W, item);
             if (I.cnt <= 0) continue;
             int crd[4] = {0, 0, 0, 0};                                   // lane l: tokens 4l .. 4l+3 (a dead one repeats the last)
             const int n_g = (I.cnt + 3) >> 2;
@@ -339,9 +357,9 @@ __global__ void __launch_bounds__(FW_THREADS, 1) k_pf_gemm_few(const lkb_pf_gemm
             for (int r = 0; r < 2; ++r) {
                 const int row = EPI ? I.rt * FW_ROWS : (2 * I.rt + r) * FW_ROWS;
                 const int seg = EPI ? r : (row < g.seg_end[0]) ? 0 : (row < g.seg_end[1]) ? 1 : 2;
-                mw[r] = seg == 0 ? &map_w0 : seg == 1 ? &map_w1 : &map_w2;
-                md[r] = seg == 0 ? &map_d0 : seg == 1 ? &map_d1 : &map_d2;
-                wrow[r] = I.expert * rpe + row - (EPI || !seg ? 0 : g.seg_end[seg - 1]);
+                mw[r] = &maps.w[I.rows < FW_ROWS][seg];
+                md[r] = &maps.d[I.rows < FW_ROWS][seg];
+                wrow[r] = I.expert * rpe + I.r0 + row - (EPI || !seg ? 0 : g.seg_end[seg - 1]);
             }
             for (int ks = 0; ks < nstage; ++ks, ++it) {
                 const unsigned stg = it % S.NS;
@@ -349,7 +367,7 @@ __global__ void __launch_bounds__(FW_THREADS, 1) k_pf_gemm_few(const lkb_pf_gemm
                 FwStage<TOK> & T = S.st[stg];
                 if (warp == FW_W_WARP) {
                     if (lane == 0) {
-                        tc_mbar_arrive_tx(&S.full[stg], 2u * FW_ROWS * (128u + 16u) + (unsigned) n_g * (4u * 64u));
+                        tc_mbar_arrive_tx(&S.full[stg], 2u * (unsigned) I.rows * (128u + 16u) + (unsigned) n_g * (4u * 64u));
 #pragma unroll
                         for (int r = 0; r < 2; ++r) tc_tma_tile(T.q + r * (FW_ROWS * 128), mw[r], ks * (FW_KB * 16), wrow[r], &S.full[stg]);
 #pragma unroll
@@ -373,8 +391,8 @@ __global__ void __launch_bounds__(FW_THREADS, 1) k_pf_gemm_few(const lkb_pf_gemm
         // ============================ token constants (one warp) =====================
         bool ok = true;
         unsigned n_item = 0;
-        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++n_item) {
-            const FwItem I = fw_item<TOK>(S, g, tw, n_rt, item);
+        for (int item = blockIdx.x; item < W.n && ok; item += gridDim.x, ++n_item) {
+            const FwItem I = fw_item<TOK>(S, g, tw, n_rt, W, item);
             if (I.cnt <= 0) { --n_item; continue; }                      // (only items with tokens count)
             if (lane < TOK) {                                            // (no later than the item's first constants)
                 const int slot = lane < I.cnt ? (g.perm ? __ldg(g.perm + I.tstart + lane) : I.tstart + lane) : 0;
@@ -405,9 +423,16 @@ __global__ void __launch_bounds__(FW_THREADS, 1) k_pf_gemm_few(const lkb_pf_gemm
         // ============================ dots (eight warps) =============================
         bool ok = true;
         unsigned n_item = 0;
-        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++n_item) {
-            const FwItem I = fw_item<TOK>(S, g, tw, n_rt, item);
+        for (int item = blockIdx.x; item < W.n && ok; item += gridDim.x, ++n_item) {
+            const FwItem I = fw_item<TOK>(S, g, tw, n_rt, W, item);
             if (I.cnt <= 0) { --n_item; continue; }                      // (only items with tokens count)
+            if (16 * warp >= I.rows) {                                   // not a row of this part (the block's last): its stages as they come
+                for (int ks = 0; ks < nstage && ok; ++ks, ++it) {
+                    ok = tc_wait(S, &S.full[it % S.NS], (it / S.NS) & 1u, 33u);
+                    tc_mbar_arrive_if(&S.empty[it % S.NS], lane == 0 && ok);
+                }
+                continue;
+            }
             const int nt = (I.cnt + 7) >> 3;
             if (nt == 1) ok = fw_do_item<EPI, FOLD, TOK, 1>(S, it, n_item, g, I, nstage, warp, lane);
             if (nt == 2) ok = fw_do_item<EPI, FOLD, TOK, 2>(S, it, n_item, g, I, nstage, warp, lane);
@@ -424,7 +449,7 @@ __global__ void __launch_bounds__(FW_THREADS, 1) k_pf_gemm_few(const lkb_pf_gemm
 int lkb_tc_make_map(CUtensorMap * m, const void * base, unsigned row_bytes, unsigned long long pitch, unsigned long long rows,
                     unsigned box_bytes, unsigned box_rows, CUtensorMapSwizzle sw, CUtensorMapL2promotion l2);           // lkb_gemm_tc.cu
 
-typedef void (*FwKernel)(lkb_pf_gemm, int, int, int, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap);
+typedef void (*FwKernel)(lkb_pf_gemm, int, int, int, int, CUtensorMap, CUtensorMap, FwMaps);
 template <int TOK> static FwKernel fw_form(int epi, int fold) {
     return epi ? (fold ? k_pf_gemm_few<1, 1, TOK> : k_pf_gemm_few<1, 0, TOK>) : (fold ? k_pf_gemm_few<0, 1, TOK> : k_pf_gemm_few<0, 0, TOK>);
 }
@@ -505,6 +530,12 @@ extern "C" __attribute__((visibility("default"))) int lkb_debug_silu(unsigned fi
     return lkb_check_launch();
 }
 
+// Parts of an item in a last wave (fw_work), as a shift: halves, or quarters where they fit.  Grouped the host does not know the items: halves.
+static int fw_cut(long long items, int sms) {
+    const long long rem = items % sms;
+    return 4 * rem <= sms ? 2 : 2 * rem <= sms ? 1 : 0;
+}
+
 // LKB_ERR_UNSUPPORTED where another form is the better one or the planes do not have the alignment the copies ask for.
 int lkb_gemm_few_launch(const lkb_pf_gemm * g, int epi, int fold, int max_tiles, cudaStream_t st) {
     if (!lkb_tensor_map_encoder()) return LKB_ERR_UNSUPPORTED;
@@ -518,19 +549,23 @@ int lkb_gemm_few_launch(const lkb_pf_gemm * g, int epi, int fold, int max_tiles,
     // L2 fetches 256 bytes at a time (with 64-byte pieces of a row gate|up at 37 tokens took 12 us less so)
     const CUtensorMapL2promotion l2 = CU_TENSOR_MAP_L2_PROMOTION_L2_256B;
     const unsigned long long any = 1ull << 30;              // row bound of a plane whose extent the caller does not state: it only clips
-    CUtensorMap ma, ms, mw[3], md[3];
+    CUtensorMap ma, ms;
+    FwMaps maps;
     const unsigned long long rows = g->perm ? any : (unsigned long long) g->ntok;
     int r = lkb_tc_make_map(&ma, g->aqs, (unsigned) g->bpr * 32u, (unsigned) g->bpr * 32u, rows, FW_KB * 16u, 1u, CU_TENSOR_MAP_SWIZZLE_128B, l2);
     if (r == LKB_OK) r = lkb_tc_make_map(&ms, g->asc, (unsigned) g->bpr * 8u, (unsigned) g->bpr * 8u, rows, FW_KB * 8u, 1u, CU_TENSOR_MAP_SWIZZLE_NONE, l2);
-    for (int s = 0; s < 3 && r == LKB_OK; ++s) {
-        const int src = s < nseg ? s : 0;
-        r = lkb_tc_make_map(&mw[s], g->qs[src], (unsigned) g->bpr * 16u, (unsigned) g->bpr * 16u, any, FW_KB * 16u, FW_ROWS, CU_TENSOR_MAP_SWIZZLE_128B, l2);
-        if (r == LKB_OK) r = lkb_tc_make_map(&md[s], g->d[src], (unsigned) g->bpr * 2u, (unsigned) g->bpr * 2u, any, 16u, FW_ROWS, CU_TENSOR_MAP_SWIZZLE_NONE, l2);
-    }
+    const int sms = lkb_context().sm_count, cut = g->perm ? 1 : fw_cut((long long) ((g->ntok + tw - 1) / tw) * (g->N / (epi ? FW_ROWS : 2 * FW_ROWS)), sms);
+    for (int p = 0; p < 2; ++p)
+        for (int s = 0; s < 3 && r == LKB_OK; ++s) {
+            const unsigned box = p ? FW_ROWS >> cut : FW_ROWS;
+            if (s >= nseg || (p && !cut)) { const int f = s < nseg ? s : 0; maps.w[p][s] = maps.w[0][f]; maps.d[p][s] = maps.d[0][f]; continue; }
+            r = lkb_tc_make_map(&maps.w[p][s], g->qs[s], (unsigned) g->bpr * 16u, (unsigned) g->bpr * 16u, any, FW_KB * 16u, box, CU_TENSOR_MAP_SWIZZLE_128B, l2);
+            if (r == LKB_OK) r = lkb_tc_make_map(&maps.d[p][s], g->d[s], (unsigned) g->bpr * 2u, (unsigned) g->bpr * 2u, any, 16u, box, CU_TENSOR_MAP_SWIZZLE_NONE, l2);
+        }
     if (r != LKB_OK) return r;
     const int rpe = (int) (g->exp_stride / g->bpr);
-    const dim3 grid(lkb_context().sm_count), block(FW_THREADS);
-    if (tw <= 16) LKB_PF_LAUNCH(fw_form<16>(epi, fold), grid, block, fw_smem<16>(), st, *g, max_tiles, rpe, tw, ma, ms, mw[0], mw[1], mw[2], md[0], md[1], md[2]);
-    else           LKB_PF_LAUNCH(fw_form<32>(epi, fold), grid, block, fw_smem<32>(), st, *g, max_tiles, rpe, tw, ma, ms, mw[0], mw[1], mw[2], md[0], md[1], md[2]);
+    const dim3 grid(sms), block(FW_THREADS);
+    if (tw <= 16) LKB_PF_LAUNCH(fw_form<16>(epi, fold), grid, block, fw_smem<16>(), st, *g, max_tiles, rpe, tw, cut, ma, ms, maps);
+    else           LKB_PF_LAUNCH(fw_form<32>(epi, fold), grid, block, fw_smem<32>(), st, *g, max_tiles, rpe, tw, cut, ma, ms, maps);
     return lkb_check_launch();
 }

@@ -1,5 +1,6 @@
 """The few-token form of the GEMM beyond its first 47 tokens, at its edges: plan tiles cut into parts of 16 or 32 tokens, the MMA's groups of
-eight tokens, one stage of K and an odd number, more items than the stages hold, more parts than its list holds, dense chunks of every width.
+eight tokens, one stage of K and an odd number, more items than the stages hold, more parts than its list holds, dense chunks of every width, last
+waves cut into halves and quarters of rows, alone and behind whole ones.
 Bit for bit against the CPU checker; the fused SwiGLU form against the CUDA-core form (itself checked in test_gpu_prefill.py)."""
 import ctypes
 
@@ -42,7 +43,7 @@ def _width(L, g, max_tiles=MAX_TILES):
 
 
 @pytest.mark.parametrize("width", [16, 32])
-@pytest.mark.parametrize("N,bpr", [(256, 8), (1024, 24)])
+@pytest.mark.parametrize("N,bpr", [(256, 8), (1024, 24), (1280, 8), (2048, 8)])       # 22 to 256 items on 148 SMs
 def test_grouped(L, orc, N, bpr, width):
     rng = np.random.default_rng(N + width)
     perm, tiles = _plan(rng, COUNTS[width])
@@ -94,7 +95,7 @@ def test_more_parts_than_are_listed_swiglu(L, orc):
 
 
 @pytest.mark.parametrize("width", [16, 32])
-@pytest.mark.parametrize("I,bpr", [(128, 8), (384, 40)])
+@pytest.mark.parametrize("I,bpr", [(128, 8), (384, 40), (640, 8), (1024, 8)])          # 22 to 256 items
 @pytest.mark.parametrize("off", [0, 1])
 def test_swiglu(L, orc, I, bpr, width, off):
     """off: the quants' plane starts on an odd byte, which this form's stores cannot take; the call is served all the same."""
@@ -121,7 +122,7 @@ def test_swiglu(L, orc, I, bpr, width, off):
     assert int(got[1][0].float().abs().max()) > 0 and torch.isfinite(got[1][1][:, 0, 0]).any()
 
 
-@pytest.mark.parametrize("m,N,ends,bpr,width", [(5, 256, (256,) * 3, 64, 8), (37, 1024, (512, 640, 1024), 40, 8), (130, 2048, (2048,) * 3, 64, 8), (251, 2048, (2048,) * 3, 64, 16),
+@pytest.mark.parametrize("m,N,ends,bpr,width", [(5, 256, (256,) * 3, 64, 8), (37, 1024, (512, 640, 1024), 40, 8), (130, 2048, (2048,) * 3, 64, 8), (64, 2048, (1024, 1152, 2048), 64, 8), (3, 38912, (38912,) * 3, 8, 8), (160, 2304, (2304,) * 3, 64, 16), (251, 2048, (2048,) * 3, 64, 16),
                                                 (90, 6144, (6144,) * 3, 64, 16), (97, 6144, (6144,) * 3, 64, 24), (143, 6144, (2048, 4096, 6144), 64, 24), (300, 2048, (2048,) * 3, 64, 24), (145, 6144, (6144,) * 3, 64, 0), (37, 256, (256,) * 3, 8, 0)])
 def test_dense(L, orc, m, N, ends, bpr, width):
     rng = np.random.default_rng(7 * m + N)
