@@ -342,8 +342,8 @@ int lkb_pf_gemm_dense(const lkb_pf_gemm * g, lkb_stream_t st);
 int lkb_pf_gemm_moe(const lkb_pf_gemm * g, int max_tiles, lkb_stream_t st);
 int lkb_pf_gemm_swiglu(const lkb_pf_gemm * g, int max_tiles, lkb_stream_t st);
 /* Kernel-configuration selector of the three launchers above: -1 (default) the
- * tensor-core form wherever it covers the shape, and for a few tokens -- dense up to 4, MoE up to 188
- * slots (g->ntok) with max_tiles >= 64 -- a form that streams the weights once; 0 the CUDA-core form, 1 the
+ * tensor-core form wherever it covers the shape, and for a few tokens -- dense where its waves of items are
+ * shorter, MoE up to 1920 slots (g->ntok) with max_tiles >= 64 -- a form that streams the weights once; 0 the CUDA-core form, 1 the
  * tensor-core form or an error.  The results are the same bits in every form.  max_tiles bounds the tiles the plan may
  * have and says nothing about how full they are.  Also read once from the environment variable
  * LKB_PF_CFG by lkb_init().  ref: src/prefill.cu:813-848 (LK_PF_CFG_DENSE/MOE/SWIGLU) */

@@ -10,11 +10,11 @@
 //
 // One MMA per 32-element block (K = 32 int8 is one Q4_0 / Q8_1 block): the per-block scales forbid accumulating across
 // blocks in the tensor core, so every block's int32 sums come back through TMEM and are folded into fp32 register
-// accumulators, two FMAs per value.  That fold bounds the kernel: a packed fma.rn.f32x2 takes 2.1 cycles of a scheduler when
+// accumulators, two FMAs per value.  That fold and the constants it reads bound the kernel: a packed fma.rn.f32x2 takes 2.1 cycles of a scheduler when
 // it fetches two register pairs and 2.9 when it fetches three (measured, two warps a scheduler), and both FMAs of the fold
 // have three operands that differ, so the 128 of a 16384-value block cost 370 cycles.  Integer instructions do not hide under
-// them: one or two lop3 beside each make it 4.8 or 6.9 cycles.  In gate|up at 4096 tokens packed FMAs are half of the cycles,
-// and with the integer and the remaining FMA-pipe instructions four fifths (ncu's counts times these costs).
+// them: one or two lop3 beside each make it 4.8 or 6.9 cycles.  And a 16-byte shared load costs the SM four cycles of return path,
+// broadcasts too: the block's 128 loads of constants are 512 of its 600 or so cycles.
 //
 //   * TMEM lanes = weight rows, TMEM columns = tokens.  A work item is 256 weight rows (two 128-lane MMA tiles; the SwiGLU
 //     form: 128 gate rows and the same 128 up rows) x the 1..64 tokens of one plan tile, and the MMA's N is the token count
@@ -40,7 +40,8 @@
 //   ... weight scales in a ring of their own, expansion a stage at a time, no scale barriers, two issuers (this form)
 //                                                    70 / 117 / 569         47 /  64 / 268           23 / 51 / 238
 //   ... dense items cut to fill the waves (tc_dense_form)                                            20 / 45 / 236
-// (by itself the launcher takes this form above 188 slots (47 tokens of four) grouped and above 4 tokens dense, below them that of lkb_gemm_few.cu)
+//   ... SwiGLU stores two values at a time         gate|up at 4096 tokens 530
+// (by itself the launcher takes this form above 1920 slots (480 tokens of four) grouped, and dense where that of lkb_gemm_few.cu would need the longer waves)
 // With few tokens the hand-over of every block is the bound (300 to 440 cycles of polls, commits and arrivals).
 // No copy in this file is a multicast one; every tensor map covers memory of the GPU the kernel runs on.
 // Every wait is bounded; on expiry a status word is set and all roles drain and exit, freeing TMEM.
