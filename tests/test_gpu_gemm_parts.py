@@ -1,7 +1,7 @@
 """The few-token form of the GEMM beyond its first 47 tokens, at its edges: plan tiles cut into parts of 16 or 32 tokens, the MMA's groups of
 eight tokens, one stage of K and an odd number, more items than the stages hold, more parts than its list holds, dense chunks of every width, last
 waves cut into halves and quarters of rows, alone and behind whole ones.
-Bit for bit against the CPU checker; the fused SwiGLU form against the CUDA-core form (itself checked in test_gpu_prefill.py)."""
+Bit for bit against the oracle; the fused SwiGLU form against the CUDA-core form (itself checked in test_gpu_prefill.py)."""
 import ctypes
 
 import numpy as np
