@@ -44,6 +44,11 @@ else:
         return torch.cuda.current_stream().cuda_stream
 
 
+class _ArgumentError(C.ArgumentError, TypeError):
+    """An argument of another type than an entry point takes: what ctypes raises for one, and what it raises for a structure's field."""
+
+
+_fast.set_types(PfAct, C.Structure.__mro__[1], _ArgumentError)
 _fast.set_stream_lookup(*((_raw_stream, _device) if _raw_stream and _device else (stream, None)))
 
 

@@ -10,6 +10,7 @@
 #include "../../include/lkb.h"
 
 static PyObject * g_stream, * g_device;
+static PyObject * g_act_type, * g_ctypes_object, * g_argument_error;        // PfAct, the base of every ctypes object, what a refused argument raises
 
 // A tensor's address; NULL for None.  Sets *bad with an exception pending.
 static void * as_ptr(PyObject * t, int * bad) {
@@ -37,15 +38,24 @@ static float as_float(PyObject * o, int * bad) {
     if (v == -1.0 && PyErr_Occurred()) *bad = 1;
     return (float) v;
 }
-// The bytes of a ctypes structure.  They stay where they are while the caller holds the object, as it does for the call.
-static void * as_struct(PyObject * o, size_t size, int * bad) {
+// The bytes of an object of the ctypes type given; a subclass may be longer.  They stay where they are while the caller holds the object, as it does for the call.
+static void * as_struct(PyObject * o, PyObject * type, size_t size, int * bad) {
     if (*bad) return nullptr;
+    *bad = 1;
+    const int is = type ? PyObject_IsInstance(o, type) : 0;
+    if (is < 0) return nullptr;
     Py_buffer b;
-    if (PyObject_GetBuffer(o, &b, PyBUF_WRITABLE)) { *bad = 1; return nullptr; }
+    if (!is || PyObject_GetBuffer(o, &b, PyBUF_WRITABLE)) {
+        PyErr_Clear();
+        if (!g_argument_error || !type) PyErr_SetString(PyExc_RuntimeError, "no types set");
+        else PyErr_Format(g_argument_error, "expected %s instance instead of %s", ((PyTypeObject *) type)->tp_name, Py_TYPE(o)->tp_name);
+        return nullptr;
+    }
     void * const p = b.buf;
     const size_t len = (size_t) b.len;
     PyBuffer_Release(&b);
-    if (len != size) { PyErr_SetString(PyExc_TypeError, "a structure of another type"); *bad = 1; return nullptr; }
+    if (len < size) { PyErr_SetString(g_argument_error, "a shorter structure than the one wanted"); return nullptr; }
+    *bad = 0;
     return p;
 }
 // What lookup(device()) gives, or lookup() where there is no device function.
@@ -67,8 +77,8 @@ struct Ptr { void * p; template <class T> operator T *() const { return (T *) p;
 #define P(i) Ptr{as_ptr(a[i], &bad)}
 #define I(i) (int) as_int(a[i], &bad)
 #define F(i) as_float(a[i], &bad)
-#define ACT(i) const lkb_pf_act * act = (const lkb_pf_act *) as_struct(a[i], sizeof(lkb_pf_act), &bad)
-#define GEMM(i) const lkb_pf_gemm * g = (const lkb_pf_gemm *) as_struct(a[i], sizeof(lkb_pf_gemm), &bad)
+#define ACT(i) const lkb_pf_act * act = (const lkb_pf_act *) as_struct(a[i], g_act_type, sizeof(lkb_pf_act), &bad)
+#define GEMM(i) const lkb_pf_gemm * g = (const lkb_pf_gemm *) as_struct(a[i], g_ctypes_object, sizeof(lkb_pf_gemm), &bad)      /* any type, as by ctypes.byref */
 // Arguments first, in order; then the call, without the interpreter's lock (a launch may block when the device's queue is full).
 #define ENTRY(name, count, args, call) \
     static PyObject * f_##name(PyObject * self, PyObject * const * a, Py_ssize_t n) { \
@@ -115,7 +125,7 @@ static PyObject * f_fill_pf_gemm(PyObject * self, PyObject * const * a, Py_ssize
     (void) self;
     if (n != 20) { PyErr_SetString(PyExc_TypeError, "fill_pf_gemm takes 20 arguments"); return NULL; }
     int bad = 0;
-    lkb_pf_gemm * const g = (lkb_pf_gemm *) as_struct(a[0], sizeof(lkb_pf_gemm), &bad);
+    lkb_pf_gemm * const g = (lkb_pf_gemm *) as_struct(a[0], g_ctypes_object, sizeof(lkb_pf_gemm), &bad);
     PyObject * segs = bad ? NULL : PySequence_Fast(a[1], "segs: a sequence of (qs, d)"), * ends = segs ? PySequence_Fast(a[2], "seg_end: a sequence") : NULL;
     const Py_ssize_t ns = segs ? PySequence_Fast_GET_SIZE(segs) : 0, ne = ends ? PySequence_Fast_GET_SIZE(ends) : 0;
     if (!ends) bad = 1;
@@ -159,11 +169,23 @@ static PyObject * f_set_stream_lookup(PyObject * self, PyObject * const * a, Py_
     Py_RETURN_NONE;
 }
 
+static PyObject * f_set_types(PyObject * self, PyObject * const * a, Py_ssize_t n) {
+    (void) self;
+    if (n != 3 || !PyType_Check(a[0]) || !PyType_Check(a[1]) || !PyExceptionClass_Check(a[2])) {
+        PyErr_SetString(PyExc_TypeError, "set_types takes PfAct, the base of ctypes objects and an exception");
+        return NULL;
+    }
+    Py_INCREF(a[0]); Py_XSETREF(g_act_type, a[0]);
+    Py_INCREF(a[1]); Py_XSETREF(g_ctypes_object, a[1]);
+    Py_INCREF(a[2]); Py_XSETREF(g_argument_error, a[2]);
+    Py_RETURN_NONE;
+}
+
 #define M(name) {#name, (PyCFunction) (void (*)(void)) f_##name, METH_FASTCALL, NULL}
 static PyMethodDef methods[] = {
     M(rmsnorm_q8_1), M(gemv_q4_0), M(gemv_q6_K), M(argmax_part), M(argmax_final), M(pf_embed), M(pf_norm), M(pf_norm_router_select), M(pf_moe_route),
     M(pf_gemm_dense), M(pf_gemm_moe), M(pf_gemm_swiglu), M(pf_moe_combine_norm), M(pf_conv_next), M(pf_qknr), M(pf_attn), M(pf_quant_rows), M(fill_pf_gemm),
-    M(set_stream_lookup), {"ptr", f_ptr, METH_O, NULL}, {NULL, NULL, 0, NULL}};
+    M(set_stream_lookup), M(set_types), {"ptr", f_ptr, METH_O, NULL}, {NULL, NULL, 0, NULL}};
 static struct PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fast", NULL, -1, methods, NULL, NULL, NULL, NULL};
 PyMODINIT_FUNC PyInit__fast(void) {
     return PyModule_Create(&module);

@@ -24,6 +24,44 @@ def test_refusals(lkb):
         fast.fill_pf_gemm(lkb.PfGemm(), [], [1], *range(17))
 
 
+def _buffer(n):
+    return pytest.importorskip("numpy").zeros(n, "uint8")
+
+
+@pytest.mark.parametrize("wrong", [lambda lkb: lkb.StepScratch(), lambda lkb: (ctypes.c_void_p * 2)(), lambda lkb: _buffer(16), lambda lkb: bytearray(16),
+                                   lambda lkb: ctypes.byref(lkb.PfAct()), lambda lkb: None, lambda lkb: 0])
+def test_an_activation_is_a_pf_act(lkb, wrong):
+    """Sixteen writable bytes of another kind are refused, with the exception that a ctypes call raises."""
+    for call in (lambda a: lkb.k_pf_norm(None, None, 0, a, None, None, 4), lambda a: lkb.k_pf_quant_rows(None, 2048, 64, a, 4),
+                 lambda a: lkb.k_pf_conv_next(None, None, None, a, 4), lambda a: lkb.k_pf_moe_combine_norm(None, None, None, None, a, None, 4),
+                 lambda a: lkb.k_pf_norm_router_select(None, None, a, None, None, 4, 1, None, None, None, None, None, None)):
+        with pytest.raises(ctypes.ArgumentError):
+            call(wrong(lkb))
+
+
+def test_a_gemm_descriptor_is_a_ctypes_object(lkb):
+    """As ctypes.byref has it: no other buffer, and nothing shorter than the descriptor."""
+    n = ctypes.sizeof(lkb.PfGemm)
+    for g in (_buffer(n), bytearray(n), None, ctypes.byref(lkb.PfGemm()), lkb.PfAct(), (ctypes.c_byte * (n - 1))()):
+        for call in (lkb.pf_gemm_dense, lambda g: lkb.pf_gemm_moe(g, 4), lambda g: lkb.pf_gemm_swiglu(g, 4)):
+            with pytest.raises(TypeError):
+                call(g)
+
+
+def test_subclasses_and_arrays_are_taken(lkb):
+    """What ctypes took: a subclass by value, and whatever starts with a descriptor by reference.  Without a GPU the call ends at the stream or at
+    the entry point, behind its arguments."""
+    class Act(lkb.PfAct):
+        _fields_ = [("more", ctypes.c_int)]
+    for call in (lambda: lkb.k_pf_norm(None, None, 0, Act(), None, None, 4), lambda: lkb.pf_gemm_dense((lkb.PfGemm * 2)())):
+        try:
+            call()
+        except (TypeError, ctypes.ArgumentError):
+            raise
+        except Exception:
+            pass
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("n_seg", [1, 2, 3])
 def test_descriptor_fields(lkb, n_seg):
