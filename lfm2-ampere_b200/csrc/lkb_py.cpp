@@ -26,16 +26,24 @@ static void * as_ptr(PyObject * t, int * bad) {
         return nullptr;
     }
 }
-static long long as_int(PyObject * o, int * bad) {
+// What a number of another type raises: the same text under ctypes' exception.
+static void refuse() {
+    if (!PyErr_ExceptionMatches(PyExc_TypeError) || !g_argument_error) return;
+    PyObject * type, * value, * trace;
+    PyErr_Fetch(&type, &value, &trace);
+    PyErr_Format(g_argument_error, "%S", value ? value : type);
+    Py_XDECREF(type); Py_XDECREF(value); Py_XDECREF(trace);
+}
+static long long as_int(PyObject * o, int * bad) {               // masked to the field it goes into, as ctypes does
     if (*bad) return 0;
-    const long long v = PyLong_AsLongLong(o);
-    if (v == -1 && PyErr_Occurred()) *bad = 1;
-    return v;
+    const unsigned long long v = PyLong_AsUnsignedLongLongMask(o);
+    if (v == (unsigned long long) -1 && PyErr_Occurred()) { refuse(); *bad = 1; }
+    return (long long) v;
 }
 static float as_float(PyObject * o, int * bad) {
     if (*bad) return 0.0f;
     const double v = PyFloat_AsDouble(o);
-    if (v == -1.0 && PyErr_Occurred()) *bad = 1;
+    if (v == -1.0 && PyErr_Occurred()) { refuse(); *bad = 1; }
     return (float) v;
 }
 // The bytes of an object of the ctypes type given; a subclass may be longer.  They stay where they are while the caller holds the object, as it does for the call.

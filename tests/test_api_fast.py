@@ -48,6 +48,19 @@ def test_a_gemm_descriptor_is_a_ctypes_object(lkb):
                 call(g)
 
 
+def test_numbers_as_ctypes_takes_them(lkb):
+    """An argument of another type raises ctypes' exception; whole numbers are masked to the field, as in a ctypes structure."""
+    for bad in (None, "4", 4.0):
+        with pytest.raises(ctypes.ArgumentError):
+            lkb.k_pf_moe_route(None, bad, None, None, None, None, None)
+    with pytest.raises(ctypes.ArgumentError):
+        lkb.k_gemv_q4_0(None, None, None, 32, 64, None, eps="1e-5")
+    g, wide = lkb.make_pf_gemm([(None, None)], [(1 << 70) + 5, -3], 1 << 32 | 7, 64, None, None, ntok=True, exp_stride=-(1 << 63)), lkb.PfGemm()
+    wide.N, wide.bpr, wide.ntok, wide.exp_stride = 1 << 32 | 7, 64, True, -(1 << 63)
+    wide.seg_end[:] = [(1 << 70) + 5, -3, -3]
+    assert bytes(g) == bytes(wide)
+
+
 def test_subclasses_and_arrays_are_taken(lkb):
     """What ctypes took: a subclass by value, and whatever starts with a descriptor by reference.  Without a GPU the call ends at the stream or at
     the entry point, behind its arguments."""
