@@ -13,6 +13,7 @@ B200, and raises otherwise.
 from __future__ import annotations
 
 import ctypes as C
+import importlib
 import pathlib
 import re
 
@@ -112,7 +113,21 @@ def load_library():
     return lib
 
 
+def load_bindings():
+    """The native module that reads tensors of the installed torch (csrc/lkb_py.cpp): one of another build is not used."""
+    import torch
+    try:
+        fast = importlib.import_module("._fast", __name__)
+    except ImportError as e:
+        raise LkbError(f"the native bindings cannot be loaded ({e}): build them with `python lfm2-ampere_b200/build.py`") from e
+    built = getattr(fast, "built_for", "another version")
+    if built != f"torch {torch.__version__};":
+        raise LkbError(f"the native bindings were built for {built} and torch is {torch.__version__}: build them with `python lfm2-ampere_b200/build.py`")
+    return fast
+
+
 lib = load_library()
+_fast = load_bindings()
 _inited = set()
 
 

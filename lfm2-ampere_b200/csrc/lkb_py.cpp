@@ -196,5 +196,7 @@ static PyMethodDef methods[] = {
     M(set_stream_lookup), M(set_types), {"ptr", f_ptr, METH_O, NULL}, {NULL, NULL, 0, NULL}};
 static struct PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fast", NULL, -1, methods, NULL, NULL, NULL, NULL};
 PyMODINIT_FUNC PyInit__fast(void) {
-    return PyModule_Create(&module);
+    PyObject * m = PyModule_Create(&module);
+    if (m && PyModule_AddStringConstant(m, "built_for", LKB_BUILT_FOR)) Py_CLEAR(m);       // the torch whose objects it reads; the package looks at it
+    return m;
 }
