@@ -61,7 +61,7 @@ def build_bindings():
     inc = [x for p in cpp_extension.include_paths() + [sysconfig.get_paths()["include"]] for x in ("-isystem", p)]
     cmd = ["g++", "-O2", "-std=c++17", "-Wall", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
            f'-DLKB_BUILT_FOR="torch {torch.__version__};"'] + inc + [
-        "-o", str(PY_OUT), str(CSRC / "lkb_py.cpp"), "-L", str(HERE), "-l:liblkb.so", "-Wl,-rpath,$ORIGIN",
+        "-o", str(PY_OUT), str(CSRC / "lkb_py.cpp"), "-L", str(HERE), "-l:liblkb.so", "-Wl,-rpath,$ORIGIN,--disable-new-dtags",      # RPATH: before LD_LIBRARY_PATH
         "-L", str(pathlib.Path(torch.__file__).parent / "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode:

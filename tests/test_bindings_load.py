@@ -1,5 +1,6 @@
 """The native bindings that the package loads: built for this interpreter and this torch, or refused with advice."""
 import importlib.util
+import os
 import pathlib
 import shutil
 import subprocess
@@ -71,3 +72,12 @@ def test_rebuilt_for_another_torch(tmp_path, monkeypatch):
     monkeypatch.setattr(build.subprocess, "run", lambda cmd, **k: ran.append(cmd[0]) or subprocess.CompletedProcess(cmd, 0, "", ""))
     build.build()
     assert ran == ["g++"]
+
+
+def test_one_library_whatever_the_loader_s_path(tmp_path):
+    """The bindings call into the library that the package loaded, not into a second copy (never initialised) found on LD_LIBRARY_PATH."""
+    shutil.copy(PKG / "liblkb.so", tmp_path)
+    code = ("import importlib; importlib.import_module('lfm2-ampere_b200')\n"
+            "print({l.split(None, 5)[-1].strip() for l in open('/proc/self/maps') if 'liblkb.so' in l})")
+    r = subprocess.run([sys.executable, "-c", code], cwd=PKG.parent, capture_output=True, text=True, check=True, env={**os.environ, "LD_LIBRARY_PATH": str(tmp_path)})
+    assert r.stdout.strip() == repr({str(PKG / "liblkb.so")})
