@@ -384,9 +384,7 @@ __global__ void __launch_bounds__(FW_THREADS, 1) k_pf_gemm_few(const lkb_pf_gemm
                 __syncwarp();
             }
         }
-        if (!ok)                                                         // copies in flight land before the block leaves (bounded)
-            for (unsigned k = it < S.NS ? 0u : it - S.NS; k < it; ++k)
-                for (unsigned i = 0; i < 4096u && !tc_mbar_try<TC_HINT_PROD>(&S.full[k % S.NS], (k / S.NS) & 1u); ++i) { }
+        tc_drain<S.NS>(S.full, it);
     } else if (warp == FW_C_WARP) {
         // ============================ token constants (one warp) =====================
         bool ok = true;

@@ -62,6 +62,13 @@ __device__ __forceinline__ bool tc_wait(SM & S, unsigned long long * b, unsigned
 }
 #define TC_HINT_PROD 2000           // ns
 #define TC_HINT_MMA  500
+// How a copying role leaves, whoever gave up: the copies of the last N stages before `it` land before the block ends (bounded).  On the
+// ordinary path another role needs them all the same.
+template <int N> __device__ __forceinline__ void tc_drain(unsigned long long * full, unsigned it) {
+#pragma unroll 1
+    for (unsigned k = it < N ? 0u : it - N; k < it; ++k)
+        for (unsigned i = 0; i < 4096u && !tc_mbar_try<TC_HINT_PROD>(&full[k % N], (k / N) & 1u); ++i) { }
+}
 __device__ __forceinline__ bool tc_elect() {
     unsigned p;
     asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(p));
