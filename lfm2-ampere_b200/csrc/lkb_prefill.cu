@@ -499,9 +499,7 @@ __global__ void __launch_bounds__(32 * NW + 32) k_pf_router_tma(int m, const __g
                 tc_tma_tile(st + lane * F::SUB + LKB_N_EXPERTS * 128, &map_h, (tile * RT_KT + lane * 32) * 4, t0, &full[stg]);
             }
         }
-        if (tile < NTILES)                                             // copies in flight land before the block leaves (bounded)
-            for (int k = max(0, tile - RT_STAGES); k < tile; ++k)
-                for (unsigned i = 0; i < 4096u && !tc_mbar_try<TC_HINT_PROD>(&full[k % RT_STAGES], (unsigned) (k / RT_STAGES) & 1u); ++i) { }
+        tc_drain<RT_STAGES>(full, tile);
     } else for (int tile = 0; tile < NTILES; ++tile) {
         const int stg = tile % RT_STAGES;
         if (!tc_wait(S, &full[stg], (unsigned) (tile / RT_STAGES) & 1u, 42u)) break;
