@@ -567,6 +567,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_pf_gemm_tc(const lkb_pf_gemm 
                     if (glive) tc_tma_gather4(T.act + lane * 512, &map_a, ks * 128, crd[0], crd[1], crd[2], crd[3], &S.full[stg]);
                 }
             }
+            tc_drain<TC_NS>(S.full, it);
         }
         // ============================ MMA issuers (two warps) ========================
         // Issuer q serves column half q (free halves) or block-sum buffer q, that is blocks q and q + 2 of every stage: polls,
