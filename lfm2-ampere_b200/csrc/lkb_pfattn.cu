@@ -204,7 +204,8 @@ __global__ void __launch_bounds__(FaCfg<NT>::THREADS, FaCfg<NT>::CTAS) k_pf_attn
         __syncwarp();
         int slot = 0;
         unsigned par = 1;                                       // every slot starts out empty
-        for (int t = 0; t < 2 * nkt; ++t) {                     // K0 V0 K1 V1 ...
+        int t = 0;
+        for (; t < 2 * nkt; ++t) {                              // K0 V0 K1 V1 ...
             if (!tc_wait<TC_HINT_PROD>(S, &S.empty[slot], par, 50u)) break;
             if (leader) {
                 tc_mbar_arrive_tx(&S.full[slot], FA_TILE);
@@ -213,6 +214,8 @@ __global__ void __launch_bounds__(FaCfg<NT>::THREADS, FaCfg<NT>::CTAS) k_pf_attn
             __syncwarp();
             if (++slot == C::SLOTS) { slot = 0; par ^= 1u; }
         }
+        tc_drain<1>(&S.qfull, q_rows ? 0 : 1);
+        tc_drain<C::SLOTS>(S.full, t);
     } else if (warp == C::MMA_WARP) {
         const bool leader = tc_elect();
         int slot = 0;

@@ -10,6 +10,7 @@ CSRC = pathlib.Path(__file__).resolve().parent.parent / "lfm2-ampere_b200" / "cs
 # file, what names the copying warps' code, what follows it
 COPIERS = {"few": ("lkb_gemm_few.cu", "producers (three warps)", "token constants (one warp)"),
            "tensor-core GEMM": ("lkb_gemm_tc.cu", "producer (one warp)", "MMA issuers (two warps)"),
+           "attention": ("lkb_pfattn.cu", "if (warp == C::TMA_WARP) {", "} else if (warp == C::MMA_WARP) {"),
            "router": ("lkb_prefill.cu", "if (warp == NW) {\n", "} else for (int tile")}
 
 
