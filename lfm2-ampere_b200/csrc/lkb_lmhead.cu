@@ -135,6 +135,7 @@ __global__ void __launch_bounds__(LM_THREADS, 1) k_gemv_q6_K_stream(const unsign
                 if (id >= total) {
                     S.row[b] = -1;
                     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(lm_u32(&S.full[b])) : "memory");
+                    ++c;
                     return false;
                 }
                 const int row = (int) id * LM_ROWS, n = min(LM_ROWS, out_rows - row);
@@ -159,6 +160,9 @@ __global__ void __launch_bounds__(LM_THREADS, 1) k_gemv_q6_K_stream(const unsign
             if (ok) while (ticketed(t0) && ticketed(t1) && ticketed(t2) && ticketed(t3)) { }
             __threadfence();
             if (atomicAdd(&ctr[1], 1u) == gridDim.x - 1) { ctr[0] = 0u; ctr[1] = 0u; __threadfence(); }
+            // whoever gave up, the copies of the last slots land before the block leaves (bounded; on the ordinary path a consumer needs them all the same)
+            for (int k = max(0, c - LM_NBUF); k < c; ++k)
+                for (unsigned i = 0; i < LM_SPIN && !lm_try(&S.full[k % LM_NBUF], (unsigned) (k / LM_NBUF) & 1u); ++i) { }
         }
         return;
     }

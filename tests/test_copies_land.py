@@ -11,6 +11,7 @@ CSRC = pathlib.Path(__file__).resolve().parent.parent / "lfm2-ampere_b200" / "cs
 COPIERS = {"few": ("lkb_gemm_few.cu", "producers (three warps)", "token constants (one warp)"),
            "tensor-core GEMM": ("lkb_gemm_tc.cu", "producer (one warp)", "MMA issuers (two warps)"),
            "attention": ("lkb_pfattn.cu", "if (warp == C::TMA_WARP) {", "} else if (warp == C::MMA_WARP) {"),
+           "output projection": ("lkb_lmhead.cu", "if (warp == LM_WARPS) {", "// consumers: the activation"),
            "router": ("lkb_prefill.cu", "if (warp == NW) {\n", "} else for (int tile")}
 
 
@@ -20,7 +21,7 @@ def _drains(name):
     text = (CSRC / file).read_text()
     part = text[text.index(a):text.index(b, text.index(a))]
     part = re.sub(r"//[^\n]*", "", part)
-    d = re.search(r"tc_drain|tc_mbar_try", part)
+    d = re.search(r"tc_drain|tc_mbar_try|\blm_try", part)
     if not d:
         return "never"
     return "own" if re.search(r"if \((?:!ok|tile < NTILES)\)", part[:d.start()]) else "always"
