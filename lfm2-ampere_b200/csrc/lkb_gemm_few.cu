@@ -482,31 +482,33 @@ static bool fw_better(const lkb_pf_gemm * g, int max_tiles) {
 // Test hook (not in the public header): whether a call takes this form whatever the other's time.
 extern "C" __attribute__((visibility("default"))) int lkb_debug_gemm_few_better(const lkb_pf_gemm * g, int max_tiles) { return fw_better(g, max_tiles); }
 
+static int fw_row_tiles(int N, int epi) { return N / (epi ? FW_ROWS : 2 * FW_ROWS); }       // of an item: two tiles, SwiGLU form: of 128 output rows
 // The token width of a dense problem's items, or 0 where the tensor-core form is faster: waves x the time of an item's block, which is 95, 128 or
 // 176 ns at 8, 16 or 24 tokens here (64 blocks a row: a wave more takes 6.1, 8.2 or 11.3 us; 225 ns at 32, never better) against tc_dense_ns there, and 5 us more
 // an item for launch, fill and drain.  us in the tensor-core form and here, caches flushed: in_proj (6144 rows) at 37 / 64 / 96 / 128 / 144 / 432 tokens
 // 19.5 / 24.6 / 24.6 / 23.6 / 24.6 / 46.1 -> 14.3 / 16.4 / 16.4 / 18.9 / 19.0 / 39.9 (at 256 28.7 there, 32.8 here), out_proj (2048 rows) at 37 / 128 / 256 / 300 / 432
 // 18.4 / 20.5 / 24.6 / 23.5 / 24.0 -> 12.3 / 12.3 / 16.4 / 17.9 / 18.9.
-int lkb_gemm_tc_dense_ns(int ntok, int N, int sms);      // lkb_gemm_tc.cu
-static int fw_dense_width(int ntok, int N, int bpr, int sms, bool always) {
+int lkb_gemm_tc_dense_ns(int ntok, int N, int sms, int epi);      // lkb_gemm_tc.cu
+static int fw_dense_width(int ntok, int N, int bpr, int sms, int epi, bool always) {
     static const int ns[3] = {95, 128, 176};
     int best = 0;
-    long long least = always ? 1ll << 62 : lkb_gemm_tc_dense_ns(ntok, N, sms) - 5000 / bpr;
+    long long least = always ? 1ll << 62 : lkb_gemm_tc_dense_ns(ntok, N, sms, epi) - 5000 / bpr;
     for (int i = 0; i < 3; ++i) {
         const int tw = 8 * (i + 1);
-        const long long items = (long long) ((ntok + tw - 1) / tw) * (N / (2 * FW_ROWS)), t = (items + sms - 1) / sms * ns[i];
+        const long long items = (long long) ((ntok + tw - 1) / tw) * fw_row_tiles(N, epi), t = (items + sms - 1) / sms * ns[i];
         if (t < least) { least = t; best = tw; }
     }
     return best;
 }
-static int fw_width(const lkb_pf_gemm * g, int max_tiles, int sms) {
+static int fw_width(const lkb_pf_gemm * g, int epi, int max_tiles, int sms) {
     const bool always = fw_better(g, max_tiles);
-    if (!g->perm) return fw_dense_width(g->ntok, g->N, g->bpr, sms, always);
+    if (!g->perm) return fw_dense_width(g->ntok, g->N, g->bpr, sms, epi, always);
     if (!always && (max_tiles < FW_MIN_TILES || g->ntok <= 0 || g->ntok > FW_MORE_SLOTS)) return 0;
     return g->ntok <= FW_16_SLOTS ? 16 : 32;
 }
-// Test hook (not in the public header): the items' token width where a call takes this form, if its planes allow it; else 0.
-extern "C" __attribute__((visibility("default"))) int lkb_debug_gemm_few_width(const lkb_pf_gemm * g, int max_tiles, int sms) { return fw_width(g, max_tiles, sms); }
+// Test hook (not in the public header): the items' token width where a call (with planes for quants: of the SwiGLU form) takes this form, if its
+// planes allow it; else 0.
+extern "C" __attribute__((visibility("default"))) int lkb_debug_gemm_few_width(const lkb_pf_gemm * g, int max_tiles, int sms) { return fw_width(g, g->oqs != nullptr, max_tiles, sms); }
 
 // Test hook (not in the public header): over `count` float bit patterns from `first` on, counts[0] += those whose tc_silu2 is sure of another
 // result than lkb_silu's, counts[1] += those it is not sure of.
@@ -537,7 +539,7 @@ static int fw_cut(long long items, int sms) {
 // LKB_ERR_UNSUPPORTED where another form is the better one or the planes do not have the alignment the copies ask for.
 int lkb_gemm_few_launch(const lkb_pf_gemm * g, int epi, int fold, int max_tiles, cudaStream_t st) {
     if (!lkb_tensor_map_encoder()) return LKB_ERR_UNSUPPORTED;
-    const int tw = fw_width(g, max_tiles, lkb_context().sm_count);
+    const int tw = fw_width(g, epi, max_tiles, lkb_context().sm_count);
     if (!tw) return LKB_ERR_UNSUPPORTED;
     if (epi ? (g->N % FW_ROWS) : (g->N % (2 * FW_ROWS))) return LKB_ERR_UNSUPPORTED;
     if (g->bpr % 8 || (((size_t) g->aqs | (size_t) g->asc) & 15) || g->exp_stride % g->bpr) return LKB_ERR_UNSUPPORTED;
@@ -552,7 +554,7 @@ int lkb_gemm_few_launch(const lkb_pf_gemm * g, int epi, int fold, int max_tiles,
     const unsigned long long rows = g->perm ? any : (unsigned long long) g->ntok;
     int r = lkb_tc_make_map(&ma, g->aqs, (unsigned) g->bpr * 32u, (unsigned) g->bpr * 32u, rows, FW_KB * 16u, 1u, CU_TENSOR_MAP_SWIZZLE_128B, l2);
     if (r == LKB_OK) r = lkb_tc_make_map(&ms, g->asc, (unsigned) g->bpr * 8u, (unsigned) g->bpr * 8u, rows, FW_KB * 8u, 1u, CU_TENSOR_MAP_SWIZZLE_NONE, l2);
-    const int sms = lkb_context().sm_count, cut = g->perm ? 1 : fw_cut((long long) ((g->ntok + tw - 1) / tw) * (g->N / (epi ? FW_ROWS : 2 * FW_ROWS)), sms);
+    const int sms = lkb_context().sm_count, cut = g->perm ? 1 : fw_cut((long long) ((g->ntok + tw - 1) / tw) * fw_row_tiles(g->N, epi), sms);
     for (int p = 0; p < 2; ++p)
         for (int s = 0; s < 3 && r == LKB_OK; ++s) {
             const unsigned box = p ? FW_ROWS >> cut : FW_ROWS;

@@ -815,13 +815,14 @@ int lkb_tc_make_map(CUtensorMap * m, const void * base, unsigned row_bytes, unsi
 // cut into narrow items (each reads the weights again, from L2), and one that would leave most of its last wave empty is cut
 // so that the waves fill.  us with 64-token items and with these, caches flushed: in_proj (6144 rows) at 37 / 130 / 509 tokens
 // 22.5 / 26.6 / 51.2 -> 19.5 / 24.6 / 45.0, out_proj (2048 rows) 24.6 / 26.6 / 28.7 -> 18.4 / 20.5 / 26.6; at 4096 tokens the
-// choice is 64 x 256 as before.
-static TcDense tc_dense_form(int ntok, int N, int sms, long long * cost = nullptr) {
+// choice is 64 x 256 as before.  SwiGLU form: an item is 128 rows of either weight, two tiles always.
+static TcDense tc_dense_form(int ntok, int N, int sms, int epi, long long * cost = nullptr) {
     TcDense best = {TC_TOK, 1};
     long long least = 0;
-    for (int wide = 1; wide >= 0; --wide)
+    for (int wide = 1; wide >= (epi ? 1 : 0); --wide)
         for (int tw = TC_TOK; tw >= 16; tw -= 16) {
-            const long long items = (long long) ((ntok + tw - 1) / tw) * ((N + (wide ? 2 : 1) * TC_ROWS - 1) / ((wide ? 2 : 1) * TC_ROWS));
+            const int rows = wide && !epi ? 2 * TC_ROWS : TC_ROWS;
+            const long long items = (long long) ((ntok + tw - 1) / tw) * ((N + rows - 1) / rows);
             const long long t = (items + sms - 1) / sms * (wide ? 3500 + 62 * tw : 3300 + 60 * tw);
             if (!least || t < least) { least = t; best = {tw, wide}; }
         }
@@ -829,15 +830,15 @@ static TcDense tc_dense_form(int ntok, int N, int sms, long long * cost = nullpt
     return best;
 }
 // What a block of all its items' waves takes, in ns: the above at 1.87 GHz.
-int lkb_gemm_tc_dense_ns(int ntok, int N, int sms) {
+int lkb_gemm_tc_dense_ns(int ntok, int N, int sms, int epi) {
     long long c = 0;
-    tc_dense_form(ntok, N, sms, &c);
+    tc_dense_form(ntok, N, sms, epi, &c);
     return (int) (c * 100 / 1870 < (1 << 30) ? c * 100 / 1870 : 1 << 30);
 }
 
-// Test hook (not in the public header): the items a dense problem is cut into, tokens * 1000 + weight rows.
+// Test hook (not in the public header): the items a plain dense problem is cut into, tokens * 1000 + weight rows.
 extern "C" __attribute__((visibility("default"))) int lkb_debug_gemm_dense_item(int ntok, int N) {
-    const TcDense d = tc_dense_form(ntok, N, lkb_context().sm_count);
+    const TcDense d = tc_dense_form(ntok, N, lkb_context().sm_count, 0);
     return d.tw * 1000 + (d.wide ? 2 : 1) * TC_ROWS;
 }
 
@@ -876,7 +877,7 @@ int lkb_gemm_tc_launch(const lkb_pf_gemm * g, int epi, int fold, int max_tiles, 
     const dim3 grid(lkb_context().sm_count), block(TC_THREADS);
     const size_t sm = sizeof(TcSmem) + 1024;
     LKB_PF_LAUNCH(TC_FORMS[(epi ? 4 : 0) + (fold ? 2 : 0) + wcopy], grid, block, sm, st, *g, max_tiles, rpe, sc_plane, s_pitch, ma, mw[0], mw[1], mw[2],
-                  md[0], md[1], md[2], out_rows, g->perm ? TcDense{TC_TOK, 1} : tc_dense_form(g->ntok, g->N, lkb_context().sm_count));
+                  md[0], md[1], md[2], out_rows, g->perm ? TcDense{TC_TOK, 1} : tc_dense_form(g->ntok, g->N, lkb_context().sm_count, epi));
     return lkb_check_launch();
 }
 

@@ -42,3 +42,11 @@ def test_width_of_dense_items(lkb, m, N, bpr, width):
     g = lkb.PfGemm()
     g.ntok, g.N, g.bpr = m, N, bpr
     assert lkb.lib.lkb_debug_gemm_few_width(ctypes.byref(g), 0, 148) == width
+
+
+@pytest.mark.parametrize("m,N,bpr,width", [(5, 128, 64, 8), (37, 1536, 64, 8), (100, 1536, 64, 16), (130, 1536, 64, 16), (200, 1536, 64, 24), (300, 1536, 64, 0)])
+def test_width_of_dense_swiglu_items(lkb, m, N, bpr, width):
+    """An item of the SwiGLU form is 128 output rows (128 gate and 128 up rows): N / 128 of them a width of tokens, in either form."""
+    g = lkb.PfGemm()
+    g.ntok, g.N, g.bpr, g.oqs = m, N, bpr, 64
+    assert lkb.lib.lkb_debug_gemm_few_width(ctypes.byref(g), 0, 148) == width
