@@ -41,9 +41,9 @@ def needs_build():
 
 def build(force=False, verbose=False):
     if force or needs_library():
-        nvcc = str(pathlib.Path(os.environ.get("CUDA_HOME", "/usr/local/cuda")) / "bin" / "nvcc")
-        cmd = [nvcc] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) + ["-o", str(OUT)] + [str(CSRC / s) for s in SOURCES]
-        print(" ".join(map(shlex.quote, cmd)))
+        srcs = [str(CSRC / s) for s in SOURCES if (CSRC / s).exists()]
+        extra = shlex.split(os.environ.get("LKB_NVCC_EXTRA", ""))          # e.g. -DTC_MAGIC=0 while tuning
+        cmd = ["nvcc"] + NVCC_FLAGS + extra + (["-Xptxas", "-v"] if verbose else []) + ["-o", str(OUT)] + srcs + ["-lcuda"]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if verbose or r.returncode:
             sys.stderr.write(r.stdout + r.stderr)

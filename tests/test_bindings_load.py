@@ -81,3 +81,15 @@ def test_one_library_whatever_the_loader_s_path(tmp_path):
             "print({l.split(None, 5)[-1].strip() for l in open('/proc/self/maps') if 'liblkb.so' in l})")
     r = subprocess.run([sys.executable, "-c", code], cwd=PKG.parent, capture_output=True, text=True, check=True, env={**os.environ, "LD_LIBRARY_PATH": str(tmp_path)})
     assert r.stdout.strip() == repr({str(PKG / "liblkb.so")})
+
+
+def test_build_takes_extra_compiler_options(monkeypatch):
+    """LKB_NVCC_EXTRA reaches the compiler that PATH has, between the fixed options and the sources."""
+    build = _load(PKG / "build.py", "lkb_build_copy")
+    ran = []
+    monkeypatch.setattr(build.subprocess, "run", lambda cmd, **k: ran.append(cmd) or subprocess.CompletedProcess(cmd, 0, "", ""))
+    monkeypatch.setenv("LKB_NVCC_EXTRA", "-DSOME=1 '-DOTHER=a b'")
+    build.build(force=True)
+    n = len(build.NVCC_FLAGS)
+    assert ran[0][0] == "nvcc" and ran[0][1:n + 1] == build.NVCC_FLAGS and ran[0][n + 1:n + 3] == ["-DSOME=1", "-DOTHER=a b"]
+    assert [c[0] for c in ran] == ["nvcc", "g++"]
