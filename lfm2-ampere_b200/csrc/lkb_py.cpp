@@ -12,10 +12,23 @@
 static PyObject * g_stream, * g_device;
 static PyObject * g_act_type, * g_ctypes_object, * g_argument_error;        // PfAct, the base of every ctypes object, what a refused argument raises
 
+// The address of anything else with a tensor's is_cuda, is_contiguous() and data_ptr(): subclasses that override them, wrappers of memory of their own.
+static void * other_ptr(PyObject * t, int * bad) {
+    PyObject * cuda = PyObject_GetAttrString(t, "is_cuda"), * whole = NULL, * at = NULL;
+    int yes = cuda ? PyObject_IsTrue(cuda) : -1;
+    if (yes > 0) whole = PyObject_CallMethod(t, "is_contiguous", NULL), yes = whole ? PyObject_IsTrue(whole) : -1;
+    if (!yes) PyErr_SetString(PyExc_AssertionError, "device-resident contiguous tensors only");
+    else if (yes < 0 && PyErr_ExceptionMatches(PyExc_AttributeError)) PyErr_SetString(PyExc_TypeError, "a tensor is wanted");
+    void * p = NULL;
+    if (yes > 0) at = PyObject_CallMethod(t, "data_ptr", NULL), p = at ? PyLong_AsVoidPtr(at) : NULL;
+    Py_XDECREF(cuda); Py_XDECREF(whole); Py_XDECREF(at);
+    if (PyErr_Occurred()) *bad = 1;
+    return p;
+}
 // A tensor's address; NULL for None.  Sets *bad with an exception pending.
 static void * as_ptr(PyObject * t, int * bad) {
     if (*bad || t == Py_None) return nullptr;
-    if (!THPVariable_Check(t)) { PyErr_SetString(PyExc_TypeError, "a tensor is wanted"); *bad = 1; return nullptr; }
+    if (!THPVariable_CheckExact(t)) return other_ptr(t, bad);
     try {
         const at::Tensor & v = THPVariable_Unpack(t);
         if (!v.is_cuda() || !v.is_contiguous()) { PyErr_SetString(PyExc_AssertionError, "device-resident contiguous tensors only"); *bad = 1; return nullptr; }

@@ -95,3 +95,41 @@ def test_descriptor_fields(lkb, n_seg):
     assert h.perm is None and h.out is None and h.ntok == 0 and ctypes.sizeof(h) == ctypes.sizeof(g)
     with pytest.raises(AssertionError):
         lkb.make_pf_gemm([(segs[0][0][::2], segs[0][1])], ends, 384, 24, t["aqs"], t["asc"])        # not contiguous
+
+
+class _Memory:
+    """What a wrapper of device memory shows of a tensor."""
+    is_cuda = True
+
+    def __init__(self, at, whole=True):
+        self.at, self.whole = at, whole
+
+    def is_contiguous(self):
+        return self.whole
+
+    def data_ptr(self):
+        return self.at
+
+
+class _Subclass(torch.Tensor):
+    is_cuda = property(lambda self: True)
+
+    def data_ptr(self):
+        return 4096
+
+
+def test_whatever_has_a_tensor_s_address(lkb):
+    """An address is asked for through is_cuda, is_contiguous() and data_ptr(), which subclasses and wrappers may have of their own."""
+    api = importlib.import_module("lfm2-ampere_b200.api")
+    assert api.ptr(_Memory(1 << 40)) == 1 << 40 and api.ptr(torch.zeros(4).as_subclass(_Subclass)) == 4096
+    assert api.pf_act(_Memory(64), _Memory(128)).sc == 128
+    g = lkb.make_pf_gemm([(_Memory(16), _Memory(32))], [128], 128, 8, _Memory(48), None)
+    assert (g.qs[0], g.d[2], g.aqs, g.asc) == (16, 32, 48, None)
+    assert api.ptr(_Memory(0)) == 0
+    for refused in (_Memory(64, whole=False), torch.zeros(4, 4).t(), torch.nn.Parameter(torch.zeros(4))):
+        with pytest.raises(AssertionError):
+            api.ptr(refused)
+    with pytest.raises(TypeError):
+        api.ptr("64")
+    with pytest.raises(ZeroDivisionError):
+        api.ptr(_Memory(64, whole=type("", (), {"__bool__": lambda self: 1 // 0})()))
