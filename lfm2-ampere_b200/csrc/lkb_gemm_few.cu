@@ -510,17 +510,21 @@ static int fw_width(const lkb_pf_gemm * g, int epi, int max_tiles, int sms) {
 // planes allow it; else 0.
 extern "C" __attribute__((visibility("default"))) int lkb_debug_gemm_few_width(const lkb_pf_gemm * g, int max_tiles, int sms) { return fw_width(g, g->oqs != nullptr, max_tiles, sms); }
 
-// Test hook (not in the public header): over `count` float bit patterns from `first` on, counts[0] += those whose tc_silu2 is sure of another
-// result than lkb_silu's, counts[1] += those it is not sure of.
+// Test hook (not in the public header): over `count` float bit patterns from `first` on, in either half of a pair whose other is 1:
+// counts[0] += halves where tc_silu2 is sure of another result than lkb_silu's, counts[1] += those it is not sure of.
 __global__ void k_debug_silu(unsigned first, unsigned long long count, unsigned long long * __restrict__ counts) {
     unsigned long long wrong = 0, unsure = 0;
     for (unsigned long long i = blockIdx.x * (unsigned long long) blockDim.x + threadIdx.x; i < count; i += (unsigned long long) gridDim.x * blockDim.x) {
         const float v = __uint_as_float(first + (unsigned) i);
-        bool sure = true;
-        float q, o;
-        tc_unpack(tc_silu2(tc_pack(v, 1.0f), sure), q, o);
-        unsure += !sure;
-        wrong += sure && __float_as_uint(q) != __float_as_uint(lkb_silu(v));
+        const unsigned want = __float_as_uint(lkb_silu(v));
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            bool sure = true;
+            float q[2];
+            tc_unpack(tc_silu2(half ? tc_pack(1.0f, v) : tc_pack(v, 1.0f), sure), q[0], q[1]);
+            unsure += !sure;
+            wrong += sure && __float_as_uint(q[half]) != want;
+        }
     }
     if (wrong) atomicAdd(counts, wrong);
     if (unsure) atomicAdd(counts + 1, unsure);
