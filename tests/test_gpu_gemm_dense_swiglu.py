@@ -38,4 +38,4 @@ def test_dense_swiglu(lkb, orc, m, I, bpr, width, fold):
     assert lkb.lib.lkb_pf_gemm_status() == 0
     for q, s in got[1:]:
         assert torch.equal(q, got[0][0]) and torch.equal(s.view(torch.int32), got[0][1].view(torch.int32))
-    assert int(got[0][0].float().abs().max()) > 0
+    assert (int(got[0][0].float().abs().max()) > 0) == (m > 1)         # one token is the row of zeros
