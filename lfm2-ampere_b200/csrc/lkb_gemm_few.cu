@@ -213,9 +213,10 @@ __device__ __forceinline__ bool fw_store_swiglu(FwSmem<TOK> & S, const int * slo
         float x[2][2];                                                   // [row][token]
         const float s0 = scls[8 * n + 2 * q], s1 = scls[8 * n + 2 * q + 1];
         const unsigned long long scl = tc_pack(s0, s1);
+        const bool live0 = 8 * n + 2 * q < I.cnt, live1 = 8 * n + 2 * q + 1 < I.cnt;       // sums of no token are whatever the stages held
         bool sure = true;
 #pragma unroll
-        for (int k = 0; k < 2; ++k) tc_unpack(tc_fmul2(tc_silu2(tc_fmul2(acc[0][n][k], scl), sure), tc_fmul2(acc[1][n][k], scl)), x[k][0], x[k][1]);
+        for (int k = 0; k < 2; ++k) tc_unpack(tc_fmul2(tc_silu2(tc_fmul2(acc[0][n][k], scl), sure, live0, live1), tc_fmul2(acc[1][n][k], scl)), x[k][0], x[k][1]);
         if (!sure) {
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
@@ -510,21 +511,25 @@ static int fw_width(const lkb_pf_gemm * g, int epi, int max_tiles, int sms) {
 // planes allow it; else 0.
 extern "C" __attribute__((visibility("default"))) int lkb_debug_gemm_few_width(const lkb_pf_gemm * g, int max_tiles, int sms) { return fw_width(g, g->oqs != nullptr, max_tiles, sms); }
 
-// Test hook (not in the public header): over `count` float bit patterns from `first` on, in either half of a pair whose other is 1:
-// counts[0] += halves where tc_silu2 is sure of another result than lkb_silu's, counts[1] += those it is not sure of.
+// Test hook (not in the public header): over `count` float bit patterns from `first` on, in either half of a pair whose other is 1, or any value that
+// does not count: counts[0] += halves where tc_silu2 is sure of another result than lkb_silu's, counts[1] += those it is not sure of.
 __global__ void k_debug_silu(unsigned first, unsigned long long count, unsigned long long * __restrict__ counts) {
     unsigned long long wrong = 0, unsure = 0;
     for (unsigned long long i = blockIdx.x * (unsigned long long) blockDim.x + threadIdx.x; i < count; i += (unsigned long long) gridDim.x * blockDim.x) {
-        const float v = __uint_as_float(first + (unsigned) i);
+        const unsigned bits = first + (unsigned) i;
+        const float v = __uint_as_float(bits), other = __uint_as_float(bits * 2654435761u);
         const unsigned want = __float_as_uint(lkb_silu(v));
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            bool sure = true;
-            float q[2];
-            tc_unpack(tc_silu2(half ? tc_pack(1.0f, v) : tc_pack(v, 1.0f), sure), q[0], q[1]);
-            unsure += !sure;
-            wrong += sure && __float_as_uint(q[half]) != want;
-        }
+        for (int half = 0; half < 2; ++half)
+#pragma unroll
+            for (int counts2 = 0; counts2 < 2; ++counts2) {
+                const float o = counts2 ? 1.0f : (i & 1) ? other : (i & 2) ? __int_as_float(0x7FC00000) : 0.0f;
+                bool sure = true;
+                float q[2];
+                tc_unpack(tc_silu2(half ? tc_pack(o, v) : tc_pack(v, o), sure, half ? counts2 : true, half ? true : counts2), q[0], q[1]);
+                unsure += !sure;
+                wrong += sure && __float_as_uint(q[half]) != want;
+            }
     }
     if (wrong) atomicAdd(counts, wrong);
     if (unsure) atomicAdd(counts + 1, unsure);

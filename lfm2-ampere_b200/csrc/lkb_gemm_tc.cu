@@ -335,7 +335,13 @@ __device__ __forceinline__ void tc_store_swiglu(const lkb_pf_gemm & g, const TcI
         const unsigned long long s = tc_pack(__shfl_sync(LKB_FULL, K.scl, c0 + c), __shfl_sync(LKB_FULL, K.scl, c0 + c + 1));
         bool ok = true;
         tc_unpack(tc_fmul2(tc_silu2(tc_fmul2(acc[0][(c0 + c) / 2], s), ok), tc_fmul2(acc[1][(c0 + c) / 2], s)), v[c], v[c + 1]);
-        sure = sure && (ok || c >= nlive);
+        sure = sure && (ok || c + 1 >= nlive);
+    }
+    if ((nlive & 1) && nlive < NT) {                                                  // the last token, whose pair has another that is none
+        float last = 0.0f;
+#pragma unroll
+        for (int c = 0; c < NT; c += 2) if (c + 1 == nlive) last = tc_col<NC>(acc[0], c0 + c);
+        tc_silu2(tc_pack(__fmul_rn(last, __shfl_sync(LKB_FULL, K.scl, c0 + nlive - 1)), 1.0f), sure);
     }
     if (!__all_sync(LKB_FULL, sure)) {
 #pragma unroll

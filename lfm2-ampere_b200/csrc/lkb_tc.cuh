@@ -164,10 +164,10 @@ __device__ __forceinline__ void tc_unpack(unsigned long long v, float & x, float
 }
 // lkb_silu of two values without the divide's branches, so that many are in flight: a reciprocal refined once (Newton), the quotient
 // corrected by its exact remainder (Markstein 1990), which rounds as the IEEE division does unless something under- or overflows on
-// the way.  `sure` is cleared where that may be (results of 0 and up to 1e-17, infinities, NaN): the caller takes lkb_silu there.
+// the way.  `sure` is cleared where that may be (results of 0 and up to 1e-17, infinities, NaN) and the value counts: the caller takes lkb_silu there.
 // Equal to it for every other float (test_gpu_silu.py).  gate|up, whose SwiGLU stores it is for, at 384 / 509 / 1237 / 4096 tokens 105 / 121 / 242 / 570 us
 // with lkb_silu, 96 / 115 / 223 / 530 with this (without any silu 512 at 4096).
-__device__ __forceinline__ unsigned long long tc_silu2(unsigned long long v, bool & sure) {
+__device__ __forceinline__ unsigned long long tc_silu2(unsigned long long v, bool & sure, bool counts0 = true, bool counts1 = true) {
     float v0, v1, d0, d1, y0, y1;
     tc_unpack(v, v0, v1);
     const unsigned long long one = tc_pack(1.0f, 1.0f), d = tc_fadd2(one, tc_pack(__expf(-v0), __expf(-v1)));
@@ -181,7 +181,7 @@ __device__ __forceinline__ unsigned long long tc_silu2(unsigned long long v, boo
     q = tc_ffma2(tc_ffma2(nd, q, v), y, q);
     float q0, q1;
     tc_unpack(q, q0, q1);
-    sure = sure && fabsf(q0) > 1e-17f && fabsf(q1) > 1e-17f;
+    sure = sure && (!counts0 || fabsf(q0) > 1e-17f) && (!counts1 || fabsf(q1) > 1e-17f);
     return q;
 }
 // one tile of a 2-D tensor: box at (x, y) -> shared memory, bytes counted on the mbarrier
