@@ -466,23 +466,16 @@ int lkb_gemm_few_init() {
 }
 int lkb_gemm_few_take_status() { return tc_take_status(); }
 
-// Where the forms cross.  Grouped: by the slots the caller states, spread over 64 experts.  Up to FW_MAX_SLOTS this form is better whatever the
-// skew; beyond, a MoE layer at 400 / 440 / 480 / 520 / 600 tokens of four slots takes 196 / 214 / 223 / 241 / 268 us here and 212 / 220 / 224 / 240 / 260 in the
+// Where the forms cross.  Grouped: by the slots the caller states, spread over 64 experts.  A MoE layer at 400 / 440 / 480 / 520 / 600 tokens of four slots
+// takes 196 / 214 / 223 / 241 / 268 us here and 212 / 220 / 224 / 240 / 260 in the
 // tensor-core form with balanced routing, 209 / 212 / 223 / 235 / 260 and 235 / 239 / 242 / 250 / 270 with Zipf(1.1): the line lies at 480.  Items of 16 tokens to 200 tokens (at
 // 180 gate|up 64 us, 68 with 32; the fifth stage is worth 7 % of a layer at 37 tokens), of 32 beyond.  A plan that cannot have a tile per expert is one of fewer experts, whose tiles may be
 // full; it takes the other form, as does a call that does not state its slots.
 #define FW_MIN_TILES LKB_N_EXPERTS
-#define FW_MAX_SLOTS (47 * LKB_TOP_K)
-#define FW_MORE_SLOTS (480 * LKB_TOP_K)
+#define FW_MAX_SLOTS (480 * LKB_TOP_K)
 #define FW_16_SLOTS  (200 * LKB_TOP_K)
 // Dense: up to FW_MAX_DENSE tokens always, beyond by the time of either form's waves of items (fw_dense_width).
 #define FW_MAX_DENSE 4
-static bool fw_better(const lkb_pf_gemm * g, int max_tiles) {
-    return g->perm ? max_tiles >= FW_MIN_TILES && g->ntok > 0 && g->ntok <= FW_MAX_SLOTS : g->ntok <= FW_MAX_DENSE;
-}
-// Test hook (not in the public header): whether a call takes this form whatever the other's time.
-extern "C" __attribute__((visibility("default"))) int lkb_debug_gemm_few_better(const lkb_pf_gemm * g, int max_tiles) { return fw_better(g, max_tiles); }
-
 static int fw_row_tiles(int N, int epi) { return N / (epi ? FW_ROWS : 2 * FW_ROWS); }       // of an item: two tiles, SwiGLU form: of 128 output rows
 // The token width of a dense problem's items, or 0 where the tensor-core form is faster: waves x the time of an item's block, which is 95, 128 or
 // 176 ns at 8, 16 or 24 tokens here (64 blocks a row: a wave more takes 6.1, 8.2 or 11.3 us; 225 ns at 32, never better) against tc_dense_ns there, and 5 us more
@@ -502,14 +495,18 @@ static int fw_dense_width(int ntok, int N, int bpr, int sms, int epi, bool alway
     return best;
 }
 static int fw_width(const lkb_pf_gemm * g, int epi, int max_tiles, int sms) {
-    const bool always = fw_better(g, max_tiles);
-    if (!g->perm) return fw_dense_width(g->ntok, g->N, g->bpr, sms, epi, always);
-    if (!always && (max_tiles < FW_MIN_TILES || g->ntok <= 0 || g->ntok > FW_MORE_SLOTS)) return 0;
+    if (!g->perm) return fw_dense_width(g->ntok, g->N, g->bpr, sms, epi, g->ntok <= FW_MAX_DENSE);
+    if (max_tiles < FW_MIN_TILES || g->ntok <= 0 || g->ntok > FW_MAX_SLOTS) return 0;
     return g->ntok <= FW_16_SLOTS ? 16 : 32;
 }
 // Test hook (not in the public header): the items' token width where a call (with planes for quants: of the SwiGLU form) takes this form, if its
 // planes allow it; else 0.
 extern "C" __attribute__((visibility("default"))) int lkb_debug_gemm_few_width(const lkb_pf_gemm * g, int max_tiles, int sms) { return fw_width(g, g->oqs != nullptr, max_tiles, sms); }
+// Test hook (not in the public header): the same for a call that this form serves whatever the other's time, at the smallest sizes: up to four dense
+// tokens, or 47 routed ones.
+extern "C" __attribute__((visibility("default"))) int lkb_debug_gemm_few_better(const lkb_pf_gemm * g, int max_tiles) {
+    return g->ntok <= (g->perm ? 47 * LKB_TOP_K : FW_MAX_DENSE) && fw_width(g, 0, max_tiles, 148) > 0;
+}
 
 // Test hook (not in the public header): over `count` float bit patterns from `first` on, in either half of a pair whose other is 1, or any value that
 // does not count: counts[0] += halves where tc_silu2 is sure of another result than lkb_silu's, counts[1] += those it is not sure of.

@@ -35,6 +35,19 @@ def test_width_of_grouped_items(lkb, slots, max_tiles, width):
     assert lkb.lib.lkb_debug_gemm_few_width(ctypes.byref(g), max_tiles, 148) == width
 
 
+@pytest.mark.parametrize("slots,max_tiles,width", [
+    (4096, 64, 0), (1921, 320, 0), (1920, 320, 32), (800, 320, 16), (148, 320, 16), (1, 64, 16),       # the bound on the tiles decides nothing
+    (100, 8, 0), (1920, 63, 0),          # a plan of a few experts
+    (0, 65, 0), (-4, 65, 0),             # slots not stated
+])
+def test_grouped_calls_that_take_the_form(lkb, slots, max_tiles, width):
+    """The launcher's own rule, over its whole range of slots (test_grouped: the sizes where the form is the better one whatever the routing)."""
+    g = lkb.PfGemm()
+    g.ntok, g.perm, g.N, g.bpr = slots, 64, 2048, 64
+    assert lkb.lib.lkb_debug_gemm_few_width(ctypes.byref(g), max_tiles, 148) == width
+    assert not _better(lkb, ntok=slots, perm=64, max_tiles=max_tiles) or width
+
+
 @pytest.mark.parametrize("m,N,bpr,width", [(1, 2048, 64, 8), (4, 6144, 8, 8), (5, 2048, 8, 0), (37, 6144, 64, 8), (64, 6144, 64, 16), (96, 6144, 64, 16), (97, 6144, 64, 24), (144, 6144, 64, 24), (145, 6144, 64, 0),
                                            (144, 2048, 64, 8), (180, 2048, 64, 16), (289, 2048, 64, 24), (432, 2048, 64, 24), (433, 2048, 64, 0), (4096, 6144, 64, 0)])
 def test_width_of_dense_items(lkb, m, N, bpr, width):
