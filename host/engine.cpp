@@ -245,7 +245,7 @@ void prefill_chunk(Engine & e, lk::stream_t st, const int * toks_host, int m, in
         }
         // MoE FFN.  ref: src/engine.cu:1170-1241
         const lkb_moe_layer & l = e.moe[i];
-        if (m <= 160) {                                                       // one launch
+        if (m <= LKB_PF_NORM_ROUTER_TOKENS) {                                 // one launch
             lk::check(lkb_pf_norm_router_select(e.X, l.norm_w, a, e.inv, e.h32, m, 1, l.router, l.rbias, e.sel, e.sig, e.idx, e.w, st),
                       "k_pf_norm + k_pf_router + k_pf_select");
         } else {

@@ -324,7 +324,8 @@ int lkb_pf_select(const float * sel, const float * sig, int m, int * idx, float 
  * results as the two calls.  No counterpart in the reference (its engine launches the two kernels, src/engine.cu:1170-1180). */
 int lkb_pf_router_select(const float * H, int m, int small_form, const float * Wr, const float * bias, const float * inv,
                          float * sel, float * sig, int * idx, float * w, lkb_stream_t st);
-/* lkb_pf_norm (plain = 0) followed by lkb_pf_router_select on its h32: up to 160 tokens of the small form in one launch, which
+#define LKB_PF_NORM_ROUTER_TOKENS 160
+/* lkb_pf_norm (plain = 0) followed by lkb_pf_router_select on its h32: up to LKB_PF_NORM_ROUTER_TOKENS of the small form in one launch, which
  * leaves h32 (m x 2048 floats of the caller's) untouched.  Same results as the two calls. */
 int lkb_pf_norm_router_select(const float * X, const float * nw, lkb_pf_act a, float * inv, float * h32, int m, int small_form,
                               const float * Wr, const float * bias, float * sel, float * sig, int * idx, float * w, lkb_stream_t st);

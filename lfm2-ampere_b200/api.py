@@ -22,7 +22,7 @@ __all__ = [
     "k_pf_pack_q8_1", "zero_i32", "moe_layer_desc", "moe_scratch", "moe_ffn_decode", "moe_ffn_decode_stack",
     "layer_descs_to_device", "ep_pack_rows", "ep_unpack_rows", "k_pf_moe_combine_norm_gather", "moe_ffn_decode_stack_static", "set_pdl", "pf_gemm_config", "pf_gemm_arith", "pf_gemm_workspace_bytes", "pf_gemm_set_workspace", "sm_count",
     "k_gemv_q6_K", "k_argmax_part", "k_argmax_final", "k_embed_q6_K", "gemv_q6_K_status",
-    "k_attn_split", "k_attn_combine", "k_qk_norm_rope", "k_shortconv", "ATTN_SPLIT", "ATTN_PARTW",
+    "k_attn_split", "k_attn_combine", "k_qk_norm_rope", "k_shortconv", "ATTN_SPLIT", "ATTN_PARTW", "PF_NORM_ROUTER_TOKENS",
     "mixer_layer_desc", "step_scratch", "decode_layers",
     "k_pf_embed", "k_pf_conv", "k_pf_conv_hist", "k_pf_conv_next", "k_pf_qknr", "k_pf_attn",
     "decode_set_expert_prefetch", "decode_expert_prefetch_hits", "ep_peers", "EP_ROW_BYTES", "ep_set_wait_limit_ms", "ep_route_exchange", "ep_route_experts", "pf_gemm_moe_rows", "pf_gemm_swiglu_packed", "ep_publish_wait", "ep_pack_push", "ep_wait",
@@ -348,6 +348,7 @@ def k_embed_q6_K(ql, qh, sc, d, d_token, n, x):
 
 # ------------------------------------------------------------ sequence mixers --
 ATTN_SPLIT, ATTN_PARTW = 18, 66          # LKB_ATTN_SPLIT / LKB_ATTN_PARTW of include/lkb.h
+PF_NORM_ROUTER_TOKENS = 160              # LKB_PF_NORM_ROUTER_TOKENS
 
 
 def k_attn_split(q, kc, vc, d_pos, part):

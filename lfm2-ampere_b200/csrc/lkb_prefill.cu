@@ -201,7 +201,6 @@ __global__ void __launch_bounds__(256) k_pf_router_token(const float * __restric
 // The same for fewer tokens still: a cluster of eight CTAs per token, a warp per expert.  The selection needs all 64 logits: they meet in
 // the shared memory of the cluster's first CTA.  Bound by the latency of a warp's two rows; see router_small for where it pays.
 #define RC_CTAS 8
-#define RC_MAX_TOKENS 160            // see router_small
 __global__ void __cluster_dims__(RC_CTAS, 1, 1) __launch_bounds__(256) k_pf_router_cluster(const float * __restrict__ H, const float * __restrict__ Wr,
                                                          const float * __restrict__ bias, const float * __restrict__ inv,
                                                          float * __restrict__ sel, float * __restrict__ sig,
@@ -1039,7 +1038,7 @@ static int router_small(const float * H, int m, const float * Wr, const float * 
     if (m > 65535) return LKB_ERR_SHAPE;
     // A cluster of CTAs a token while that is about a wave: a MoE layer at 2 / 9 / 37 / 64 / 100 tokens 47 / 63 / 114 / 152 / 155 -> 41 / 58 / 109 /
     // 146 / 150 us; at 180 equal, at 256 182 -> 186.
-    if (m <= RC_MAX_TOKENS) {
+    if (m <= LKB_PF_NORM_ROUTER_TOKENS) {
         LKB_PF_LAUNCH(k_pf_router_cluster, dim3(m * RC_CTAS), dim3(256), 0, (cudaStream_t) st, H, Wr, bias, inv, sel, sig,
                       reinterpret_cast<int4 *>(idx), reinterpret_cast<float4 *>(w));
         return lkb_check_launch();
@@ -1093,7 +1092,7 @@ int lkb_pf_norm_router_select(const float * X, const float * nw, lkb_pf_act a, f
     LKB_REQUIRE_INIT();
     if (!X || !nw || !a.qs || !a.sc || !inv || !h32 || !Wr || !bias || !sel || !sig || !idx || !w) return LKB_ERR_NULL;
     if (m <= 0) return m == 0 ? LKB_OK : LKB_ERR_SHAPE;
-    if (small_form && m <= RC_MAX_TOKENS) {
+    if (small_form && m <= LKB_PF_NORM_ROUTER_TOKENS) {
         LKB_PF_LAUNCH(k_pf_norm_router_cluster, dim3(m * RC_CTAS), dim3(256), 0, (cudaStream_t) st, X, nw, a.qs, reinterpret_cast<float2 *>(a.sc), inv, Wr, bias, sel, sig,
                       reinterpret_cast<int4 *>(idx), reinterpret_cast<float4 *>(w));
         return lkb_check_launch();

@@ -221,7 +221,7 @@ class PrefillChunk:
         self.o = torch.zeros(m, H, **f32)
         self.toks = torch.zeros(m, dtype=torch.int32, device=device)
         n_attn = sum(mx.is_attn for mx in model.mixers)
-        self.launches_per_step = 1 + 1 + sum((6 if mx.is_attn else 3) for mx in model.mixers) + (5 if m <= 160 else 6 if 4 * m <= 2048 else 8) * len(model.mixers)
+        self.launches_per_step = 1 + 1 + sum((6 if mx.is_attn else 3) for mx in model.mixers) + (5 if m <= api.PF_NORM_ROUTER_TOKENS else 6 if 4 * m <= 2048 else 8) * len(model.mixers)
 
     def macs_per_step(self):
         m, n = self.m_, len(self.model.mixers)

@@ -57,7 +57,7 @@ class PrefillStack:
         self.a = api.pf_act(self.a_qs, self.a_sc)
         self.a2 = api.pf_act(self.a2_qs, self.a2_sc)
         self.an = api.pf_act(self.n_qs, self.n_sc)
-        self.launches_per_step = (5 if m <= 160 else 6 if self.ns <= 2048 else 8) * len(layers)       # kernels per layer (the memset is not a kernel)
+        self.launches_per_step = (5 if m <= api.PF_NORM_ROUTER_TOKENS else 6 if self.ns <= 2048 else 8) * len(layers)       # kernels per layer (the memset is not a kernel)
 
     def layer(self, i, next_norm_w=None, next_act=None):
         """One MoE FFN layer over the chunk.  next_norm_w / next_act = (PfAct, inv): where the fused combine + norm

@@ -83,3 +83,11 @@ int main() { return lkb_sm_count() < 0; }
     subprocess.run(["g++", "-std=c++17", "-I", str(lkb.ROOT / "include"), str(src), "-o", str(exe),
                     str(lkb.LIB_PATH), f"-Wl,-rpath,{lkb.LIB_PATH.parent}"], check=True)
     assert subprocess.run([str(exe)]).returncode == 0
+
+
+def test_numbers_that_python_shares_with_the_header(lkb):
+    """Limits of the C ABI that the Python host counts by, and the C++ host's use of the name instead of the number."""
+    header = dict(re.findall(r"#define LKB_(\w+)\s+(\d+)\b", lkb.HEADER.read_text()))
+    for name in ("ATTN_SPLIT", "ATTN_PARTW", "PF_NORM_ROUTER_TOKENS"):
+        assert getattr(lkb, name) == int(header[name]), name
+    assert "m <= LKB_PF_NORM_ROUTER_TOKENS" in (lkb.HEADER.parent.parent / "host" / "engine.cpp").read_text()
