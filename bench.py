@@ -534,9 +534,9 @@ def run_ours(args):
                 "gemm_share_of_step": (float(np.sum(gemm_ms)) / pms) if gemm_ms else None,
                 "traffic": profile_traffic("k_pf_gemm_tc_prefill_4096tok.txt"),
                 "vs_ref_kernel": vs_ref_kernel,
-                "co_bound": "the exact per-block scale arithmetic: two fp32 FMAs per int32 block sum on the CUDA cores are 128 packed FMAs a "
-                            "scheduler for a block of 256 rows x 64 tokens, 2.9 cycles each, and the integer instructions beside them add their "
-                            "own two cycles: about 80 % of the kernel's cycles, with the tensor pipe 18 to 19 % busy (profiles/)",
+                "co_bound": "the exact per-block scale arithmetic and the constants it reads: two fp32 FMAs per int32 block sum on the CUDA cores are "
+                            "128 packed FMAs a scheduler for a block of 256 rows x 64 tokens, 2.9 cycles each, and the block's 128 shared loads of "
+                            "constants 512 cycles of the SM's return path, of 600 or so a block, with the tensor pipe 19 to 20 % busy (profiles/)",
                 "whole_step_TMACs": macs / (pms * 1e-3) / 1e12}
     pf_cfg = {"workload": WORKLOAD, "tokens": m, "layers": args.layers, "resident_weight_bytes": args.layers * 339738624,
               "cold_cache": "each step streams the whole 13.6 GB expert set (inputs larger than L2)",

@@ -362,9 +362,9 @@ int lkb_pf_gemm_arith(int fold);
 int lkb_pf_gemm_workspace_bytes(int max_tiles, int k_max, size_t * bytes_out);
 int lkb_pf_gemm_set_workspace(void * ptr, size_t bytes);
 /* Every device-side wait of the tensor-core kernels is bounded; this SYNCHRONISES the device and
- * returns 0, or the code of the first wait that expired since the last call (10 producer, 11 / 33 few-token form,
- * 15/16 expansion, 20-22 MMA issuer, 30/31 epilogue; 50-63 the
- * chunk attention) and clears it.  No counterpart in the reference. */
+ * returns 0, or the code of the first wait that expired since the last call (tensor-core GEMM: 10 producer,
+ * 15/16 expansion, 20-22 MMA issuer, 31 epilogue; few-token GEMM: 11 producers, 33 dots, 34/35 SwiGLU hand-over, 36 token constants;
+ * router of longer chunks: 41 copies, 42 logits; 50-63 the chunk attention) and clears it.  No counterpart in the reference. */
 int lkb_pf_gemm_status(void);
 /* ref: src/prefill.cuh:123-127  k_pf_moe_combine / k_pf_moe_combine_norm / k_pf_pack_q8_1 */
 int lkb_pf_moe_combine(float * X, const float * D, const float * w, int m, lkb_stream_t st);

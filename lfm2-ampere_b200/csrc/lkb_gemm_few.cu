@@ -14,10 +14,10 @@
 //     one that turns a stage's (d8, 8sum) into the constants of token pairs (in the dot warps, eight times over, that doubled a block's time).
 //   * Stages of eight blocks: 128 bytes of a weight row, half the copies and waits of four (m = 128: gate|up 78 -> 66 us).
 //   * 16 or 32 tokens an item; the part of a stage that activations leave goes into stages: five or four, 110 to 180 KB in flight.
-// Measured, 64 experts, balanced routing, caches flushed before every call, us at 9 / 20 / 37 / 64 / 128 / 256 / 384 / 509 tokens:
-//   gate|up  dp4a form, three CTAs an SM (before, to 47 tokens)  32 / 50 / 62;  tensor-core form  80 / 82 / 89 / 103 / 121 from 64 on
-//            this form                                           33 / 43 / 52 / 57 / 61 / 72 / 93 / 117
-//   down     before  22 / 30 / 40;  49 / 53 / 59 / 58 / 65       this form  21 / 29 / 33 / 35 / 39 / 41 / 50 / 66
+// Measured in one run, 64 experts, balanced routing, caches flushed before every call, us at 9 / 20 / 37 / 64 / 128 / 256 / 384 / 480 tokens:
+//   gate|up  dp4a form, three CTAs an SM (before, to 47 tokens)  32 / 48 / 63;  tensor-core form  80 / 81 / 92 / 96 / 114 from 64 on
+//            this form                                           34 / 44 / 55 / 58 / 64 / 75 / 95 / 115
+//   down     before  21 / 28 / 40;  51 / 53 / 57 / 58 / 62       this form  21 / 28 / 34 / 35 / 37 / 43 / 49 / 59
 // What bounds it: to some 100 tokens whole waves of items (768 on 148 SMs: 5.2) of 4.5 TB/s each and 5 to 7 us of launch, fill and drain;
 // then the MMAs and the fold.
 // No copy in this file is a multicast one; every tensor map covers memory of the GPU the kernel runs on.
@@ -56,7 +56,7 @@ template <int TOK> struct FwSmem {
 
 struct FwItem { int expert, tstart, cnt, rt, r0, rows; };   // cnt <= 0: nothing to do; rows r0 .. r0 + rows - 1 of both tiles
 // The blocks' work: items, of which those from `whole` on -- a last wave that would leave half of the blocks or more without one -- are cut
-// into 1 << cut parts of fewer rows, one a block, whose first warps have rows (an item's time is its weights' way into one SM).  us, whole -> cut, caches
+// into 1 << cut parts of fewer rows, one a block, whose first warps have rows (an item's time is its weights' way into one SM).  us, whole -> cut in a run of its own, caches
 // flushed: down at 2 / 20 tokens 15.3 -> 13.3, 29.7 -> 27.7; out_proj (2048 rows) at 2 to 64 tokens 13.3 -> 11.3, in_proj at 2 13.3 -> 11.3; a layer of 2 / 9 / 20 / 37 /
 // 64 tokens 59.4 / 84.4 / 100.6 / 114.3 / 122.3 -> 55.6 / 79.2 / 96.3 / 111.3 / 119.8.  A choice of the width that counts a part as 0.6 of an item
 // changed nothing (-1 % at 70 tokens, +0.5 % at 200).

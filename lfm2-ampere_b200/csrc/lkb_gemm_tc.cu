@@ -40,7 +40,7 @@
 //   ... weight scales in a ring of their own, expansion a stage at a time, no scale barriers, two issuers (this form)
 //                                                    70 / 117 / 569         47 /  64 / 268           23 / 51 / 238
 //   ... dense items cut to fill the waves (tc_dense_form)                                            20 / 45 / 236
-//   ... SwiGLU stores two values at a time         gate|up at 4096 tokens 530
+//   ... SwiGLU stores two values at a time         gate|up at 4096 tokens 530; values of no token not asked 514
 // (by itself the launcher takes this form above 1920 slots (480 tokens of four) grouped, and dense where that of lkb_gemm_few.cu would need the longer waves)
 // With few tokens the hand-over of every block is the bound (300 to 440 cycles of polls, commits and arrivals).
 // No copy in this file is a multicast one; every tensor map covers memory of the GPU the kernel runs on.

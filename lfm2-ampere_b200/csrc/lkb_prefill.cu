@@ -447,8 +447,9 @@ static int rt_launch(const float * H, int m, const float * Wr, const float * bia
 // 32 experts (a thread: tokens l / 8, + 4, ..., experts l % 8, + 8, + 16, + 24), 4 * TPT independent chains a thread, and one warp that copies:
 // k-tiles of the CTA's token rows and of all 64 router rows travel global -> shared by tensor copies, 128 bytes of every row at a time
 // (swizzled: 128-bit loads of eight neighbouring rows are conflict-free), through a ring of RT_STAGES buffers handed over by mbarriers.
-// us at 1184 / 2048 / 4096 / 8192 tokens: 31.5 / 36.4 / 54.5 / 106 in the form above, 26.9 / 30.5 / 44.6 / 86 here (without the shared loads 16 / 17 / 22 /
-// 39; with a bulk copy per row, 67 cycles each, 44 / 54 / 118 / 234).  At 509 tokens 22.8 there, 29.4 here with the same four-token CTAs.
+// us, calls back to back, at 1184 / 2048 / 4096 / 8192 tokens: 29.7 / 35.2 / 53.4 / 105 in the form above, 25.2 / 28.8 / 43.3 / 85 here (in an earlier run, where this took
+// 26.9 / 30.5 / 44.6 / 86, 16 / 17 / 22 / 39 without the shared loads; with a bulk copy per row, 67 cycles each, 44 / 54 / 118 / 234).  At 509 tokens 21.2 there,
+// 27.8 here with the same four-token CTAs.
 // Waits are bounded; on expiry a status word is set and all roles leave, the copying warp after its copies have landed.
 __device__ __forceinline__ float4 rt_lds(unsigned addr) {
     float4 v;
@@ -1054,12 +1055,13 @@ static int router_tiled(const float * H, int m, const float * Wr, const float * 
     if (!H || !Wr || !bias || !inv || !sel || !sig) return LKB_ERR_NULL;
     if (m <= 0) return m == 0 ? LKB_OK : LKB_ERR_SHAPE;
     // The k loop of one CTA is the critical path and its length grows with the tokens per CTA, so a token range takes the smallest
-    // CTA that still fits one wave.  Measured on B200, us, copies by every thread and by tensor copies:
-    //   4-token CTAs (two warps)         up to 592 tokens   22.8   29.4
-    //   8-token CTAs (two warps)         up to 1184         31.0   26.9
-    //   16-token CTAs                    up to 2368         36.3   30.5
-    //   32-token CTAs, 64 k-values a tile  at 4096          54.5   44.6
-    // A rank's share of an expert-parallel chunk lands in the first three.  LKB_ROUTER_FORM = 4 / 8 / 16 / 32 forces a shape (tuning).
+    // CTA that still fits one wave.  Measured on B200, us, calls back to back, copies by every thread and by tensor copies:
+    //   4-token CTAs (two warps)         up to 592 tokens   21.2   27.8
+    //   8-token CTAs (two warps)         up to 1184         29.7   25.2
+    //   16-token CTAs                    up to 2368         35.2   28.9
+    //   32-token CTAs, 64 k-values a tile  at 4096          53.4   43.3
+    // A rank's share of an expert-parallel chunk lands in the first three.  LKB_ROUTER_FORM = 4 / 8 / 16 / 32 forces a shape (tuning): 4 with copies by
+    // every thread, the others with tensor copies.
     static const int form = [] { const char * e = getenv("LKB_ROUTER_FORM"); return e ? atoi(e) : 0; }();
     const int sms = lkb_context().sm_count;
     if (form == 4 || (form == 0 && m <= 4 * sms)) return rt_launch<1, 2, 128, 4>(H, m, Wr, bias, inv, sel, sig, idx, w, (cudaStream_t) st);

@@ -166,7 +166,7 @@ __device__ __forceinline__ void tc_unpack(unsigned long long v, float & x, float
 // corrected by its exact remainder (Markstein 1990), which rounds as the IEEE division does unless something under- or overflows on
 // the way.  `sure` is cleared where that may be (results of 0 and up to 1e-17, infinities, NaN) and the value counts: the caller takes lkb_silu there.
 // Equal to it for every other float (test_gpu_silu.py).  gate|up, whose SwiGLU stores it is for, at 384 / 509 / 1237 / 4096 tokens 105 / 121 / 242 / 570 us
-// with lkb_silu, 96 / 115 / 223 / 530 with this (without any silu 512 at 4096).
+// with lkb_silu, 96 / 115 / 223 / 530 with this (without any silu 512 at 4096), 95 / 114 / 208 / 514 since a value of no token does not count.
 __device__ __forceinline__ unsigned long long tc_silu2(unsigned long long v, bool & sure, bool counts0 = true, bool counts1 = true) {
     float v0, v1, d0, d1, y0, y1;
     tc_unpack(v, v0, v1);
